@@ -1626,9 +1626,11 @@ extern "C" int grmp_stokes_batch_solve(grmp_matrix A, grmp_vector bf, grmp_vecto
             m.U_doubles = C.max_U;
             m.L_doubles = C.max_L;
             m.uv_doubles = std::max<long long>(1, C.max_uv);
-            // groups of 128 threads factoring small fronts concurrently, as many as
-            // the pivot-column and panel buffers (sized for the largest front) hold
-            m.fact_groups = std::max(1, std::min(4, C.max_f / kGroupFront));
+            // groups of threads factoring small fronts concurrently, as many as the
+            // pivot-column and panel buffers (sized for the largest front) hold: 4, 2
+            // or 1, so that the block's 512 threads split into whole warps (a group
+            // synchronises on a named barrier, which counts whole warps only)
+            m.fact_groups = C.max_f >= 4 * kGroupFront ? 4 : (C.max_f >= 2 * kGroupFront ? 2 : 1);
             m.slot_doubles = m.F_doubles + m.U_doubles + C.max_L + m.uv_doubles +
                              (m.fact_groups > 1 ? (long long)m.fact_groups * kGroupFront * kGroupFront : 0);
             m.max_f = C.max_f;
