@@ -6,9 +6,17 @@
 // each problem of a batch gets a multifrontal Cholesky factorisation, done
 // once and reused by every sweep.  This file computes, for a symmetric
 // pattern:
-//   * a nested-dissection elimination order: level-set separators of a
-//     breadth-first search started at a pseudo-peripheral DoF, recursively,
-//     down to leaves of at most kLeaf DoFs;
+//   * a nested-dissection elimination order: separators from the level sets of
+//     a breadth-first search started at a pseudo-peripheral DoF (the DoFs of
+//     one level that touch the next one), recursively, down to leaves of at
+//     most kLeaf DoFs.  On these meshes a whole level holds two lines of DoFs
+//     where one separates: factor flops on 256 x 256 P2 elasticity (526k DoFs)
+//     1.12e11 with whole levels, 2.49e10 with the touching DoFs (largest front
+//     3,500 and 1,956 rows, factor 159M and 74M entries); 96 x 96
+//     Bernardi-Raugel 1.51e9 and 5.8e8; 6^3 Bernardi-Raugel cubes 6.0e8 and
+//     8.3e7 (largest front 969 and 345).  Choosing the level of the smallest
+//     separator near the median takes the same time as the median level did,
+//     with three searches per separator instead of up to six;
 //   * the assembly tree in post-order (children before parents, which is
 //     the elimination order), each node with its front = its own DoFs
 //     followed by its structure (later-eliminated DoFs coupled to them);
@@ -37,7 +45,7 @@ struct Builder {
     std::vector<std::vector<int>> own;   // own DoFs per node (creation = post-order)
     std::vector<std::vector<int>> kids;
 
-    int bfs(const std::vector<int> &set, int start, int setstamp, std::vector<int> &order_out) {
+    int bfs(int start, int setstamp, std::vector<int> &order_out) {
         // returns the eccentricity of `start` in the subgraph; order_out = BFS order
         order_out.clear();
         ++cur;
@@ -67,10 +75,8 @@ struct Builder {
         ++cur;
         const int setstamp = cur;
         for (int v : set) stamp[v] = setstamp;
-        std::vector<int> ord;
-        // pseudo-peripheral start: repeat BFS from a farthest DoF while the eccentricity grows
-        int start = set[0];
-        int ecc = bfs(set, start, setstamp, ord);
+        std::vector<int> ord, o2;
+        int ecc = bfs(set[0], setstamp, ord);
         if (ord.size() < set.size()) {
             // disconnected: split off the component of set[0]
             std::vector<int> a = ord, b;
@@ -82,35 +88,55 @@ struct Builder {
             int cb = dissect(std::move(b));
             return join({}, {ca, cb});
         }
-        for (int rep = 0; rep < 4; rep++) {
-            int cand = ord.back();
-            std::vector<int> o2;
-            int e2 = bfs(set, cand, setstamp, o2);
-            if (e2 <= ecc) break;
-            ecc = e2;
-            start = cand;
+        // pseudo-peripheral start: the levels of the last of three searches,
+        // each from the DoF that the one before it reached last
+        for (int rep = 0; rep < 2; rep++) {
+            const int e2 = bfs(ord.back(), setstamp, o2);
             ord.swap(o2);
+            if (e2 <= ecc) { ecc = e2; break; }
+            ecc = e2;
         }
-        bfs(set, start, setstamp, ord);   // levels from the chosen start
         if (ecc < 2) return leaf(std::move(set));
-        // median level as the separator
-        std::vector<int> cnt(ecc + 1, 0);
-        for (int v : ord) cnt[level[v]]++;
-        int acc = 0, L = 1;
-        const int half = (int)set.size() / 2;
-        for (int l = 0; l <= ecc; l++) {
-            acc += cnt[l];
-            if (acc >= half) {
+        // Separator of level l: its DoFs with a neighbour in level l + 1 (the
+        // rest of the level has none there and stays with the lower part).
+        // Taken is the level whose separator is smallest, weighted by how far
+        // the larger part exceeds half, among those that leave at most 0.65 of
+        // the DoFs on one side (the median level where none does).
+        std::vector<int> first(ecc + 2, (int)ord.size()), touching(ecc + 1, 0);
+        std::vector<char> touch(ord.size(), 0);
+        for (int h = (int)ord.size() - 1; h >= 0; h--) first[level[ord[h]]] = h;
+        for (size_t h = 0; h < ord.size(); h++) {
+            const int v = ord[h], up = level[v] + 1;
+            for (int k = rp[v]; k < rp[v + 1]; k++) {
+                const int w = ci[k];
+                if (level[w] == up && stamp[w] == setstamp) {
+                    touch[h] = 1;
+                    break;
+                }
+            }
+            touching[level[v]] += touch[h];
+        }
+        const double tot = (double)set.size();
+        int L = 1;
+        while (L < ecc - 1 && first[L + 1] < 0.5 * tot) L++;
+        double best = -1.0;
+        const int median = L;
+        for (int l = 1; l < ecc; l++) {
+            const double lower = first[l + 1] - touching[l], upper = tot - first[l + 1];
+            const double share = std::max(lower, upper) / tot;
+            if (share > 0.65 && l != median) continue;
+            const double cost = touching[l] * (1.0 + 2.0 * (share - 0.5));
+            if (best < 0 || cost < best) {
+                best = cost;
                 L = l;
-                break;
             }
         }
-        L = std::min(std::max(L, 1), ecc - 1);
         std::vector<int> a, b, sep;
-        for (int v : ord) {
-            if (level[v] < L) a.push_back(v);
-            else if (level[v] > L) b.push_back(v);
-            else sep.push_back(v);
+        for (size_t h = 0; h < ord.size(); h++) {
+            const int v = ord[h];
+            if (level[v] > L) b.push_back(v);
+            else if (level[v] == L && touch[h]) sep.push_back(v);
+            else a.push_back(v);
         }
         std::vector<int> ch;
         if (!a.empty()) ch.push_back(dissect(std::move(a)));
