@@ -647,6 +647,8 @@ int grmp_p2b_rhs(grmp_space s, const grmp_rhs *rhs, grmp_vector b);
 int grmp_assemble_bilinear_impl(grmp_matrix A, int nterms, const grmp_bilinear_term *terms, int precision) {
     grmp_space s = A->space;
     grmp_context ctx = s->mesh->ctx;
+    A->elliptic = false;
+    for (int i = 0; i < nterms; i++) A->elliptic = A->elliptic || terms[i].op_kind == GRMP_OP_LAPLACE;
     if (s->fe == GRMP_FE_H1BR) {
         int rc = precision == GRMP_FP64_FP32 ? grmp_br_assemble(A, nterms, terms, GRMP_FP64)
                                              : grmp_br_assemble(A, nterms, terms, precision);

@@ -137,6 +137,12 @@ struct grmp_matrix_s {
     struct DirectCache *direct = nullptr;
     // single-problem direct solvers: symbolic analysis + factor storage
     struct MfCache *mf = nullptr;
+    // multilevel preconditioner: hierarchy, 0 = not built, 1 = built, -1 = not
+    // for this matrix; elliptic: the last assembly had a diffusion term
+    struct MgCache *mg = nullptr;
+    int mg_state = 0;
+    size_t mg_budget = SIZE_MAX;    // device bytes it may take (served requests: what their estimate leaves)
+    bool elliptic = false;
 };
 
 void grmp_duo_free(grmp_matrix A);   // duo copy of mixed solves (solve.cu)

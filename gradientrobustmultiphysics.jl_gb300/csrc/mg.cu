@@ -1,0 +1,1170 @@
+// Multilevel preconditioned conjugate gradients for scalar elliptic matrices
+// (H1P1 / H1P2 spaces with a diffusion term), FP64 and mixed.
+//
+// Jacobi-PCG needs O(1/h) iterations (64^3 P2 Poisson 1,031, 128^2 P2 1,203)
+// and each is bound by the latency of its gathers and grid barriers, so what
+// pays is fewer iterations.  The preconditioner is one multilevel cycle:
+//
+//   z = c D_0 r + P_0 V(P_0^T r)
+//
+// additive on the fine level (its Jacobi part costs no product with the fine
+// matrix, so an iteration keeps one fine SpMV; multiplicative smoothing there
+// needs two more and saves less than half of the iterations: 47 against 27 on
+// 24^3 P2), and a symmetric V(1,1) cycle below.  P_0 of a P2 space
+// interpolates from the vertices (P1 is in P2); all other levels are smoothed
+// aggregation, P = (I - w D A) P_agg.  D = 1 / sum_j |a_ij| (l1-Jacobi:
+// convergent for every SPD matrix without an eigenvalue estimate).  With
+// S = w D the cycle on level l is
+//
+//   r_{l+1} = Q^T r_l,      e_l = 2 S r_l - S A S r_l + Q e_{l+1},
+//   Q = P - S A P,
+//
+// which is one pre- and one post-smoothing step written with the smoothed
+// prolongation Q: one phase down and one up per level (two grid barriers
+// instead of four); Q is formed with the coarse matrices from A P.
+//
+// The hierarchy's patterns are built once per matrix pattern on the host
+// (mg_symbolic.cpp); its values are formed on the device at every solve, from
+// the matrix as it is then.  Rows without off-diagonal values (Dirichlet rows
+// of either kind) are left out of the coarse spaces.  Everything is in the
+// precision of the iteration (FP32 inside the FP64 refinement of mixed
+// solves, FP64 throughout in FP64 solves), every sum has a fixed order.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "mg.h"
+#include "mg_symbolic.h"
+#include "pcg_device.cuh"
+
+namespace {
+
+constexpr int kTB = 256;
+constexpr int kCl = 8;            // lanes per row of k_mg_rows
+constexpr int kMgT = 384;         // threads per block of the solvers: two blocks fit an SM at 85 registers a thread
+constexpr int kLongRow = 48;      // mean entries from which a warp takes a row (transposes of wide aggregates)
+constexpr double kSmooth = 1.7;   // w of the smoothing steps and c of the fine level (l1-scaled: spectrum in (0, 1])
+constexpr double kProlong = 1.32; // w of the prolongation smoothing
+// reaction-dominated matrices (energy of the constant function against the
+// diagonal) converge in a few dozen Jacobi iterations: they keep that solver
+constexpr double kMaxReaction = 0.02;
+constexpr int kMinRows = 400;
+
+template <typename T>
+struct alignas(2 * sizeof(T)) Pair {
+    T a, b;
+};
+
+template <typename T>
+struct MgLv {
+    int n;
+    const int32_t *rp, *ci;       // A
+    const T *v, *D;
+    const int32_t *qrp, *qci;     // Q: n x next n
+    const T *qv;
+    const int32_t *trp, *tci;     // Q^T
+    const T *tv;
+    int along, qlong, tlong;      // a warp per row of A, Q, Q^T
+    T *r, *y, *e;
+};
+
+template <typename T>
+struct MgDev {
+    int nl, dense, rlong;         // levels, dense inverse at the bottom, a warp per row of P_0^T
+    const int32_t *prp, *pci;     // P_0 and its transpose
+    const T *pv;
+    const int2 *ell;              // P_0 of a P2 space as two entries a row (nullptr: CSR)
+    const Pair<T> *ellv;
+    const int32_t *rrp, *rci;
+    const T *rv;
+    const T *D0, *binv;
+    MgLv<T> lv[kMgMaxLevels + 1];
+};
+
+// ------------------------------------------------------------------ values of the hierarchy
+// D, the rows without coupling, and (level 0) per-block sums of the positive
+// row sums and diagonals of the rows away from eliminated DoFs, bad diagonals
+template <typename T>
+__global__ void __launch_bounds__(kTB) k_mg_rows(int n, const int32_t *rp, const int32_t *ci, const T *v, T *D,
+                                                 uint8_t *iso, double2 *part, int *bad) {
+    __shared__ double sh[32 * 2];
+    const int lane = threadIdx.x & (kCl - 1);
+    double s0 = 0.0, s1 = 0.0;
+    for (long long base = blockIdx.x * (long long)(kTB / kCl); base < n; base += (long long)gridDim.x * (kTB / kCl)) {
+        const int i = (int)base + threadIdx.x / kCl;
+        T off = 0, d = 0, sum = 0;
+        int zero = 0;
+        if (i < n)
+            for (int k = rp[i] + lane; k < rp[i + 1]; k += kCl) {
+                const T a = v[k];
+                sum += a;
+                if (ci[k] == i) d = a;
+                else {
+                    off += fabs(a);
+                    zero |= a == T(0);
+                }
+            }
+        for (int o = kCl / 2; o > 0; o >>= 1) {
+            off += __shfl_xor_sync(0xffffffffu, off, o);
+            d += __shfl_xor_sync(0xffffffffu, d, o);
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            zero |= __shfl_xor_sync(0xffffffffu, zero, o);
+        }
+        if (i < n && lane == 0) {
+            const T s = off + fabs(d);
+            const bool lone = off <= T(1e-8) * fabs(d);
+            D[i] = s > T(0) ? T(1) / s : T(1);
+            iso[i] = lone;
+            if (bad && (!(d > T(0)) || !isfinite((double)s))) atomicExch(bad, 1);
+            if (!lone && !zero) {
+                s0 += sum > T(0) ? (double)sum : 0.0;
+                s1 += (double)d;
+            }
+        }
+    }
+    if (!part) return;
+    double v2[2] = {s0, s1};
+    block_sum<2>(v2, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = make_double2(v2[0], v2[1]);
+}
+
+// vertex interpolation: 1 at a vertex, 1/2 from the two ends of an edge; fixed DoFs neither receive nor give
+template <typename T>
+__global__ void k_mg_prol_geo(int n, const int32_t *prp, const int32_t *pci, const int32_t *vrow, const uint8_t *iso,
+                              T *pv, Pair<T> *ellv) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int b = prp[i], e = prp[i + 1];
+    T w[2] = {T(0), T(0)};
+    for (int q = b; q < e; q++) {
+        w[q - b] = iso[i] || iso[vrow[pci[q]]] ? T(0) : (e - b == 1 ? T(1) : T(0.5));
+        pv[q] = w[q - b];
+    }
+    ellv[i] = Pair<T>{w[0], w[1]};
+}
+
+// P = (I - w D A) P_agg
+template <typename T>
+__global__ void k_mg_prol_agg(int n, const int32_t *rp, const int32_t *ci, const T *v, const T *D, const uint8_t *iso,
+                              const int32_t *agg, const int32_t *prp, const int32_t *pci, T *pv) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int kb = rp[i], ke = rp[i + 1], own = agg[i];
+    const bool lone = iso[i];
+    const T w = (T)kProlong * D[i];
+    for (int q = prp[i]; q < prp[i + 1]; q++) {
+        const int t = pci[q];
+        T s = 0;
+        for (int k = kb; k < ke; k++)
+            if (agg[ci[k]] == t) s += v[k];
+        pv[q] = lone ? T(0) : (t == own ? T(1) : T(0)) - w * s;
+    }
+}
+
+// A P, a group of L lanes per row, a lane per entry of the row of A P (L >= the
+// longest of them where 32 allows it): the lanes load the row's entries and
+// the rows of P they meet, and pass them round by shuffles (A is read
+// coalesced, nothing is searched, the order is fixed).  Bound by the
+// shuffles: 64^3 P2 (55.6M entries times two) 1.4 ms with a warp per row,
+// half of it with two rows per warp.
+template <typename T, int L>
+__global__ void __launch_bounds__(kTB) k_mg_ap(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                                               const T *__restrict__ v, const int32_t *__restrict__ prp,
+                                               const int32_t *__restrict__ pci, const T *__restrict__ pv,
+                                               const int32_t *__restrict__ arp, const int32_t *__restrict__ aci, T *av) {
+    const int lane = threadIdx.x & (L - 1);
+    const int ng = gridDim.x * blockDim.x / L;
+    const int pad = (n + 32 / L - 1) / (32 / L) * (32 / L);   // whole warps take part in the shuffles
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) / L; i < pad; i += ng) {
+        const int kb = i < n ? rp[i] : 0, ke = i < n ? rp[i + 1] : 0;
+        const int t0 = i < n ? arp[i] : 0, te = i < n ? arp[i + 1] : 0;
+        const int chunks = __reduce_max_sync(0xffffffffu, (te - t0 + L - 1) / L);
+        const int steps = __reduce_max_sync(0xffffffffu, (ke - kb + L - 1) / L);
+        for (int tc = 0; tc < chunks; tc++) {
+            const int tb = t0 + tc * L + lane;
+            const int mine = tb < te ? aci[tb] : -1;
+            T acc = 0;
+            for (int kc = 0; kc < steps; kc++) {
+                const int k0 = kb + kc * L + lane;
+                int p0 = 0, len = 0;
+                T a = 0;
+                if (k0 < ke) {
+                    const int j = ci[k0];
+                    a = v[k0];
+                    p0 = prp[j];
+                    len = prp[j + 1] - p0;
+                }
+                const int m = __reduce_max_sync(0xffffffffu, min(L, max(0, ke - kb - kc * L)));
+                const int longest = __reduce_max_sync(0xffffffffu, len);
+                for (int q = 0; q < longest; q++) {
+                    const int c = q < len ? pci[p0 + q] : -2;
+                    const T w = q < len ? a * pv[p0 + q] : T(0);
+                    for (int k = 0; k < m; k++) {
+                        const int cc = __shfl_sync(0xffffffffu, c, k, L);
+                        const T ww = __shfl_sync(0xffffffffu, w, k, L);
+                        if (cc == mine) acc += ww;
+                    }
+                }
+            }
+            if (tb < te) av[tb] = acc;
+        }
+    }
+}
+
+// next level's matrix P^T (A P), L lanes per row, a lane per entry; a row
+// without values (only fixed DoFs below it) becomes the identity's.  LUMP:
+// the pattern leaves out couplings, whose values are added to the diagonal.
+template <typename T, int L, bool LUMP>
+__global__ void __launch_bounds__(kTB) k_mg_rap(int nc, const int32_t *__restrict__ rrp, const int32_t *__restrict__ rci,
+                                                const int32_t *__restrict__ rperm, const T *__restrict__ pv,
+                                                const int32_t *__restrict__ arp, const int32_t *__restrict__ aci,
+                                                const T *__restrict__ av, const int32_t *__restrict__ crp,
+                                                const int32_t *__restrict__ cci, T *cv) {
+    const int lane = threadIdx.x & (L - 1);
+    const int ng = gridDim.x * blockDim.x / L;
+    const int pad = (nc + 32 / L - 1) / (32 / L) * (32 / L);
+    for (int I = (blockIdx.x * blockDim.x + threadIdx.x) / L; I < pad; I += ng) {
+        const int t0 = I < nc ? crp[I] : 0, te = I < nc ? crp[I + 1] : 0;
+        const int kb = I < nc ? rrp[I] : 0, ke = I < nc ? rrp[I + 1] : 0;
+        const int chunks = __reduce_max_sync(0xffffffffu, (te - t0 + L - 1) / L);
+        const int steps = __reduce_max_sync(0xffffffffu, (ke - kb + L - 1) / L);
+        bool any = false;
+        T total = 0, kept = 0;
+        for (int tc = 0; tc < chunks; tc++) {
+            const int tb = t0 + tc * L + lane;
+            const int mine = tb < te ? cci[tb] : -1;
+            T acc = 0;
+            for (int kc = 0; kc < steps; kc++) {
+                const int k0 = kb + kc * L + lane;
+                int a0 = 0, a1 = 0;
+                T w = 0;
+                if (k0 < ke) {
+                    const int i = rci[k0];
+                    w = pv[rperm[k0]];
+                    a0 = arp[i];
+                    a1 = w == T(0) ? a0 : arp[i + 1];
+                }
+                const int m = __reduce_max_sync(0xffffffffu, min(L, max(0, ke - kb - kc * L)));
+                for (int k = 0; k < m; k++) {
+                    const int b = __shfl_sync(0xffffffffu, a0, k, L), e = __shfl_sync(0xffffffffu, a1, k, L);
+                    const T wk = __shfl_sync(0xffffffffu, w, k, L);
+                    const int longest = __reduce_max_sync(0xffffffffu, e - b);
+                    for (int q0 = 0; q0 < longest; q0 += L) {
+                        const int at = b + q0 + lane;
+                        const int c = at < e ? aci[at] : -2;
+                        const T x = at < e ? wk * av[at] : T(0);
+                        const int len = min(L, longest - q0);
+                        for (int q = 0; q < len; q++) {
+                            const int cc = __shfl_sync(0xffffffffu, c, q, L);
+                            const T xx = __shfl_sync(0xffffffffu, x, q, L);
+                            if (cc == mine) acc += xx;
+                            if (LUMP && tc == 0) total += xx;
+                        }
+                    }
+                }
+            }
+            any = any || acc != T(0);
+            kept += acc;
+            if (tb < te) cv[tb] = acc;
+        }
+        for (int o = L / 2; o > 0; o >>= 1) any = __shfl_xor_sync(0xffffffffu, (int)any, o) || any;
+        if (LUMP) {   // lanes of a row hold the same total
+            for (int o = L / 2; o > 0; o >>= 1) kept += __shfl_xor_sync(0xffffffffu, kept, o);
+            if (any)
+                for (int t = t0 + lane; t < te; t += L)
+                    if (cci[t] == I) cv[t] += total - kept;
+        }
+        if (!any)
+            for (int t = t0 + lane; t < te; t += L)
+                if (cci[t] == I) cv[t] = T(1);
+    }
+}
+
+// Q = P - w D (A P), in place of A P (both rows ascending)
+template <typename T>
+__global__ void k_mg_q(int n, const int32_t *prp, const int32_t *pci, const T *pv, const int32_t *arp,
+                       const int32_t *aci, const T *D, T *av) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int q = prp[i];
+    const int qe = prp[i + 1];
+    const T w = (T)kSmooth * D[i];
+    for (int t = arp[i]; t < arp[i + 1]; t++) {
+        T x = -w * av[t];
+        while (q < qe && pci[q] < aci[t]) q++;
+        if (q < qe && pci[q] == aci[t]) x += pv[q];
+        av[t] = x;
+    }
+}
+
+template <typename T>
+__global__ void k_mg_perm(int n, const int32_t *perm, const T *a, T *b) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) b[i] = a[perm[i]];
+}
+
+// dense inverse of the bottom matrix (n <= kMgBottom) by Gauss-Jordan in
+// shared memory, one block; a direction that is zero to rounding (pure
+// Neumann problems) is left out
+template <typename T>
+__global__ void __launch_bounds__(512) k_mg_binv(int n, const int32_t *rp, const int32_t *ci, const T *v, T *inv) {
+    extern __shared__ __align__(16) unsigned char mg_smem[];
+    T *M = reinterpret_cast<T *>(mg_smem);
+    __shared__ T col[kMgBottom], row[kMgBottom], diag[kMgBottom];
+    const int ld = n | 1;
+    for (int k = threadIdx.x; k < n * ld; k += blockDim.x) M[k] = T(0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        for (int k = rp[i]; k < rp[i + 1]; k++) {
+            M[i * ld + ci[k]] = v[k];
+            if (ci[k] == i) diag[i] = v[k];
+        }
+    __syncthreads();
+    const T eps = sizeof(T) == 8 ? T(1e-13) : T(1e-5);
+    for (int k = 0; k < n; k++) {
+        const T d = M[k * ld + k];
+        const T p = d > eps * diag[k] ? T(1) / d : T(0);
+        __syncthreads();
+        for (int j = threadIdx.x; j < n; j += blockDim.x) {
+            col[j] = M[j * ld + k];
+            row[j] = M[k * ld + j] * p;
+        }
+        __syncthreads();
+        for (int q = threadIdx.x; q < n * n; q += blockDim.x) {
+            const int i = q / n, j = q - i * n;
+            T x;
+            if (i == k) x = j == k ? p : row[j];
+            else x = j == k ? -col[i] * p : M[i * ld + j] - col[i] * row[j];
+            M[i * ld + j] = x;
+        }
+        __syncthreads();
+    }
+    for (int q = threadIdx.x; q < n * n; q += blockDim.x) inv[q] = M[q / n * ld + q % n];
+}
+
+// ------------------------------------------------------------------ the cycle
+// One block: a system whose iteration fits one SM's L1 needs no grid barrier
+// at all (about 3 us a phase), only __syncthreads.
+struct BlockSync {
+    __device__ __forceinline__ BlockSync(SolveState *, double *, long long) {}
+    __device__ __forceinline__ bool barrier() {
+        __syncthreads();
+        return true;
+    }
+    template <int NV>
+    __device__ __forceinline__ bool sum(double *v, double *sh) {
+        block_sum<NV>(v, sh);
+        return true;
+    }
+    template <int NV>
+    __device__ __forceinline__ bool sumf(float *v, float *sh) {
+        block_sum_f<NV>(v, sh);
+        return true;
+    }
+};
+struct MgGridSync : GridSync {
+    __device__ __forceinline__ MgGridSync(SolveState *st, double *part, long long spin) : GridSync{st, part, spin, 0} {}
+};
+
+// rows of a coarse operator over the grid: 8 lanes a row, or a warp where rows are long
+template <typename T, typename G, typename E>
+__device__ __forceinline__ void mg_rows(int n, const int32_t *rp, const int32_t *ci, const T *v, int longrows, G gather,
+                                        E epi) {
+    if (longrows) spmv_rows<32, 4, false, T>(n, rp, CsrSource<T>{ci, v}, gather, epi);
+    else spmv_rows<8, 2, true, T>(n, rp, CsrSource<T>{ci, v}, gather, epi);
+}
+
+// r, y of a level from the one above it
+template <typename T>
+__device__ __forceinline__ void mg_down(const int32_t *rp, const int32_t *ci, const T *v, int longrows, const T *src,
+                                        const MgLv<T> &to) {
+    mg_rows(
+        to.n, rp, ci, v, longrows, [&](int c) { return src[c]; },
+        [&](int i, T s) {
+            to.r[i] = s;
+            to.y[i] = (T)kSmooth * to.D[i] * s;
+        });
+}
+
+// e of a level: 2 y - w D A y, then + Q e of the next (both products with
+// 8 lanes a row, so the same lane writes and adds; a barrier between them
+// where a warp takes the rows of only one)
+template <typename T, class SY>
+__device__ __forceinline__ bool mg_up(const MgLv<T> &l, const T *enext, SY &sy) {
+    mg_rows(
+        l.n, l.rp, l.ci, l.v, l.along, [&](int c) { return ((const T *)l.y)[c]; },
+        [&](int i, T s) { l.e[i] = T(2) * l.y[i] - (T)kSmooth * l.D[i] * s; });
+    if (l.along != l.qlong && !sy.barrier()) return false;
+    mg_rows(
+        l.n, l.qrp, l.qci, l.qv, l.qlong, [&](int c) { return enext[c]; }, [&](int i, T s) { l.e[i] += s; });
+    return true;
+}
+
+// e of level 1 from r: restriction, the levels below, back up.  The caller
+// has passed a barrier since r was written; returns after the barrier that
+// follows e.  False: a barrier wait gave up.  Every block solves the bottom
+// level for itself (its product with the dense inverse costs less than a
+// barrier).
+template <typename T, class SY>
+__device__ __forceinline__ bool mg_cycle(const MgDev<T> &m, const T *r, T *eb, SY &sy) {
+    mg_down(m.rrp, m.rci, m.rv, m.rlong, r, m.lv[1]);
+    if (!sy.barrier()) return false;
+    const int bottom = m.nl - 1;
+    for (int l = 1; l < bottom; l++) {
+        mg_down(m.lv[l].trp, m.lv[l].tci, m.lv[l].tv, m.lv[l].tlong, (const T *)m.lv[l].r, m.lv[l + 1]);
+        if (!sy.barrier()) return false;
+    }
+    const MgLv<T> &b = m.lv[bottom];
+    const T *enext = b.y;   // no dense inverse: the smoothing step
+    if (m.dense) {
+        T *rb = eb + kMgBottom;
+        for (int i = threadIdx.x; i < b.n; i += blockDim.x) rb[i] = b.r[i];
+        __syncthreads();
+        const int lane = threadIdx.x & 3;
+        const int pad = (b.n + 7) & ~7;   // whole warps take part in the shuffles
+        for (int i = threadIdx.x >> 2; i < pad; i += blockDim.x >> 2) {
+            T s = 0;
+            if (i < b.n)
+                for (int j = lane; j < b.n; j += 4) s += __ldg(m.binv + i * b.n + j) * rb[j];
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            if (i < b.n && lane == 0) eb[i] = s;
+        }
+        __syncthreads();
+        enext = eb;
+    }
+    if (bottom == 1) {   // two levels: the fine level reads e from memory
+        if (blockIdx.x == 0)
+            for (int i = threadIdx.x; i < b.n; i += blockDim.x) b.e[i] = enext[i];
+        return sy.barrier();
+    }
+    for (int l = bottom - 1; l >= 1; l--) {
+        if (!mg_up(m.lv[l], enext, sy)) return false;
+        enext = m.lv[l].e;
+        if (!sy.barrier()) return false;
+    }
+    return true;
+}
+
+// z_i of the fine level
+template <typename T>
+__device__ __forceinline__ T mg_fine(const MgDev<T> &m, int i, T ri) {
+    T z = (T)kSmooth * __ldg(m.D0 + i) * ri;
+    if (m.ell) {
+        const int2 c = __ldg(m.ell + i);
+        const Pair<T> w = m.ellv[i];
+        const T *e = m.lv[1].e;
+        return z + (w.a * e[c.x] + w.b * e[c.y]);
+    }
+    const int e = __ldg(m.prp + i + 1);
+    for (int q = __ldg(m.prp + i); q < e; q++) z += __ldg(m.pv + q) * m.lv[1].e[__ldg(m.pci + q)];
+    return z;
+}
+
+// ------------------------------------------------------------------ FP64 solver
+template <int TPR, int U, bool PIPE, class SY>
+__global__ void __launch_bounds__(kMgT, std::is_same<SY, BlockSync>::value ? 1 : 2)
+    k_mgcg64(int n, const int32_t *rowptr, const int32_t *cols, const double *vals, const double *b, double *x, double *r,
+             double *z, double *p, double *q, double *partial, SolveState *st, double abstol, double reltol, int maxit,
+             int guess, long long spin, const __grid_constant__ MgDev<double> m) {
+    __shared__ double sh[32 * 4];
+    __shared__ double eb[2 * kMgBottom];
+    SY sy(st, partial, spin);
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gsz = gridDim.x * blockDim.x;
+    if (guess) spmv_grid<TPR, U, PIPE, double, double, double, false, true>(n, rowptr, cols, vals, x, r, nullptr, b);
+    if (!sy.barrier()) return;
+    double v[2] = {0, 0};
+    for (int i = gtid; i < n; i += gsz) {
+        const double ri = guess ? r[i] : b[i];
+        if (!guess) {
+            r[i] = ri;
+            x[i] = 0.0;
+        }
+        p[i] = 0.0;
+        v[0] += ri * ri;
+        v[1] += b[i] * b[i];
+    }
+    if (!sy.template sum<2>(v, sh)) return;
+    const double bn = sqrt(v[1]);
+    const double tol = fmax(abstol, reltol * bn);
+    int it = 0;
+    bool conv = sqrt(v[0]) <= tol;
+    double rz = 0.0;
+    while (!conv && it < maxit) {
+        if (!mg_cycle(m, (const double *)r, eb, sy)) return;
+        double w[1] = {0};
+        for (int i = gtid; i < n; i += gsz) {
+            const double ri = r[i], zi = mg_fine(m, i, ri);
+            z[i] = zi;
+            w[0] += ri * zi;
+        }
+        if (!sy.template sum<1>(w, sh)) return;
+        const double beta = it == 0 ? 0.0 : w[0] / rz;
+        rz = w[0];
+        for (int i = gtid; i < n; i += gsz) p[i] = z[i] + beta * p[i];
+        if (!sy.barrier()) return;
+        double d[1];
+        d[0] = spmv_grid<TPR, U, PIPE, double, double, double, true, false>(n, rowptr, cols, vals, p, q, p, nullptr);
+        if (!sy.template sum<1>(d, sh)) return;
+        const double pq = d[0];
+        if (!(pq > 0) || !isfinite(pq) || !isfinite(rz)) {
+            if (gtid == 0) atomicCAS(&st->status, 0, (int)GRMP_ERR_NAN);
+            break;
+        }
+        const double alpha = rz / pq;
+        double rr[1] = {0};
+        for (int i = gtid; i < n; i += gsz) {
+            x[i] += alpha * p[i];
+            const double ri = r[i] - alpha * q[i];
+            r[i] = ri;
+            rr[0] += ri * ri;
+        }
+        if (!sy.template sum<1>(rr, sh)) return;
+        it++;
+        conv = sqrt(rr[0]) <= tol;
+    }
+    if (!sy.barrier()) return;
+    double t[1];
+    t[0] = spmv_grid<TPR, U, PIPE, double, double, double, true, true>(n, rowptr, cols, vals, x, r, nullptr, b);
+    if (!sy.template sum<1>(t, sh)) return;
+    if (gtid == 0) {
+        st->iters = it;
+        st->outer = 0;
+        st->relres = sqrt(t[0]) / (bn > 0 ? bn : 1.0);
+        if (st->status == 0 && !(sqrt(t[0]) <= fmax(tol, 0.0) || conv)) st->status = GRMP_ERR_NOT_CONVERGED;
+    }
+}
+
+// ------------------------------------------------------------------ mixed solver
+// FP32 conjugate gradients with the FP32 cycle inside the FP64 refinement
+// loop of the Jacobi mixed solver (solve.cu): the FP32 correction is folded
+// into x when the FP32 residual has fallen by `delta`, the FP64 residual
+// replaces it, the direction is kept unless the true residual stopped falling.
+template <int TPR, int U, bool PIPE, class SY>
+__global__ void __launch_bounds__(kMgT, std::is_same<SY, BlockSync>::value ? 1 : 2)
+    k_mgcg_mixed(int n, const int32_t *rowptr, const int32_t *cols, const double *vals64, const float *vals32,
+                 const double *b, double *x, float *r, float *q, float *xc, float2 *zp0, float2 *zp1, double *r64,
+                 double *partial, SolveState *st, double abstol, double reltol, double delta, int maxit, int maxouter,
+                 int guess, long long spin, const __grid_constant__ MgDev<float> m) {
+    __shared__ double sh[32 * 4];
+    __shared__ float shf[32 * 4];
+    __shared__ float eb[2 * kMgBottom];
+    SY sy(st, partial, spin);
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gsz = gridDim.x * blockDim.x;
+    double v[2] = {0, 0};
+    if (guess) {
+        v[0] = spmv_grid<TPR, U, PIPE, double, double, double, true, true>(n, rowptr, cols, vals64, x, r64, nullptr, b);
+    } else {
+        for (int i = gtid; i < n; i += gsz) {
+            x[i] = 0.0;
+            r64[i] = b[i];
+            v[0] += b[i] * b[i];
+        }
+    }
+    for (int i = gtid; i < n; i += gsz) v[1] += b[i] * b[i];
+    if (!sy.template sum<2>(v, sh)) return;
+    const double bn = sqrt(v[1]);
+    const double tol = fmax(abstol, reltol * bn);
+    double rn64 = sqrt(v[0]), prev_rn64 = rn64;
+    // the FP32 system is solved for the residual scaled to norm 1: the
+    // correction and its residual stay in FP32's range at any size of b
+    double scale = rn64 > 0 ? rn64 : 1.0;
+    for (int i = gtid; i < n; i += gsz) {
+        r[i] = (float)(r64[i] / scale);
+        zp0[i] = make_float2(0.f, 0.f);
+        xc[i] = 0.f;
+    }
+    if (!sy.barrier()) return;
+    int it = 0, outer = 0, stall = 0;
+    bool conv = rn64 <= tol;
+    float rz = 0.f, rmax = 1.f;
+    bool restart = true;
+    float2 *cur = zp0, *nxt = zp1;
+    while (!conv && it < maxit && outer < maxouter) {
+        if (!mg_cycle(m, (const float *)r, eb, sy)) return;
+        float w[1] = {0.f};
+#pragma unroll 4
+        for (int i = gtid; i < n; i += gsz) {
+            const float ri = r[i], zi = mg_fine(m, i, ri);
+            cur[i].x = zi;
+            w[0] += ri * zi;
+        }
+        if (!sy.template sumf<1>(w, shf)) return;
+        const float beta = restart ? 0.f : w[0] / rz;
+        rz = w[0];
+        // q = A p with p = z + beta p formed while gathering; the owner of a row stores p
+        float dot = 0.f;
+        spmv_rows<TPR, U, PIPE, float>(
+            n, rowptr, CsrSource<float>{cols, vals32},
+            [&](int c) {
+                const float2 e = cur[c];
+                return fmaf(beta, e.y, e.x);
+            },
+            [&](int i, float s) {
+                const float2 e = cur[i];
+                const float pi = fmaf(beta, e.y, e.x);
+                nxt[i].y = pi;
+                q[i] = s;
+                dot += pi * s;
+            });
+        float d[1] = {dot};
+        if (!sy.template sumf<1>(d, shf)) return;
+        const float pq = d[0];
+        if (!(pq > 0.f) || !isfinite(pq) || !isfinite(rz)) {
+            if (gtid == 0) atomicCAS(&st->status, 0, (int)GRMP_ERR_NAN);
+            break;
+        }
+        const float alpha = rz / pq;
+        float u[1] = {0.f};
+        {   // four rows a thread, 16-byte accesses
+            float4 *xc4 = reinterpret_cast<float4 *>(xc), *r4 = reinterpret_cast<float4 *>(r);
+            const float4 *q4 = reinterpret_cast<const float4 *>(q), *nx4 = reinterpret_cast<const float4 *>(nxt);
+            const int n4 = n >> 2;
+            for (int i = gtid; i < n4; i += gsz) {
+                const float4 a = nx4[2 * i], c = nx4[2 * i + 1], qq = q4[i];
+                float4 rr = r4[i], xx = xc4[i];
+                xx.x += alpha * a.y;
+                xx.y += alpha * a.w;
+                xx.z += alpha * c.y;
+                xx.w += alpha * c.w;
+                rr.x -= alpha * qq.x;
+                rr.y -= alpha * qq.y;
+                rr.z -= alpha * qq.z;
+                rr.w -= alpha * qq.w;
+                xc4[i] = xx;
+                r4[i] = rr;
+                u[0] += rr.x * rr.x + rr.y * rr.y + rr.z * rr.z + rr.w * rr.w;
+            }
+            for (int i = 4 * n4 + gtid; i < n; i += gsz) {
+                xc[i] += alpha * nxt[i].y;
+                const float ri = r[i] - alpha * q[i];
+                r[i] = ri;
+                u[0] += ri * ri;
+            }
+        }
+        if (!sy.template sumf<1>(u, shf)) return;
+        it++;
+        const float rn32 = sqrtf(u[0]);
+        restart = false;
+        if (rn32 <= (float)delta * rmax || (double)rn32 * scale <= tol || it >= maxit) {
+            for (int i = gtid; i < n; i += gsz) {
+                x[i] += (double)xc[i] * scale;
+                xc[i] = 0.f;
+            }
+            if (!sy.barrier()) return;
+            double t[1];
+            t[0] = spmv_grid<TPR, U, PIPE, double, double, double, true, true>(n, rowptr, cols, vals64, x, r64, nullptr, b);
+            if (!sy.template sum<1>(t, sh)) return;
+            outer++;
+            rn64 = sqrt(t[0]);
+            conv = rn64 <= tol;
+            if (conv || it >= maxit) break;
+            restart = rn64 > 0.5 * prev_rn64;
+            stall = (rn64 > 0.9 * prev_rn64) ? stall + 1 : 0;
+            prev_rn64 = rn64;
+            if (stall >= 16) break;
+            // rescale: directions and rz are of the old scale
+            const float f = (float)(scale / rn64);
+            scale = rn64;
+            rz *= f * f;
+            for (int i = gtid; i < n; i += gsz) {
+                r[i] = (float)(r64[i] / scale);
+                nxt[i].y *= f;
+            }
+            rmax = 1.f;
+            if (!sy.barrier()) return;
+        }
+        float2 *tmp = cur;
+        cur = nxt;
+        nxt = tmp;
+    }
+    if (gtid == 0) {
+        st->iters = it;
+        st->outer = outer;
+        st->relres = rn64 / (bn > 0 ? bn : 1.0);
+        if (st->status == 0 && !conv) st->status = GRMP_ERR_NOT_CONVERGED;
+    }
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------- host side
+struct MgCache {
+    MgSymbolic S;
+    std::vector<std::pair<void *, size_t>> bufs;   // patterns
+    struct Step {
+        int32_t *agg = nullptr, *vrow = nullptr;
+        int2 *ell = nullptr;
+        int32_t *prp, *pci, *rrp, *rci, *rperm, *arp, *aci, *trp = nullptr, *tci = nullptr, *tperm = nullptr, *crp, *cci;
+        size_t np, na, nt, nc;   // entries of P, A P, Q^T, next A
+        int amax, cmax;          // longest row of A P, next A
+    };
+    std::vector<Step> step;
+    // numeric storage per precision (0: FP64, 1: FP32), one allocation each
+    struct Num {
+        void *p = nullptr;
+        size_t bytes = 0;
+        std::vector<char *> pv, av, tv, cv, D, iso, r, y, e;
+        char *rv0 = nullptr, *ellv = nullptr, *binv = nullptr, *part = nullptr, *vec = nullptr;
+        int *bad = nullptr;
+    } num[2];
+    double react[2] = {0, 0};
+    char *state = nullptr;
+};
+
+namespace {
+
+inline size_t al(size_t v) { return (v + 255) & ~(size_t)255; }
+
+template <typename V>
+int mg_up_vec(grmp_context ctx, MgCache &C, const std::vector<V> &v, V **out) {
+    const size_t bytes = std::max<size_t>(1, v.size()) * sizeof(V);
+    void *p = nullptr;
+    int rc = grmp_alloc(ctx, &p, bytes);
+    if (rc) return rc;
+    C.bufs.push_back({p, bytes});
+    *out = (V *)p;
+    if (v.empty()) return GRMP_OK;
+    cudaError_t e = cudaMemcpyAsync(p, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, ctx->stream);
+    return e == cudaSuccess ? GRMP_OK : grmp_cuda_fail(ctx, e, "multilevel patterns");
+}
+
+int mg_build(grmp_matrix A) {
+    grmp_space s = A->space;
+    grmp_context ctx = s->mesh->ctx;
+    const int n = A->nrows;
+    std::vector<int32_t> rp((size_t)n + 1), ci((size_t)A->nnz), cd, cells;
+    std::vector<double> coords;
+    cudaError_t e = cudaMemcpyAsync(rp.data(), A->d_rowptr, rp.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ci.data(), A->d_cols, ci.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
+    if (s->fe == GRMP_FE_H1P2) {
+        cd.resize((size_t)s->mesh->ncells * s->ldofs);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(cd.data(), s->d_celldofs, cd.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
+        cells.resize((size_t)s->mesh->ncells * (s->mesh->dim + 1));
+        coords.resize((size_t)s->mesh->nverts * s->mesh->dim);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(cells.data(), s->mesh->d_cells, cells.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(coords.data(), s->mesh->d_coords, coords.size() * 8, cudaMemcpyDeviceToHost, ctx->stream);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multilevel: pattern download");
+    MgCache *C = new MgCache;
+    A->mg = C;
+    if (mg_symbolic_build(n, rp.data(), ci.data(), s->mesh->dim, s->mesh->ncells, s->ldofs, cd.empty() ? nullptr : cd.data(),
+                          coords.data(), cells.data(), &C->S)) {
+        A->mg_state = -1;
+        return GRMP_OK;
+    }
+    int rc = GRMP_OK;
+    const int ns = (int)C->S.step.size();
+    C->step.resize(ns);
+    for (int k = 0; k < ns && !rc; k++) {
+        MgStep &t = C->S.step[k];
+        MgCache::Step &d = C->step[k];
+        d.np = t.P.ci.size();
+        d.na = t.AP.ci.size();
+        d.nt = t.QT.ci.size();
+        d.nc = t.Ac.ci.size();
+        d.amax = d.cmax = 0;
+        for (int i = 0; i < t.n; i++) d.amax = std::max(d.amax, t.AP.rp[i + 1] - t.AP.rp[i]);
+        for (int i = 0; i < t.nc; i++) d.cmax = std::max(d.cmax, t.Ac.rp[i + 1] - t.Ac.rp[i]);
+        auto up = [&](std::vector<int32_t> &v, int32_t **p) {
+            if (!rc) rc = mg_up_vec(ctx, *C, v, p);
+        };
+        if (t.geometric) {
+            std::vector<int32_t> vrow(t.nc);
+            for (int i = 0; i < t.n; i++)
+                if (t.P.rp[i + 1] - t.P.rp[i] == 1) vrow[t.P.ci[t.P.rp[i]]] = i;
+            up(vrow, &d.vrow);
+            std::vector<int2> ell(t.n);
+            for (int i = 0; i < t.n; i++) ell[i] = make_int2(t.P.ci[t.P.rp[i]], t.P.ci[t.P.rp[i + 1] - 1]);
+            if (!rc) rc = mg_up_vec(ctx, *C, ell, &d.ell);
+            if (!rc && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = GRMP_ERR_DEVICE;
+        } else {
+            up(t.agg, &d.agg);
+        }
+        up(t.P.rp, &d.prp);
+        up(t.P.ci, &d.pci);
+        up(t.R.rp, &d.rrp);
+        up(t.R.ci, &d.rci);
+        up(t.Rperm, &d.rperm);
+        up(t.AP.rp, &d.arp);
+        up(t.AP.ci, &d.aci);
+        up(t.Ac.rp, &d.crp);
+        up(t.Ac.ci, &d.cci);
+        if (k > 0) {
+            up(t.QT.rp, &d.trp);
+            up(t.QT.ci, &d.tci);
+            up(t.QTperm, &d.tperm);
+        }
+        if (!rc && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = GRMP_ERR_DEVICE;
+        t.P = t.R = t.AP = t.QT = t.Ac = MgCsr();   // the sizes stay
+        t.Rperm = t.QTperm = t.agg = std::vector<int32_t>();
+    }
+    if (rc) return rc;
+    A->mg_state = 1;
+    return GRMP_OK;
+}
+
+size_t mg_bytes(const MgCache &C) {
+    size_t b = 0;
+    for (auto &x : C.bufs) b += x.second;
+    for (auto &N : C.num) b += N.bytes;
+    return b;
+}
+
+// numeric storage of one precision: values of every level, vectors, state
+template <typename T>
+int mg_storage(grmp_matrix A) {
+    grmp_context ctx = A->space->mesh->ctx;
+    MgCache &C = *A->mg;
+    MgCache::Num &N = C.num[sizeof(T) == 8 ? 0 : 1];
+    if (N.p) return GRMP_OK;
+    const int ns = (int)C.step.size();
+    for (int pass = 0; pass < 2; pass++) {
+        size_t at = 0;
+        auto take = [&](size_t bytes) -> char * {
+            const size_t o = at;
+            at += al(bytes);
+            return pass ? (char *)N.p + o : nullptr;
+        };
+        N.pv.assign(ns, nullptr);
+        N.av = N.tv = N.cv = N.pv;
+        N.D.assign(ns + 1, nullptr);
+        N.iso = N.r = N.y = N.e = N.D;
+        for (int k = 0; k < ns; k++) {
+            const MgCache::Step &d = C.step[k];
+            N.pv[k] = take(d.np * sizeof(T));
+            N.av[k] = take(d.na * sizeof(T));
+            N.cv[k] = take(d.nc * sizeof(T));
+            N.tv[k] = take(d.nt * sizeof(T));
+        }
+        N.rv0 = take(C.step[0].np * sizeof(T));
+        N.ellv = take(C.step[0].ell ? (size_t)A->nrows * 2 * sizeof(T) : 0);
+        for (int k = 0; k <= ns; k++) {
+            const size_t n = k < ns ? C.S.step[k].n : C.S.step[ns - 1].nc;
+            N.D[k] = take(n * sizeof(T));
+            N.iso[k] = take(n);
+            if (k > 0) {
+                N.r[k] = take(n * sizeof(T));
+                N.y[k] = take(n * sizeof(T));
+                N.e[k] = take(n * sizeof(T));
+            }
+        }
+        N.binv = take((size_t)kMgBottom * kMgBottom * sizeof(T));
+        N.part = take((size_t)4096 * 16);
+        N.bad = (int *)take(4);
+        // FP64: r z p q; mixed: r q xc, two pairs, FP64 residual
+        const size_t n0 = A->nrows;
+        N.vec = take(sizeof(T) == 8 ? 4 * al(n0 * 8) : 3 * al(n0 * 4) + 2 * al(n0 * 8) + al(n0 * 8));
+        if (pass == 0) {
+            N.bytes = at + al((size_t)2 * kPartStride * 8) + al(sizeof(SolveState));
+            int rc = mg_bytes(C) > A->mg_budget ? (int)GRMP_ERR_BUDGET : grmp_alloc(ctx, &N.p, N.bytes);
+            if (rc) {
+                N.p = nullptr;
+                N.bytes = 0;
+                return rc;
+            }
+        }
+    }
+    return GRMP_OK;
+}
+
+template <typename T>
+const T *fine_values(grmp_matrix A);
+template <>
+const double *fine_values<double>(grmp_matrix A) { return A->d_vals64; }
+template <>
+const float *fine_values<float>(grmp_matrix A) { return A->d_vals32; }
+
+// D of the fine level, the diagonal check and the reaction share
+template <typename T>
+int mg_probe(grmp_matrix A, double *react) {
+    grmp_context ctx = A->space->mesh->ctx;
+    MgCache &C = *A->mg;
+    MgCache::Num &N = C.num[sizeof(T) == 8 ? 0 : 1];
+    const int n = A->nrows, grid = std::max(1, std::min(nblk(n, kTB / kCl), 4 * ctx->num_sms));
+    cudaMemsetAsync(N.bad, 0, 4, ctx->stream);
+    k_mg_rows<T><<<grid, kTB, 0, ctx->stream>>>(n, A->d_rowptr, A->d_cols, fine_values<T>(A), (T *)N.D[0],
+                                                (uint8_t *)N.iso[0], (double2 *)N.part, N.bad);
+    GRMP_LAUNCHED(ctx);
+    double h[2 * 4096];
+    int bad = 0;
+    cudaError_t e = cudaMemcpyAsync(h, N.part, (size_t)grid * 16, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, N.bad, 4, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multilevel: diagonal");
+    if (bad) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "solve: non-positive or non-finite diagonal entry");
+    double s = 0, d = 0;
+    for (int b = 0; b < grid; b++) s += h[2 * b], d += h[2 * b + 1];
+    *react = d > 0 ? s / d : 1.0;
+    return GRMP_OK;
+}
+
+template <typename T>
+void mg_values(grmp_matrix A) {
+    grmp_context ctx = A->space->mesh->ctx;
+    cudaStream_t st = ctx->stream;
+    MgCache &C = *A->mg;
+    MgCache::Num &N = C.num[sizeof(T) == 8 ? 0 : 1];
+    const int ns = (int)C.step.size();
+    const int32_t *rp = A->d_rowptr, *ci = A->d_cols;
+    const T *v = fine_values<T>(A);
+    const int wide = 8 * ctx->num_sms;
+    for (int k = 0; k < ns; k++) {
+        const MgCache::Step &d = C.step[k];
+        const int n = C.S.step[k].n, nc = C.S.step[k].nc;
+        T *pv = (T *)N.pv[k], *av = (T *)N.av[k], *cv = (T *)N.cv[k], *D = (T *)N.D[k];
+        if (k > 0) {
+            k_mg_rows<T><<<std::max(1, std::min(nblk(n, kTB / kCl), wide)), kTB, 0, st>>>(
+                n, rp, ci, v, D, (uint8_t *)N.iso[k], nullptr, nullptr);
+            GRMP_LAUNCHED(ctx);
+        }
+        if (d.vrow)
+            k_mg_prol_geo<T><<<nblk(n), 256, 0, st>>>(n, d.prp, d.pci, d.vrow, (const uint8_t *)N.iso[k], pv,
+                                                        (Pair<T> *)N.ellv);
+        else
+            k_mg_prol_agg<T><<<nblk(n, 128), 128, 0, st>>>(n, rp, ci, v, D, (const uint8_t *)N.iso[k], d.agg, d.prp, d.pci,
+                                                           pv);
+        // lanes per row: the smallest power of two that holds the longest row of the product
+        const int la = d.amax <= 8 ? 8 : (d.amax <= 16 ? 16 : 32), lc = d.cmax <= 8 ? 8 : (d.cmax <= 16 ? 16 : 32);
+        auto ap = la == 8 ? k_mg_ap<T, 8> : (la == 16 ? k_mg_ap<T, 16> : k_mg_ap<T, 32>);
+        auto rap = lc == 8 ? k_mg_rap<T, 8, false> : (lc == 16 ? k_mg_rap<T, 16, false> : k_mg_rap<T, 32, false>);
+        if (C.S.step[k].filtered)
+            rap = lc == 8 ? k_mg_rap<T, 8, true> : (lc == 16 ? k_mg_rap<T, 16, true> : k_mg_rap<T, 32, true>);
+        ap<<<std::max(1, std::min(nblk((long long)n * la), wide)), kTB, 0, st>>>(n, rp, ci, v, d.prp, d.pci, pv, d.arp,
+                                                                                d.aci, av);
+        rap<<<std::max(1, std::min(nblk((long long)nc * lc), wide)), kTB, 0, st>>>(nc, d.rrp, d.rci, d.rperm, pv, d.arp,
+                                                                                  d.aci, av, d.crp, d.cci, cv);
+        ctx->launches += 3;
+        if (k > 0) {
+            k_mg_q<T><<<nblk(n, 128), 128, 0, st>>>(n, d.prp, d.pci, pv, d.arp, d.aci, D, av);
+            k_mg_perm<T><<<nblk((long long)d.nt), 256, 0, st>>>((int)d.nt, d.tperm, av, (T *)N.tv[k]);
+            ctx->launches += 2;
+        } else {
+            k_mg_perm<T><<<nblk((long long)d.np), 256, 0, st>>>((int)d.np, d.rperm, pv, (T *)N.rv0);
+            GRMP_LAUNCHED(ctx);
+        }
+        rp = d.crp;
+        ci = d.cci;
+        v = cv;
+    }
+    const int nb = C.S.step[ns - 1].nc;
+    k_mg_rows<T><<<std::max(1, std::min(nblk(nb, kTB / kCl), wide)), kTB, 0, st>>>(
+        nb, rp, ci, v, (T *)N.D[ns], (uint8_t *)N.iso[ns], nullptr, nullptr);
+    GRMP_LAUNCHED(ctx);
+    if (nb <= kMgBottom) {
+        const size_t smem = (size_t)nb * (nb | 1) * sizeof(T);
+        cudaFuncSetAttribute(k_mg_binv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_mg_binv<T><<<1, 512, smem, st>>>(nb, rp, ci, v, (T *)N.binv);
+        GRMP_LAUNCHED(ctx);
+    }
+}
+
+template <typename T>
+MgDev<T> mg_device(grmp_matrix A) {
+    MgCache &C = *A->mg;
+    MgCache::Num &N = C.num[sizeof(T) == 8 ? 0 : 1];
+    const int ns = (int)C.step.size();
+    MgDev<T> m;
+    std::memset(&m, 0, sizeof(m));
+    m.nl = ns + 1;
+    m.prp = C.step[0].prp;
+    m.pci = C.step[0].pci;
+    m.pv = (const T *)N.pv[0];
+    m.rrp = C.step[0].rrp;
+    m.rci = C.step[0].rci;
+    m.rv = (const T *)N.rv0;
+    m.ell = C.step[0].ell;
+    m.ellv = (const Pair<T> *)N.ellv;
+    m.D0 = (const T *)N.D[0];
+    m.binv = (const T *)N.binv;
+    m.dense = C.S.step[ns - 1].nc <= kMgBottom;
+    auto lng = [](size_t entries, int rows) { return (int)(entries > (size_t)kLongRow * rows); };
+    m.rlong = lng(C.step[0].np, C.S.step[0].nc);
+    for (int l = 1; l <= ns; l++) {
+        MgLv<T> &L = m.lv[l];
+        L.n = C.S.step[l - 1].nc;
+        L.rp = C.step[l - 1].crp;
+        L.ci = C.step[l - 1].cci;
+        L.v = (const T *)N.cv[l - 1];
+        L.D = (const T *)N.D[l];
+        L.along = lng(C.step[l - 1].nc, L.n);
+        if (l < ns) {
+            L.qlong = lng(C.step[l].na, L.n);
+            L.tlong = lng(C.step[l].nt, C.S.step[l].nc);
+            L.qrp = C.step[l].arp;
+            L.qci = C.step[l].aci;
+            L.qv = (const T *)N.av[l];
+            L.trp = C.step[l].trp;
+            L.tci = C.step[l].tci;
+            L.tv = (const T *)N.tv[l];
+        }
+        L.r = (T *)N.r[l];
+        L.y = (T *)N.y[l];
+        L.e = (T *)N.e[l];
+    }
+    return m;
+}
+
+// Systems of at most this many rows run in one block (its L1 holds matrix and
+// vectors; on the FP64 pipe of one SM, two FMAs a clock, only smaller ones gain)
+constexpr int kOneBlock32 = 6000, kOneBlock64 = 1200;
+
+// grid: enough blocks for the rows, at most what fits; small systems take
+// one block per SM, which makes the barriers cheaper
+template <typename K>
+int mg_grid(grmp_context ctx, K kern, int n, int tpr, int want) {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kMgT, 0);
+    const int maxg = std::max(1, per_sm) * ctx->num_sms;
+    if (want > 0) return std::min(want, maxg);
+    const int need = std::max(1, nblk((long long)n * tpr, kMgT));
+    const int cap = n <= 150000 ? ctx->num_sms : maxg;
+    return std::min({need, cap, maxg});
+}
+
+template <typename K>
+cudaError_t mg_start(grmp_context ctx, K kern, bool one, int n, int tpr, int want, void **args, int *grid) {
+    *grid = one ? 1 : mg_grid(ctx, kern, n, tpr, want);
+    GRMP_LAUNCHED(ctx);
+    if (one) return cudaLaunchKernel((const void *)kern, dim3(1), dim3(kMgT), args, 0, ctx->stream);
+    return cudaLaunchCooperativeKernel((const void *)kern, dim3(*grid), dim3(kMgT), args, 0, ctx->stream);
+}
+
+template <int TPR, int U, bool PIPE>
+int mg_launch(grmp_matrix A, const double *b, double *x, const grmp_solve_params *p, bool mixed, int *grid) {
+    grmp_context ctx = A->space->mesh->ctx;
+    MgCache::Num &N = A->mg->num[mixed ? 1 : 0];
+    const size_t n0 = A->nrows;
+    char *part = (char *)N.p + N.bytes - al(sizeof(SolveState)) - al((size_t)2 * kPartStride * 8);
+    SolveState *dst = (SolveState *)((char *)N.p + N.bytes - al(sizeof(SolveState)));
+    double *partial = (double *)part;
+    int n = A->nrows, mi = p->maxiter, guess = p->use_initial_guess ? 1 : 0;
+    double at = p->abstol, rt = p->reltol;
+    const int32_t *rp = A->d_rowptr, *ci = A->d_cols;
+    const double *v64 = A->d_vals64;
+    long long spin = ctx->wait_limit;
+    cudaMemsetAsync(dst, 0, sizeof(SolveState), ctx->stream);
+    cudaError_t e;
+    if (!mixed) {
+        const bool one = n <= kOneBlock64 && p->grid_blocks <= 0;
+        auto kern = one ? k_mgcg64<TPR, U, PIPE, BlockSync> : k_mgcg64<TPR, U, PIPE, MgGridSync>;
+        MgDev<double> m = mg_device<double>(A);
+        double *r = (double *)N.vec, *z = (double *)(N.vec + al(n0 * 8)), *pp = (double *)(N.vec + 2 * al(n0 * 8));
+        double *q = (double *)(N.vec + 3 * al(n0 * 8));
+        void *args[] = {&n, &rp, &ci, &v64, &b, &x, &r, &z, &pp, &q, &partial, &dst, &at, &rt, &mi, &guess, &spin, &m};
+        e = mg_start(ctx, kern, one, n, TPR, p->grid_blocks, args, grid);
+    } else {
+        const bool one = n <= kOneBlock32 && p->grid_blocks <= 0;
+        auto kern = one ? k_mgcg_mixed<TPR, U, PIPE, BlockSync> : k_mgcg_mixed<TPR, U, PIPE, MgGridSync>;
+        MgDev<float> m = mg_device<float>(A);
+        const float *v32 = A->d_vals32;
+        float *r = (float *)N.vec, *q = (float *)(N.vec + al(n0 * 4)), *xc = (float *)(N.vec + 2 * al(n0 * 4));
+        char *w = N.vec + 3 * al(n0 * 4);
+        float2 *zp0 = (float2 *)w, *zp1 = (float2 *)(w + al(n0 * 8));
+        double *r64 = (double *)(w + 2 * al(n0 * 8));
+        int mo = p->max_outer > 0 ? p->max_outer : 1000;
+        // an iteration of this solver gains about as much as ten of the Jacobi one, a
+        // refinement costs the same: it waits for three times as many digits
+        const double d1 = p->inner_reltol > 0 && p->inner_reltol < 1 ? p->inner_reltol : 0.1;
+        double delta = std::max(1e-4, d1 * d1 * d1);
+        void *args[] = {&n, &rp, &ci, &v64, &v32, &b, &x, &r, &q, &xc, &zp0, &zp1, &r64, &partial, &dst,
+                        &at, &rt, &delta, &mi, &mo, &guess, &spin, &m};
+        e = mg_start(ctx, kern, one, n, TPR, p->grid_blocks, args, grid);
+    }
+    return e == cudaSuccess ? GRMP_OK : grmp_cuda_fail(ctx, e, "multilevel solve launch");
+}
+
+}  // namespace
+
+void grmp_mg_free(grmp_matrix A) {
+    if (!A || !A->mg) return;
+    grmp_context ctx = A->space->mesh->ctx;
+    for (auto &b : A->mg->bufs) grmp_free(ctx, b.first, b.second);
+    for (auto &N : A->mg->num) grmp_free(ctx, N.p, N.bytes);
+    delete A->mg;
+    A->mg = nullptr;
+}
+
+bool grmp_mg_ready(grmp_matrix A, bool mixed) { return A->mg_state > 0 && A->mg && A->mg->num[mixed ? 1 : 0].p; }
+
+int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use) {
+    *use = 0;
+    grmp_space s = A->space;
+    grmp_context ctx = s->mesh->ctx;
+    if (A->mg_state < 0 || A->imported || !A->elliptic || A->nrows < kMinRows || s->ncomp != 1 ||
+        (s->fe != GRMP_FE_H1P1 && s->fe != GRMP_FE_H1P2))
+        return GRMP_OK;
+    int rc = GRMP_OK;
+    if (!A->mg) rc = mg_build(A);
+    if (!rc && A->mg_state > 0) rc = mixed ? mg_storage<float>(A) : mg_storage<double>(A);
+    if (rc == GRMP_ERR_BUDGET || rc == GRMP_ERR_OUT_OF_MEMORY) {   // no room for the hierarchy: the Jacobi solvers
+        grmp_mg_free(A);
+        A->mg_state = -1;
+        ctx->last_error.clear();
+        cudaGetLastError();
+        return GRMP_OK;
+    }
+    if (rc || A->mg_state < 0) return rc;
+    double react = 0.0;
+    rc = mixed ? mg_probe<float>(A, &react) : mg_probe<double>(A, &react);
+    if (rc) return rc;
+    if (react > kMaxReaction) return GRMP_OK;
+    if (mixed) mg_values<float>(A);
+    else mg_values<double>(A);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multilevel values");
+    *use = 1;
+    return GRMP_OK;
+}
+
+int grmp_mg_solve(grmp_matrix A, const double *b, double *x, const grmp_solve_params *p, grmp_solve_stats *st) {
+    grmp_context ctx = A->space->mesh->ctx;
+    const bool mixed = p->mode == GRMP_SOLVE_MIXED;
+    const double avg = (double)A->nnz / std::max(1, A->nrows);
+    MgCache::Num &N = A->mg->num[mixed ? 1 : 0];
+    const SolveState *dst = (const SolveState *)((char *)N.p + N.bytes - al(sizeof(SolveState)));
+    cudaEvent_t e0, e1;
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+    cudaEventRecord(e0, ctx->stream);
+    int grid = 0, code, rc;
+    if (avg <= 8) {
+        code = 204;
+        rc = mg_launch<2, 4, true>(A, b, x, p, mixed, &grid);
+    } else if (avg <= 20) {
+        code = 404;
+        rc = mg_launch<4, 4, true>(A, b, x, p, mixed, &grid);
+    } else {
+        code = 408;
+        rc = mg_launch<4, 8, true>(A, b, x, p, mixed, &grid);
+    }
+    cudaEventRecord(e1, ctx->stream);
+    SolveState hs;
+    cudaError_t e = rc ? cudaSuccess : cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream);
+    if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    float ms = 0;
+    if (!rc && e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    if (rc) return rc;
+    if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multilevel solve");
+    st->status = hs.status;
+    st->iterations = hs.iters;
+    st->outer_iterations = hs.outer;
+    st->final_relres = hs.relres;
+    st->spmv_config = kMgConfig + code;
+    st->grid_blocks = grid;
+    st->solve_ms = ms;
+    if (hs.status == GRMP_ERR_NOT_CONVERGED)
+        return grmp_fail(ctx, GRMP_ERR_NOT_CONVERGED, "PCG: %d iterations, relative residual %.3e", hs.iters, hs.relres);
+    if (hs.status == GRMP_ERR_TIMEOUT) return grmp_fail(ctx, GRMP_ERR_TIMEOUT, "PCG: a grid barrier wait timed out");
+    if (hs.status == GRMP_ERR_NAN) return grmp_fail(ctx, GRMP_ERR_NAN, "PCG: breakdown (non-positive or non-finite p.Ap)");
+    return hs.status;
+}

@@ -1,0 +1,17 @@
+// Multilevel preconditioner of the scalar elliptic solves (mg.cu).
+#pragma once
+#include "grmp_internal.h"
+
+// spmv_config reported by a solve that the multilevel preconditioner ran
+// (plus the row-loop code of its SpMV, e.g. 90404)
+constexpr int kMgConfig = 90000;
+
+// Whether grmp_solve takes the multilevel solver for this matrix (scalar
+// H1P1 / H1P2 with a diffusion term, not reaction dominated); builds or
+// refreshes what it needs.  *use = 0: the Jacobi solvers.
+int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use);
+// Jacobi-free conjugate gradients with the prepared hierarchy; allocates nothing.
+int grmp_mg_solve(grmp_matrix A, const double *b, double *x, const grmp_solve_params *p, grmp_solve_stats *st);
+// Whether a hierarchy with numeric storage of this precision exists.
+bool grmp_mg_ready(grmp_matrix A, bool mixed);
+void grmp_mg_free(grmp_matrix A);

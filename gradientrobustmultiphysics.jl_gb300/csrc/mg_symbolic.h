@@ -1,0 +1,36 @@
+// Multilevel hierarchy of a scalar elliptic matrix: the patterns (host side).
+#pragma once
+#include <cstdint>
+#include <vector>
+
+struct MgCsr {
+    std::vector<int32_t> rp, ci;   // rows, ascending columns
+};
+
+// One coarsening step from a level of n rows to nc: the prolongation P, its
+// transpose R, the product A P (also the pattern of the smoothed
+// prolongation Q), its transpose, and the next level's matrix P^T A P.
+// perm arrays give, for each entry of a transpose, its position in the
+// original.
+struct MgStep {
+    int n = 0, nc = 0;
+    bool geometric = false;              // P2 -> P1 interpolation, else smoothed aggregation
+    bool filtered = false;               // Ac leaves out couplings (their values go to the diagonal)
+    std::vector<int32_t> agg;            // aggregate of each row (smoothed aggregation)
+    MgCsr P, R, AP, QT, Ac;
+    std::vector<int32_t> Rperm, QTperm;
+};
+
+struct MgSymbolic {
+    std::vector<MgStep> step;            // step[0]: fine level
+};
+
+constexpr int kMgBottom = 96;            // rows of a level that is solved densely
+constexpr int kMgMaxLevels = 14;
+
+// Builds the steps of a matrix with pattern (n, rp, ci).  celldofs != nullptr:
+// a P2 space's cell DoFs [ncells][ld] (dim + 1 vertices, then edges) on the
+// mesh (coords, cells); the first step then interpolates from the vertices.
+// Returns 0, or 1 when the matrix does not coarsen.
+int mg_symbolic_build(int n, const int32_t *rp, const int32_t *ci, int dim, int ncells, int ld, const int32_t *celldofs,
+                      const double *coords, const int32_t *cells, MgSymbolic *S);

@@ -12,6 +12,7 @@
 
 #include "element.cuh"
 #include "grmp_internal.h"
+#include "mg.h"
 
 namespace {
 
@@ -616,6 +617,7 @@ extern "C" int grmp_matrix_destroy(grmp_matrix A) {
     grmp_free(ctx, A->d_cellfac, A->cellfac_bytes);
     grmp_direct_cache_free(A);
     grmp_mf_cache_free(A);
+    grmp_mg_free(A);
     grmp_import_free(A);
     cudaStreamSynchronize(ctx->stream);
     if (A->imported) {   // the placeholder mesh / space of a CSC import belong to the matrix

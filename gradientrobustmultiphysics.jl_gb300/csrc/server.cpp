@@ -129,6 +129,7 @@ size_t estimate_bytes(const Request &r) {
 
 // Mesh, DoF map, pattern, vectors and Dirichlet DoFs of a request.
 int build_resident(grmp_context ctx, Request &r, Resident &res) {
+    const size_t before = ctx->in_use;
     int rc = grmp_mesh_upload(ctx, r.dim, r.nverts, r.coords.data(), r.ncells, r.cells.data(), &res.mesh);
     if (!rc) {
         if (r.device_dofmap) {
@@ -165,6 +166,17 @@ int build_resident(grmp_context ctx, Request &r, Resident &res) {
         // other requests sharing the GPU while they run)
         if (!rc)
             for (int &t : res.A->asm_tpb) t = -1;
+        // A one-off request does not pay the analysis that the multilevel solver
+        // makes once per pattern; a resident pattern's hierarchy takes what the
+        // request's estimate leaves of the budget after the matrix values, the
+        // cell factors, the vectors and a linear form's cell vectors.
+        if (!rc) {
+            if (r.key == 0) res.A->mg_state = -1;
+            const size_t ld = (size_t)grmp_fe_ldofs(r.fe, r.dim, r.ncomp);
+            const size_t used = (ctx->in_use - before) + (size_t)res.A->nnz * 12 + (size_t)r.ncells * (ld * 8 + 16 * 12) +
+                                (size_t)res.ndofs * 60;
+            res.A->mg_budget = r.bytes > used ? r.bytes - used : 0;
+        }
     }
     if (!rc) rc = grmp_vector_create(ctx, res.ndofs, &res.b);
     if (!rc) rc = grmp_vector_create(ctx, res.ndofs, &res.x);
