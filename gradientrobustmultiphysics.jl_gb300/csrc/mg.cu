@@ -43,13 +43,29 @@ namespace {
 constexpr int kTB = 256;
 constexpr int kCl = 8;            // lanes per row of k_mg_rows
 constexpr int kMgT = 384;         // threads per block of the solvers: two blocks fit an SM at 85 registers a thread
-constexpr int kLongRow = 48;      // mean entries from which a warp takes a row (transposes of wide aggregates)
+// lanes per row of the coarse operators by mean entries a row: 4 up to
+// kShortRow (vertex level on right angles: 7), 8, and a warp from kLongRow
+// (transposes of wide aggregates: 100-600)
+constexpr int kShortRow = 10, kLongRow = 48;
 constexpr double kSmooth = 1.7;   // w of the smoothing steps and c of the fine level (l1-scaled: spectrum in (0, 1])
 constexpr double kProlong = 1.32; // w of the prolongation smoothing
 // reaction-dominated matrices (energy of the constant function against the
 // diagonal) converge in a few dozen Jacobi iterations: they keep that solver
 constexpr double kMaxReaction = 0.02;
-constexpr int kMinRows = 400;
+
+// Rows from which the multilevel solver is taken.  An iteration costs three to
+// four Jacobi iterations on small systems (the cycle's phases) and the values
+// about 0.4 ms, so it pays once Jacobi-PCG needs some 150 iterations, about 6
+// per DoF along an axis.  Whole passes, multilevel / Jacobi, lognormal
+// coefficient, ms: 2D 441 rows 0.80 / 0.94, 1,089 rows 0.93 / 1.69; 3D P1
+// mixed 15,625 rows 1.78 / 1.52, FP64 4,913 rows 1.82 / 1.73, 15,625 rows 2.25 /
+// 2.54; 3D P2 mixed 1,331 rows 1.33 / 1.15, 4,913 rows 1.83 / 1.99, FP64 2.64 /
+// 2.54.
+int min_rows(int dim, int fe, bool mixed) {
+    if (dim == 2) return 600;
+    if (fe == GRMP_FE_H1P2) return mixed ? 4500 : 6000;
+    return mixed ? 30000 : 12000;
+}
 
 template <typename T>
 struct alignas(2 * sizeof(T)) Pair {
@@ -65,13 +81,13 @@ struct MgLv {
     const T *qv;
     const int32_t *trp, *tci;     // Q^T
     const T *tv;
-    int along, qlong, tlong;      // a warp per row of A, Q, Q^T
+    int lanes, tlanes;            // lanes per row of A and Q (one choice: the same lane owns a row in both), of Q^T
     T *r, *y, *e;
 };
 
 template <typename T>
 struct MgDev {
-    int nl, dense, rlong;         // levels, dense inverse at the bottom, a warp per row of P_0^T
+    int nl, dense, rlanes;        // levels, dense inverse at the bottom, lanes per row of P_0^T
     const int32_t *prp, *pci;     // P_0 and its transpose
     const T *pv;
     const int2 *ell;              // P_0 of a P2 space as two entries a row (nullptr: CSR)
@@ -162,49 +178,114 @@ __global__ void k_mg_prol_agg(int n, const int32_t *rp, const int32_t *ci, const
     }
 }
 
-// A P, a group of L lanes per row, a lane per entry of the row of A P (L >= the
-// longest of them where 32 allows it): the lanes load the row's entries and
-// the rows of P they meet, and pass them round by shuffles (A is read
-// coalesced, nothing is searched, the order is fixed).  Bound by the
-// shuffles: 64^3 P2 (55.6M entries times two) 1.4 ms with a warp per row,
-// half of it with two rows per warp.
-template <typename T, int L>
+// position of column c in a row's ascending columns, -1 if it is not there
+__device__ __forceinline__ int mg_find(const int32_t *cols, int n, int c) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (cols[mid] < c) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo < n && cols[lo] == c ? lo : -1;
+}
+
+// Sparse products, a group of lanes per row of the result.  The factor rows
+// that make up a result row are taken one after another, the lanes take the
+// entries of one of them (distinct columns: no two lanes add to one place, so
+// the order is fixed) and add into the row's accumulators in shared memory;
+// rows longer than kRowCap accumulate in the result itself.  FP64: passing
+// the entries round by shuffles to a lane per result entry issued a 32-lane
+// FP64 addition for each one (2 lanes a clock): 61^3 P1, all levels, 2.9 ms a
+// pass with that, see the caller for this form.
+constexpr int kRowCap = 64;
+
+// A P, 8 lanes a row
+template <typename T>
 __global__ void __launch_bounds__(kTB) k_mg_ap(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
                                                const T *__restrict__ v, const int32_t *__restrict__ prp,
                                                const int32_t *__restrict__ pci, const T *__restrict__ pv,
-                                               const int32_t *__restrict__ arp, const int32_t *__restrict__ aci, T *av) {
+                                               const int32_t *__restrict__ arp, const int32_t *aci, T *av) {
+    constexpr int L = 8;
+    __shared__ T sacc[kTB / L][kRowCap];
+    __shared__ int32_t scol[kTB / L][kRowCap];
+    const int lane = threadIdx.x & (L - 1), g = threadIdx.x / L;
+    const int ng = gridDim.x * (kTB / L), pad = (n + 3) & ~3;   // whole warps go round together
+    for (int i = blockIdx.x * (kTB / L) + g; i < pad; i += ng) {
+        const int kb = i < n ? rp[i] : 0, m = i < n ? rp[i + 1] - kb : 0;
+        const int t0 = i < n ? arp[i] : 0, nt = i < n ? arp[i + 1] - t0 : 0;
+        const bool small = nt <= kRowCap;
+        T *acc = small ? sacc[g] : av + t0;
+        const int32_t *cols = small ? scol[g] : aci + t0;
+        for (int t = lane; t < nt; t += L) {
+            acc[t] = T(0);
+            if (small) scol[g][t] = aci[t0 + t];
+        }
+        __syncwarp();
+        const int longest = __reduce_max_sync(0xffffffffu, m);
+        for (int k0 = 0; k0 < longest; k0 += L) {
+            int p0 = 0, len = 0;
+            T a = 0;
+            if (k0 + lane < m) {
+                const int j = ci[kb + k0 + lane];
+                a = v[kb + k0 + lane];
+                p0 = prp[j];
+                len = prp[j + 1] - p0;
+            }
+            const int steps = min(L, longest - k0);
+            for (int k = 0; k < steps; k++) {
+                const int b = __shfl_sync(0xffffffffu, p0, k, L), ln = __shfl_sync(0xffffffffu, len, k, L);
+                const T ak = __shfl_sync(0xffffffffu, a, k, L);
+                for (int q = lane; q < ln; q += L) {
+                    const int s = mg_find(cols, nt, pci[b + q]);
+                    if (s >= 0) acc[s] += ak * pv[b + q];
+                }
+                __syncwarp();
+            }
+        }
+        if (small)
+            for (int t = lane; t < nt; t += L) av[t0 + t] = acc[t];
+        __syncwarp();
+    }
+}
+
+// The same for the vertex interpolation (two entries a row of P), 16 lanes a
+// row and a lane per result entry: the row's entries and their pairs are
+// passed round by shuffles.  64^3 P2 (55.6M entries), FP32: 1.95 ms a pass
+// with the form above, 0.85 ms with this one, bound by the shuffles.
+template <typename T>
+__global__ void __launch_bounds__(kTB) k_mg_ap_geo(int n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                                                   const T *__restrict__ v, const int2 *__restrict__ ell,
+                                                   const Pair<T> *__restrict__ ellv, const int32_t *__restrict__ arp,
+                                                   const int32_t *__restrict__ aci, T *av) {
+    constexpr int L = 16;
     const int lane = threadIdx.x & (L - 1);
-    const int ng = gridDim.x * blockDim.x / L;
-    const int pad = (n + 32 / L - 1) / (32 / L) * (32 / L);   // whole warps take part in the shuffles
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) / L; i < pad; i += ng) {
+    const int ng = gridDim.x * (kTB / L), pad = (n + 1) & ~1;
+    for (int i = blockIdx.x * (kTB / L) + threadIdx.x / L; i < pad; i += ng) {
         const int kb = i < n ? rp[i] : 0, ke = i < n ? rp[i + 1] : 0;
         const int t0 = i < n ? arp[i] : 0, te = i < n ? arp[i + 1] : 0;
         const int chunks = __reduce_max_sync(0xffffffffu, (te - t0 + L - 1) / L);
-        const int steps = __reduce_max_sync(0xffffffffu, (ke - kb + L - 1) / L);
+        const int longest = __reduce_max_sync(0xffffffffu, ke - kb);
         for (int tc = 0; tc < chunks; tc++) {
             const int tb = t0 + tc * L + lane;
             const int mine = tb < te ? aci[tb] : -1;
             T acc = 0;
-            for (int kc = 0; kc < steps; kc++) {
-                const int k0 = kb + kc * L + lane;
-                int p0 = 0, len = 0;
-                T a = 0;
-                if (k0 < ke) {
-                    const int j = ci[k0];
-                    a = v[k0];
-                    p0 = prp[j];
-                    len = prp[j + 1] - p0;
+            for (int k0 = 0; k0 < longest; k0 += L) {
+                int2 c = make_int2(-2, -2);
+                T wa = 0, wb = 0;
+                if (kb + k0 + lane < ke) {
+                    const int j = ci[kb + k0 + lane];
+                    const T a = v[kb + k0 + lane];
+                    c = ell[j];
+                    const Pair<T> w = ellv[j];
+                    wa = a * w.a;
+                    wb = a * w.b;
                 }
-                const int m = __reduce_max_sync(0xffffffffu, min(L, max(0, ke - kb - kc * L)));
-                const int longest = __reduce_max_sync(0xffffffffu, len);
-                for (int q = 0; q < longest; q++) {
-                    const int c = q < len ? pci[p0 + q] : -2;
-                    const T w = q < len ? a * pv[p0 + q] : T(0);
-                    for (int k = 0; k < m; k++) {
-                        const int cc = __shfl_sync(0xffffffffu, c, k, L);
-                        const T ww = __shfl_sync(0xffffffffu, w, k, L);
-                        if (cc == mine) acc += ww;
-                    }
+                const int m = min(L, longest - k0);
+                for (int k = 0; k < m; k++) {
+                    const int ca = __shfl_sync(0xffffffffu, c.x, k, L), cb = __shfl_sync(0xffffffffu, c.y, k, L);
+                    const T xa = __shfl_sync(0xffffffffu, wa, k, L), xb = __shfl_sync(0xffffffffu, wb, k, L);
+                    if (ca == mine) acc += xa;
+                    if (cb == mine) acc += xb;
                 }
             }
             if (tb < te) av[tb] = acc;
@@ -212,72 +293,63 @@ __global__ void __launch_bounds__(kTB) k_mg_ap(int n, const int32_t *__restrict_
     }
 }
 
-// next level's matrix P^T (A P), L lanes per row, a lane per entry; a row
-// without values (only fixed DoFs below it) becomes the identity's.  LUMP:
-// the pattern leaves out couplings, whose values are added to the diagonal.
-template <typename T, int L, bool LUMP>
+// next level's matrix P^T (A P), 16 lanes a row; a row without values (only
+// fixed DoFs below it) becomes the identity's.  Couplings that the pattern
+// leaves out (filtered vertex level) are added to the diagonal.
+template <typename T>
 __global__ void __launch_bounds__(kTB) k_mg_rap(int nc, const int32_t *__restrict__ rrp, const int32_t *__restrict__ rci,
                                                 const int32_t *__restrict__ rperm, const T *__restrict__ pv,
                                                 const int32_t *__restrict__ arp, const int32_t *__restrict__ aci,
                                                 const T *__restrict__ av, const int32_t *__restrict__ crp,
-                                                const int32_t *__restrict__ cci, T *cv) {
-    const int lane = threadIdx.x & (L - 1);
-    const int ng = gridDim.x * blockDim.x / L;
-    const int pad = (nc + 32 / L - 1) / (32 / L) * (32 / L);
-    for (int I = (blockIdx.x * blockDim.x + threadIdx.x) / L; I < pad; I += ng) {
-        const int t0 = I < nc ? crp[I] : 0, te = I < nc ? crp[I + 1] : 0;
-        const int kb = I < nc ? rrp[I] : 0, ke = I < nc ? rrp[I + 1] : 0;
-        const int chunks = __reduce_max_sync(0xffffffffu, (te - t0 + L - 1) / L);
-        const int steps = __reduce_max_sync(0xffffffffu, (ke - kb + L - 1) / L);
-        bool any = false;
-        T total = 0, kept = 0;
-        for (int tc = 0; tc < chunks; tc++) {
-            const int tb = t0 + tc * L + lane;
-            const int mine = tb < te ? cci[tb] : -1;
-            T acc = 0;
-            for (int kc = 0; kc < steps; kc++) {
-                const int k0 = kb + kc * L + lane;
-                int a0 = 0, a1 = 0;
-                T w = 0;
-                if (k0 < ke) {
-                    const int i = rci[k0];
-                    w = pv[rperm[k0]];
-                    a0 = arp[i];
-                    a1 = w == T(0) ? a0 : arp[i + 1];
-                }
-                const int m = __reduce_max_sync(0xffffffffu, min(L, max(0, ke - kb - kc * L)));
-                for (int k = 0; k < m; k++) {
-                    const int b = __shfl_sync(0xffffffffu, a0, k, L), e = __shfl_sync(0xffffffffu, a1, k, L);
-                    const T wk = __shfl_sync(0xffffffffu, w, k, L);
-                    const int longest = __reduce_max_sync(0xffffffffu, e - b);
-                    for (int q0 = 0; q0 < longest; q0 += L) {
-                        const int at = b + q0 + lane;
-                        const int c = at < e ? aci[at] : -2;
-                        const T x = at < e ? wk * av[at] : T(0);
-                        const int len = min(L, longest - q0);
-                        for (int q = 0; q < len; q++) {
-                            const int cc = __shfl_sync(0xffffffffu, c, q, L);
-                            const T xx = __shfl_sync(0xffffffffu, x, q, L);
-                            if (cc == mine) acc += xx;
-                            if (LUMP && tc == 0) total += xx;
-                        }
-                    }
-                }
+                                                const int32_t *cci, T *cv) {
+    constexpr int L = 16;
+    __shared__ T sacc[kTB / L][kRowCap];
+    __shared__ int32_t scol[kTB / L][kRowCap];
+    const int lane = threadIdx.x & (L - 1), g = threadIdx.x / L;
+    const int ng = gridDim.x * (kTB / L), pad = (nc + 1) & ~1;
+    for (int I = blockIdx.x * (kTB / L) + g; I < pad; I += ng) {
+        const int t0 = I < nc ? crp[I] : 0, nt = I < nc ? crp[I + 1] - t0 : 0;
+        const int kb = I < nc ? rrp[I] : 0, m = I < nc ? rrp[I + 1] - kb : 0;
+        const bool small = nt <= kRowCap;
+        T *acc = small ? sacc[g] : cv + t0;
+        const int32_t *cols = small ? scol[g] : cci + t0;
+        for (int t = lane; t < nt; t += L) {
+            acc[t] = T(0);
+            if (small) scol[g][t] = cci[t0 + t];
+        }
+        __syncwarp();
+        T lump = 0;
+        const int longest = __reduce_max_sync(0xffffffffu, m);
+        for (int k0 = 0; k0 < longest; k0 += L) {
+            int a0 = 0, len = 0;
+            T w = 0;
+            if (k0 + lane < m) {
+                const int i = rci[kb + k0 + lane];
+                w = pv[rperm[kb + k0 + lane]];
+                a0 = arp[i];
+                len = w == T(0) ? 0 : arp[i + 1] - a0;
             }
-            any = any || acc != T(0);
-            kept += acc;
-            if (tb < te) cv[tb] = acc;
+            const int steps = min(L, longest - k0);
+            for (int k = 0; k < steps; k++) {
+                const int b = __shfl_sync(0xffffffffu, a0, k, L), ln = __shfl_sync(0xffffffffu, len, k, L);
+                const T wk = __shfl_sync(0xffffffffu, w, k, L);
+                for (int q = lane; q < ln; q += L) {
+                    const int s = mg_find(cols, nt, aci[b + q]);
+                    const T x = wk * av[b + q];
+                    if (s >= 0) acc[s] += x;
+                    else lump += x;
+                }
+                __syncwarp();
+            }
         }
-        for (int o = L / 2; o > 0; o >>= 1) any = __shfl_xor_sync(0xffffffffu, (int)any, o) || any;
-        if (LUMP) {   // lanes of a row hold the same total
-            for (int o = L / 2; o > 0; o >>= 1) kept += __shfl_xor_sync(0xffffffffu, kept, o);
-            if (any)
-                for (int t = t0 + lane; t < te; t += L)
-                    if (cci[t] == I) cv[t] += total - kept;
+        bool any = false;
+        for (int t = lane; t < nt; t += L) any = any || acc[t] != T(0);
+        for (int o = L / 2; o > 0; o >>= 1) {
+            any = __shfl_xor_sync(0xffffffffu, (int)any, o) || any;
+            lump += __shfl_xor_sync(0xffffffffu, lump, o);
         }
-        if (!any)
-            for (int t = t0 + lane; t < te; t += L)
-                if (cci[t] == I) cv[t] = T(1);
+        for (int t = lane; t < nt; t += L) cv[t0 + t] = acc[t] + (cols[t] == I ? (any ? lump : T(1)) : T(0));
+        __syncwarp();
     }
 }
 
@@ -347,6 +419,7 @@ __global__ void __launch_bounds__(512) k_mg_binv(int n, const int32_t *rp, const
 // One block: a system whose iteration fits one SM's L1 needs no grid barrier
 // at all (about 3 us a phase), only __syncthreads.
 struct BlockSync {
+    static constexpr int kThreads = 1024, kBlocks = 1;
     __device__ __forceinline__ BlockSync(SolveState *, double *, long long) {}
     __device__ __forceinline__ bool barrier() {
         __syncthreads();
@@ -364,41 +437,40 @@ struct BlockSync {
     }
 };
 struct MgGridSync : GridSync {
+    static constexpr int kThreads = kMgT, kBlocks = 2;
     __device__ __forceinline__ MgGridSync(SolveState *st, double *part, long long spin) : GridSync{st, part, spin, 0} {}
 };
 
-// rows of a coarse operator over the grid: 8 lanes a row, or a warp where rows are long
+// rows of a coarse operator over the grid
 template <typename T, typename G, typename E>
-__device__ __forceinline__ void mg_rows(int n, const int32_t *rp, const int32_t *ci, const T *v, int longrows, G gather,
+__device__ __forceinline__ void mg_rows(int n, const int32_t *rp, const int32_t *ci, const T *v, int lanes, G gather,
                                         E epi) {
-    if (longrows) spmv_rows<32, 4, false, T>(n, rp, CsrSource<T>{ci, v}, gather, epi);
-    else spmv_rows<8, 2, true, T>(n, rp, CsrSource<T>{ci, v}, gather, epi);
+    const CsrSource<T> src{ci, v};
+    if (lanes == 4) spmv_rows<4, 2, true, T>(n, rp, src, gather, epi);
+    else if (lanes == 8) spmv_rows<8, 2, true, T>(n, rp, src, gather, epi);
+    else spmv_rows<32, 4, false, T>(n, rp, src, gather, epi);
 }
 
 // r, y of a level from the one above it
 template <typename T>
-__device__ __forceinline__ void mg_down(const int32_t *rp, const int32_t *ci, const T *v, int longrows, const T *src,
+__device__ __forceinline__ void mg_down(const int32_t *rp, const int32_t *ci, const T *v, int lanes, const T *src,
                                         const MgLv<T> &to) {
     mg_rows(
-        to.n, rp, ci, v, longrows, [&](int c) { return src[c]; },
+        to.n, rp, ci, v, lanes, [&](int c) { return src[c]; },
         [&](int i, T s) {
             to.r[i] = s;
             to.y[i] = (T)kSmooth * to.D[i] * s;
         });
 }
 
-// e of a level: 2 y - w D A y, then + Q e of the next (both products with
-// 8 lanes a row, so the same lane writes and adds; a barrier between them
-// where a warp takes the rows of only one)
-template <typename T, class SY>
-__device__ __forceinline__ bool mg_up(const MgLv<T> &l, const T *enext, SY &sy) {
+// e of a level: 2 y - w D A y, then + Q e of the next
+template <typename T>
+__device__ __forceinline__ void mg_up(const MgLv<T> &l, const T *enext) {
     mg_rows(
-        l.n, l.rp, l.ci, l.v, l.along, [&](int c) { return ((const T *)l.y)[c]; },
+        l.n, l.rp, l.ci, l.v, l.lanes, [&](int c) { return ((const T *)l.y)[c]; },
         [&](int i, T s) { l.e[i] = T(2) * l.y[i] - (T)kSmooth * l.D[i] * s; });
-    if (l.along != l.qlong && !sy.barrier()) return false;
     mg_rows(
-        l.n, l.qrp, l.qci, l.qv, l.qlong, [&](int c) { return enext[c]; }, [&](int i, T s) { l.e[i] += s; });
-    return true;
+        l.n, l.qrp, l.qci, l.qv, l.lanes, [&](int c) { return enext[c]; }, [&](int i, T s) { l.e[i] += s; });
 }
 
 // e of level 1 from r: restriction, the levels below, back up.  The caller
@@ -408,11 +480,11 @@ __device__ __forceinline__ bool mg_up(const MgLv<T> &l, const T *enext, SY &sy) 
 // barrier).
 template <typename T, class SY>
 __device__ __forceinline__ bool mg_cycle(const MgDev<T> &m, const T *r, T *eb, SY &sy) {
-    mg_down(m.rrp, m.rci, m.rv, m.rlong, r, m.lv[1]);
+    mg_down(m.rrp, m.rci, m.rv, m.rlanes, r, m.lv[1]);
     if (!sy.barrier()) return false;
     const int bottom = m.nl - 1;
     for (int l = 1; l < bottom; l++) {
-        mg_down(m.lv[l].trp, m.lv[l].tci, m.lv[l].tv, m.lv[l].tlong, (const T *)m.lv[l].r, m.lv[l + 1]);
+        mg_down(m.lv[l].trp, m.lv[l].tci, m.lv[l].tv, m.lv[l].tlanes, (const T *)m.lv[l].r, m.lv[l + 1]);
         if (!sy.barrier()) return false;
     }
     const MgLv<T> &b = m.lv[bottom];
@@ -440,7 +512,7 @@ __device__ __forceinline__ bool mg_cycle(const MgDev<T> &m, const T *r, T *eb, S
         return sy.barrier();
     }
     for (int l = bottom - 1; l >= 1; l--) {
-        if (!mg_up(m.lv[l], enext, sy)) return false;
+        mg_up(m.lv[l], enext);
         enext = m.lv[l].e;
         if (!sy.barrier()) return false;
     }
@@ -464,7 +536,7 @@ __device__ __forceinline__ T mg_fine(const MgDev<T> &m, int i, T ri) {
 
 // ------------------------------------------------------------------ FP64 solver
 template <int TPR, int U, bool PIPE, class SY>
-__global__ void __launch_bounds__(kMgT, std::is_same<SY, BlockSync>::value ? 1 : 2)
+__global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     k_mgcg64(int n, const int32_t *rowptr, const int32_t *cols, const double *vals, const double *b, double *x, double *r,
              double *z, double *p, double *q, double *partial, SolveState *st, double abstol, double reltol, int maxit,
              int guess, long long spin, const __grid_constant__ MgDev<double> m) {
@@ -543,7 +615,7 @@ __global__ void __launch_bounds__(kMgT, std::is_same<SY, BlockSync>::value ? 1 :
 // into x when the FP32 residual has fallen by `delta`, the FP64 residual
 // replaces it, the direction is kept unless the true residual stopped falling.
 template <int TPR, int U, bool PIPE, class SY>
-__global__ void __launch_bounds__(kMgT, std::is_same<SY, BlockSync>::value ? 1 : 2)
+__global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     k_mgcg_mixed(int n, const int32_t *rowptr, const int32_t *cols, const double *vals64, const float *vals32,
                  const double *b, double *x, float *r, float *q, float *xc, float2 *zp0, float2 *zp1, double *r64,
                  double *partial, SolveState *st, double abstol, double reltol, double delta, int maxit, int maxouter,
@@ -700,7 +772,6 @@ struct MgCache {
         int2 *ell = nullptr;
         int32_t *prp, *pci, *rrp, *rci, *rperm, *arp, *aci, *trp = nullptr, *tci = nullptr, *tperm = nullptr, *crp, *cci;
         size_t np, na, nt, nc;   // entries of P, A P, Q^T, next A
-        int amax, cmax;          // longest row of A P, next A
     };
     std::vector<Step> step;
     // numeric storage per precision (0: FP64, 1: FP32), one allocation each
@@ -770,9 +841,6 @@ int mg_build(grmp_matrix A) {
         d.na = t.AP.ci.size();
         d.nt = t.QT.ci.size();
         d.nc = t.Ac.ci.size();
-        d.amax = d.cmax = 0;
-        for (int i = 0; i < t.n; i++) d.amax = std::max(d.amax, t.AP.rp[i + 1] - t.AP.rp[i]);
-        for (int i = 0; i < t.nc; i++) d.cmax = std::max(d.cmax, t.Ac.rp[i + 1] - t.Ac.rp[i]);
         auto up = [&](std::vector<int32_t> &v, int32_t **p) {
             if (!rc) rc = mg_up_vec(ctx, *C, v, p);
         };
@@ -931,16 +999,14 @@ void mg_values(grmp_matrix A) {
         else
             k_mg_prol_agg<T><<<nblk(n, 128), 128, 0, st>>>(n, rp, ci, v, D, (const uint8_t *)N.iso[k], d.agg, d.prp, d.pci,
                                                            pv);
-        // lanes per row: the smallest power of two that holds the longest row of the product
-        const int la = d.amax <= 8 ? 8 : (d.amax <= 16 ? 16 : 32), lc = d.cmax <= 8 ? 8 : (d.cmax <= 16 ? 16 : 32);
-        auto ap = la == 8 ? k_mg_ap<T, 8> : (la == 16 ? k_mg_ap<T, 16> : k_mg_ap<T, 32>);
-        auto rap = lc == 8 ? k_mg_rap<T, 8, false> : (lc == 16 ? k_mg_rap<T, 16, false> : k_mg_rap<T, 32, false>);
-        if (C.S.step[k].filtered)
-            rap = lc == 8 ? k_mg_rap<T, 8, true> : (lc == 16 ? k_mg_rap<T, 16, true> : k_mg_rap<T, 32, true>);
-        ap<<<std::max(1, std::min(nblk((long long)n * la), wide)), kTB, 0, st>>>(n, rp, ci, v, d.prp, d.pci, pv, d.arp,
-                                                                                d.aci, av);
-        rap<<<std::max(1, std::min(nblk((long long)nc * lc), wide)), kTB, 0, st>>>(nc, d.rrp, d.rci, d.rperm, pv, d.arp,
-                                                                                  d.aci, av, d.crp, d.cci, cv);
+        if (d.vrow)
+            k_mg_ap_geo<T><<<std::max(1, std::min(nblk((long long)n * 16), wide)), kTB, 0, st>>>(
+                n, rp, ci, v, d.ell, (const Pair<T> *)N.ellv, d.arp, d.aci, av);
+        else
+            k_mg_ap<T><<<std::max(1, std::min(nblk((long long)n * 8), wide)), kTB, 0, st>>>(n, rp, ci, v, d.prp, d.pci,
+                                                                                           pv, d.arp, d.aci, av);
+        k_mg_rap<T><<<std::max(1, std::min(nblk((long long)nc * 16), wide)), kTB, 0, st>>>(
+            nc, d.rrp, d.rci, d.rperm, pv, d.arp, d.aci, av, d.crp, d.cci, cv);
         ctx->launches += 3;
         if (k > 0) {
             k_mg_q<T><<<nblk(n, 128), 128, 0, st>>>(n, d.prp, d.pci, pv, d.arp, d.aci, D, av);
@@ -985,8 +1051,10 @@ MgDev<T> mg_device(grmp_matrix A) {
     m.D0 = (const T *)N.D[0];
     m.binv = (const T *)N.binv;
     m.dense = C.S.step[ns - 1].nc <= kMgBottom;
-    auto lng = [](size_t entries, int rows) { return (int)(entries > (size_t)kLongRow * rows); };
-    m.rlong = lng(C.step[0].np, C.S.step[0].nc);
+    auto lanes = [](size_t entries, int rows) {
+        return entries <= (size_t)kShortRow * rows ? 4 : (entries <= (size_t)kLongRow * rows ? 8 : 32);
+    };
+    m.rlanes = lanes(C.step[0].np, C.S.step[0].nc);
     for (int l = 1; l <= ns; l++) {
         MgLv<T> &L = m.lv[l];
         L.n = C.S.step[l - 1].nc;
@@ -994,10 +1062,9 @@ MgDev<T> mg_device(grmp_matrix A) {
         L.ci = C.step[l - 1].cci;
         L.v = (const T *)N.cv[l - 1];
         L.D = (const T *)N.D[l];
-        L.along = lng(C.step[l - 1].nc, L.n);
         if (l < ns) {
-            L.qlong = lng(C.step[l].na, L.n);
-            L.tlong = lng(C.step[l].nt, C.S.step[l].nc);
+            L.lanes = lanes(std::max(C.step[l - 1].nc, C.step[l].na), L.n);
+            L.tlanes = lanes(C.step[l].nt, C.S.step[l].nc);
             L.qrp = C.step[l].arp;
             L.qci = C.step[l].aci;
             L.qv = (const T *)N.av[l];
@@ -1013,8 +1080,11 @@ MgDev<T> mg_device(grmp_matrix A) {
 }
 
 // Systems of at most this many rows run in one block (its L1 holds matrix and
-// vectors; on the FP64 pipe of one SM, two FMAs a clock, only smaller ones gain)
-constexpr int kOneBlock32 = 6000, kOneBlock64 = 1200;
+// vectors; on the FP64 pipe of one SM, two FMAs a clock, only smaller ones
+// gain).  2D lognormal, solve in one block / on the grid: mixed 1,089 rows
+// 0.56 / 0.86 ms, 3,249 1.15 / 1.19, 5,041 1.85 / 1.55; FP64 625 0.93 / 1.07,
+// 1,089 1.38 / 1.28.
+constexpr int kOneBlock32 = 3300, kOneBlock64 = 700;
 
 // grid: enough blocks for the rows, at most what fits; small systems take
 // one block per SM, which makes the barriers cheaper
@@ -1033,7 +1103,7 @@ template <typename K>
 cudaError_t mg_start(grmp_context ctx, K kern, bool one, int n, int tpr, int want, void **args, int *grid) {
     *grid = one ? 1 : mg_grid(ctx, kern, n, tpr, want);
     GRMP_LAUNCHED(ctx);
-    if (one) return cudaLaunchKernel((const void *)kern, dim3(1), dim3(kMgT), args, 0, ctx->stream);
+    if (one) return cudaLaunchKernel((const void *)kern, dim3(1), dim3(BlockSync::kThreads), args, 0, ctx->stream);
     return cudaLaunchCooperativeKernel((const void *)kern, dim3(*grid), dim3(kMgT), args, 0, ctx->stream);
 }
 
@@ -1098,8 +1168,8 @@ int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use) {
     *use = 0;
     grmp_space s = A->space;
     grmp_context ctx = s->mesh->ctx;
-    if (A->mg_state < 0 || A->imported || !A->elliptic || A->nrows < kMinRows || s->ncomp != 1 ||
-        (s->fe != GRMP_FE_H1P1 && s->fe != GRMP_FE_H1P2))
+    if (A->mg_state < 0 || A->imported || !A->elliptic || s->ncomp != 1 ||
+        (s->fe != GRMP_FE_H1P1 && s->fe != GRMP_FE_H1P2) || A->nrows < min_rows(s->mesh->dim, s->fe, mixed))
         return GRMP_OK;
     int rc = GRMP_OK;
     if (!A->mg) rc = mg_build(A);
