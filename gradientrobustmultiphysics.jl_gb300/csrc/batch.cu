@@ -24,6 +24,7 @@
 
 #include "grmp_internal.h"
 #include "mf_device.cuh"
+#include "forest.h"
 #include "nd_symbolic.h"
 
 int grmp_br_divergence(grmp_space s, double **Dv, double **vol);
@@ -987,14 +988,13 @@ __device__ void mf_prec32(const BatchDev &d, const DirectDev &m, int pid, int r0
     __syncthreads();
 }
 
-// MIXED = false: FP64 factorisation, each sweep refined against the FP64
-// matrix.  MIXED = true: FP32 factorisation (GB300's FP32 rate is ~64x its
+// MIXED_DIRECT: FP32 factorisation (GB300's FP32 rate is ~64x its
 // FP64 rate), each sweep solved by FP64 conjugate gradients on the FP64
 // matrix preconditioned by the FP32 factor, warm-started from the previous
 // sweep's velocity; a problem whose FP32 factorisation meets a non-positive
 // pivot, or whose preconditioned CG stalls above the tolerance, is factored
 // again in FP64 and finishes in the FP64 mode (counted in fallbacks).
-template <int TPR, bool MIXED>
+template <int TPR>
 __global__ void __launch_bounds__(512, 1) k_stokes_direct(BatchDev d, DirectDev m) {
     extern __shared__ double dsm[];
     __shared__ double sh[32 * 4];
@@ -1020,17 +1020,14 @@ __global__ void __launch_bounds__(512, 1) k_stokes_direct(BatchDev d, DirectDev 
         for (int i = r0 + tid; i < r1; i += bs) d.u[i] = 0.0;
         for (int c = c0 + tid; c < c1; c += bs) d.p[c] = 0.0;
         __syncthreads();
-        bool use32 = MIXED;
+        bool use32 = true;
         int nfall = 0;
-        bool fact_ok = false;
-        if (MIXED) {
-            fact_ok = mf_factor_lv<float>(d, m, m.prob_lvl0[pid], m.prob_nlev[pid], (long long)d.rowptr[r0], (float *)F,
-                                          (float *)U, (float *)L, (float *)colk, (float *)P, (float *)Fg, &fail_flag);
-            __syncthreads();
-            if (!fact_ok) {
-                use32 = false;
-                nfall = 1;
-            }
+        bool fact_ok = mf_factor_lv<float>(d, m, m.prob_lvl0[pid], m.prob_nlev[pid], (long long)d.rowptr[r0], (float *)F,
+                                           (float *)U, (float *)L, (float *)colk, (float *)P, (float *)Fg, &fail_flag);
+        __syncthreads();
+        if (!fact_ok) {
+            use32 = false;
+            nfall = 1;
         }
         if (!use32)
             fact_ok = mf_factor_lv<double>(d, m, m.prob_lvl0[pid], m.prob_nlev[pid], (long long)d.rowptr[r0], F, U, L,
@@ -1058,7 +1055,7 @@ __global__ void __launch_bounds__(512, 1) k_stokes_direct(BatchDev d, DirectDev 
                 double rel = 0.0, prev = INFINITY, eta = 0.0;
                 bool floor = false;
                 bool done32 = false;
-                if (MIXED && use32) {
+                if (use32) {
                     // FP64 CG preconditioned by the FP32 factor (x = u, r = rhs - A u)
                     double *z = d.w64a, *pp = d.w64b, *q = d.w64c, *r = d.r64;
                     double v[1] = {block_spmv<TPR, double, double, true>(d, r0, r1, d.v64, d.u, r, nullptr, d.rhs)};
@@ -1180,6 +1177,168 @@ __global__ void __launch_bounds__(512, 1) k_stokes_direct(BatchDev d, DirectDev 
     }
 }
 
+// ------------------------------------------------------------------------
+// DIRECT mode: every problem's FP64 factorisation and solves through the
+// forest (forest.cu), all problems of the batch sweeping together.  Rows are
+// handled in chunks of kChunk rows of one problem (a block each), a problem's
+// norms are the sums of its chunks in order, so its bits do not depend on the
+// batch.  Problems that have met the tolerance (or the FP64 floor) are skipped
+// by every kernel until the next sweep.
+constexpr int kChunk = 2048;
+
+struct SweepDev {
+    const int4 *chunk;      // {problem, first row, last row + 1, -}
+    const int2 *pchunk;     // first chunk and end of each problem
+    const int *pid;         // problem in the batch
+    const int *err;         // factorisation failures
+    double *part;           // [chunk][3]
+    double *anorm, *bn, *prev, *rel, *worst;
+    int *act, *fin, *ok, *nsolve, *sweeps, *count;
+    int max_solves;
+};
+
+__global__ void k_sb_init(int np, SweepDev s) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= np) return;
+    const bool good = s.err[p] == 0;
+    s.fin[p] = !good;
+    s.ok[p] = good;
+    s.act[p] = 0;
+    s.nsolve[p] = s.sweeps[p] = 0;
+    s.worst[p] = good ? 0.0 : INFINITY;
+}
+
+// per chunk: largest row sum of |A|
+__global__ void __launch_bounds__(256) k_sb_anorm(BatchDev d, SweepDev s) {
+    __shared__ double sh[32 * 4];
+    const int4 c = s.chunk[blockIdx.x];
+    double an[1] = {0.0};
+    for (int i = c.y + threadIdx.x; i < c.z; i += blockDim.x) {
+        double rs = 0.0;
+        for (int k = d.rowptr[i]; k < d.rowptr[i + 1]; k++) rs += fabs(d.v64[k]);
+        an[0] = fmax(an[0], rs);
+    }
+    bmax1(an, sh);
+    if (threadIdx.x == 0) s.part[3 * blockIdx.x] = an[0];
+}
+__global__ void k_sb_anorm2(int np, SweepDev s) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= np) return;
+    double a = 0.0;
+    for (int c = s.pchunk[p].x; c < s.pchunk[p].y; c++) a = fmax(a, s.part[3 * c]);
+    s.anorm[p] = a;
+}
+
+// right-hand side of a sweep and the chunk's share of its norm
+__global__ void __launch_bounds__(256) k_sb_rhs(BatchDev d, SweepDev s) {
+    __shared__ double sh[32 * 4];
+    const int4 c = s.chunk[blockIdx.x];
+    if (s.fin[c.x]) return;
+    double v[1] = {0.0};
+    for (int i = c.y + threadIdx.x; i < c.z; i += blockDim.x) {
+        double acc = d.bf[i];
+        if (!d.fixed[i])
+            for (int q = d.inc_ptr[i]; q < d.inc_ptr[i + 1]; q++) {
+                const int cell = d.inc_cell[q];
+                acc += d.Dv[(size_t)cell * d.ld + d.inc_loc[q]] * d.p[cell];
+            }
+        d.rhs[i] = acc;
+        v[0] += acc * acc;
+    }
+    bsum<1>(v, sh);
+    if (threadIdx.x == 0) s.part[3 * blockIdx.x + 2] = v[0];
+}
+
+// r = rhs - A u, shares of r.r and u.u (8 lanes per row)
+__global__ void __launch_bounds__(256) k_sb_resid(BatchDev d, SweepDev s, int ref) {
+    __shared__ double sh[32 * 4];
+    const int4 c = s.chunk[blockIdx.x];
+    if (s.fin[c.x] || (ref > 0 && !s.act[c.x])) return;
+    const int lane = threadIdx.x & 7, rows = c.z - c.y, pad = (rows + 31) & ~31;
+    double v[2] = {0.0, 0.0};
+    for (int o = threadIdx.x >> 3; o < pad; o += 32) {
+        const int i = c.y + o;
+        double t = 0.0;
+        if (o < rows)
+            for (int k = d.rowptr[i] + lane; k < d.rowptr[i + 1]; k += 8) t += d.v64[k] * d.u[d.cols[k]];
+        for (int q = 4; q > 0; q >>= 1) t += __shfl_xor_sync(0xffffffffu, t, q);
+        if (o < rows && lane == 0) {
+            const double r = d.rhs[i] - t, u = d.u[i];
+            d.r64[i] = r;
+            v[0] += r * r;
+            v[1] += u * u;
+        }
+    }
+    bsum<2>(v, sh);
+    if (threadIdx.x == 0) {
+        s.part[3 * blockIdx.x] = v[0];
+        s.part[3 * blockIdx.x + 1] = v[1];
+    }
+}
+
+// which problems solve once more: stop at reltol, or when the residual stops
+// falling (the FP64 floor of an ill-conditioned system, accepted by the
+// normwise backward error), or after max_solves
+__global__ void k_sb_decide(int np, SweepDev s, int ref, double reltol) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= np) return;
+    if (s.fin[p] || (ref > 0 && !s.act[p])) {
+        s.act[p] = 0;
+        return;
+    }
+    double rr = 0.0, uu = 0.0, bb = 0.0;
+    for (int c = s.pchunk[p].x; c < s.pchunk[p].y; c++) {
+        rr += s.part[3 * c];
+        uu += s.part[3 * c + 1];
+        if (ref == 0) bb += s.part[3 * c + 2];
+    }
+    if (ref == 0) s.bn[p] = sqrt(bb);
+    const double bn = s.bn[p], rel = bn > 0 ? sqrt(rr) / bn : 0.0;
+    const double eta = sqrt(rr) / (s.anorm[p] * sqrt(uu) + bn + 1e-300);
+    bool stop = rel <= reltol, floor = false;
+    if (!stop && ref > 0 && rel > 0.5 * s.prev[p]) stop = floor = true;
+    if (ref >= s.max_solves) stop = true;
+    s.prev[p] = rel;
+    s.act[p] = !stop;
+    if (stop) {
+        s.worst[p] = fmax(s.worst[p], rel);
+        if (!(rel <= reltol || (floor && eta <= kDirectBackwardMax))) s.ok[p] = 0;
+    } else {
+        s.nsolve[p]++;
+        atomicAdd(s.count, 1);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_sb_add(BatchDev d, SweepDev s) {
+    const int4 c = s.chunk[blockIdx.x];
+    if (!s.act[c.x]) return;
+    for (int i = c.y + threadIdx.x; i < c.z; i += blockDim.x) d.u[i] += d.r64[i];
+}
+
+__global__ void __launch_bounds__(512) k_sb_pressure(BatchDev d, SweepDev s) {
+    __shared__ double sh[32 * 4];
+    const int p = blockIdx.x;
+    if (s.fin[p]) return;
+    const int pid = s.pid[p];
+    const bool met = block_pressure_update(d, d.cell_off[pid], d.cell_off[pid + 1], sh);
+    if (threadIdx.x == 0) {
+        s.sweeps[p]++;
+        if (met) s.fin[p] = 1;
+        else atomicAdd(s.count + 1, 1);
+    }
+}
+
+__global__ void k_sb_result(int np, BatchDev d, SweepDev s) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= np) return;
+    const int pid = s.pid[p];
+    d.iters[pid] = s.nsolve[p];
+    d.sweeps_done[pid] = s.sweeps[p];
+    d.relres[pid] = s.worst[p];
+    d.fallbacks[pid] = 0;
+    d.status[pid] = s.err[p] ? (int)GRMP_ERR_NAN : (s.ok[p] ? 0 : (int)GRMP_ERR_NOT_CONVERGED);
+}
+
 // 64-bit fingerprint of each problem's local pattern (row lengths and
 // row-relative columns), summed over nonzeros so the reduction order does
 // not matter.
@@ -1246,6 +1405,20 @@ __global__ void k_check_blocks(int nprob, const int32_t *row_off, const int32_t 
 
 struct DirectCache {
     std::vector<int32_t> row_offsets;
+    std::vector<NdSymbolic> S;            // one per distinct local pattern
+    std::vector<int> group_of;            // of each problem
+    std::vector<long long> nnz0;          // first value of each problem
+    // DIRECT: the problems in batches that fit the memory together
+    struct Part {
+        MfForest *F = nullptr;
+        int np = 0, nchunk = 0;
+        const int4 *chunk = nullptr;
+        const int2 *pchunk = nullptr;
+        const int *pid = nullptr;
+    };
+    std::vector<Part> parts;
+    size_t parts_allow = 0;
+    bool tables = false;                  // MIXED_DIRECT's arrays are uploaded
     std::vector<std::pair<void *, size_t>> bufs;
     const DNode *node = nullptr;
     const int32_t *front = nullptr, *child = nullptr, *ent_rel = nullptr, *ent_pos = nullptr, *ext = nullptr;
@@ -1359,7 +1532,10 @@ int build_direct_cache(grmp_matrix A, int np, const int32_t *row_off, const int3
         const int r0 = row_off[reps[g]];
         for (auto &c : lci[g]) c -= r0;
     }
-    std::vector<NdSymbolic> S(ng);
+    DirectCache *C = new DirectCache;
+    A->direct = C;
+    C->S.resize(ng);
+    std::vector<NdSymbolic> &S = C->S;
     std::vector<int> src(ng, 0);
     {
         const int nthr = std::max(1, std::min<int>(ng, (int)std::thread::hardware_concurrency()));
@@ -1374,9 +1550,21 @@ int build_direct_cache(grmp_matrix A, int np, const int32_t *row_off, const int3
     }
     for (int g = 0; g < ng; g++)
         if (src[g]) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "direct: symbolic analysis failed (%d)", src[g]);
-    // concatenate
-    DirectCache *C = new DirectCache;
     C->row_offsets.assign(row_off, row_off + np + 1);
+    C->group_of = group_of;
+    for (int k = 0; k < np; k++) C->nnz0.push_back(rowptr[row_off[k]]);
+    return GRMP_OK;
+}
+
+// the concatenated trees of MIXED_DIRECT (one problem per block)
+int build_direct_tables(grmp_matrix A, int np) {
+    grmp_context ctx = A->space->mesh->ctx;
+    DirectCache *C = A->direct;
+    if (C->tables) return GRMP_OK;
+    const std::vector<NdSymbolic> &S = C->S;
+    const std::vector<int> &group_of = C->group_of;
+    const int ng = (int)S.size();
+    int rc = GRMP_OK;
     C->groups = ng;
     std::vector<DNode> node;
     std::vector<int32_t> front, child, ent_rel, ent_pos, ext, gnode0(ng), pn0(np), pnn(np);
@@ -1423,7 +1611,6 @@ int build_direct_cache(grmp_matrix A, int np, const int32_t *row_off, const int3
         pl0[k] = glvl0[group_of[k]];
         pnl[k] = gnlev[group_of[k]];
     }
-    A->direct = C;
     rc = upload_vec(ctx, *C, node, &C->node);
     if (!rc) rc = upload_vec(ctx, *C, front, &C->front);
     if (!rc) rc = upload_vec(ctx, *C, child, &C->child);
@@ -1437,10 +1624,137 @@ int build_direct_cache(grmp_matrix A, int np, const int32_t *row_off, const int3
     if (!rc) rc = upload_vec(ctx, *C, pl0, &C->prob_lvl0);
     if (!rc) rc = upload_vec(ctx, *C, pnl, &C->prob_nlev);
     if (!rc) {
-        e = cudaStreamSynchronize(ctx->stream);
+        cudaError_t e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) rc = grmp_cuda_fail(ctx, e, "direct cache upload");
     }
-    if (rc) grmp_direct_cache_free(A);
+    C->tables = rc == GRMP_OK;
+    return rc;
+}
+
+void free_parts(grmp_context ctx, DirectCache &C) {
+    for (auto &p : C.parts) grmp_forest_free(ctx, p.F);
+    C.parts.clear();
+    C.parts_allow = 0;
+}
+
+// batches of DIRECT: problems in order of size, as many together as `allow` holds
+int build_parts(grmp_matrix A, const std::vector<int32_t> &order, size_t allow) {
+    grmp_context ctx = A->space->mesh->ctx;
+    DirectCache &C = *A->direct;
+    std::vector<const NdSymbolic *> groups;
+    for (auto &q : C.S) groups.push_back(&q);
+    // an earlier split stays while it still fits
+    if (!C.parts.empty() && C.parts_allow <= allow) return GRMP_OK;
+    free_parts(ctx, C);
+    size_t need = 0;
+    for (size_t at = 0; at < order.size();) {
+        std::vector<FoProblem> probs;
+        std::vector<int> pid;
+        size_t bytes = 0;
+        while (at < order.size()) {
+            const int k = order[at];
+            probs.push_back(FoProblem{C.group_of[k], C.row_offsets[k], C.nnz0[k]});
+            const size_t b = grmp_forest_bytes(groups, probs, 8);
+            if (probs.size() > 1 && b > allow) {
+                probs.pop_back();
+                break;
+            }
+            bytes = b;
+            pid.push_back(k);
+            at++;
+        }
+        need = std::max(need, bytes);
+        std::vector<int4> chunk;
+        std::vector<int2> pchunk;
+        for (size_t q = 0; q < pid.size(); q++) {
+            const int r0 = C.row_offsets[pid[q]], r1 = C.row_offsets[pid[q] + 1], c0 = (int)chunk.size();
+            for (int r = r0; r < r1; r += kChunk) chunk.push_back(make_int4((int)q, r, std::min(r1, r + kChunk), 0));
+            pchunk.push_back(make_int2(c0, (int)chunk.size()));
+        }
+        C.parts.emplace_back();
+        DirectCache::Part &p = C.parts.back();
+        p.np = (int)pid.size();
+        p.nchunk = (int)chunk.size();
+        int rc = grmp_forest_create(ctx, groups, probs, 8, &p.F);
+        if (!rc) rc = upload_vec(ctx, C, chunk, &p.chunk);
+        if (!rc) rc = upload_vec(ctx, C, pchunk, &p.pchunk);
+        if (!rc) rc = upload_vec(ctx, C, pid, &p.pid);
+        if (!rc && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = GRMP_ERR_DEVICE;
+        if (rc) {
+            free_parts(ctx, C);
+            return rc;
+        }
+    }
+    C.parts_allow = need;
+    return GRMP_OK;
+}
+
+// factor and sweep one batch
+int run_part(grmp_context ctx, DirectCache::Part &P, const BatchDev &d) {
+    const int np = P.np;
+    char *w = nullptr;
+    const size_t dbl = (size_t)P.nchunk * 3 + 5 * (size_t)np, bytes = dbl * 8 + ((size_t)np * 6 + 2) * 4;
+    int rc = grmp_alloc(ctx, (void **)&w, bytes);
+    if (rc) return rc;
+    SweepDev s;
+    s.chunk = P.chunk;
+    s.pchunk = P.pchunk;
+    s.pid = P.pid;
+    s.part = (double *)w;
+    s.anorm = s.part + (size_t)P.nchunk * 3;
+    s.bn = s.anorm + np;
+    s.prev = s.bn + np;
+    s.rel = s.prev + np;
+    s.worst = s.rel + np;
+    int *iw = (int *)(w + dbl * 8);
+    s.act = iw;
+    s.fin = iw + np;
+    s.ok = iw + 2 * np;
+    s.nsolve = iw + 3 * np;
+    s.sweeps = iw + 4 * np;
+    int *err = iw + 5 * np;
+    s.err = err;
+    s.count = iw + 6 * np;
+    s.max_solves = 4;
+    rc = grmp_forest_factor64(ctx, P.F, d.v64, err);
+    const int gp = (np + 127) / 128;
+    cudaError_t e = cudaSuccess;
+    if (!rc) {
+        k_sb_init<<<gp, 128, 0, ctx->stream>>>(np, s);
+        k_sb_anorm<<<P.nchunk, 256, 0, ctx->stream>>>(d, s);
+        k_sb_anorm2<<<gp, 128, 0, ctx->stream>>>(np, s);
+        ctx->launches += 3;
+        for (int sweep = 0; sweep < d.sweeps && e == cudaSuccess; sweep++) {
+            k_sb_rhs<<<P.nchunk, 256, 0, ctx->stream>>>(d, s);
+            GRMP_LAUNCHED(ctx);
+            int left[2] = {0, 0};
+            for (int ref = 0; ref <= s.max_solves; ref++) {
+                cudaMemsetAsync(s.count, 0, 8, ctx->stream);
+                k_sb_resid<<<P.nchunk, 256, 0, ctx->stream>>>(d, s, ref);
+                k_sb_decide<<<gp, 128, 0, ctx->stream>>>(np, s, ref, d.reltol);
+                ctx->launches += 2;
+                e = cudaMemcpyAsync(left, s.count, 8, cudaMemcpyDeviceToHost, ctx->stream);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+                if (e != cudaSuccess || left[0] == 0) break;
+                grmp_forest_solve64(ctx, P.F, d.r64, s.act);
+                k_sb_add<<<P.nchunk, 256, 0, ctx->stream>>>(d, s);
+                GRMP_LAUNCHED(ctx);
+            }
+            k_sb_pressure<<<np, 512, 0, ctx->stream>>>(d, s);
+            GRMP_LAUNCHED(ctx);
+            if (d.sweep_tol > 0 && e == cudaSuccess) {
+                e = cudaMemcpyAsync(left, s.count, 8, cudaMemcpyDeviceToHost, ctx->stream);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+                if (left[1] == 0) break;
+            }
+        }
+        k_sb_result<<<gp, 128, 0, ctx->stream>>>(np, d, s);
+        GRMP_LAUNCHED(ctx);
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e != cudaSuccess) rc = grmp_cuda_fail(ctx, e, "batched Stokes");
+    }
+    grmp_forest_release(ctx, P.F);
+    grmp_free(ctx, w, bytes);
     return rc;
 }
 
@@ -1449,6 +1763,7 @@ int build_direct_cache(grmp_matrix A, int np, const int32_t *row_off, const int3
 void grmp_direct_cache_free(grmp_matrix A) {
     if (!A || !A->direct) return;
     grmp_context ctx = A->space->mesh->ctx;
+    free_parts(ctx, *A->direct);
     for (auto &b : A->direct->bufs) grmp_free(ctx, b.first, b.second);
     delete A->direct;
     A->direct = nullptr;
@@ -1605,7 +1920,39 @@ extern "C" int grmp_stokes_batch_solve(grmp_matrix A, grmp_vector bf, grmp_vecto
         if (!A->direct || A->direct->row_offsets != std::vector<int32_t>(prm->row_offsets, prm->row_offsets + np + 1)) {
             grmp_direct_cache_free(A);
             rc = build_direct_cache(A, np, prm->row_offsets, drow);
+            if (rc) grmp_direct_cache_free(A);
         }
+    }
+    if (prm->mode == GRMP_SOLVE_DIRECT) {
+        size_t freeb = 0, totalb = 0;
+        cudaMemGetInfo(&freeb, &totalb);
+        // what the pool holds without using it counts as free
+        cudaMemPool_t pool;
+        uint64_t held = 0, used = 0;
+        if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess &&
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+            freeb += held - used;
+        size_t allow = (size_t)(0.8 * (double)freeb);
+        if (ctx->budget) allow = std::min(allow, ctx->budget > ctx->in_use ? ctx->budget - ctx->in_use : (size_t)0);
+        cudaMemsetAsync(d.u, 0, (size_t)n * 8, ctx->stream);
+        cudaMemsetAsync(d.p, 0, (size_t)nc * 8, ctx->stream);
+        if (!rc) rc = build_parts(A, order, allow);
+        cudaEventRecord(e0, ctx->stream);
+        if (!rc)
+            for (auto &part : A->direct->parts)
+                if (!rc) rc = run_part(ctx, part, d);
+        cudaEventRecord(e1, ctx->stream);
+        if (rc) {
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            release();
+            grmp_free(ctx, Dv, (size_t)nc * s->ldofs * 8);
+            grmp_free(ctx, vol, (size_t)nc * 8);
+            return rc;
+        }
+    } else if (direct) {
+        if (!rc) rc = build_direct_tables(A, np);
         DirectDev m;
         std::memset(&m, 0, sizeof(m));
         if (!rc) {
@@ -1639,10 +1986,7 @@ extern "C" int grmp_stokes_batch_solve(grmp_matrix A, grmp_vector bf, grmp_vecto
         }
         const size_t smem =
             ((size_t)m.max_f + m.max_s + 32 * 33 + (size_t)m.max_f * kPanelStride + 16 * (size_t)kWarpFront) * 8;
-        const bool mx = prm->mode == GRMP_SOLVE_MIXED_DIRECT;
-        auto kern = mx ? (tpr == 4 ? k_stokes_direct<4, true> : (tpr == 8 ? k_stokes_direct<8, true> : k_stokes_direct<16, true>))
-                       : (tpr == 4 ? k_stokes_direct<4, false>
-                                   : (tpr == 8 ? k_stokes_direct<8, false> : k_stokes_direct<16, false>));
+        auto kern = tpr == 4 ? k_stokes_direct<4> : (tpr == 8 ? k_stokes_direct<8> : k_stokes_direct<16>);
         if (!rc && smem > 220 * 1024)
             rc = grmp_fail(ctx, GRMP_ERR_UNSUPPORTED, "batch direct: front of %d DoFs too large", m.max_f);
         if (!rc) {
