@@ -309,23 +309,30 @@ __device__ bool big_front(const FoDev &m, int2 it, const double *vals, T *L, T *
     const FoProb pr = m.prob[it.x];
     const int f = nd.f, s = nd.s;
     T *Lt = L + pr.Lb + nd.L_off;
-    for (long long i = gwarp; i < f; i += nwarps)
-        for (int j = lane; j <= i; j += 32) F[i * f + j] = T(0);
+    // a warp per row: zero it and add the rows of the children's update matrices
+    // that fall on it (src names them), then the matrix entries
+    const int2 *src = m.src + nd.front_off;
+    for (long long i = gwarp; i < f; i += nwarps) {
+        T *Fi = F + i * f;
+        for (int j = lane; j <= i; j += 32) Fi[j] = T(0);
+        __syncwarp();
+        const int2 q = src[i];
+        for (int c = 0; c < nd.nchild; c++) {
+            const FoNode cn = m.node[m.child[nd.child_off + c]];
+            const int sc = cn.f - cn.s;
+            const long long ax = q.x - cn.uv_off, ay = q.y - cn.uv_off;
+            const long long a = q.x >= 0 && ax >= 0 && ax < sc ? ax : (q.y >= 0 && ay >= 0 && ay < sc ? ay : -1);
+            if (a < 0) continue;
+            const T *Uc = U + pr.Ub + cn.U_off + a * sc;
+            const int32_t *ex = m.ext + cn.ext_off;
+            for (int b = lane; b <= a; b += 32) Fi[ex[b]] += Uc[b];
+            __syncwarp();
+        }
+    }
     if (!sync()) return false;
     for (long long e = gtid; e < nd.nentry; e += gsz)
-        F[m.ent_pos[nd.entry_off + e]] = (T)vals[pr.nnz0 + m.ent_rel[nd.entry_off + e]];
+        F[m.ent_pos[nd.entry_off + e]] += (T)vals[pr.nnz0 + m.ent_rel[nd.entry_off + e]];
     if (!sync()) return false;
-    for (int c = 0; c < nd.nchild; c++) {
-        const FoNode cn = m.node[m.child[nd.child_off + c]];
-        const int sc = cn.f - cn.s;
-        const T *Uc = U + pr.Ub + cn.U_off;
-        const int32_t *ex = m.ext + cn.ext_off;
-        for (long long a = gwarp; a < sc; a += nwarps) {
-            const long long pa = (long long)ex[a] * f;
-            for (int b = lane; b <= a; b += 32) F[pa + ex[b]] += Uc[a * sc + b];
-        }
-        if (!sync()) return false;
-    }
     for (int k0 = 0; k0 < s; k0 += kWide) {
         const int kw = min(kWide, s - k0), k1 = k0 + kw, mrows = f - k1;
         for (int q = tid; q < kWide * kWide; q += kBigT) {

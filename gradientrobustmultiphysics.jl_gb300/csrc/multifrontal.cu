@@ -207,22 +207,39 @@ __global__ void __launch_bounds__(NT) k_fq_fwd(FoDev m, const int4 *tiles, const
     for (int k = tid; k < s; k += NT) b[k] = w[fr[k]] - up(k);
     __syncthreads();
     const float *Qt = Q + nd.L_off;
-    // 8 lanes per row of short rows, a warp otherwise
-    const int lp = s <= 48 ? 8 : 32, lane = tid & (lp - 1), rows = NT / lp;
-    const int span = (t.z - t.y + rows - 1) / rows * rows;
-    for (int o = tid / lp; o < span; o += rows) {
-        const int r = t.y + o;
-        float acc = 0.f;
-        if (r < t.z) {
-            const float *Qr = Qt + (long long)r * s;
-            const int kend = r < s ? r + 1 : s;
+    // 8 lanes per row of short rows, a warp otherwise, two rows at a time (the
+    // entries above a row's diagonal are stored as zeros within its 32 x 32
+    // block and not at all beyond it)
+    const int lp = s <= 64 ? 8 : 32, lane = tid & (lp - 1), rows = NT / lp;
+    const int span = (t.z - t.y + 2 * rows - 1) / (2 * rows) * (2 * rows);
+    for (int o = tid / lp; o < span; o += 2 * rows) {
+        const int r0 = t.y + o, r1 = r0 + rows;
+        const int e0 = r0 < t.z ? (r0 < s ? r0 + 1 : s) : 0, e1 = r1 < t.z ? (r1 < s ? r1 + 1 : s) : 0;
+        const float *Q0 = Qt + (long long)r0 * s, *Q1 = Qt + (long long)r1 * s;
+        float a0 = 0.f, a1 = 0.f;
+        const int both = min(e0, e1);
+        int k = lane;
 #pragma unroll 4
-            for (int k = lane; k < kend; k += lp) acc += Qr[k] * b[k];
+        for (; k < both; k += lp) {
+            const float bk = b[k];
+            a0 += Q0[k] * bk;
+            a1 += Q1[k] * bk;
         }
-        for (int d = lp / 2; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
-        if (r < t.z && lane == 0) {
-            if (r < s) wy[fr[r]] = acc;
-            else uv[nd.uv_off + r - s] = up(r) + acc;
+        for (int q = k; q < e0; q += lp) a0 += Q0[q] * b[q];
+        for (int q = k; q < e1; q += lp) a1 += Q1[q] * b[q];
+        for (int d = lp / 2; d > 0; d >>= 1) {
+            a0 += __shfl_xor_sync(0xffffffffu, a0, d);
+            a1 += __shfl_xor_sync(0xffffffffu, a1, d);
+        }
+        if (lane == 0) {
+            if (r0 < t.z) {
+                if (r0 < s) wy[fr[r0]] = a0;
+                else uv[nd.uv_off + r0 - s] = up(r0) + a0;
+            }
+            if (r1 < t.z) {
+                if (r1 < s) wy[fr[r1]] = a1;
+                else uv[nd.uv_off + r1 - s] = up(r1) + a1;
+            }
         }
     }
 }
@@ -498,8 +515,21 @@ int mf_build(grmp_matrix A) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(ci.data(), A->d_cols, (size_t)A->nnz * 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multifrontal: pattern download");
+    // separators in the mesh's graph, where the matrix was assembled on one by
+    // cell terms (face terms couple further)
+    grmp_space s = A->space;
+    NdGraph G;
+    bool mesh_graph = false;
+    if (!A->imported && s->d_celldofs && (s->fe == GRMP_FE_H1P1 || s->fe == GRMP_FE_H1P2)) {
+        std::vector<int32_t> cd((size_t)s->mesh->ncells * s->ldofs);
+        e = cudaMemcpyAsync(cd.data(), s->d_celldofs, cd.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multifrontal: cell DoFs");
+        mesh_graph = nd_cell_graph(n, s->mesh->ncells, s->ldofs, s->ncomp, cd.data(), &G) == 0;
+    }
     MfCache *C = new MfCache;
-    int src = nd_symbolic_build(n, rp.data(), ci.data(), &C->S);
+    int src = nd_symbolic_build(n, rp.data(), ci.data(), &C->S, mesh_graph ? &G : nullptr);
+    if (src == 3 && mesh_graph) src = nd_symbolic_build(n, rp.data(), ci.data(), &C->S);
     if (src) {
         delete C;
         return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "multifrontal: symbolic analysis failed (%d)", src);

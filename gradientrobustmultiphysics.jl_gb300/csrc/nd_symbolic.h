@@ -29,6 +29,19 @@ struct NdSymbolic {
     int64_t uv_size = 0;
 };
 
+// Graph that the separators are sought in: nodes of one or more DoFs each
+// (member lists mem[mptr[v] .. mptr[v + 1])), coupled wherever the mesh couples
+// them.  It covers the pattern, so its separators separate the pattern too.
+struct NdGraph {
+    int n = 0;
+    std::vector<int32_t> rp, ci, mptr, mem;
+};
+
 // rowptr/cols: the local pattern (cols local to the problem, diagonal
-// included, symmetric); ent_rel is relative to rowptr[0].  Returns 0 on success.
-int nd_symbolic_build(int n, const int32_t *rowptr, const int32_t *cols, NdSymbolic *S);
+// included, symmetric); ent_rel is relative to rowptr[0].  graph: where to
+// seek separators (nullptr: the pattern itself).  Returns 0 on success.
+int nd_symbolic_build(int n, const int32_t *rowptr, const int32_t *cols, NdSymbolic *S, const NdGraph *graph = nullptr);
+// the graph of a mesh's cells: DoFs (component c, basis function a) of one
+// basis function's components are one node; returns 1 if the cell DoFs are
+// not component-major copies of each other
+int nd_cell_graph(int n, int ncells, int ld, int ncomp, const int32_t *celldofs, NdGraph *G);
