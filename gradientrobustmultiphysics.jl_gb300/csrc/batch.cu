@@ -1184,7 +1184,7 @@ __global__ void __launch_bounds__(512, 1) k_stokes_direct(BatchDev d, DirectDev 
 // norms are the sums of its chunks in order, so its bits do not depend on the
 // batch.  Problems that have met the tolerance (or the FP64 floor) are skipped
 // by every kernel until the next sweep.
-constexpr int kChunk = 2048;
+constexpr int kChunk = 512;
 
 struct SweepDev {
     const int4 *chunk;      // {problem, first row, last row + 1, -}

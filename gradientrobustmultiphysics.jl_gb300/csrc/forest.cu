@@ -60,8 +60,8 @@ __device__ __forceinline__ bool chol16(T *A, int ld, int kw, T *inv) {
             if (!(piv > T(0)) || !isfinite((double)piv)) {
                 ok = false;
             } else {
-                const T d = sqrt(piv), iv = T(1) / d;
-                a[c] = lane == c ? d : a[c] * iv;
+                const T iv = rsqrt(piv);   // one dependent chain instead of a square root and a division
+                a[c] *= iv;
                 if (lane == 0) inv[c] = iv;
 #pragma unroll
                 for (int j = c + 1; j < kPan; j++) {
@@ -82,14 +82,19 @@ template <typename T>
 __device__ __forceinline__ void row16(T *row, const T *D, int ld, int kw, const T *inv) {
     T x[kPan];
 #pragma unroll
+    for (int j = 0; j < kPan; j++) x[j] = j < kw ? row[j] : T(0);
+    // right-looking: the updates of one step are independent of each other
+#pragma unroll
     for (int j = 0; j < kPan; j++)
         if (j < kw) {
-            T v = row[j];
+            x[j] *= inv[j];
 #pragma unroll
-            for (int l = 0; l < j; l++) v -= x[l] * D[j * ld + l];
-            x[j] = v * inv[j];
-            row[j] = x[j];
+            for (int l = j + 1; l < kPan; l++)
+                if (l < kw) x[l] -= x[j] * D[l * ld + j];
         }
+#pragma unroll
+    for (int j = 0; j < kPan; j++)
+        if (j < kw) row[j] = x[j];
 }
 
 // lower tile (bi, bj) of a linear index
@@ -383,43 +388,45 @@ __device__ bool big_front(const FoDev &m, int2 it, const double *vals, T *L, T *
             }
         __syncthreads();
         // (c) trailing update
+        constexpr int TS = sizeof(T) == 8 ? 32 : 64, R = TS / 16;
         T *Ta = Dg, *Tb = W;
-        const int nt = (mrows + kWide - 1) / kWide, ntiles = nt * (nt + 1) / 2;
+        const int nt = (mrows + TS - 1) / TS, ntiles = nt * (nt + 1) / 2;
         const int ty = tid >> 4, tx = tid & 15;
         for (int q = grank; q < ntiles; q += gblocks) {
             int bi, bj;
             tile_of(q, bi, bj);
-            for (int e = tid; e < kWide * kWide; e += kBigT) {
+            for (int e = tid; e < TS * kWide; e += kBigT) {
                 const int r = e / kWide, c = e - r * kWide;
-                const int ia = bi * kWide + r, ib = bj * kWide + r;
+                const int ia = bi * TS + r, ib = bj * TS + r;
                 Ta[r * kWs + c] = (ia < mrows && c < kw) ? P[(long long)ia * kWs + c] : T(0);
                 Tb[r * kWs + c] = (ib < mrows && c < kw) ? P[(long long)ib * kWs + c] : T(0);
             }
             __syncthreads();
-            T acc[4][4];
+            T acc[R][R];
 #pragma unroll
-            for (int a = 0; a < 4; a++)
+            for (int a = 0; a < R; a++)
 #pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = T(0);
+                for (int b = 0; b < R; b++) acc[a][b] = T(0);
+#pragma unroll 2
             for (int t = 0; t < kw; t++) {
-                T x[4], y[4];
+                T x[R], y[R];
 #pragma unroll
-                for (int a = 0; a < 4; a++) {
+                for (int a = 0; a < R; a++) {
                     x[a] = Ta[(ty + 16 * a) * kWs + t];
                     y[a] = Tb[(tx + 16 * a) * kWs + t];
                 }
 #pragma unroll
-                for (int a = 0; a < 4; a++)
+                for (int a = 0; a < R; a++)
 #pragma unroll
-                    for (int b = 0; b < 4; b++) acc[a][b] += x[a] * y[b];
+                    for (int b = 0; b < R; b++) acc[a][b] += x[a] * y[b];
             }
 #pragma unroll
-            for (int a = 0; a < 4; a++) {
-                const int i = bi * kWide + ty + 16 * a;
+            for (int a = 0; a < R; a++) {
+                const int i = bi * TS + ty + 16 * a;
                 T *Fi = F + (long long)(k1 + i) * f + k1;
 #pragma unroll
-                for (int b = 0; b < 4; b++) {
-                    const int j = bj * kWide + tx + 16 * b;
+                for (int b = 0; b < R; b++) {
+                    const int j = bj * TS + tx + 16 * b;
                     if (i < mrows && j <= i) Fi[j] -= acc[a][b];
                 }
             }
@@ -441,36 +448,57 @@ __device__ bool big_front(const FoDev &m, int2 it, const double *vals, T *L, T *
 }
 
 template <typename T, bool WB>
-__global__ void __launch_bounds__(kBigT, 2) k_ff_big(FoDev m, const int2 *items, int count, int ngroups, const double *vals,
-                                                     T *L, T *U, T *pool, long long fslot, long long pslot, CoopState *cs,
-                                                     int *err, long long spin) {
-    const int g = blockIdx.x % ngroups, grank = blockIdx.x / ngroups;
-    const int gblocks = (gridDim.x - g + ngroups - 1) / ngroups;
-    CoopState *c = cs + g;
+__global__ void __launch_bounds__(kBigT, 2) k_ff_big(FoDev m, const int2 *items, int count, const int4 *blocks, int slots,
+                                                     const double *vals, T *L, T *U, T *pool, long long fslot,
+                                                     long long pslot, CoopState *cs, int *err, long long spin) {
+    const int4 b = blocks[blockIdx.x];
+    // group b.x takes fronts b.x, b.x + groups, ...; its buffers are slot b.x (slots < groups only when
+    // memory is short: then the groups of the later slots leave their fronts to the first ones)
+    if (b.x >= slots) return;
+    const int step = min(b.w, slots);
+    CoopState *c = cs + b.x;
     extern __shared__ __align__(16) unsigned char fo_bsmem[];
     T *sm = reinterpret_cast<T *>(fo_bsmem);
-    T *F = pool + (long long)g * (fslot + pslot), *P = F + fslot;
-    auto sync = [&]() { return grid_barrier(&c->bar, gblocks, &c->status, spin); };
-    for (int q = g; q < count; q += ngroups)
-        if (!big_front<T, WB>(m, items[q], vals, L, U, F, P, grank, gblocks, sync, err, sm)) return;
+    T *F = pool + (long long)b.x * (fslot + pslot), *P = F + fslot;
+    auto sync = [&]() { return grid_barrier(&c->bar, b.z, &c->status, spin); };
+    for (int q = b.x; q < count; q += step)
+        if (!big_front<T, WB>(m, items[q], vals, L, U, F, P, b.y, b.z, sync, err, sm)) return;
 }
 
 // ------------------------------------------------------------------ FP64 solves
+// 32 columns of L (rows i0 + 8 k) times 32 values, 8 rows a warp: four lanes a
+// row, eight consecutive columns each, two shuffle additions a row.  FP64 pipe
+// time 1.25 of the multiply-adds alone; a lane per row needs the tile staged
+// through shared memory first (3 times slower on 100 to 500 rows), a warp per
+// row spends five shuffle additions a row.
+__device__ __forceinline__ double rows8(const double *Lt, int s, int i, bool in, int kb, int nb, const double *v) {
+    const int c0 = (threadIdx.x & 3) * 8;
+    double l[8];
+    const double *r = Lt + (long long)i * s + kb + c0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) l[j] = in && c0 + j < nb ? r[j] : 0.0;
+    double a = 0.0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) a += l[j] * v[kb + c0 + j];
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    a += __shfl_xor_sync(0xffffffffu, a, 2);
+    return a;
+}
+
 // Forward: the front's vector is its own entries of w minus the children's
 // update entries, and their sum for its structure (gathered: src names the
-// entries of each row); per 32 columns y = W v, then a thread per remaining
-// row subtracts (own) or adds (structure) L y, its 32 columns staged per warp.
-// The structure part is the front's update vector.
+// entries of each row); per 32 columns y = W v, then the remaining rows
+// subtract (own) or add (structure) L y.  The structure part is the front's
+// update vector.
 template <int NT>
 __global__ void __launch_bounds__(NT) k_fs_fwd(FoDev m, const int2 *items, const double *L, double *uv, double *w,
                                                const int *active) {
     extern __shared__ __align__(16) unsigned char fo_ssmem[];
-    double *stage = reinterpret_cast<double *>(fo_ssmem);   // NT / 32 warps x 32 x 33
-    double *v = stage + NT * 33;
+    double *v = reinterpret_cast<double *>(fo_ssmem);   // f + 32 (the last columns' reads run past s)
     const int2 it = items[blockIdx.x];
     if (active && !active[it.x]) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double *st = stage + warp * 32 * 33;
+    constexpr int NW = NT / 32;
     const FoNode nd = m.node[it.y];
     const FoProb pr = m.prob[it.x];
     const int f = nd.f, s = nd.s;
@@ -478,39 +506,38 @@ __global__ void __launch_bounds__(NT) k_fs_fwd(FoDev m, const int2 *items, const
     const int2 *src = m.src + nd.front_off;
     const double *Lt = L + pr.Lb + nd.L_off;
     double *u = uv + pr.uvb;
-    for (int k = tid; k < f; k += NT) {
-        const int2 q = src[k];
-        const double c = (q.x >= 0 ? u[q.x] : 0.0) + (q.y >= 0 ? u[q.y] : 0.0);
-        v[k] = k < s ? w[pr.row0 + fr[k]] - c : c;
+    for (int k = tid; k < f + 32; k += NT) {
+        double x = 0.0;
+        if (k < f) {
+            const int2 q = src[k];
+            const double c = (q.x >= 0 ? u[q.x] : 0.0) + (q.y >= 0 ? u[q.y] : 0.0);
+            x = k < s ? w[pr.row0 + fr[k]] - c : c;
+        }
+        v[k] = x;
     }
     __syncthreads();
     for (int kb = 0; kb < s; kb += 32) {
         const int nb = min(32, s - kb);
-        if (warp == 0) {
-#pragma unroll 8
-            for (int r = 0; r < nb; r++)
-                if (lane < nb) st[r * 33 + lane] = Lt[(long long)(kb + r) * s + kb + lane];
-            __syncwarp();
-            double y = 0.0;
-            if (lane < nb)
-                for (int c = 0; c <= lane; c++) y += st[lane * 33 + c] * v[kb + c];
-            __syncwarp();
-            if (lane < nb) v[kb + lane] = y;
+        // y = W v: every warp its rows, written after all have read v
+        constexpr int NY = 8 * NW < 32 ? 32 / (8 * NW) : 1;   // warps from 4 on have no row of these
+        double y[NY];
+#pragma unroll
+        for (int q = 0; q < NY; q++) {
+            const int r = (q * NW + warp) * 8 + (lane >> 2);
+            y[q] = r < 32 ? rows8(Lt, s, kb + r, r < nb, kb, nb, v) : 0.0;
         }
         __syncthreads();
-        for (int i0 = kb + nb + warp * 32; i0 < f; i0 += NT) {
-            const int rows = min(32, f - i0);
-#pragma unroll 8
-            for (int r = 0; r < rows; r++)
-                if (lane < nb) st[r * 33 + lane] = Lt[(long long)(i0 + r) * s + kb + lane];
-            __syncwarp();
-            if (lane < rows) {
-                double a = 0.0;
-                for (int c = 0; c < nb; c++) a += st[lane * 33 + c] * v[kb + c];
-                const int i = i0 + lane;
-                v[i] = i < s ? v[i] - a : v[i] + a;
-            }
-            __syncwarp();
+#pragma unroll
+        for (int q = 0; q < NY; q++) {
+            const int r = (q * NW + warp) * 8 + (lane >> 2);
+            if (r < nb && (lane & 3) == 0) v[kb + r] = y[q];
+        }
+        __syncthreads();
+#pragma unroll 2
+        for (int i0 = kb + nb + warp * 8; i0 < f; i0 += NW * 8) {
+            const int i = i0 + (lane >> 2);
+            const double a = rows8(Lt, s, i, i < f, kb, nb, v);
+            if (i < f && (lane & 3) == 0) v[i] = i < s ? v[i] - a : v[i] + a;
         }
         __syncthreads();
     }
@@ -520,7 +547,8 @@ __global__ void __launch_bounds__(NT) k_fs_fwd(FoDev m, const int2 *items, const
 }
 
 // Backward: per 32 columns from the last, z = y - L^T x over the rows below
-// (a lane per column, the warps split the rows), x = W^T z.
+// (a lane per column, the warps split the rows), x = W^T z (warp 0, its part of
+// W loaded before the sums are ready).
 template <int NT>
 __global__ void __launch_bounds__(NT) k_fs_bwd(FoDev m, const int2 *items, const double *L, double *w, const int *active) {
     extern __shared__ __align__(16) unsigned char fo_ssmem[];
@@ -539,13 +567,18 @@ __global__ void __launch_bounds__(NT) k_fs_bwd(FoDev m, const int2 *items, const
     __syncthreads();
     for (int kb = ((s + 31) / 32 - 1) * 32; kb >= 0; kb -= 32) {
         const int nb = min(32, s - kb);
+        const double *Lk = Lt + kb + lane;
+        double wr[32];
+        if (warp == 0) {
+#pragma unroll
+            for (int r = 0; r < 32; r++) wr[r] = r < nb && lane < nb ? Lk[(long long)(kb + r) * s] : 0.0;
+        }
         double a = 0.0;
         if (lane < nb) {
-            const double *Lk = Lt + kb + lane;
-#pragma unroll 4
+#pragma unroll 8
             for (int i = kb + nb + warp; i < f; i += NW) a += Lk[(long long)i * s] * v[i];
         }
-        part[warp * 32 + lane] = a;
+        part[tid] = a;
         __syncthreads();
         if (warp == 0) {
             double z = 0.0;
@@ -554,11 +587,8 @@ __global__ void __launch_bounds__(NT) k_fs_bwd(FoDev m, const int2 *items, const
                 for (int g = 0; g < NW; g++) z -= part[g * 32 + lane];
             }
             double x = 0.0;
-#pragma unroll 8
-            for (int r = 0; r < nb; r++) {
-                const double zr = __shfl_sync(0xffffffffu, z, r);
-                if (lane <= r) x += Lt[(long long)(kb + r) * s + kb + lane] * zr;
-            }
+#pragma unroll
+            for (int r = 0; r < 32; r++) x += wr[r] * __shfl_sync(0xffffffffu, z, r);
             if (lane < nb) v[kb + lane] = x;
         }
         __syncthreads();
@@ -580,18 +610,20 @@ int fo_upload(grmp_context ctx, MfForest &F, const std::vector<V> &v, const V **
     return e == cudaSuccess ? GRMP_OK : grmp_cuda_fail(ctx, e, "multifrontal upload");
 }
 
-// groups of a level's large fronts: one each, as far as the pool's bound and the blocks go
+// groups of a level's large fronts with buffers of their own
 constexpr size_t kPoolBound = (size_t)3 << 30;
+constexpr int kMaxGroups = 160;
 inline long long slot_elems(int maxf) { return (long long)maxf * maxf + (long long)maxf * kWs; }
-inline int big_groups(int count, int maxf, int esize) {
-    const long long fit = std::max<long long>(1, (long long)(kPoolBound / (slot_elems(maxf) * esize)));
-    return (int)std::min<long long>({(long long)count, fit, 152LL});
+inline int big_slots(const FoLevel &l, int num_sms, size_t poolb, int esize) {
+    const long long fit = std::max<long long>(1, (long long)(poolb / (slot_elems(l.big.maxf) * esize)));
+    return (int)std::min<long long>({(long long)l.big.count, fit, (long long)num_sms, (long long)kMaxGroups});
 }
 
-size_t pool_bytes(const MfForest &F, int esize) {
+size_t pool_bytes(const MfForest &F, int num_sms, int esize) {
     size_t b = 0;
     for (const FoLevel &l : F.level)
-        if (l.big.count) b = std::max<size_t>(b, (size_t)big_groups(l.big.count, l.big.maxf, esize) * slot_elems(l.big.maxf) * esize);
+        if (l.big.count)
+            b = std::max<size_t>(b, (size_t)big_slots(l, num_sms, kPoolBound, esize) * slot_elems(l.big.maxf) * esize);
     return b;
 }
 
@@ -600,7 +632,7 @@ int fo_storage(grmp_context ctx, MfForest *F, int esize) {
     F->Lb = std::max<size_t>(1, F->L_size) * esize;
     F->Ub = std::max<size_t>(1, F->U_size) * esize;
     F->uvb = std::max<size_t>(1, F->uv_size) * esize;
-    F->poolb = std::max<size_t>(256, pool_bytes(*F, esize));
+    F->poolb = std::max<size_t>(256, pool_bytes(*F, ctx->num_sms, esize));
     int rc = grmp_alloc(ctx, &F->L, F->Lb);
     if (!rc) rc = grmp_alloc(ctx, &F->U, F->Ub);
     if (!rc) rc = grmp_alloc(ctx, &F->uv, F->uvb);
@@ -613,7 +645,7 @@ int fo_storage(grmp_context ctx, MfForest *F, int esize) {
         if (!rc) ctx->last_error.clear();
         cudaGetLastError();
     }
-    if (!rc) rc = grmp_alloc(ctx, &F->cs, 152 * sizeof(CoopState));
+    if (!rc) rc = grmp_alloc(ctx, &F->cs, kMaxGroups * sizeof(CoopState));
     if (rc) {
         grmp_free(ctx, F->L, F->Lb);
         grmp_free(ctx, F->U, F->Ub);
@@ -651,22 +683,20 @@ int fo_factor(grmp_context ctx, MfForest *F, const double *vals, int *err) {
             }
         if (!l.big.count) continue;
         if (!coop) {
-            int per_sm = 0;
             cudaFuncSetAttribute(k_ff_big<T, WB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ff_big<T, WB>, kBigT, bsmem);
-            coop = std::max(1, std::min(per_sm, 2)) * ctx->num_sms;
+            coop = 1;
         }
-        const long long room = (long long)(F->poolb / sizeof(T)) / slot_elems(l.big.maxf);
-        int ng = (int)std::min<long long>({(long long)big_groups(l.big.count, l.big.maxf, sizeof(T)), (long long)coop, room});
-        int count = l.big.count;
-        cudaMemsetAsync(F->cs, 0, (size_t)ng * sizeof(CoopState), ctx->stream);
+        int slots = big_slots(l, ctx->num_sms, F->poolb, sizeof(T)), count = l.big.count;
+        const int ng = slots;
+        const int4 *blocks = l.blocks;
+        cudaMemsetAsync(F->cs, 0, kMaxGroups * sizeof(CoopState), ctx->stream);
         FoDev dv = F->dev;
         const int2 *items = l.big.d;
         T *Lp = (T *)F->L, *Up = (T *)F->U, *pool = (T *)F->pool;
         long long fs = (long long)l.big.maxf * l.big.maxf, ps = (long long)l.big.maxf * kWs, spin = ctx->wait_limit;
         CoopState *cs = (CoopState *)F->cs;
-        void *args[] = {&dv, &items, &count, &ng, &vals, &Lp, &Up, &pool, &fs, &ps, &cs, &err, &spin};
-        e = cudaLaunchCooperativeKernel((void *)k_ff_big<T, WB>, coop, kBigT, args, bsmem, ctx->stream);
+        void *args[] = {&dv, &items, &count, &blocks, &slots, &vals, &Lp, &Up, &pool, &fs, &ps, &cs, &err, &spin};
+        e = cudaLaunchCooperativeKernel((void *)k_ff_big<T, WB>, l.nblocks, kBigT, args, bsmem, ctx->stream);
         GRMP_LAUNCHED(ctx);
         std::vector<CoopState> hc(ng);
         if (e == cudaSuccess)
@@ -746,8 +776,8 @@ int grmp_forest_create(grmp_context ctx, const std::vector<const NdSymbolic *> &
     F->level.resize(nlev);
     int rc = GRMP_OK;
     for (size_t l = 0; l < nlev && !rc; l++) {
-        std::vector<int2> cls[7];   // 0-3 small, 4 big, 5 / 6 solve classes
-        int maxf[7] = {};
+        std::vector<int2> cls[8];   // 0-3 small, 4 big, 5-7 solve classes
+        int maxf[8] = {};
         for (int p = 0; p < F->nprob; p++) {
             const NdSymbolic &S = *groups[probs[p].group];
             if (l + 1 >= S.level_ptr.size()) continue;
@@ -759,18 +789,62 @@ int grmp_forest_create(grmp_context ctx, const std::vector<const NdSymbolic *> &
                 while (k < 4 && f > class_limit(esize, k)) k++;
                 cls[k].push_back(it);
                 maxf[k] = std::max(maxf[k], f);
-                k = f <= kFoWarpFront ? 5 : 6;
+                k = f <= kFoSolve[0] ? 5 : (f <= kFoSolve[1] ? 6 : 7);
                 cls[k].push_back(it);
                 maxf[k] = std::max(maxf[k], f);
             }
         }
         FoLevel &L = F->level[l];
-        FoItems *to[7] = {&L.small_[0], &L.small_[1], &L.small_[2], &L.small_[3], &L.big, &L.warp, &L.block};
-        for (int k = 0; k < 7 && !rc; k++) {
+        FoItems *to[8] = {&L.small_[0], &L.small_[1], &L.small_[2], &L.small_[3], &L.big, &L.solve[0], &L.solve[1], &L.solve[2]};
+        for (int k = 0; k < 8; k++) {
             std::stable_sort(cls[k].begin(), cls[k].end(), [&](int2 a, int2 b) { return node[a.y].f > node[b.y].f; });
             to[k]->count = (int)cls[k].size();
             to[k]->maxf = maxf[k];
+        }
+        // few shared-memory fronts in the level: one launch for all classes (a class is a launch,
+        // and one front's chain of panels is its time); largest first
+        int nsmall = 0;
+        for (int k = 0; k < 4; k++) nsmall += to[k]->count;
+        if (nsmall <= 2 * ctx->num_sms)
+            for (int k = 2; k >= 0; k--) {
+                cls[3].insert(cls[3].end(), cls[k].begin(), cls[k].end());
+                to[3]->count += to[k]->count;
+                to[3]->maxf = std::max(to[3]->maxf, to[k]->maxf);
+                to[k]->count = to[k]->maxf = 0;
+                cls[k].clear();
+            }
+        for (int k = 0; k < 8 && !rc; k++)
             if (to[k]->count) rc = fo_upload(ctx, *F, cls[k], &to[k]->d);
+        // large fronts: with at most one per SM each gets blocks in proportion to its flops (all run at
+        // once, the largest is the level's time), else groups of two blocks take them in turn
+        if (!rc && L.big.count) {
+            const int nblk = 2 * ctx->num_sms, cnt = L.big.count;
+            std::vector<int4> blk;
+            if (cnt <= ctx->num_sms) {
+                double tot = 0;
+                std::vector<double> wt;
+                for (int2 it : cls[4]) {
+                    const FoNode &q = node[it.y];
+                    wt.push_back((double)q.s * q.f * q.f);
+                    tot += wt.back();
+                }
+                std::vector<int> nb(cnt, 1);
+                int left = nblk - cnt;
+                for (int i = 0; i < cnt; i++) {
+                    const int add = std::min(left, (int)(wt[i] / tot * (nblk - cnt)));
+                    nb[i] += add;
+                }
+                for (int b : nb) left -= b - 1;
+                for (int i = 0; left > 0; i = (i + 1) % cnt, left--) nb[i]++;
+                for (int i = 0; i < cnt; i++)
+                    for (int r = 0; r < nb[i]; r++) blk.push_back(make_int4(i, r, nb[i], cnt));
+            } else {
+                const int g = nblk / 2;
+                for (int i = 0; i < g; i++)
+                    for (int r = 0; r < 2; r++) blk.push_back(make_int4(i, r, 2, g));
+            }
+            L.nblocks = (int)blk.size();
+            rc = fo_upload(ctx, *F, blk, &L.blocks);
         }
     }
     if (!rc) rc = fo_upload(ctx, *F, node, &F->dev.node);
@@ -790,7 +864,7 @@ void grmp_forest_release(grmp_context ctx, MfForest *F) {
     grmp_free(ctx, F->U, F->Ub);
     grmp_free(ctx, F->uv, F->uvb);
     grmp_free(ctx, F->pool, F->poolb);
-    grmp_free(ctx, F->cs, 152 * sizeof(CoopState));
+    grmp_free(ctx, F->cs, kMaxGroups * sizeof(CoopState));
     F->L = F->U = F->uv = F->pool = F->cs = nullptr;
     F->esize = 0;
 }
@@ -812,21 +886,22 @@ int grmp_forest_factor32(grmp_context ctx, MfForest *F, const double *vals, int 
 void grmp_forest_solve64(grmp_context ctx, MfForest *F, double *w, const int *active) {
     const double *L = (const double *)F->L;
     double *uv = (double *)F->uv;
-    auto smem_f = [](int nt, int maxf) { return ((size_t)nt * 33 + maxf) * 8; };
+    auto smem_f = [](int maxf) { return (size_t)(maxf + 32) * 8; };
     auto smem_b = [](int nt, int maxf) { return ((size_t)nt + maxf) * 8; };
-    cudaFuncSetAttribute(k_fs_fwd<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f(64, kFoWarpFront));
-    cudaFuncSetAttribute(k_fs_fwd<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f(128, F->max_f));
-    cudaFuncSetAttribute(k_fs_bwd<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b(128, F->max_f));
+    cudaFuncSetAttribute(k_fs_fwd<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f(F->max_f));
+    cudaFuncSetAttribute(k_fs_bwd<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b(512, F->max_f));
     for (size_t l = 0; l < F->level.size(); l++) {
-        const FoItems &a = F->level[l].warp, &b = F->level[l].block;
-        if (b.count) k_fs_fwd<128><<<b.count, 128, smem_f(128, b.maxf), ctx->stream>>>(F->dev, b.d, L, uv, w, active);
-        if (a.count) k_fs_fwd<64><<<a.count, 64, smem_f(64, a.maxf), ctx->stream>>>(F->dev, a.d, L, uv, w, active);
-        ctx->launches += (a.count > 0) + (b.count > 0);
+        const FoItems *c = F->level[l].solve;
+        if (c[2].count) k_fs_fwd<512><<<c[2].count, 512, smem_f(c[2].maxf), ctx->stream>>>(F->dev, c[2].d, L, uv, w, active);
+        if (c[1].count) k_fs_fwd<128><<<c[1].count, 128, smem_f(c[1].maxf), ctx->stream>>>(F->dev, c[1].d, L, uv, w, active);
+        if (c[0].count) k_fs_fwd<64><<<c[0].count, 64, smem_f(c[0].maxf), ctx->stream>>>(F->dev, c[0].d, L, uv, w, active);
+        for (int k = 0; k < 3; k++) ctx->launches += c[k].count > 0;
     }
     for (size_t l = F->level.size(); l-- > 0;) {
-        const FoItems &a = F->level[l].warp, &b = F->level[l].block;
-        if (b.count) k_fs_bwd<128><<<b.count, 128, smem_b(128, b.maxf), ctx->stream>>>(F->dev, b.d, L, w, active);
-        if (a.count) k_fs_bwd<64><<<a.count, 64, smem_b(64, a.maxf), ctx->stream>>>(F->dev, a.d, L, w, active);
-        ctx->launches += (a.count > 0) + (b.count > 0);
+        const FoItems *c = F->level[l].solve;
+        if (c[2].count) k_fs_bwd<512><<<c[2].count, 512, smem_b(512, c[2].maxf), ctx->stream>>>(F->dev, c[2].d, L, w, active);
+        if (c[1].count) k_fs_bwd<128><<<c[1].count, 128, smem_b(128, c[1].maxf), ctx->stream>>>(F->dev, c[1].d, L, w, active);
+        if (c[0].count) k_fs_bwd<64><<<c[0].count, 64, smem_b(64, c[0].maxf), ctx->stream>>>(F->dev, c[0].d, L, w, active);
+        for (int k = 0; k < 3; k++) ctx->launches += c[k].count > 0;
     }
 }

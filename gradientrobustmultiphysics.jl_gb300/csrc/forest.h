@@ -33,10 +33,15 @@ struct FoItems {
 struct FoLevel {
     FoItems small_[4];             // fronts factored in shared memory, by size
     FoItems big;                   // fronts factored by groups of blocks
-    FoItems warp, block;           // solve classes
+    FoItems solve[3];              // by size, for the solves
+    // blocks of the large fronts' launch: {item, rank in its group, blocks of the group, groups}
+    const int4 *blocks = nullptr;
+    int nblocks = 0;
 };
 
-constexpr int kFoWarpFront = 96;   // fronts up to this size are solved by 64 threads, larger ones by 128
+// fronts up to these sizes are solved by 64 and 128 threads, larger ones by 512
+// (96 squares, f = 550, s = 290: 130 us with 128 threads, bound by the loads in flight)
+constexpr int kFoSolve[2] = {96, 224};
 
 struct MfForest {
     FoDev dev{};

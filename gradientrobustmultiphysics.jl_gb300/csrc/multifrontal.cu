@@ -546,7 +546,7 @@ int mf_numeric_arrays(grmp_matrix A, int esize) {
     mf_free_numeric(ctx, C);
     const NdSymbolic &S = C.S;
     // shared memory of the solve kernels: the front's vector
-    if ((esize == 8 ? (size_t)(S.max_f + 128 * 33) * 8 : (size_t)(S.max_f + 512) * 4) > 220 * 1024)
+    if ((esize == 8 ? (size_t)(S.max_f + 512) * 8 : (size_t)(S.max_f + 512) * 4) > 220 * 1024)
         return grmp_fail(ctx, GRMP_ERR_UNSUPPORTED, "direct solve: front of %d DoFs exceeds shared memory", S.max_f);
     int rc = grmp_forest_create(ctx, {&S}, {FoProblem{0, 0, 0}}, esize, &C.F);
     if (!rc) rc = mf_take(ctx, C, 1, &C.err);
