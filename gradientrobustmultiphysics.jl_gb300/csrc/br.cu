@@ -247,38 +247,28 @@ __global__ void __launch_bounds__(128) k_br_rows(int32_t nrows, const int32_t *_
 // ------------------------------------------------------------------ reconstructed rhs (FP64)
 struct BrRhs {
     const double *par;     // [ngroups][nt][5] polynomial terms (component, coef, e1, e2, e3)
+    const PolyTerm *term;  // the same, decoded
     int nt;                // terms per group
     const int32_t *group;  // [ncells] group of each cell (nullptr: one group)
     double factor;
     int nq;
-    double xref[64][2];
+    double xref[64][2], lam0[64];
     double w[64];
 };
-
-// loc[cell][I] = factor*vol * sum_q w_q f(x_q) . (R Piola RT0)_I (x_q)
-// (src/feevaluator_h1.jl:342-381; src/assemblypatterns/linearform.jl:181-220)
-// BR -> BDM1 reconstruction coefficients (src/reconstructions.jl:351-379):
-// column 2f = RT0 function of face f, 2f+1 = its linear-moment BDM1 function.
-__device__ __forceinline__ void br_bdm1(const double fv[3], const double nrm[3][2], const double sg[3], double R[9][6]) {
-    const double c[2] = {-1.0 / 12.0, 1.0 / 12.0};
-    for (int i = 0; i < 9; i++)
-        for (int j = 0; j < 6; j++) R[i][j] = 0.0;
-    for (int f = 0; f < 3; f++) {
-        const int nodes[2] = {f, (f + 1) % 3};
-        for (int n = 0; n < 2; n++)
-            for (int k = 0; k < 2; k++) {
-                R[3 * k + nodes[n]][2 * f] = 0.5 * fv[f] * nrm[f][k];
-                R[3 * k + nodes[n]][2 * f + 1] = c[n] * fv[f] * nrm[f][k] * sg[f];
-            }
-        R[6 + f][2 * f] = fv[f];
-    }
-}
 
 // b += factor (f, R v) with R = BR -> RT0 (NR = 3) or BR -> BDM1 (NR = 6):
 // ReconstructionIdentity (src/feevaluator_h1.jl:342-381) with the Piola
 // transform of the H(div) basis (RT0: src/fedefs/hdiv_rt0.jl:67-116,
 // BDM1: src/fedefs/hdiv_bdm1.jl:81-92, 160-172; cell-face signs on the RT0
-// functions only).
+// functions only).  BR -> BDM1 coefficients (src/reconstructions.jl:351-379):
+// |F| n_k / 2 on the RT0 function of the face for both of its nodes, -1/12 and
+// 1/12 |F| n_k sg on its linear-moment function; a bubble has |F| on RT0.
+// The reconstructed fields are linear on the cell, so the six moments
+// M_v = sum_q w_q lambda_v f are all that the data contributes: the product
+// with a target function t is sum_v M_v . A t(vertex v) / det A.  With every
+// local function evaluated at every point from per-thread arrays the kernel
+// took 209 us for BDM1 on 64,800 cells (whole call), now 95 us (FP64 issue: 35
+// operations a point with 12 polynomial terms' evaluation on top).
 template <int NR>
 __global__ void k_br_rhs_cells(int ncells, BrMeshDev m, BrRhs r, double *loc) {
     int cell = blockIdx.x * blockDim.x + threadIdx.x;
@@ -290,55 +280,61 @@ __global__ void k_br_rhs_cells(int ncells, BrMeshDev m, BrRhs r, double *loc) {
         for (int j = 0; j < 2; j++) A[k][j] = X[(j + 1) * 2 + k] - X[k];
     const double det = A[0][0] * A[1][1] - A[0][1] * A[1][0];
     const double vol = fabs(det) / 2.0;
-    double R[9][NR];
-    if constexpr (NR == 3) {
-        br_rt0(fv, nrm, R, false);
-    } else {
-        br_bdm1(fv, nrm, sg, R);
-    }
-    const double *par = r.par + (size_t)(r.group ? r.group[cell] : 0) * r.nt * 5;
-    double lb[9];
-    for (int i = 0; i < 9; i++) lb[i] = 0;
+    const size_t g0 = (size_t)(r.group ? r.group[cell] : 0) * r.nt;
+    const double *par = r.par + g0 * 5;
+    const PolyTerm *term = r.term + g0;
+    double M[3][2] = {};
     for (int q = 0; q < r.nq; q++) {
         const double xi = r.xref[q][0], eta = r.xref[q][1];
-        double rt[NR][2], cf[NR];
-        if constexpr (NR == 3) {
-            rt[0][0] = xi, rt[0][1] = eta - 1;
-            rt[1][0] = xi, rt[1][1] = eta;
-            rt[2][0] = xi - 1, rt[2][1] = eta;
-            for (int j = 0; j < NR; j++) cf[j] = sg[j];
-        } else {
-            rt[0][0] = xi, rt[0][1] = eta - 1;
-            rt[1][0] = 6 * xi, rt[1][1] = 6 - 12 * xi - 6 * eta;
-            rt[2][0] = xi, rt[2][1] = eta;
-            rt[3][0] = -6 * xi, rt[3][1] = 6 * eta;
-            rt[4][0] = xi - 1, rt[4][1] = eta;
-            rt[5][0] = 6 * (xi - 1) + 12 * eta, rt[5][1] = -6 * eta;
-            for (int j = 0; j < NR; j++) cf[j] = (j % 2 == 0) ? sg[j / 2] : 1.0;   // signs on RT0 only
-        }
-        double te[NR][2];
-        for (int j = 0; j < NR; j++)
-            for (int k = 0; k < 2; k++) te[j][k] = (A[k][0] * rt[j][0] + A[k][1] * rt[j][1]) * (cf[j] / det);
         double x[2];
+#pragma unroll
         for (int k = 0; k < 2; k++) x[k] = X[k] + A[k][0] * xi + A[k][1] * eta;
-        double f[2] = {0, 0};
+        double f0 = 0.0, f1 = 0.0;
         for (int t = 0; t < r.nt; t++) {
-            const int c = (int)par[5 * t];
-            double v = par[5 * t + 1];
-            if (par[5 * t + 2] != 0) v *= poly_pow(x[0], par[5 * t + 2]);
-            if (par[5 * t + 3] != 0) v *= poly_pow(x[1], par[5 * t + 3]);
-            f[c] += v;
+            const PolyTerm pt = term[t];
+            double v = poly_factor(pt.coef, x[0], (pt.code >> 4) & 15, par + 5 * t + 2);
+            v = poly_factor(v, x[1], (pt.code >> 8) & 15, par + 5 * t + 3);
+            if ((pt.code & 15) == 0) f0 += v;
+            else f1 += v;
         }
-        for (int i = 0; i < 9; i++) {
-            double cv0 = 0, cv1 = 0;
-            for (int j = 0; j < NR; j++) {
-                cv0 += R[i][j] * te[j][0];
-                cv1 += R[i][j] * te[j][1];
+        const double lam[3] = {r.lam0[q], xi, eta};
+        f0 *= r.w[q], f1 *= r.w[q];
+#pragma unroll
+        for (int v = 0; v < 3; v++) M[v][0] += lam[v] * f0, M[v][1] += lam[v] * f1;
+    }
+    // values of the reference functions at the vertices (0, 0), (1, 0), (0, 1); rows 2f RT0, 2f + 1 BDM1:
+    // (x, y - 1), (6 x, 6 - 12 x - 6 y), (x, y), (-6 x, 6 y), (x - 1, y), (6 (x - 1) + 12 y, -6 y)
+    constexpr double V[6][3][2] = {{{0, -1}, {1, -1}, {0, 0}}, {{0, 6}, {6, -6}, {0, 0}}, {{0, 0}, {1, 0}, {0, 1}},
+                                   {{0, 0}, {-6, 0}, {0, 6}}, {{-1, 0}, {0, 0}, {-1, 1}}, {{-6, 0}, {0, 0}, {6, -6}}};
+    double B[3][2];   // A^T M_v
+#pragma unroll
+    for (int v = 0; v < 3; v++)
+#pragma unroll
+        for (int l = 0; l < 2; l++) B[v][l] = A[0][l] * M[v][0] + A[1][l] * M[v][1];
+    const double idet = 1.0 / det;
+    double lb[9] = {};
+#pragma unroll
+    for (int f = 0; f < 3; f++) {
+        // products of f with the functions of face f; cell-face signs on the RT0 function only
+        double h0 = 0.0, h1 = 0.0;
+#pragma unroll
+        for (int v = 0; v < 3; v++)
+#pragma unroll
+            for (int l = 0; l < 2; l++) {
+                h0 += V[2 * f][v][l] * B[v][l];
+                if (NR == 6) h1 += V[2 * f + 1][v][l] * B[v][l];
             }
-            lb[i] += (f[0] * cv0 + f[1] * cv1) * r.w[q];
-        }
+        h0 *= sg[f] * idet * fv[f];
+        h1 *= sg[f] * idet * fv[f];   // sg: the linear moment's coefficient
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+                lb[3 * k + (f + n) % 3] += nrm[f][k] * (0.5 * h0 + (n ? 1.0 / 12.0 : -1.0 / 12.0) * h1);
+        lb[6 + f] = h0;
     }
     const double itemfactor = r.factor * vol;
+#pragma unroll
     for (int i = 0; i < 9; i++) loc[(size_t)cell * 9 + i] = lb[i] * itemfactor;
 }
 
@@ -551,6 +547,7 @@ int grmp_br_rhs(grmp_space s, const grmp_rhs *rhs, grmp_vector b) {
         r.xref[q][0] = rt->xref[q][0];
         r.xref[q][1] = rt->xref[q][1];
         r.w[q] = rt->w[q];
+        r.lam0[q] = 1.0 - r.xref[q][0] - r.xref[q][1];
     }
     delete rt;
     r.nt = nt;
@@ -558,11 +555,16 @@ int grmp_br_rhs(grmp_space s, const grmp_rhs *rhs, grmp_vector b) {
     double *dpar = nullptr;
     int32_t *dgrp = nullptr;
     rc = grmp_upload(ctx, &dpar, rhs->params, (size_t)rhs->nparams);
+    std::vector<PolyTerm> term((size_t)(ng * nt));
+    for (size_t t = 0; t < term.size(); t++) term[t] = poly_term(rhs->params + 5 * t);
+    PolyTerm *dterm = nullptr;
+    if (!rc) rc = grmp_upload(ctx, &dterm, term.data(), term.size());
     if (!rc && rhs->cell_group) rc = grmp_upload(ctx, &dgrp, rhs->cell_group, (size_t)m->ncells);
     size_t ncl = (size_t)m->ncells * 9;
     if (!rc && !s->d_locbuf) rc = grmp_alloc(ctx, (void **)&s->d_locbuf, ncl * 8);
     if (!rc) {
         r.par = dpar;
+        r.term = dterm;
         r.group = dgrp;
         if (rhs->test_operator == 2)
             k_br_rhs_cells<6><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(m->ncells, br_mesh(m), r, s->d_locbuf);
@@ -577,6 +579,7 @@ int grmp_br_rhs(grmp_space s, const grmp_rhs *rhs, grmp_vector b) {
         if (e != cudaSuccess) rc = grmp_cuda_fail(ctx, e, "H1BR rhs");
     }
     grmp_free(ctx, dpar, (size_t)rhs->nparams * 8);
+    grmp_free(ctx, dterm, term.size() * sizeof(PolyTerm));
     grmp_free(ctx, dgrp, (size_t)m->ncells * 4);
     return rc;
 }

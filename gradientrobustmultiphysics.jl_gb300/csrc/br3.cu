@@ -267,150 +267,133 @@ __global__ void __launch_bounds__(128) k_br3_rows(int32_t nrows, const int32_t *
 }
 
 // ------------------------------------------------------------------ reconstructed rhs (FP64)
-// BR -> BDM1 reconstruction (src/reconstructions.jl:493-535): R phi is the
-// linear vector field whose normal-flux moments against P1 on every face
-// equal those of phi (the functionals the reference's coefficients
-// _P1_INTO_BDM1_COEFFS_3D encode; its orientation-dependent choice of two
-// linear moments per face only selects a basis of the same space).  On face
-// f with vertices V and moments m_a = int_F (phi . n_F) lambda_a, the
-// field's normal components at the face's vertices are
-// s_a = (12 / |F|) (m_a - (m_0 + m_1 + m_2) / 4); its value at vertex i
-// solves n_F . w_i = s over the three faces at i.  W[dof][vertex][component].
-__device__ void br3_bdm1_fields(const double fv[4], const double nrm[4][3], double W[16][4][3]) {
-    for (int dof = 0; dof < 16; dof++) {
-        double s[4][3];
-        for (int f = 0; f < 4; f++) {
-            double m[3] = {0.0, 0.0, 0.0};
-            for (int a = 0; a < 3; a++) {
-                const int va = kFaces3[f][a];
-                if (dof < 12) {
-                    const int k = dof / 4, p = dof % 4;
-                    const bool on = kFaces3[f][0] == p || kFaces3[f][1] == p || kFaces3[f][2] == p;
-                    if (on) m[a] = nrm[f][k] * fv[f] * (va == p ? 2.0 : 1.0) / 12.0;
-                } else if (dof - 12 == f) {
-                    m[a] = (nrm[f][0] * nrm[f][0] + nrm[f][1] * nrm[f][1] + nrm[f][2] * nrm[f][2]) * fv[f] / 3.0;
-                }
-            }
-            const double mean = (m[0] + m[1] + m[2]) / 4.0;
-            for (int a = 0; a < 3; a++) s[f][a] = (12.0 / fv[f]) * (m[a] - mean);
-        }
-        for (int i = 0; i < 4; i++) {
-            double N[3][3], r[3];
-            int row = 0;
-            for (int f = 0; f < 4; f++)
-                for (int a = 0; a < 3; a++)
-                    if (kFaces3[f][a] == i) {
-                        for (int k = 0; k < 3; k++) N[row][k] = nrm[f][k];
-                        r[row++] = s[f][a];
-                    }
-            const double det = N[0][0] * (N[1][1] * N[2][2] - N[1][2] * N[2][1]) -
-                               N[0][1] * (N[1][0] * N[2][2] - N[1][2] * N[2][0]) +
-                               N[0][2] * (N[1][0] * N[2][1] - N[1][1] * N[2][0]);
-            for (int c = 0; c < 3; c++) {   // Cramer's rule
-                double M[3][3];
-                for (int x = 0; x < 3; x++)
-                    for (int y = 0; y < 3; y++) M[x][y] = (y == c) ? r[x] : N[x][y];
-                W[dof][i][c] = (M[0][0] * (M[1][1] * M[2][2] - M[1][2] * M[2][1]) -
-                                M[0][1] * (M[1][0] * M[2][2] - M[1][2] * M[2][0]) +
-                                M[0][2] * (M[1][0] * M[2][1] - M[1][1] * M[2][0])) /
-                               det;
-            }
-        }
-    }
-}
-
 struct Br3Rhs {
     const double *par;   // [ngroups][nt][5] polynomial terms (component, coef, e1, e2, e3)
+    const PolyTerm *term;   // the same, decoded
     const int32_t *group;   // [ncells] group of each cell, or nullptr (one group)
     int nt;
     double factor;
     int bdm1;            // 0: RT0 reconstruction, 1: BDM1
     int nq;
-    double xref[64][3];
+    double xref[64][3], lam0[64];
     double w[64];
 };
 
-// loc[cell][I] = factor*vol * sum_q w_q f(x_q) . (R Piola RT0)_I (x_q)
-// (ReconstructionIdentity, src/feevaluator_h1.jl:342-381)
-__global__ void k_br3_rhs_cells(int ncells, Br3MeshDev m, Br3Rhs r, double *loc) {
+// loc[cell][I] = factor |T| sum_q w_q f(x_q) . (R phi_I)(x_q)
+// (ReconstructionIdentity, src/feevaluator_h1.jl:342-381).  R phi_I is a
+// linear field on the cell, so the twelve moments M_v = sum_q w_q lambda_v f
+// against the barycentric functions are all that the data contributes:
+//
+//   RT0: the function of face j is 2 sg_j / |det A| (x - X_opp(j)), its
+//     product with f h_j = 2 sg_j / |det A| sum_v M_v . (X_v - X_opp(j)), and
+//     loc = R h with the 16 x 4 coefficients (src/reconstructions.jl:474-491).
+//   BDM1 (src/reconstructions.jl:493-535): R phi is the linear field whose
+//     normal-flux moments against P1 on every face equal those of phi (the
+//     functionals that the coefficients _P1_INTO_BDM1_COEFFS_3D encode; their
+//     orientation-dependent choice of two linear moments per face only selects
+//     a basis of the same space).  A P1 field is its own reconstruction:
+//     loc = M_v[k].  The bubble of face f has the normal component |n_f|^2 at
+//     the vertices of f and none on the other faces: its value at vertex v
+//     solves N_v w = |n_f|^2 e_f over the three faces at v, so with
+//     y_v = N_v^-T M_v its product is |n_f|^2 sum_v y_v[f].
+//
+// Bound by FP64 issue (two lanes per clock and SM): about 60 operations a
+// quadrature point and 250 a cell.  Evaluating all 16 fields at every point
+// from per-thread arrays (16 x 4 x 3 doubles in local memory) took 2.69 ms on
+// 82,944 cells with the order-4 rule; the moments take 0.37 ms.
+__global__ void __launch_bounds__(128) k_br3_rhs_cells(int ncells, Br3MeshDev m, Br3Rhs r, double *loc) {
     const int cell = blockIdx.x * blockDim.x + threadIdx.x;
     if (cell >= ncells) return;
     double X[12], nrm[4][3], fv[4], sg[4];
     br3_load(m, cell, X, nrm, fv, sg);
-    double A[3][3], G[3][3], vol;
-    simplex_geometry<3, double>(X, G, vol, A);
-    const double adet = 6.0 * vol;
-    double R[16][4];
-    br3_rt0(fv, nrm, R, false);
-    double lb[16];
-    for (int i = 0; i < 16; i++) lb[i] = 0.0;
-    if (r.bdm1) {
-        double W[16][4][3];
-        br3_bdm1_fields(fv, nrm, W);
-        for (int q = 0; q < r.nq; q++) {
-            const double lam[4] = {1.0 - r.xref[q][0] - r.xref[q][1] - r.xref[q][2], r.xref[q][0], r.xref[q][1],
-                                   r.xref[q][2]};
-            double x[3];
-            for (int k = 0; k < 3; k++) {
-                x[k] = X[k];
-                for (int j = 0; j < 3; j++) x[k] += A[k][j] * r.xref[q][j];
-            }
-            double fq[3] = {0, 0, 0};
-            const double *gpar = r.par + (r.group ? (size_t)r.group[cell] * r.nt * 5 : 0);
-            for (int t = 0; t < r.nt; t++) {
-                const double *pt = gpar + 5 * t;
-                double v = pt[1];
-                for (int j = 0; j < 3; j++)
-                    if (pt[2 + j] != 0) v *= poly_pow(x[j], pt[2 + j]);
-                fq[(int)pt[0]] += v;
-            }
-            for (int i = 0; i < 16; i++) {
-                double t = 0;
-                for (int k = 0; k < 3; k++)
-                    t += fq[k] * (lam[0] * W[i][0][k] + lam[1] * W[i][1][k] + lam[2] * W[i][2][k] +
-                                  lam[3] * W[i][3][k]);
-                lb[i] += t * r.w[q];
-            }
-        }
-        const double itemfactor = r.factor * vol;
-        for (int i = 0; i < 16; i++) loc[(size_t)cell * 16 + i] = lb[i] * itemfactor;
-        return;
-    }
+    double A[3][3];
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) A[k][j] = X[(j + 1) * 3 + k] - X[k];
+    const double det = A[0][0] * (A[1][1] * A[2][2] - A[1][2] * A[2][1]) +
+                       A[0][1] * (A[1][2] * A[2][0] - A[1][0] * A[2][2]) +
+                       A[0][2] * (A[1][0] * A[2][1] - A[1][1] * A[2][0]);
+    const double itemfactor = r.factor * (fabs(det) / 6.0);
+    const size_t g0 = (r.group ? (size_t)r.group[cell] : 0) * r.nt;
+    const double *gpar = r.par + g0 * 5;
+    const PolyTerm *gterm = r.term + g0;
+    double M[4][3] = {};
     for (int q = 0; q < r.nq; q++) {
-        const double x0 = r.xref[q][0], y0 = r.xref[q][1], z0 = r.xref[q][2];
-        const double rt[4][3] = {{2 * x0, 2 * y0, 2 * (z0 - 1)}, {2 * x0, 2 * (y0 - 1), 2 * z0},
-                                 {2 * x0, 2 * y0, 2 * z0}, {2 * (x0 - 1), 2 * y0, 2 * z0}};
-        double te[4][3];
-        for (int j = 0; j < 4; j++)
-            for (int k = 0; k < 3; k++) {
-                double s = 0;
-                for (int l = 0; l < 3; l++) s += A[k][l] * rt[j][l];
-                te[j][k] = s * (sg[j] / adet);
-            }
-        double x[3];
-        for (int k = 0; k < 3; k++) {
-            x[k] = X[k];
-            for (int j = 0; j < 3; j++) x[k] += A[k][j] * r.xref[q][j];
-        }
-        double fq[3] = {0, 0, 0};
-        const double *gpar = r.par + (r.group ? (size_t)r.group[cell] * r.nt * 5 : 0);
+        double x[3], f0 = 0.0, f1 = 0.0, f2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            x[k] = X[k] + A[k][0] * r.xref[q][0] + A[k][1] * r.xref[q][1] + A[k][2] * r.xref[q][2];
         for (int t = 0; t < r.nt; t++) {
-            const double *pt = gpar + 5 * t;
-            double v = pt[1];
-            for (int j = 0; j < 3; j++)
-                if (pt[2 + j] != 0) v *= poly_pow(x[j], pt[2 + j]);
-            fq[(int)pt[0]] += v;
+            const PolyTerm pt = gterm[t];
+            const double *e = gpar + 5 * t + 2;
+            double v = poly_factor(pt.coef, x[0], (pt.code >> 4) & 15, e);
+            v = poly_factor(v, x[1], (pt.code >> 8) & 15, e + 1);
+            v = poly_factor(v, x[2], (pt.code >> 12) & 15, e + 2);
+            const int c = pt.code & 15;
+            if (c == 0) f0 += v;
+            else if (c == 1) f1 += v;
+            else f2 += v;
         }
-        for (int i = 0; i < 16; i++) {
-            double cv[3] = {0, 0, 0};
-            for (int j = 0; j < 4; j++)
-                if (R[i][j] != 0)
-                    for (int k = 0; k < 3; k++) cv[k] += R[i][j] * te[j][k];
-            lb[i] += (fq[0] * cv[0] + fq[1] * cv[1] + fq[2] * cv[2]) * r.w[q];
+        const double lam[4] = {r.lam0[q], r.xref[q][0], r.xref[q][1], r.xref[q][2]};
+        const double g[3] = {f0 * r.w[q], f1 * r.w[q], f2 * r.w[q]};
+#pragma unroll
+        for (int v = 0; v < 4; v++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) M[v][k] += lam[v] * g[k];
+    }
+    double lb[16];
+    constexpr int FV[4][3] = {{0, 1, 2}, {0, 1, 3}, {1, 2, 3}, {0, 2, 3}};   // kFaces3, known to the compiler
+    constexpr int OPP[4] = {3, 2, 0, 1};
+    if (r.bdm1) {
+        constexpr int AT[4][3] = {{0, 1, 3}, {0, 1, 2}, {0, 2, 3}, {1, 2, 3}};   // faces at each vertex
+        double yf[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            // rows n_a, n_b, n_c of N_v: N^-T M = (M . (n_b x n_c), M . (n_c x n_a), M . (n_a x n_b)) / det N
+            double c[3][3];
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                const double *p = nrm[AT[v][(a + 1) % 3]], *q = nrm[AT[v][(a + 2) % 3]];
+                c[a][0] = p[1] * q[2] - p[2] * q[1];
+                c[a][1] = p[2] * q[0] - p[0] * q[2];
+                c[a][2] = p[0] * q[1] - p[1] * q[0];
+            }
+            const double *n0 = nrm[AT[v][0]];
+            const double id = 1.0 / (n0[0] * c[0][0] + n0[1] * c[0][1] + n0[2] * c[0][2]);
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+                yf[AT[v][a]] += (M[v][0] * c[a][0] + M[v][1] * c[a][1] + M[v][2] * c[a][2]) * id;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+#pragma unroll
+            for (int v = 0; v < 4; v++) lb[4 * k + v] = M[v][k];
+#pragma unroll
+        for (int f = 0; f < 4; f++)
+            lb[12 + f] = (nrm[f][0] * nrm[f][0] + nrm[f][1] * nrm[f][1] + nrm[f][2] * nrm[f][2]) * yf[f];
+    } else {
+        const double sc = 2.0 / fabs(det);
+#pragma unroll
+        for (int i = 0; i < 12; i++) lb[i] = 0.0;
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            double h = 0.0;
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) h += M[FV[f][a]][k] * (X[FV[f][a] * 3 + k] - X[OPP[f] * 3 + k]);
+            h *= sc * sg[f] * fv[f];
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) lb[4 * k + FV[f][a]] += (1.0 / 3.0) * nrm[f][k] * h;
+            lb[12 + f] = h;
         }
     }
-    const double itemfactor = r.factor * vol;
-    for (int i = 0; i < 16; i++) loc[(size_t)cell * 16 + i] = lb[i] * itemfactor;
+    double2 *o = reinterpret_cast<double2 *>(loc + (size_t)cell * 16);
+#pragma unroll
+    for (int i = 0; i < 8; i++) o[i] = make_double2(lb[2 * i] * itemfactor, lb[2 * i + 1] * itemfactor);
 }
 
 __global__ void k_gather_rows_br3(int32_t nrows, const int32_t *inc_ptr, const int32_t *inc_cell,
@@ -617,6 +600,7 @@ int grmp_br3_rhs(grmp_space s, const grmp_rhs *rhs, grmp_vector b) {
     r.nq = rt->nq;
     for (int q = 0; q < rt->nq; q++) {
         for (int k = 0; k < 3; k++) r.xref[q][k] = rt->xref[q][k];
+        r.lam0[q] = 1.0 - r.xref[q][0] - r.xref[q][1] - r.xref[q][2];
         r.w[q] = rt->w[q];
     }
     delete rt;
@@ -626,11 +610,16 @@ int grmp_br3_rhs(grmp_space s, const grmp_rhs *rhs, grmp_vector b) {
     double *dpar = nullptr;
     int32_t *dgrp = nullptr;
     rc = grmp_upload(ctx, &dpar, rhs->params, (size_t)rhs->nparams);
+    std::vector<PolyTerm> term((size_t)(ng * nt));
+    for (size_t t = 0; t < term.size(); t++) term[t] = poly_term(rhs->params + 5 * t);
+    PolyTerm *dterm = nullptr;
+    if (!rc) rc = grmp_upload(ctx, &dterm, term.data(), term.size());
     if (!rc && rhs->cell_group) rc = grmp_upload(ctx, &dgrp, rhs->cell_group, (size_t)m->ncells);
     const size_t ncl = (size_t)m->ncells * 16;
     if (!rc && !s->d_locbuf) rc = grmp_alloc(ctx, (void **)&s->d_locbuf, ncl * 8);
     if (!rc) {
         r.par = dpar;
+        r.term = dterm;
         r.group = dgrp;
         k_br3_rhs_cells<<<nblk(m->ncells), TPB, 0, ctx->stream>>>(m->ncells, br3_mesh(m), r, s->d_locbuf);
         GRMP_LAUNCHED(ctx);
@@ -642,6 +631,7 @@ int grmp_br3_rhs(grmp_space s, const grmp_rhs *rhs, grmp_vector b) {
         if (e != cudaSuccess) rc = grmp_cuda_fail(ctx, e, "H1BR{3} rhs");
     }
     grmp_free(ctx, dpar, (size_t)rhs->nparams * 8);
+    grmp_free(ctx, dterm, term.size() * sizeof(PolyTerm));
     grmp_free(ctx, dgrp, (size_t)m->ncells * 4);
     return rc;
 }

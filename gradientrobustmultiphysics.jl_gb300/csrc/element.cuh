@@ -120,6 +120,32 @@ __host__ __device__ __forceinline__ double poly_pow(double x, double e) {
     return pow(x, e);
 }
 
+// A term of a polynomial with small whole exponents: coefficient, component
+// and exponents as integers (FP64 compares and conversions run at the rate of
+// FP64 multiplications, so decoding a term from five doubles costs more than
+// evaluating it).  An exponent of 15 stands for one that is not a whole number
+// of 0..8: pow of the term's exponent in the parameter array.
+struct alignas(16) PolyTerm {
+    double coef;
+    int32_t code;   // component | e1 << 4 | e2 << 8 | e3 << 12
+    int32_t pad;
+};
+inline PolyTerm poly_term(const double *p) {
+    PolyTerm t{p[1], (int32_t)p[0], 0};
+    for (int j = 0; j < 3; j++) {
+        const double e = p[2 + j];
+        t.code |= (e >= 0 && e <= 8 && e == (double)(int)e ? (int)e : 15) << (4 + 4 * j);
+    }
+    return t;
+}
+__device__ __forceinline__ double poly_factor(double v, double x, int e, const double *exact) {
+    if (e == 0) return v;
+    if (e == 15) return v * poly_pow(x, *exact);
+    double r = x;
+    for (int i = 1; i < e; i++) r = r * x;
+    return v * r;
+}
+
 // Data functions of the linear forms and item integrators evaluated on device
 // (constant, per cell, Fourier series, polynomial; grmp_rhs_kind).  f gets
 // r.ncomp values.
