@@ -12,16 +12,14 @@
 //
 // A face couples the DoFs of its two cells, so a matrix with face terms holds
 // the DoFs of the face neighbours of each row's cells (pattern.cu).  Values
-// are added row by row: each row walks its cells in ascending order and their
-// interior faces (a face shared by two of the row's cells is taken once, from
-// the lower cell), evaluates the jumps of its own basis function and of every
-// function of the two cells at the face's quadrature points and adds the
-// products into its CSR entries (deterministic, no atomics).  Quadrature points
+// come face by face into face matrices and are added row by row (deterministic,
+// no atomics).  Quadrature points
 // of a face are placed by barycentric weights over the face's vertices in
 // ascending global vertex order, so both cells see the same points.
 #include "element.cuh"
 #include "grmp_internal.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -92,98 +90,96 @@ __device__ __forceinline__ void face_canon(const int32_t *cells, int cell, int f
         }
 }
 
-// reference coordinates of the point with barycentric weights lam over the
-// face's canonical vertices: reference vertex 0 is the origin, vertex v >= 1
-// the unit vector e_{v-1}
+// end points of the P2 edge functions (h1_p2.jl:134-165)
 template <int DIM>
-__device__ __forceinline__ void face_point(const double *lam, const int loc[DIM], double xh[DIM]) {
-    for (int j = 0; j < DIM; j++) {
-        double s = 0.0;
-        for (int k = 0; k < DIM; k++) s += loc[k] == j + 1 ? lam[k] : 0.0;
-        xh[j] = s;
-    }
+__device__ __forceinline__ int edge_vertex(int e, int k) {
+    if (DIM == 2) return (e + k) % 3;
+    const int t[6][2] = {{0, 1}, {0, 2}, {0, 3}, {1, 2}, {1, 3}, {2, 3}};
+    return t[e][k];
 }
 
-struct Dd {
-    double v, d[3];
-};
-__device__ __forceinline__ Dd dmul(Dd x, Dd y) {
-    Dd r;
-    r.v = x.v * y.v;
-    for (int i = 0; i < 3; i++) r.d[i] = y.v * x.d[i] + x.v * y.d[i];
-    return r;
-}
-__device__ __forceinline__ Dd dscal(double c, Dd x) {
-    Dd r;
-    r.v = c * x.v;
-    for (int i = 0; i < 3; i++) r.d[i] = c * x.d[i];
-    return r;
-}
-__device__ __forceinline__ Dd dsubc(Dd x, double c) {
-    x.v -= c;
-    return x;
-}
-__device__ __forceinline__ Dd dcsub(double c, Dd x) {
-    Dd r;
-    r.v = c - x.v;
-    for (int i = 0; i < 3; i++) r.d[i] = -x.d[i];
-    return r;
-}
-__device__ __forceinline__ Dd dsub(Dd x, Dd y) {
-    Dd r;
-    r.v = x.v - y.v;
-    for (int i = 0; i < 3; i++) r.d[i] = x.d[i] - y.d[i];
-    return r;
-}
-
-// physical gradients of the scalar P1 / P2 basis (h1_p1.jl:64-75,
-// h1_p2.jl:134-165; forward-mode derivative order) at reference point xh
+// gradient of local basis function a at barycentric coordinates lam from the
+// gradients gl of those: grad lam_a (P1); (4 lam_a - 1) grad lam_a at the
+// vertices and 4 (lam_i grad lam_j + lam_j grad lam_i) on the edges (P2)
 template <int DIM, int NB>
-__device__ void basis_grads(const double *xh, const double G[3][3], double g[NB][DIM]) {
-    Dd x[3];
-    for (int j = 0; j < 3; j++) {
-        x[j].v = j < DIM ? xh[j] : 0.0;
-        for (int i = 0; i < 3; i++) x[j].d[i] = i == j ? 1.0 : 0.0;
-    }
-    Dd o[NB];
-    Dd r = dcsub(1.0, x[0]);
-    for (int j = 1; j < DIM; j++) r = dsub(r, x[j]);
-    if constexpr (NB == DIM + 1) {
-        o[0] = r;
-        for (int j = 0; j < DIM; j++) o[1 + j] = x[j];
-    } else if constexpr (DIM == 2) {
-        o[0] = dmul(dscal(2.0, r), dsubc(r, 0.5));
-        o[1] = dmul(dscal(2.0, x[0]), dsubc(x[0], 0.5));
-        o[2] = dmul(dscal(2.0, x[1]), dsubc(x[1], 0.5));
-        o[3] = dmul(dscal(4.0, r), x[0]);
-        o[4] = dmul(dscal(4.0, x[0]), x[1]);
-        o[5] = dmul(dscal(4.0, x[1]), r);
+__device__ __forceinline__ void basis_grad(int a, const double lam[DIM + 1], const double gl[DIM + 1][DIM], double g[DIM]) {
+    if (a <= DIM) {
+        const double c = NB == DIM + 1 ? 1.0 : 4.0 * lam[a] - 1.0;
+#pragma unroll
+        for (int k = 0; k < DIM; k++) g[k] = c * gl[a][k];
     } else {
-        o[0] = dmul(dscal(2.0, r), dsubc(r, 0.5));
-        o[1] = dmul(dscal(2.0, x[0]), dsubc(x[0], 0.5));
-        o[2] = dmul(dscal(2.0, x[1]), dsubc(x[1], 0.5));
-        o[3] = dmul(dscal(2.0, x[2]), dsubc(x[2], 0.5));
-        o[4] = dmul(dscal(4.0, r), x[0]);
-        o[5] = dmul(dscal(4.0, r), x[1]);
-        o[6] = dmul(dscal(4.0, r), x[2]);
-        o[7] = dmul(dscal(4.0, x[0]), x[1]);
-        o[8] = dmul(dscal(4.0, x[0]), x[2]);
-        o[9] = dmul(dscal(4.0, x[1]), x[2]);
+        const int i = edge_vertex<DIM>(a - DIM - 1, 0), j = edge_vertex<DIM>(a - DIM - 1, 1);
+        const double ci = 4.0 * lam[i], cj = 4.0 * lam[j];
+#pragma unroll
+        for (int k = 0; k < DIM; k++) g[k] = ci * gl[j][k] + cj * gl[i][k];
     }
-    for (int a = 0; a < NB; a++)
-        for (int k = 0; k < DIM; k++) {
-            double s = 0.0;
-            for (int j = 0; j < DIM; j++) s += G[k][j] * o[a].d[j];
-            g[a][k] = s;
-        }
+}
+
+// barycentric coordinates in the cell of the point with weights w over the face's canonical vertices
+template <int DIM>
+__device__ __forceinline__ void face_point(const double *w, const int loc[DIM], double lam[DIM + 1]) {
+#pragma unroll
+    for (int v = 0; v <= DIM; v++) {
+        lam[v] = 0.0;
+#pragma unroll
+        for (int k = 0; k < DIM; k++) lam[v] = loc[k] == v ? w[k] : lam[v];
+    }
 }
 
 template <int DIM>
-__device__ __forceinline__ void cell_geometry(const double *coords, const int32_t *cells, int c, double G[3][3]) {
-    double X[(DIM + 1) * DIM], A[3][3], vol;
+__device__ __forceinline__ void cell_grad(const double *coords, const int32_t *cells, int c, double g[DIM + 1][DIM]) {
+    double X[(DIM + 1) * DIM], A[3][3], G[3][3], vol;
+#pragma unroll
     for (int v = 0; v <= DIM; v++)
+#pragma unroll
         for (int k = 0; k < DIM; k++) X[v * DIM + k] = coords[(size_t)cells[(size_t)c * (DIM + 1) + v] * DIM + k];
     simplex_geometry_rn<DIM>(X, A, G, vol);
+#pragma unroll
+    for (int k = 0; k < DIM; k++) {
+        double s = 0.0;
+#pragma unroll
+        for (int j = 0; j < DIM; j++) {
+            g[j + 1][k] = G[k][j];
+            s -= G[k][j];
+        }
+        g[0][k] = s;
+    }
+}
+
+// gradients of the barycentric coordinates of every cell, [cell][vertex][k]:
+// once per cell instead of once per face and side (nine or four FP64 divisions)
+template <int DIM>
+__global__ void k_cell_grads(int ncells, const double *coords, const int32_t *cells, double *gl) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= ncells) return;
+    double g[DIM + 1][DIM];
+    cell_grad<DIM>(coords, cells, c, g);
+#pragma unroll
+    for (int v = 0; v <= DIM; v++)
+#pragma unroll
+        for (int k = 0; k < DIM; k++) gl[((size_t)c * (DIM + 1) + v) * DIM + k] = g[v][k];
+}
+
+// (where memory is short there is no table, gl == nullptr, and they are computed here)
+template <int DIM>
+__device__ __forceinline__ void load_grads(const double *gl, const double *coords, const int32_t *cells, int c,
+                                           double g[DIM + 1][DIM]) {
+    if (!gl) {
+        cell_grad<DIM>(coords, cells, c, g);
+        return;
+    }
+#pragma unroll
+    for (int v = 0; v <= DIM; v++)
+#pragma unroll
+        for (int k = 0; k < DIM; k++) g[v][k] = gl[((size_t)c * (DIM + 1) + v) * DIM + k];
+}
+
+template <int DIM>
+__device__ __forceinline__ int face_in_cell(const int32_t *cell_faces, int c, int F) {
+    int f = 0;
+    for (int g = 0; g <= DIM; g++)
+        if (cell_faces[(size_t)c * (DIM + 1) + g] == F) f = g;
+    return f;
 }
 
 __device__ __forceinline__ double power_of(double x, double p) {
@@ -207,101 +203,186 @@ struct FaceTermDev {
 };
 
 // ------------------------------------------------------------------ face bilinear terms
+// Face matrices, then rows.  k_face_mats: a block takes fb faces; a thread per
+// (face, point) puts the jump of every function of the two cells into shared
+// memory, then a thread per entry i <= j of a face's matrix sums over the
+// points and writes both halves.  The functions are numbered: the lower cell's,
+// then those of the upper cell that the lower one lacks (fcol: their DoFs,
+// fn: their number).  k_face_add: LPR lanes per row, a lane per column, walk
+// the row's cells in ascending order and their interior faces (a face that two
+// cells of the row share comes from the lower one) and add the row of the
+// face's matrix: the same order of additions as adding face by face in one
+// thread, no atomics.
+//
+// Bound by FP64 issue in k_face_mats (45 entries x 2 points x 3 operations a
+// face for P2 triangles) and by the face matrices' write and read (63 MB for
+// 96,840 faces).  A thread per row that evaluated the jumps of both cells again
+// for every (row, face) took 1.58 ms on 129,600 P2 rows; now 134 + 111 us.
 template <int DIM, int NB>
-__global__ void __launch_bounds__(128) k_face_rows(int32_t nrows, const int32_t *inc_ptr, const int32_t *inc_cell,
-                                                   const uint8_t *inc_loc, const int32_t *celldofs,
-                                                   const int32_t *cells, const double *coords,
-                                                   const int32_t *cell_faces, const double *fvol, const int32_t *nbr,
-                                                   const int32_t *rowptr, const int32_t *cols, FaceTermDev t,
-                                                   FaceRule r, double *v64, float *v32, int *missing) {
-    constexpr int NF = DIM + 1, LD = NB;
-    const int row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= nrows) return;
-    const int r0 = rowptr[row], r1 = rowptr[row + 1];
+__global__ void __launch_bounds__(128) k_face_mats(int F0, int nf, int fb, const int32_t *face_cells,
+                                                   const int32_t *cell_faces, const int32_t *cells, const double *coords,
+                                                   const int32_t *celldofs, const double *gl, const double *fvol,
+                                                   FaceTermDev t, FaceRule r, double *mats, int32_t *fcol, int32_t *fn) {
+    constexpr int NC = 2 * NB;
+    extern __shared__ __align__(16) unsigned char fsm[];
+    double *J = reinterpret_cast<double *>(fsm);                      // [fb][nq][NC][DIM]
+    double *sc = J + (size_t)fb * r.nq * NC * DIM;                    // [fb]
+    int *num = reinterpret_cast<int *>(sc + fb), *map = num + fb;     // [fb], [fb][NB] column of the upper cell's function
+    const int base = blockIdx.x * fb, cnt = min(fb, nf - base);
+    __shared__ int nmax;
+    if (threadIdx.x == 0) nmax = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+        const int F = F0 + base + i, c1 = face_cells[2 * (size_t)F], c2 = face_cells[2 * (size_t)F + 1];
+        int n = 0;
+        if (c1 >= 0 && c2 >= 0) {
+            int32_t d1[NB];
+            int32_t *col = fcol + (size_t)(base + i) * NC;
+            n = NB;
+#pragma unroll
+            for (int b = 0; b < NB; b++) col[b] = d1[b] = celldofs[(size_t)c1 * NB + b];
+            for (int b = 0; b < NB; b++) {
+                const int32_t d = celldofs[(size_t)c2 * NB + b];
+                int m = -1;
+#pragma unroll
+                for (int e = 0; e < NB; e++)
+                    if (d1[e] == d) m = e;
+                if (m < 0) {
+                    m = n++;
+                    col[m] = d;
+                }
+                map[i * NB + b] = m;
+            }
+            const double fv = fvol[F];
+            sc[i] = t.factor * fv * power_of(fv, t.power);
+        }
+        num[i] = n;
+        fn[base + i] = n;
+        atomicMax(&nmax, n);
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < cnt * r.nq; w += blockDim.x) {
+        const int i = w / r.nq, q = w - i * r.nq;
+        if (!num[i]) continue;
+        const int F = F0 + base + i;
+        double *Jq = J + (size_t)w * NC * DIM;
+#pragma unroll 1
+        for (int side = 0; side < 2; side++) {
+            const int c = face_cells[2 * (size_t)F + side];
+            int loc[DIM];
+            double lam[DIM + 1], g[DIM + 1][DIM];
+            face_canon<DIM>(cells, c, face_in_cell<DIM>(cell_faces, c, F), loc);
+            face_point<DIM>(r.lam[q], loc, lam);
+            load_grads<DIM>(gl, coords, cells, c, g);
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                double d[DIM];
+                basis_grad<DIM, NB>(b, lam, g, d);
+                const int m = side ? map[i * NB + b] : b;
+#pragma unroll
+                for (int k = 0; k < DIM; k++) {
+                    if (!side) Jq[m * DIM + k] = d[k];
+                    else Jq[m * DIM + k] = m < NB ? Jq[m * DIM + k] - d[k] : -d[k];
+                }
+            }
+        }
+    }
+    __syncthreads();
+    const int NP = max(1, nmax * (nmax + 1) / 2);
+    for (int w = threadIdx.x; w < cnt * NP; w += blockDim.x) {
+        const int i = w / NP, e = w - i * NP, n = num[i];
+        // entry e of the lower triangle, row by row
+        int a = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+        if ((a + 1) * (a + 2) / 2 <= e) a++;
+        if (a * (a + 1) / 2 > e) a--;
+        const int b = e - a * (a + 1) / 2;
+        if (a >= n) continue;
+        const double *Ja = J + (size_t)i * r.nq * NC * DIM + a * DIM, *Jb = Ja + (b - a) * DIM;
+        double s = 0.0;
+        for (int q = 0; q < r.nq; q++, Ja += NC * DIM, Jb += NC * DIM) {
+            double d = 0.0;
+#pragma unroll
+            for (int k = 0; k < DIM; k++) d += Ja[k] * Jb[k];
+            s += r.w[q] * d;
+        }
+        s *= sc[i];
+        double *M = mats + (size_t)(base + i) * NC * NC;
+        M[a * n + b] = s;
+        M[b * n + a] = s;
+    }
+}
+
+template <int DIM, int NB, int LPR>
+__global__ void __launch_bounds__(128) k_face_add(int32_t nrows, int F0, int nf, const int32_t *inc_ptr,
+                                                  const int32_t *inc_cell, const int32_t *cell_faces,
+                                                  const int32_t *nbr, const double *mats, const int32_t *fcol,
+                                                  const int32_t *fn, const int32_t *rowptr, const int32_t *cols,
+                                                  double *v64, float *v32, int *missing) {
+    constexpr int NC = 2 * NB, NF = DIM + 1;
+    static_assert(NC <= LPR, "a lane per column");
+    const long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / LPR;
+    const int lane = threadIdx.x & 31, sub = lane & (LPR - 1), first = lane & ~(LPR - 1);
+    const unsigned mask = (LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1u) << first);
+    if (g >= nrows) return;
+    const int row = (int)g, r0 = rowptr[row], r1 = rowptr[row + 1];
     for (int p = inc_ptr[row]; p < inc_ptr[row + 1]; p++) {
-        const int c = inc_cell[p], a = inc_loc[p];
+        const int c = inc_cell[p];
         for (int f = 0; f < NF; f++) {
             const int c2 = nbr[(size_t)c * NF + f];
             if (c2 < 0) continue;
-            int a2 = -1;
-            for (int b = 0; b < LD; b++)
-                if (celldofs[(size_t)c2 * LD + b] == row) a2 = b;
-            if (a2 >= 0 && c2 < c) continue;   // taken from the lower of the row's two cells
-            const int F = cell_faces[(size_t)c * NF + f];
-            int f2 = 0;
-            for (int g = 0; g < NF; g++)
-                if (cell_faces[(size_t)c2 * NF + g] == F) f2 = g;
-            int loc1[DIM], loc2[DIM];
-            face_canon<DIM>(cells, c, f, loc1);
-            face_canon<DIM>(cells, c2, f2, loc2);
-            double G1[3][3], G2[3][3];
-            cell_geometry<DIM>(coords, cells, c, G1);
-            cell_geometry<DIM>(coords, cells, c2, G2);
-            const double s1 = c < c2 ? 1.0 : -1.0, s2 = -s1;
-            // columns: the DoFs of c, then those of c2 that c lacks
-            int32_t colid[2 * LD];
-            int l1[2 * LD], l2[2 * LD], ncol = 0;
-            for (int b = 0; b < LD; b++) {
-                const int32_t col = celldofs[(size_t)c * LD + b];
-                int b2 = -1;
-                for (int e = 0; e < LD; e++)
-                    if (celldofs[(size_t)c2 * LD + e] == col) b2 = e;
-                colid[ncol] = col, l1[ncol] = b, l2[ncol] = b2, ncol++;
-            }
-            for (int b2 = 0; b2 < LD; b2++) {
-                const int32_t col = celldofs[(size_t)c2 * LD + b2];
-                bool inc1 = false;
-                for (int e = 0; e < LD; e++) inc1 = inc1 || celldofs[(size_t)c * LD + e] == col;
-                if (inc1) continue;
-                colid[ncol] = col, l1[ncol] = -1, l2[ncol] = b2, ncol++;
-            }
-            double acc[2 * LD];
-            for (int k = 0; k < ncol; k++) acc[k] = 0.0;
-            for (int q = 0; q < r.nq; q++) {
-                double xh1[DIM], xh2[DIM], g1[NB][DIM], g2[NB][DIM];
-                face_point<DIM>(r.lam[q], loc1, xh1);
-                face_point<DIM>(r.lam[q], loc2, xh2);
-                basis_grads<DIM, NB>(xh1, G1, g1);
-                basis_grads<DIM, NB>(xh2, G2, g2);
-                double Ji[DIM];
-                for (int k = 0; k < DIM; k++) Ji[k] = s1 * g1[a][k] + (a2 >= 0 ? s2 * g2[a2][k] : 0.0);
-                for (int m = 0; m < ncol; m++) {
-                    double d = 0.0;
-                    for (int k = 0; k < DIM; k++) {
-                        const double Jj = (l1[m] >= 0 ? s1 * g1[l1[m]][k] : 0.0) + (l2[m] >= 0 ? s2 * g2[l2[m]][k] : 0.0);
-                        d += Ji[k] * Jj;
-                    }
-                    acc[m] += r.w[q] * d;
-                }
-            }
-            const double fv = fvol[F];
-            const double scale = t.factor * fv * power_of(fv, t.power);
-            for (int m = 0; m < ncol; m++) {
+            const int i = cell_faces[(size_t)c * NF + f] - F0;
+            if (i < 0 || i >= nf) continue;
+            const int n = fn[i];
+            const int32_t col = sub < n ? fcol[(size_t)i * NC + sub] : -1;
+            const unsigned own = __ballot_sync(mask, col == row);
+            const int a = __ffs(own >> first) - 1;
+            if (c2 < c && a < NB) continue;   // taken from the lower of the row's two cells
+            if (col >= 0) {
                 int lo = r0, hi = r1;
                 while (lo < hi) {
                     const int mid = (lo + hi) >> 1;
-                    if (cols[mid] < colid[m]) lo = mid + 1;
+                    if (cols[mid] < col) lo = mid + 1;
                     else hi = mid;
                 }
-                if (lo >= r1 || cols[lo] != colid[m]) {
+                if (lo >= r1 || cols[lo] != col) {
                     atomicExch(missing, 1);
-                    continue;
+                } else {
+                    const double v = mats[(size_t)i * NC * NC + a * n + sub];
+                    v64[lo] += v;
+                    if (v32) v32[lo] += (float)v;
                 }
-                const double v = acc[m] * scale;
-                v64[lo] += v;
-                if (v32) v32[lo] += (float)v;
             }
+            __syncwarp(mask);   // the next face may meet the same entries from other lanes
         }
     }
 }
 
 // ------------------------------------------------------------------ jump integrator
+// coefficients of the barycentric gradients in the gradient of a P1 / P2 function
 template <int DIM, int NB>
-__global__ void k_face_jumps(int32_t nfaces, const int32_t *face_cells, const int32_t *cell_faces,
-                             const int32_t *cells, const double *coords, const int32_t *celldofs, const double *u,
-                             const double *fnormals, const double *fvol, int kind, double power, double factor,
-                             FaceRule r, double *out) {
-    constexpr int NF = DIM + 1, LD = NB;
+__device__ __forceinline__ void grad_coefs(const double u[NB], const double lam[DIM + 1], double cf[DIM + 1]) {
+#pragma unroll
+    for (int v = 0; v <= DIM; v++) cf[v] = NB == DIM + 1 ? u[v] : u[v] * (4.0 * lam[v] - 1.0);
+    if constexpr (NB > DIM + 1) {
+#pragma unroll
+        for (int e = 0; e < NB - DIM - 1; e++) {
+            const int i = edge_vertex<DIM>(e, 0), j = edge_vertex<DIM>(e, 1);
+            cf[j] += u[DIM + 1 + e] * (4.0 * lam[i]);
+            cf[i] += u[DIM + 1 + e] * (4.0 * lam[j]);
+        }
+    }
+}
+
+// A thread per face; grad u = sum_v cf_v grad lam_v on either side.  With the
+// derivative of every basis function at every point and the geometry of both
+// cells taken per face it was 130 us for 97,200 faces (P2, two points), now
+// 38 us; bound by FP64 issue.
+template <int DIM, int NB>
+__global__ void __launch_bounds__(128) k_face_jumps(int32_t nfaces, const int32_t *face_cells, const int32_t *cell_faces,
+                                                    const int32_t *cells, const double *coords, const double *gl,
+                                                    const int32_t *celldofs,
+                                                    const double *u, const double *fnormals, const double *fvol,
+                                                    int kind, double power, double factor, FaceRule r, double *out) {
     const int F = blockIdx.x * blockDim.x + threadIdx.x;
     if (F >= nfaces) return;
     const int c1 = face_cells[2 * (size_t)F], c2 = face_cells[2 * (size_t)F + 1];
@@ -309,37 +390,43 @@ __global__ void k_face_jumps(int32_t nfaces, const int32_t *face_cells, const in
         out[F] = 0.0;
         return;
     }
-    int f1 = 0, f2 = 0;
-    for (int g = 0; g < NF; g++) {
-        if (cell_faces[(size_t)c1 * NF + g] == F) f1 = g;
-        if (cell_faces[(size_t)c2 * NF + g] == F) f2 = g;
-    }
     int loc1[DIM], loc2[DIM];
-    face_canon<DIM>(cells, c1, f1, loc1);
-    face_canon<DIM>(cells, c2, f2, loc2);
-    double G1[3][3], G2[3][3];
-    cell_geometry<DIM>(coords, cells, c1, G1);
-    cell_geometry<DIM>(coords, cells, c2, G2);
+    face_canon<DIM>(cells, c1, face_in_cell<DIM>(cell_faces, c1, F), loc1);
+    face_canon<DIM>(cells, c2, face_in_cell<DIM>(cell_faces, c2, F), loc2);
+    double g1[DIM + 1][DIM], g2[DIM + 1][DIM], u1[NB], u2[NB];
+    load_grads<DIM>(gl, coords, cells, c1, g1);
+    load_grads<DIM>(gl, coords, cells, c2, g2);
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+        u1[b] = u[celldofs[(size_t)c1 * NB + b]];
+        u2[b] = u[celldofs[(size_t)c2 * NB + b]];
+    }
     double acc = 0.0;
     for (int q = 0; q < r.nq; q++) {
-        double xh1[DIM], xh2[DIM], g1[NB][DIM], g2[NB][DIM];
-        face_point<DIM>(r.lam[q], loc1, xh1);
-        face_point<DIM>(r.lam[q], loc2, xh2);
-        basis_grads<DIM, NB>(xh1, G1, g1);
-        basis_grads<DIM, NB>(xh2, G2, g2);
+        double lam[DIM + 1], a1[DIM + 1], a2[DIM + 1];
+        face_point<DIM>(r.lam[q], loc1, lam);
+        grad_coefs<DIM, NB>(u1, lam, a1);
+        face_point<DIM>(r.lam[q], loc2, lam);
+        grad_coefs<DIM, NB>(u2, lam, a2);
         double J[DIM];
-        for (int k = 0; k < DIM; k++) J[k] = 0.0;
-        for (int b = 0; b < LD; b++) {
-            const double u1 = u[celldofs[(size_t)c1 * LD + b]], u2 = u[celldofs[(size_t)c2 * LD + b]];
-            for (int k = 0; k < DIM; k++) J[k] += u1 * g1[b][k] - u2 * g2[b][k];
+#pragma unroll
+        for (int k = 0; k < DIM; k++) {
+            double p = 0.0, m = 0.0;
+#pragma unroll
+            for (int v = 0; v <= DIM; v++) {
+                p += a1[v] * g1[v][k];
+                m += a2[v] * g2[v][k];
+            }
+            J[k] = p - m;
         }
-        double val;
+        double val = 0.0;
         if (kind == 1) {
             double jn = 0.0;
+#pragma unroll
             for (int k = 0; k < DIM; k++) jn += J[k] * fnormals[(size_t)F * DIM + k];
             val = jn * jn;
         } else {
-            val = 0.0;
+#pragma unroll
             for (int k = 0; k < DIM; k++) val += J[k] * J[k];
         }
         acc += r.w[q] * val;
@@ -347,6 +434,23 @@ __global__ void k_face_jumps(int32_t nfaces, const int32_t *face_cells, const in
     const double fv = fvol[F];
     out[F] = acc * power_of(fv, power) * fv * factor;
 }
+
+// the table, or nullptr where it does not fit
+double *cell_grads(grmp_mesh m) {
+    grmp_context ctx = m->ctx;
+    double *gl = nullptr;
+    if (grmp_alloc(ctx, (void **)&gl, (size_t)m->ncells * (m->dim + 1) * m->dim * 8)) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (m->dim == 2) k_cell_grads<2><<<nblk(m->ncells, 128), 128, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, gl);
+    else k_cell_grads<3><<<nblk(m->ncells, 128), 128, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, gl);
+    ctx->launches++;
+    return gl;
+}
+
+// face matrices in flight: a chunk of faces at a time where all would take more
+constexpr size_t kFaceBytes = (size_t)512 << 20;
 
 // rule on the face's reference element (edge or triangle) as barycentric weights
 int face_rule(grmp_context ctx, int dim, int order, FaceRule *r) {
@@ -429,6 +533,31 @@ int grmp_face_assemble(grmp_matrix A, int nterms, const grmp_bilinear_term *term
     rc = grmp_alloc(ctx, (void **)&dmiss, 4);
     if (rc) return rc;
     cudaMemsetAsync(dmiss, 0, 4, ctx->stream);
+    // scratch: gradients of the cells, matrices and columns of a chunk of faces (halved until it fits)
+    double *gl = nullptr, *mats = nullptr;
+    int32_t *fcol = nullptr, *fn = nullptr;
+    const int nc = 2 * s->nb;
+    const size_t per = (size_t)nc * nc * 8;
+    int chunk = (int)std::min<size_t>((size_t)m->nfaces, kFaceBytes / per);
+    gl = cell_grads(m);
+    // matrices, columns and numbers of a chunk in one piece
+    while ((rc = grmp_alloc(ctx, (void **)&mats, (size_t)chunk * (per + nc * 4 + 4))) && chunk > 32) {
+        cudaGetLastError();
+        chunk = (chunk + 1) / 2;
+    }
+    if (!rc) {
+        fcol = reinterpret_cast<int32_t *>(mats + (size_t)chunk * nc * nc);
+        fn = fcol + (size_t)chunk * nc;
+    }
+    auto release = [&]() {
+        grmp_free(ctx, dmiss, 4);
+        grmp_free(ctx, gl, (size_t)m->ncells * (dim + 1) * dim * 8);
+        grmp_free(ctx, mats, (size_t)chunk * (per + nc * 4 + 4));
+    };
+    if (rc) {
+        release();
+        return rc;
+    }
     double *v64 = precision != GRMP_FP32 ? A->d_vals64 : nullptr;
     float *v32 = precision != GRMP_FP64 ? A->d_vals32 : nullptr;
     const int p = grmp_fe_polyorder(s->fe, dim);
@@ -448,23 +577,32 @@ int grmp_face_assemble(grmp_matrix A, int nterms, const grmp_bilinear_term *term
             rc = grmp_fail(ctx, GRMP_ERR_UNSUPPORTED, "face terms: FP64 values are required (use FP64 or FP64_FP32)");
             break;
         }
-        auto go = [&](auto kern) {
-            kern<<<nblk(A->nrows, 128), 128, 0, ctx->stream>>>(A->nrows, s->d_inc_ptr, s->d_inc_cell, s->d_inc_loc,
-                                                               s->d_celldofs, m->d_cells, m->d_coords, m->d_cell_faces,
-                                                               m->d_face_volumes, m->d_cell_nbr, A->d_rowptr,
-                                                               A->d_cols, t, r, w64, w32, dmiss);
+        auto go = [&](auto mat, auto add, int nb, int lpr) {
+            const int nc = 2 * nb;
+            const size_t fsm = ((size_t)r.nq * nc * dim + 1) * 8 + (1 + nb) * 4;
+            const int fb = (int)std::max<size_t>(1, std::min<size_t>(32, (size_t)46 * 1024 / fsm));
+            for (int F0 = 0; F0 < m->nfaces; F0 += chunk) {
+                const int nf = std::min(chunk, m->nfaces - F0);
+                mat<<<nblk(nf, fb), 128, fb * fsm + 8, ctx->stream>>>(F0, nf, fb, m->d_face_cells, m->d_cell_faces,
+                                                                      m->d_cells, m->d_coords, s->d_celldofs, gl, m->d_face_volumes,
+                                                                      t, r, mats, fcol, fn);
+                GRMP_LAUNCHED(ctx);
+                add<<<nblk((long long)A->nrows * lpr, 128), 128, 0, ctx->stream>>>(
+                    A->nrows, F0, nf, s->d_inc_ptr, s->d_inc_cell, m->d_cell_faces, m->d_cell_nbr, mats, fcol, fn,
+                    A->d_rowptr, A->d_cols, w64, w32, dmiss);
+                GRMP_LAUNCHED(ctx);
+            }
         };
-        if (dim == 2 && s->nb == 3) go(k_face_rows<2, 3>);
-        else if (dim == 2 && s->nb == 6) go(k_face_rows<2, 6>);
-        else if (dim == 3 && s->nb == 4) go(k_face_rows<3, 4>);
-        else go(k_face_rows<3, 10>);
-        GRMP_LAUNCHED(ctx);
+        if (dim == 2 && s->nb == 3) go(k_face_mats<2, 3>, k_face_add<2, 3, 8>, 3, 8);
+        else if (dim == 2 && s->nb == 6) go(k_face_mats<2, 6>, k_face_add<2, 6, 16>, 6, 16);
+        else if (dim == 3 && s->nb == 4) go(k_face_mats<3, 4>, k_face_add<3, 4, 8>, 4, 8);
+        else go(k_face_mats<3, 10>, k_face_add<3, 10, 32>, 10, 32);
     }
     int hmiss = 0;
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(&hmiss, dmiss, 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    grmp_free(ctx, dmiss, 4);
+    release();
     if (!rc && e != cudaSuccess) rc = grmp_cuda_fail(ctx, e, "face terms");
     if (!rc && hmiss)
         rc = grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "face terms: the pattern lacks face couplings (build it with the face terms)");
@@ -492,9 +630,11 @@ extern "C" int grmp_item_face_jumps(grmp_space s, grmp_vector u, int kind, doubl
     double *dout = nullptr;
     rc = grmp_alloc(ctx, (void **)&dout, (size_t)m->nfaces * 8);
     if (rc) return rc;
+    double *gl = cell_grads(m);
+    const size_t glb = (size_t)m->ncells * (dim + 1) * dim * 8;
     auto go = [&](auto kern) {
-        kern<<<nblk(m->nfaces), TPB, 0, ctx->stream>>>(m->nfaces, m->d_face_cells, m->d_cell_faces, m->d_cells,
-                                                       m->d_coords, s->d_celldofs, u->d, m->d_face_normals,
+        kern<<<nblk(m->nfaces, 128), 128, 0, ctx->stream>>>(m->nfaces, m->d_face_cells, m->d_cell_faces, m->d_cells, m->d_coords, gl,
+                                                       s->d_celldofs, u->d, m->d_face_normals,
                                                        m->d_face_volumes, kind, power, factor, r, dout);
     };
     if (dim == 2 && s->nb == 3) go(k_face_jumps<2, 3>);
@@ -507,6 +647,7 @@ extern "C" int grmp_item_face_jumps(grmp_space s, grmp_vector u, int kind, doubl
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), dout, h.size() * 8, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     grmp_free(ctx, dout, (size_t)m->nfaces * 8);
+    grmp_free(ctx, gl, glb);
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "face jumps");
     double sum = 0.0;   // ascending face order (evaluate!, itemintegrator.jl:314-330)
     for (double v : h) sum += v;
