@@ -5,13 +5,21 @@
 // spmv_config reported by a solve that the multilevel preconditioner ran
 // (plus the row-loop code of its SpMV, e.g. 90404)
 constexpr int kMgConfig = 90000;
+// rows of a Jacobian from which BiCGStab takes the cycle
+constexpr int kMgBicgRows = 0;
 
 // Whether grmp_solve takes the multilevel solver for this matrix (scalar
 // H1P1 / H1P2 with a diffusion term, not reaction dominated); builds or
 // refreshes what it needs.  *use = 0: the Jacobi solvers.
-int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use);
+// `least`: rows below which it is not taken (besides the rule by element).
+int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, int least = 0);
 // Jacobi-free conjugate gradients with the prepared hierarchy; allocates nothing.
 int grmp_mg_solve(grmp_matrix A, const double *b, double *x, const grmp_solve_params *p, grmp_solve_stats *st);
+// BiCGStab with the prepared FP64 hierarchy for the scalar Jacobian of a Newton
+// step; vec: nine vectors of the matrix's rows.  *done = false: it did not
+// converge and x is as it was.
+int grmp_mg_bicgstab(grmp_matrix A, const double *b, double *x, const grmp_solve_params *p, double *const vec[9],
+                     double *partial, void *state, grmp_solve_stats *st, bool *done);
 // Whether a hierarchy with numeric storage of this precision exists.
 bool grmp_mg_ready(grmp_matrix A, bool mixed);
 void grmp_mg_free(grmp_matrix A);

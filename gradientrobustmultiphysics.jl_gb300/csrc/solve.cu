@@ -1973,6 +1973,18 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
     SolveState *dst = (SolveState *)(work + off_state);
     WorkLayout lay{vec, off_r64, off_part};
     cudaMemsetAsync(dst, 0, sizeof(SolveState), ctx->stream);
+    if (bicg) {   // scalar Jacobians: multilevel, else (and where that fails) Jacobi
+        int use = 0;
+        int rc = grmp_mg_prepare(A, false, &use, kMgBicgRows);
+        if (rc) return rc;
+        if (use) {
+            double *vv[9];
+            for (int k = 0; k < 9; k++) vv[k] = (double *)(work + (size_t)k * vec);
+            bool done = false;
+            rc = grmp_mg_bicgstab(A, b->d, x->d, p, vv, (double *)(work + off_part), dst, st, &done);
+            if (rc || done) return rc;
+        }
+    }
     // Jacobi preconditioner (not for the Jacobi-scaled configurations, which
     // form and check their own row scales)
     const int known = p->spmv_config != 0 ? p->spmv_config : (mixed ? A->tuned_cfg32 : A->tuned_cfg);
