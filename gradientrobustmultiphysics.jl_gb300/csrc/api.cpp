@@ -1,5 +1,6 @@
 // C-ABI entry points: contexts, meshes, spaces, vectors and the thin
 // wrappers around the pattern / assembly / solve implementations.
+#include <cstring>
 #include <cstdarg>
 #include <new>
 
@@ -47,6 +48,14 @@ void grmp_free(grmp_context ctx, void *p, size_t bytes) {
     ctx->in_use -= bytes;
 }
 
+cudaError_t grmp_readback(grmp_context ctx, void *host, const void *dev, size_t bytes) {
+    void *to = ctx->pin && bytes <= kPinBytes ? ctx->pin : host;
+    cudaError_t e = cudaMemcpyAsync(to, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess && to != host) std::memcpy(host, to, bytes);
+    return e;
+}
+
 extern "C" {
 
 int grmp_version(void) { return 10000; }
@@ -75,6 +84,10 @@ int grmp_create_context(int device, size_t hbm_budget_bytes, grmp_context *out) 
         uint64_t thr = UINT64_MAX;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
+    if (cudaHostAlloc(&c->pin, kPinBytes, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        c->pin = nullptr;
+    }
     *out = c;
     return GRMP_OK;
 }
@@ -84,6 +97,7 @@ int grmp_destroy_context(grmp_context ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);
+    if (ctx->pin) cudaFreeHost(ctx->pin);
     delete ctx;
     return GRMP_OK;
 }

@@ -1071,16 +1071,15 @@ int mg_probe(grmp_matrix A, double *react) {
     grmp_context ctx = A->space->mesh->ctx;
     MgCache &C = *A->mg;
     MgCache::Num &N = C.num[sizeof(T) == 8 ? 0 : 1];
-    const int n = A->nrows, grid = std::max(1, std::min(nblk(n, kTB / kCl), 4 * ctx->num_sms));
+    const int n = A->nrows, grid = std::max(1, std::min({nblk(n, kTB / kCl), 4 * ctx->num_sms, 2048}));
     cudaMemsetAsync(N.bad, 0, 4, ctx->stream);
     k_mg_rows<T><<<grid, kTB, 0, ctx->stream>>>(n, A->d_rowptr, A->d_cols, fine_values<T>(A), (T *)N.D[0],
                                                 (uint8_t *)N.iso[0], (double2 *)N.part, N.bad);
     GRMP_LAUNCHED(ctx);
-    double h[2 * 4096];
+    double h[2 * 2048];
     int bad = 0;
-    cudaError_t e = cudaMemcpyAsync(h, N.part, (size_t)grid * 16, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, N.bad, 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    cudaError_t e = grmp_readback(ctx, h, N.part, (size_t)grid * 16);
+    if (e == cudaSuccess) e = grmp_readback(ctx, &bad, N.bad, 4);
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multilevel: diagonal");
     if (bad) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "solve: non-positive or non-finite diagonal entry");
     double s = 0, d = 0;
@@ -1356,8 +1355,7 @@ int grmp_mg_solve(grmp_matrix A, const double *b, double *x, const grmp_solve_pa
     }
     cudaEventRecord(e1, ctx->stream);
     SolveState hs;
-    cudaError_t e = rc ? cudaSuccess : cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream);
-    if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    cudaError_t e = rc ? cudaSuccess : grmp_readback(ctx, &hs, dst, sizeof(hs));
     float ms = 0;
     if (!rc && e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1394,8 +1392,7 @@ int grmp_mg_bicgstab(grmp_matrix A, const double *b, double *x, const grmp_solve
                       : mg_launch_bicg<4, 4, true>(A, b, x, p, vec, partial, dst, &grid);
     cudaEventRecord(e1, ctx->stream);
     SolveState hs;
-    cudaError_t e = rc ? cudaSuccess : cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream);
-    if (!rc && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    cudaError_t e = rc ? cudaSuccess : grmp_readback(ctx, &hs, dst, sizeof(hs));
     float ms = 0;
     if (!rc && e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);

@@ -1351,8 +1351,7 @@ int ensure_duo_scaled(grmp_matrix A) {
             (float2 *)A->d_duo_sval);
         GRMP_LAUNCHED(ctx);
         int hbad = 0;
-        cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, ctx->stream);
-        cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        cudaError_t e = grmp_readback(ctx, &hbad, bad, 4);
         grmp_free(ctx, bad, 4);
         if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "scaled duo values");
         if (hbad) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "solve: non-positive or non-finite diagonal entry");
@@ -1527,8 +1526,7 @@ int launch_pcg(grmp_matrix A, const double *bvec, double *xvec, const grmp_solve
         cudaEventRecord(e1, ctx->stream);
     }
     SolveState hs;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) e = grmp_readback(ctx, &hs, dst, sizeof(hs));
     float ms = 0;
     if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1600,8 +1598,7 @@ int launch_pcg_staged(grmp_matrix A, const double *bvec, double *xvec, const grm
     GRMP_LAUNCHED(ctx);
     cudaEventRecord(e1, ctx->stream);
     SolveState hs;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) e = grmp_readback(ctx, &hs, dst, sizeof(hs));
     float ms = 0;
     if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1661,8 +1658,7 @@ int launch_pcg_duo(grmp_matrix A, const double *bvec, double *xvec, const grmp_s
     cudaEventRecord(e1, ctx->stream);
     SolveState hs;
     std::memset(&hs, 0, sizeof(hs));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) e = grmp_readback(ctx, &hs, dst, sizeof(hs));
     float ms = 0;
     if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1757,8 +1753,7 @@ int launch_pcg_duo_keep(grmp_matrix A, const double *bvec, double *xvec, const g
     cudaEventRecord(e1, ctx->stream);
     SolveState hs;
     std::memset(&hs, 0, sizeof(hs));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) e = grmp_readback(ctx, &hs, dst, sizeof(hs));
     float ms = 0;
     if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -1903,8 +1898,7 @@ int launch_bicgstab_t(grmp_matrix A, const double *bvec, double *xvec, const grm
     GRMP_LAUNCHED(ctx);
     cudaEventRecord(e1, ctx->stream);
     SolveState hs;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) e = grmp_readback(ctx, &hs, dst, sizeof(hs));
     float ms = 0;
     if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
@@ -2000,8 +1994,7 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
                                                              bad);
         GRMP_LAUNCHED(ctx);
         int hbad = 0;
-        cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, ctx->stream);
-        cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        cudaError_t e = grmp_readback(ctx, &hbad, bad, 4);
         grmp_free(ctx, bad, 4);
         if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "jacobi diagonal");
         if (hbad) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "solve: non-positive or non-finite diagonal entry");
@@ -2103,8 +2096,7 @@ extern "C" int grmp_selftest_wait_timeout(grmp_context ctx, int64_t polls, int32
     GRMP_LAUNCHED(ctx);
     Words h;
     std::memset(&h, 0, sizeof(h));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) e = grmp_readback(ctx, &h, d, sizeof(h));
     grmp_free(ctx, d, sizeof(Words));
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "wait self-test launch");
     *grid_status = h.grid_status;
@@ -2217,8 +2209,7 @@ extern "C" int grmp_solve_fp64_noalloc(grmp_matrix A, grmp_vector b, grmp_vector
         e = cudaGetLastError();
     }
     int hbad = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) e = grmp_readback(ctx, &hbad, bad, 4);
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "noalloc solve: jacobi diagonal");
     if (hbad) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "noalloc solve: non-positive or non-finite diagonal entry");
     // spmv_config 0 takes grmp_solve's tuned configuration and grid when there are
@@ -2249,8 +2240,7 @@ extern "C" int grmp_solve_fp64_noalloc(grmp_matrix A, grmp_vector b, grmp_vector
     }
     SolveState hs;
     std::memset(&hs, 0, sizeof(hs));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) e = grmp_readback(ctx, &hs, dst, sizeof(hs));
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "noalloc solve: persistent PCG launch");
     st->status = hs.status;
     st->iterations = hs.iters;
