@@ -107,7 +107,7 @@ struct MgDev {
 // row sums and diagonals of the rows away from eliminated DoFs, bad diagonals
 template <typename T>
 __global__ void __launch_bounds__(kTB) k_mg_rows(int n, const int32_t *rp, const int32_t *ci, const T *v, T *D,
-                                                 uint8_t *iso, double2 *part, int *bad) {
+                                                 uint8_t *iso, const uint8_t *fixed, double2 *part, int *bad) {
     __shared__ double sh[32 * 2];
     const int lane = threadIdx.x & (kCl - 1);
     double s0 = 0.0, s1 = 0.0;
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kTB) k_mg_rows(int n, const int32_t *rp, const
                 if (ci[k] == i) d = a;
                 else {
                     off += fabs(a);
-                    zero |= a == T(0);
+                    if (a == T(0) && fixed) zero |= fixed[ci[k]];   // an eliminated coupling
                 }
             }
         for (int o = kCl / 2; o > 0; o >>= 1) {
@@ -164,21 +164,26 @@ __global__ void k_mg_prol_geo(int n, const int32_t *prp, const int32_t *pci, con
     ellv[i] = Pair<T>{w[0], w[1]};
 }
 
-// P = (I - w D A) P_agg
-template <typename T>
+// P = (I - w D A) P_agg, L lanes a row (1 on long levels; 16 on short ones,
+// whose rows hold hundreds of entries: 3,000 rows 57 us with one lane)
+template <typename T, int L>
 __global__ void k_mg_prol_agg(int n, const int32_t *rp, const int32_t *ci, const T *v, const T *D, const uint8_t *iso,
                               const int32_t *agg, const int32_t *prp, const int32_t *pci, T *pv) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int kb = rp[i], ke = rp[i + 1], own = agg[i];
-    const bool lone = iso[i];
-    const T w = (T)kProlong * D[i];
-    for (int q = prp[i]; q < prp[i + 1]; q++) {
-        const int t = pci[q];
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / L, lane = threadIdx.x & (L - 1);
+    const bool in = i < n;   // whole warps take part in the shuffles
+    const int kb = in ? rp[i] : 0, ke = in ? rp[i + 1] : 0, own = in ? agg[i] : -1;
+    const bool lone = in && iso[i];
+    const T w = in ? (T)kProlong * D[i] : T(0);
+    const int q0 = in ? prp[i] : 0;
+    int nq = in ? prp[i + 1] - q0 : 0;
+    if (L > 1) nq = __reduce_max_sync(0xffffffffu, nq);
+    for (int q = q0; q < q0 + nq; q++) {
+        const int t = in && q < prp[i + 1] ? pci[q] : -1;
         T s = 0;
-        for (int k = kb; k < ke; k++)
+        for (int k = kb + lane; k < ke; k += L)
             if (agg[ci[k]] == t) s += v[k];
-        pv[q] = lone ? T(0) : (t == own ? T(1) : T(0)) - w * s;
+        for (int o = L / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0 && t >= 0) pv[q] = lone ? T(0) : (t == own ? T(1) : T(0)) - w * s;
     }
 }
 
@@ -357,6 +362,67 @@ __global__ void __launch_bounds__(kTB) k_mg_rap(int nc, const int32_t *__restric
     }
 }
 
+// The two products on short levels: a block per result row.  Its entries are
+// many (aggregates of hundreds of rows) and the rows few, so one group of
+// lanes a row is a serial chain on a few SMs (61^3 P1, levels of 779 and 16
+// rows: P^T A P 283 and 240 us, A P 63 and 47).  32 groups of 8 lanes take
+// the factor rows in turn into accumulators of their own in shared memory,
+// summed in the groups' order.  RAP = false: A P; true: P^T (A P), with the
+// lumping and the identity rows of k_mg_rap.
+constexpr int kWideG = 32;
+template <typename T, bool RAP>
+__global__ void __launch_bounds__(kTB) k_mg_wide(const int32_t *__restrict__ lrp, const int32_t *__restrict__ lci, const int32_t *__restrict__ lperm,
+                                                 const T *__restrict__ lv, const int32_t *__restrict__ frp,
+                                                 const int32_t *__restrict__ fci, const T *__restrict__ fv,
+                                                 const int32_t *__restrict__ orp, const int32_t *__restrict__ oci, T *ov) {
+    constexpr int L = kTB / kWideG;
+    extern __shared__ __align__(16) unsigned char wsm[];
+    T *acc = reinterpret_cast<T *>(wsm);   // [kWideG][nt], then the row's columns
+    __shared__ T slump[kWideG];
+    __shared__ int sany;
+    const int I = blockIdx.x, lane = threadIdx.x & (L - 1), g = threadIdx.x / L;
+    const int t0 = orp[I], nt = orp[I + 1] - t0, kb = lrp[I], m = lrp[I + 1] - kb;
+    int32_t *cols = reinterpret_cast<int32_t *>(acc + kWideG * nt);
+    for (int t = threadIdx.x; t < nt; t += kTB) cols[t] = oci[t0 + t];
+    for (int t = threadIdx.x; t < kWideG * nt; t += kTB) acc[t] = T(0);
+    if (threadIdx.x == 0) sany = 0;
+    __syncthreads();
+    T *mine = acc + g * nt;
+    T lump = 0;
+    const unsigned mask = ((1u << L) - 1u) << (threadIdx.x & 31 & ~(L - 1));
+    for (int k = g; k < m; k += kWideG) {
+        const int j = lci[kb + k];
+        const T w = lv[RAP ? lperm[kb + k] : kb + k];
+        const int b = frp[j], ln = RAP && w == T(0) ? 0 : frp[j + 1] - b;
+        for (int q = lane; q < ln; q += L) {
+            const int s = mg_find(cols, nt, fci[b + q]);
+            const T x = w * fv[b + q];
+            if (s >= 0) mine[s] += x;
+            else lump += x;
+        }
+        __syncwarp(mask);
+    }
+    if (RAP) {
+        for (int o = L / 2; o > 0; o >>= 1) lump += __shfl_xor_sync(0xffffffffu, lump, o);
+        if (lane == 0) slump[g] = lump;
+    }
+    __syncthreads();
+    bool any = false;
+    for (int t = threadIdx.x; t < nt; t += kTB) {
+        T s = 0;
+        for (int q = 0; q < kWideG; q++) s += acc[q * nt + t];
+        any = any || s != T(0);
+        if (RAP) acc[t] = s;   // this thread's column of group 0: read by nobody else
+        else ov[t0 + t] = s;
+    }
+    if (!RAP) return;
+    if (any) sany = 1;
+    __syncthreads();
+    T all = 0;
+    for (int q = 0; q < kWideG; q++) all += slump[q];
+    for (int t = threadIdx.x; t < nt; t += kTB) ov[t0 + t] = acc[t] + (cols[t] == I ? (sany ? all : T(1)) : T(0));
+}
+
 // Q = P - w D (A P), in place of A P (both rows ascending)
 template <typename T>
 __global__ void k_mg_q(int n, const int32_t *prp, const int32_t *pci, const T *pv, const int32_t *arp,
@@ -380,43 +446,80 @@ __global__ void k_mg_perm(int n, const int32_t *perm, const T *a, T *b) {
     if (i < n) b[i] = a[perm[i]];
 }
 
-// dense inverse of the bottom matrix (n <= kMgBottom) by Gauss-Jordan in
-// shared memory, one block; a direction that is zero to rounding (pure
-// Neumann problems) is left out
+// dense inverse of the bottom matrix (n <= kMgBottom = 96) by Gauss-Jordan,
+// one block: 16 warps by 32 lanes hold six rows by three columns each in
+// registers, row and column k of a step come through shared memory (two
+// buffers: one barrier a step).  With the matrix in shared memory and a
+// division per element index it took 0.9 us a step (81 rows FP32 76 us), now
+// 23 us.  A direction that is zero to rounding (pure Neumann problems) is
+// left out.
 template <typename T>
 __global__ void __launch_bounds__(512) k_mg_binv(int n, const int32_t *rp, const int32_t *ci, const T *v, T *inv) {
+    static_assert(kMgBottom == 96, "six rows by three columns a thread");
     extern __shared__ __align__(16) unsigned char mg_smem[];
     T *M = reinterpret_cast<T *>(mg_smem);
-    __shared__ T col[kMgBottom], row[kMgBottom], diag[kMgBottom];
-    const int ld = n | 1;
-    for (int k = threadIdx.x; k < n * ld; k += blockDim.x) M[k] = T(0);
+    __shared__ T col[2][kMgBottom], row[2][kMgBottom], diag[kMgBottom];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int k = threadIdx.x; k < n * n; k += blockDim.x) M[k] = T(0);
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-        for (int k = rp[i]; k < rp[i + 1]; k++) {
-            M[i * ld + ci[k]] = v[k];
-            if (ci[k] == i) diag[i] = v[k];
+    for (int i = warp; i < n; i += 16)
+        for (int k = rp[i] + lane; k < rp[i + 1]; k += 32) {
+            const int j = ci[k];
+            M[i * n + j] = v[k];
+            if (j == i) diag[i] = v[k];
         }
     __syncthreads();
+    T m[6][3];
+#pragma unroll
+    for (int a = 0; a < 6; a++)
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const int i = warp + 16 * a, j = lane + 32 * b;
+            m[a][b] = i < n && j < n ? M[i * n + j] : T(0);
+        }
     const T eps = sizeof(T) == 8 ? T(1e-13) : T(1e-5);
-    for (int k = 0; k < n; k++) {
-        const T d = M[k * ld + k];
-        const T p = d > eps * diag[k] ? T(1) / d : T(0);
-        __syncthreads();
-        for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            col[j] = M[j * ld + k];
-            row[j] = M[k * ld + j] * p;
+    // k = 16 ka + q: the register row ka and column ka / 2 of step k are known to the compiler
+#pragma unroll
+    for (int ka = 0; ka < 6; ka++) {
+        const int kb = ka / 2;
+#pragma unroll 1
+        for (int q = 0; q < 16; q++) {
+            const int k = 16 * ka + q;
+            if (k >= n) break;
+            T *ck = col[k & 1], *rk = row[k & 1];
+            const bool mycol = lane == (k & 31), myrow = warp == q;
+            if (mycol)
+#pragma unroll
+                for (int a = 0; a < 6; a++) ck[warp + 16 * a] = m[a][kb];
+            if (myrow)
+#pragma unroll
+                for (int b = 0; b < 3; b++) rk[lane + 32 * b] = m[ka][b];
+            __syncthreads();
+            const T d = ck[k];
+            const T p = d > eps * diag[k] ? T(1) / d : T(0);
+            // column k takes -c p and row k takes r: zero the column, then r with p in its place
+            T r[3];
+#pragma unroll
+            for (int b = 0; b < 3; b++) r[b] = rk[lane + 32 * b] * p;
+            r[kb] = mycol ? p : r[kb];
+#pragma unroll
+            for (int a = 0; a < 6; a++) {
+                const T c = ck[warp + 16 * a];
+                m[a][kb] = mycol ? T(0) : m[a][kb];
+#pragma unroll
+                for (int b = 0; b < 3; b++) m[a][b] -= c * r[b];
+            }
+#pragma unroll
+            for (int b = 0; b < 3; b++) m[ka][b] = myrow ? r[b] : m[ka][b];
         }
-        __syncthreads();
-        for (int q = threadIdx.x; q < n * n; q += blockDim.x) {
-            const int i = q / n, j = q - i * n;
-            T x;
-            if (i == k) x = j == k ? p : row[j];
-            else x = j == k ? -col[i] * p : M[i * ld + j] - col[i] * row[j];
-            M[i * ld + j] = x;
-        }
-        __syncthreads();
     }
-    for (int q = threadIdx.x; q < n * n; q += blockDim.x) inv[q] = M[q / n * ld + q % n];
+#pragma unroll
+    for (int a = 0; a < 6; a++)
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const int i = warp + 16 * a, j = lane + 32 * b;
+            if (i < n && j < n) inv[i * n + j] = m[a][b];
+        }
 }
 
 // ------------------------------------------------------------------ the cycle
@@ -887,6 +990,7 @@ struct MgCache {
         int2 *ell = nullptr;
         int32_t *prp, *pci, *rrp, *rci, *rperm, *arp, *aci, *trp = nullptr, *tci = nullptr, *tperm = nullptr, *crp, *cci;
         size_t np, na, nt, nc;   // entries of P, A P, Q^T, next A
+        int longa, longc;        // longest rows of A P and the next A
     };
     std::vector<Step> step;
     // numeric storage per precision (0: FP64, 1: FP32), one allocation each
@@ -956,6 +1060,13 @@ int mg_build(grmp_matrix A) {
         d.na = t.AP.ci.size();
         d.nt = t.QT.ci.size();
         d.nc = t.Ac.ci.size();
+        auto longest = [](const std::vector<int32_t> &r) {
+            int l = 0;
+            for (size_t i = 1; i < r.size(); i++) l = std::max(l, r[i] - r[i - 1]);
+            return l;
+        };
+        d.longa = longest(t.AP.rp);
+        d.longc = longest(t.Ac.rp);
         auto up = [&](std::vector<int32_t> &v, int32_t **p) {
             if (!rc) rc = mg_up_vec(ctx, *C, v, p);
         };
@@ -1074,7 +1185,8 @@ int mg_probe(grmp_matrix A, double *react) {
     const int n = A->nrows, grid = std::max(1, std::min({nblk(n, kTB / kCl), 4 * ctx->num_sms, 2048}));
     cudaMemsetAsync(N.bad, 0, 4, ctx->stream);
     k_mg_rows<T><<<grid, kTB, 0, ctx->stream>>>(n, A->d_rowptr, A->d_cols, fine_values<T>(A), (T *)N.D[0],
-                                                (uint8_t *)N.iso[0], (double2 *)N.part, N.bad);
+                                                (uint8_t *)N.iso[0], A->eliminated ? A->d_fixed : nullptr,
+                                                (double2 *)N.part, N.bad);
     GRMP_LAUNCHED(ctx);
     double h[2 * 2048];
     int bad = 0;
@@ -1086,6 +1198,17 @@ int mg_probe(grmp_matrix A, double *react) {
     for (int b = 0; b < grid; b++) s += h[2 * b], d += h[2 * b + 1];
     *react = d > 0 ? s / d : 1.0;
     return GRMP_OK;
+}
+
+// levels of at most kShortLevel rows give a row 16 lanes (k_mg_prol_agg) or a
+// block; a row of a product with at most kWideCap columns fits the accumulators
+// of k_mg_wide (kWideG x 700 x 8 bytes = 179 KB)
+constexpr int kShortLevel = 4096, kWideCap = 700;
+template <typename T, bool RAP>
+size_t mg_wide_smem(int longest) {
+    const size_t b = (size_t)kWideG * longest * sizeof(T) + (size_t)longest * 4;
+    cudaFuncSetAttribute(k_mg_wide<T, RAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+    return b;
 }
 
 template <typename T>
@@ -1104,23 +1227,33 @@ void mg_values(grmp_matrix A) {
         T *pv = (T *)N.pv[k], *av = (T *)N.av[k], *cv = (T *)N.cv[k], *D = (T *)N.D[k];
         if (k > 0) {
             k_mg_rows<T><<<std::max(1, std::min(nblk(n, kTB / kCl), wide)), kTB, 0, st>>>(
-                n, rp, ci, v, D, (uint8_t *)N.iso[k], nullptr, nullptr);
+                n, rp, ci, v, D, (uint8_t *)N.iso[k], nullptr, nullptr, nullptr);
             GRMP_LAUNCHED(ctx);
         }
         if (d.vrow)
             k_mg_prol_geo<T><<<nblk(n), 256, 0, st>>>(n, d.prp, d.pci, d.vrow, (const uint8_t *)N.iso[k], pv,
                                                         (Pair<T> *)N.ellv);
+        else if (n > kShortLevel)
+            k_mg_prol_agg<T, 1><<<nblk(n, 128), 128, 0, st>>>(n, rp, ci, v, D, (const uint8_t *)N.iso[k], d.agg, d.prp,
+                                                              d.pci, pv);
         else
-            k_mg_prol_agg<T><<<nblk(n, 128), 128, 0, st>>>(n, rp, ci, v, D, (const uint8_t *)N.iso[k], d.agg, d.prp, d.pci,
-                                                           pv);
+            k_mg_prol_agg<T, 16><<<nblk((long long)n * 16, 128), 128, 0, st>>>(n, rp, ci, v, D, (const uint8_t *)N.iso[k],
+                                                                               d.agg, d.prp, d.pci, pv);
         if (d.vrow)
             k_mg_ap_geo<T><<<std::max(1, std::min(nblk((long long)n * 16), wide)), kTB, 0, st>>>(
                 n, rp, ci, v, d.ell, (const Pair<T> *)N.ellv, d.arp, d.aci, av);
+        else if (n <= kShortLevel && d.longa <= kWideCap)
+            k_mg_wide<T, false><<<n, kTB, mg_wide_smem<T, false>(d.longa), st>>>(rp, ci, nullptr, v, d.prp, d.pci, pv,
+                                                                                 d.arp, d.aci, av);
         else
             k_mg_ap<T><<<std::max(1, std::min(nblk((long long)n * 8), wide)), kTB, 0, st>>>(n, rp, ci, v, d.prp, d.pci,
                                                                                            pv, d.arp, d.aci, av);
-        k_mg_rap<T><<<std::max(1, std::min(nblk((long long)nc * 16), wide)), kTB, 0, st>>>(
-            nc, d.rrp, d.rci, d.rperm, pv, d.arp, d.aci, av, d.crp, d.cci, cv);
+        if (nc <= kShortLevel && d.longc <= kWideCap)
+            k_mg_wide<T, true><<<nc, kTB, mg_wide_smem<T, true>(d.longc), st>>>(d.rrp, d.rci, d.rperm, pv, d.arp, d.aci, av,
+                                                                                d.crp, d.cci, cv);
+        else
+            k_mg_rap<T><<<std::max(1, std::min(nblk((long long)nc * 16), wide)), kTB, 0, st>>>(
+                nc, d.rrp, d.rci, d.rperm, pv, d.arp, d.aci, av, d.crp, d.cci, cv);
         ctx->launches += 3;
         if (k > 0) {
             k_mg_q<T><<<nblk(n, 128), 128, 0, st>>>(n, d.prp, d.pci, pv, d.arp, d.aci, D, av);
@@ -1136,10 +1269,10 @@ void mg_values(grmp_matrix A) {
     }
     const int nb = C.S.step[ns - 1].nc;
     k_mg_rows<T><<<std::max(1, std::min(nblk(nb, kTB / kCl), wide)), kTB, 0, st>>>(
-        nb, rp, ci, v, (T *)N.D[ns], (uint8_t *)N.iso[ns], nullptr, nullptr);
+        nb, rp, ci, v, (T *)N.D[ns], (uint8_t *)N.iso[ns], nullptr, nullptr, nullptr);
     GRMP_LAUNCHED(ctx);
     if (nb <= kMgBottom) {
-        const size_t smem = (size_t)nb * (nb | 1) * sizeof(T);
+        const size_t smem = (size_t)nb * nb * sizeof(T);
         cudaFuncSetAttribute(k_mg_binv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_mg_binv<T><<<1, 512, smem, st>>>(nb, rp, ci, v, (T *)N.binv);
         GRMP_LAUNCHED(ctx);
@@ -1261,6 +1394,7 @@ int mg_launch(grmp_matrix A, const double *b, double *x, const grmp_solve_params
         // then (33 iterations at 1e-2, 33 to 142 at 1e-3, depending on the right-hand side)
         const double d1 = p->inner_reltol > 0 && p->inner_reltol < 1 ? p->inner_reltol : 0.1;
         double delta = std::max(1e-3, d1 * d1);
+        if (one) delta = std::max(1e-4, delta * delta);   // small systems: FP32 directions stay good
         void *args[] = {&n, &rp, &ci, &v64, &v32, &b, &x, &r, &q, &xc, &zp0, &zp1, &r64, &partial, &dst,
                         &at, &rt, &delta, &mi, &mo, &guess, &spin, &m};
         e = mg_start(ctx, kern, one, n, TPR, p->grid_blocks, args, grid);
