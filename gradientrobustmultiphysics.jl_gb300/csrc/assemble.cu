@@ -39,6 +39,7 @@ struct FastTerm {
     int foff;        // offset of this term's factors in a cell's factor record
     int toff;        // offset of this term's reference tensors (elements)
     int ntens;       // number of NB x NB tensors
+    int exact;       // the quadrature rule integrates the term's polynomial exactly
 };
 
 struct FastTerms {
@@ -102,6 +103,163 @@ __global__ void k_cell_factors(int ncells, const double *coords, const int32_t *
     }
 }
 
+// ---- one Laplace term (LAP1): closed form
+// The factors of a cell are h_ij = |T| f coef grad lambda_i . grad lambda_j,
+// i < j, in lexicographic order; h_ii = -sum_j h_ij.  With m = 1 / ((d+1)(d+2))
+// (the mean of lambda_i lambda_j over T, twice that for i = j), e = 16 m and
+// g = 4 (4 m - 1 / (d+1)) (0 in 2D, -1/5 in 3D) the P2 matrix is
+//   vertices i, j        (e - 8 / (d+1) + 1) h_ij          (2 e for i = j)
+//   vertex m, edge (i,j) g H_m + e h_ij [m = i or j]        H_m = h_im + h_jm
+//   edges (i,j), (k,l)   e (H_k + H_l + h_jl [k = i] + h_jk [l = i] + h_il [k = j] + h_ik [l = j])
+// and the P1 matrix is h.  About 30 FP64 operations a (row, cell) in place of
+// the 60 multiplications with the reference tensors, which bound the kernel
+// (FP64 issue, two lanes a clock and SM): 64^3 P2 in both precisions, factors
+// and rows 3.1 ms before, 1.6 ms now.  Products are kept apart from the sums
+// (__dmul_rn) or explicit fma, so that every instantiation rounds alike.
+template <int DIM, bool W64, bool W32>
+__global__ void k_lap_factors(int ncells, const double *coords, const int32_t *cells, double factor, const double *coef,
+                              double *f64, float *f32) {
+    constexpr int NT = DIM * (DIM + 1) / 2;
+    const int cell = blockIdx.x * blockDim.x + threadIdx.x;
+    if (cell >= ncells) return;
+    double X[(DIM + 1) * DIM], G[3][3], A[3][3], vol, M[3][3], h[NT];
+    for (int v = 0; v <= DIM; v++)
+        for (int k = 0; k < DIM; k++) X[v * DIM + k] = coords[(size_t)cells[(size_t)cell * (DIM + 1) + v] * DIM + k];
+    simplex_geometry<DIM, double>(X, G, vol, A);
+    double scale = vol * factor;
+    if (coef) scale *= coef[cell];
+#pragma unroll
+    for (int p = 0; p < DIM; p++)
+#pragma unroll
+        for (int s = p; s < DIM; s++) {
+            double m = 0;
+#pragma unroll
+            for (int k = 0; k < DIM; k++) m += G[k][p] * G[k][s];
+            M[p][s] = M[s][p] = scale * m;
+        }
+    int q = 0;
+#pragma unroll
+    for (int j = 0; j < DIM; j++) {
+        double m = M[j][0];
+#pragma unroll
+        for (int s = 1; s < DIM; s++) m += M[j][s];
+        h[q++] = -m;
+    }
+#pragma unroll
+    for (int i = 0; i < DIM; i++)
+#pragma unroll
+        for (int j = i + 1; j < DIM; j++) h[q++] = M[i][j];
+#pragma unroll
+    for (int k = 0; k < NT; k++) {
+        if (W64) f64[(size_t)cell * NT + k] = h[k];
+        if (W32) f32[(size_t)cell * NT + k] = (float)h[k];
+    }
+}
+
+// one or both precisions of a value
+struct Dual {
+    double d;
+    float f;
+};
+template <typename V> __device__ __forceinline__ V lap_const(double c);
+template <> __device__ __forceinline__ double lap_const<double>(double c) { return c; }
+template <> __device__ __forceinline__ float lap_const<float>(double c) { return (float)c; }
+template <> __device__ __forceinline__ Dual lap_const<Dual>(double c) { return {c, (float)c}; }
+__device__ __forceinline__ double vadd(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ Dual vadd(Dual a, Dual b) { return {vadd(a.d, b.d), vadd(a.f, b.f)}; }
+__device__ __forceinline__ double vmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ Dual vmul(Dual a, Dual b) { return {vmul(a.d, b.d), vmul(a.f, b.f)}; }
+__device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ Dual vfma(Dual a, Dual b, Dual c) { return {vfma(a.d, b.d, c.d), vfma(a.f, b.f, c.f)}; }
+__device__ __forceinline__ double vneg(double a) { return -a; }
+__device__ __forceinline__ float vneg(float a) { return -a; }
+__device__ __forceinline__ Dual vneg(Dual a) { return {-a.d, -a.f}; }
+
+// index of the pair i != j in the factors; local DoF of the P2 function of edge (i, j)
+template <int DIM>
+__device__ __forceinline__ int lap_pair(int i, int j) {
+    return DIM == 2 ? i + j - 1 : i + j - 1 + (min(i, j) > 0);
+}
+template <int DIM>
+__device__ __forceinline__ int lap_edge(int i, int j) {
+    if (DIM == 3) return 4 + lap_pair<3>(i, j);
+    return i + j == 1 ? 3 : 7 - i - j;   // (0, 1), (1, 2), (0, 2)
+}
+
+// contributions of a cell to the row of its local function a: load(pair) and add(function, value)
+template <int DIM, int NB, typename V, typename LD, typename AD>
+__device__ __forceinline__ void lap_row(int a, LD load, AD add) {
+    constexpr double m = 1.0 / ((DIM + 1) * (DIM + 2)), ce = 16 * m;
+    if (a <= DIM) {
+        V h[DIM], sum;
+        int o[DIM];
+#pragma unroll
+        for (int r = 0; r < DIM; r++) {
+            o[r] = r + (r >= a);
+            h[r] = load(lap_pair<DIM>(a, o[r]));
+            sum = r ? vadd(sum, h[r]) : h[r];
+        }
+        const V hd = vneg(sum);
+        if constexpr (NB == DIM + 1) {
+            add(a, hd);
+#pragma unroll
+            for (int r = 0; r < DIM; r++) add(o[r], h[r]);
+        } else {
+            const V e = lap_const<V>(ce), g = lap_const<V>(4 * (4 * m - 1.0 / (DIM + 1)));
+            const V vd = lap_const<V>(2 * ce - 8.0 / (DIM + 1) + 1), vo = lap_const<V>(ce - 8.0 / (DIM + 1) + 1);
+            add(a, vmul(vd, hd));
+#pragma unroll
+            for (int r = 0; r < DIM; r++) {
+                add(o[r], vmul(vo, h[r]));
+                const V t = vmul(e, h[r]);
+                add(lap_edge<DIM>(a, o[r]), DIM == 2 ? t : vfma(g, vadd(h[r], hd), t));
+            }
+            if (DIM == 3) {   // g = 0 on triangles
+#pragma unroll
+                for (int r = 0; r < DIM; r++)
+#pragma unroll
+                    for (int s = r + 1; s < DIM; s++) add(lap_edge<DIM>(o[r], o[s]), vmul(g, vadd(h[r], h[s])));
+            }
+        }
+    } else if constexpr (NB > DIM + 1) {
+        const V e = lap_const<V>(ce), e2 = lap_const<V>(2 * ce);
+        if constexpr (DIM == 2) {
+            const int i = a - 3, j = (a - 2) % 3, k = 3 - i - j;
+            const V hij = load(lap_pair<2>(i, j)), hik = load(lap_pair<2>(i, k)), hjk = load(lap_pair<2>(j, k));
+            const V ev = vmul(e, hij);
+            add(i, ev);
+            add(j, ev);
+            // H_i = -h_ik, H_j = -h_jk, H_k = h_ik + h_jk
+            add(a, vneg(vmul(e2, vadd(vadd(hik, hjk), hij))));
+            add(lap_edge<2>(i, k), vmul(e2, hjk));
+            add(lap_edge<2>(j, k), vmul(e2, hik));
+        } else {
+            // edge (i, j), the other vertices k < l
+            const int i = a < 7 ? 0 : (a < 9 ? 1 : 2);
+            const int j = a < 7 ? a - 3 : (a < 9 ? a - 5 : 3);
+            const int k = i > 0 ? 0 : (j == 1 ? 2 : 1), l = 6 - i - j - k;
+            const V hij = load(lap_pair<3>(i, j)), hik = load(lap_pair<3>(i, k)), hil = load(lap_pair<3>(i, l));
+            const V hjk = load(lap_pair<3>(j, k)), hjl = load(lap_pair<3>(j, l));
+            const V g = lap_const<V>(4 * (4 * m - 1.0 / (DIM + 1)));
+            const V Hi = vneg(vadd(hik, hil)), Hj = vneg(vadd(hjk, hjl)), Hk = vadd(hik, hjk), Hl = vadd(hil, hjl);
+            const V ev = vmul(e, hij);
+            add(i, vfma(g, Hi, ev));
+            add(j, vfma(g, Hj, ev));
+            add(k, vmul(g, Hk));
+            add(l, vmul(g, Hl));
+            add(a, vmul(e2, vadd(vadd(Hi, Hj), vneg(hij))));
+            add(lap_edge<3>(i, k), vmul(e, vadd(vadd(Hi, Hk), hjk)));
+            add(lap_edge<3>(i, l), vmul(e, vadd(vadd(Hi, Hl), hjl)));
+            add(lap_edge<3>(j, k), vmul(e, vadd(vadd(Hj, Hk), hik)));
+            add(lap_edge<3>(j, l), vmul(e, vadd(vadd(Hj, Hl), hil)));
+            add(lap_edge<3>(k, l), vmul(e, vadd(Hk, Hl)));
+        }
+    }
+}
+
 // Row-centric assembly.  S = slot index type (uint8_t / uint16_t).  A block
 // owns blockDim.x consecutive rows; their values (contiguous in the CSR) are
 // accumulated in shared memory, each thread adding its row's contributions in
@@ -116,11 +274,12 @@ __global__ void __launch_bounds__(128) k_assemble_rows(int32_t nrows, const int3
     constexpr int LD = NB * NC;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *tens = reinterpret_cast<T *>(smem_raw);
-    T *acc = tens + ((ft.tens_total + 1) & ~1);
+    const int ntens = LAP1 ? 0 : ft.tens_total;
+    T *acc = tens + ((ntens + 1) & ~1);
     const int row0 = blockIdx.x * blockDim.x;
     const int row1 = min(row0 + (int)blockDim.x, nrows);
     const int v0 = rowptr[row0], nv = rowptr[row1] - v0;
-    for (int i = threadIdx.x; i < ft.tens_total; i += blockDim.x) tens[i] = gtens[i];
+    for (int i = threadIdx.x; i < ntens; i += blockDim.x) tens[i] = gtens[i];
     for (int i = threadIdx.x; i < nv; i += blockDim.x) acc[i] = T(0);
     __syncthreads();
     const int row = row0 + threadIdx.x;
@@ -134,23 +293,14 @@ __global__ void __launch_bounds__(128) k_assemble_rows(int32_t nrows, const int3
             const int c1 = A / NB, a = A - c1 * NB;
             const T *cf = fac + (size_t)cell * ft.nf_total;
             const S *sl = slot + (size_t)p * LD;
-            if (LAP1) {   // one Laplace term: its DIM(DIM+1)/2 factors in registers
-                constexpr int NT = DIM * (DIM + 1) / 2;
-                T fl[NT];
-#pragma unroll
-                for (int q = 0; q < NT; q++) fl[q] = cf[q];
-#pragma unroll
-                for (int B = 0; B < LD; B++) {
-                    const S s = sl[B];
-                    if (s == DROP) continue;
-                    const int c2 = B / NB, b = B - c2 * NB;
-                    if (c1 != c2) continue;
-                    const T *tt = tens + a * NB + b;
-                    T v = 0;
-#pragma unroll
-                    for (int q = 0; q < NT; q++) v += fl[q] * tt[q * NB * NB];
-                    rv[s] += v;
-                }
+            if constexpr (LAP1) {
+                const S *sc = sl + c1 * NB;
+                lap_row<DIM, NB, T>(
+                    a, [&](int q) { return cf[q]; },
+                    [&](int b, T v) {
+                        const S k = sc[b];
+                        if (k != DROP) rv[k] = vadd(rv[k], v);
+                    });
                 continue;
             }
             T f[GRMP_MAX_TERMS * 16];
@@ -197,13 +347,14 @@ __global__ void __launch_bounds__(128) k_assemble_rows2(int32_t nrows, const int
     constexpr int LD = NB * NC;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *tens64 = reinterpret_cast<double *>(smem_raw);
-    double *acc64 = tens64 + ft.tens_total;
+    const int ntens = LAP1 ? 0 : ft.tens_total;
+    double *acc64 = tens64 + ntens;
     float *tens32 = reinterpret_cast<float *>(acc64 + block_nnz);
-    float *acc32 = tens32 + ((ft.tens_total + 1) & ~1);
+    float *acc32 = tens32 + ((ntens + 1) & ~1);
     const int row0 = blockIdx.x * blockDim.x;
     const int row1 = min(row0 + (int)blockDim.x, nrows);
     const int v0 = rowptr[row0], nv = rowptr[row1] - v0;
-    for (int i = threadIdx.x; i < ft.tens_total; i += blockDim.x) {
+    for (int i = threadIdx.x; i < ntens; i += blockDim.x) {
         tens64[i] = gtens64[i];
         tens32[i] = gtens32[i];
     }
@@ -225,32 +376,17 @@ __global__ void __launch_bounds__(128) k_assemble_rows2(int32_t nrows, const int
             const double *cf64 = fac64 + (size_t)cell * ft.nf_total;
             const float *cf32 = fac32 + (size_t)cell * ft.nf_total;
             const S *sl = slot + (size_t)p * LD;
-            if (LAP1) {   // one Laplace term: both precisions' factors in registers
-                constexpr int NT = DIM * (DIM + 1) / 2;
-                double g64[NT];
-                float g32[NT];
-#pragma unroll
-                for (int q = 0; q < NT; q++) {
-                    g64[q] = cf64[q];
-                    g32[q] = cf32[q];
-                }
-#pragma unroll
-                for (int B = 0; B < LD; B++) {
-                    const S s = sl[B];
-                    if (s == DROP) continue;
-                    const int c2 = B / NB, b = B - c2 * NB;
-                    if (c1 != c2) continue;
-                    const int to = a * NB + b;
-                    double v = 0;
-                    float w = 0;
-#pragma unroll
-                    for (int q = 0; q < NT; q++) {
-                        v += g64[q] * tens64[to + q * NB * NB];
-                        w += g32[q] * tens32[to + q * NB * NB];
-                    }
-                    rv64[s] += v;
-                    rv32[s] += w;
-                }
+            if constexpr (LAP1) {
+                const S *sc = sl + c1 * NB;
+                lap_row<DIM, NB, Dual>(
+                    a, [&](int q) { return Dual{cf64[q], cf32[q]}; },
+                    [&](int b, Dual v) {
+                        const S k = sc[b];
+                        if (k != DROP) {
+                            rv64[k] = vadd(rv64[k], v.d);
+                            rv32[k] = vadd(rv32[k], v.f);
+                        }
+                    });
                 continue;
             }
             double f64[GRMP_MAX_TERMS * 16];
@@ -395,8 +531,8 @@ int assemble_rows_tuned(grmp_matrix A, size_t tens_b, size_t per_nnz, int *cache
     return GRMP_OK;
 }
 
-// a single Laplace term: the register-resident kernel variants
-inline bool single_laplace(const FastTerms &ft) { return ft.n == 1 && ft.t[0].op == GRMP_OP_LAPLACE; }
+// a single Laplace term integrated exactly: the closed form
+inline bool single_laplace(const FastTerms &ft) { return ft.n == 1 && ft.t[0].op == GRMP_OP_LAPLACE && ft.t[0].exact; }
 
 template <int DIM, int NB, int NC>
 int run_assembly_dual(grmp_matrix A, const FastTerms &ft, const std::vector<double> &tens64) {
@@ -430,20 +566,26 @@ int run_assembly_dual(grmp_matrix A, const FastTerms &ft, const std::vector<doub
     }
     double *fac64 = (double *)A->d_cellfac;
     float *fac32 = (float *)((char *)A->d_cellfac + ((f64b + 255) & ~(size_t)255));
-    k_cell_factors<DIM, NC, double><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, ft,
-                                                                              fac64);
-    GRMP_LAUNCHED(ctx);
-    k_cell_factors<DIM, NC, float><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, ft,
-                                                                             fac32);
-    GRMP_LAUNCHED(ctx);
+    const bool lap1 = single_laplace(ft);
+    if (lap1) {
+        k_lap_factors<DIM, true, true><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(
+            m->ncells, m->d_coords, m->d_cells, ft.factor[0], ft.coef[0], fac64, fac32);
+        GRMP_LAUNCHED(ctx);
+    } else {
+        k_cell_factors<DIM, NC, double><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, ft,
+                                                                                  fac64);
+        GRMP_LAUNCHED(ctx);
+        k_cell_factors<DIM, NC, float><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, ft,
+                                                                                 fac32);
+        GRMP_LAUNCHED(ctx);
+    }
     if (!A->d_vals64) rc = grmp_alloc(ctx, (void **)&A->d_vals64, (size_t)A->nnz * 8);
     if (!rc && !A->d_vals32) rc = grmp_alloc(ctx, (void **)&A->d_vals32, (size_t)A->nnz * 4);
     if (rc) {
         release();
         return rc;
     }
-    const size_t tens_b = tens64.size() * 8 + ((tens32.size() + 1) & ~(size_t)1) * 4;
-    const bool lap1 = single_laplace(ft);
+    const size_t tens_b = lap1 ? 0 : tens64.size() * 8 + ((tens32.size() + 1) & ~(size_t)1) * 4;
     auto go = [&](int tpb, size_t shm) {
         int bnz = 0;
         block_nnz_max(A, tpb, &bnz);   // counted by the caller already: no download here
@@ -497,7 +639,13 @@ int run_assembly(grmp_matrix A, const FastTerms &ft, const std::vector<double> &
         A->cellfac_bytes = fbytes;
     }
     T *fac = (T *)A->d_cellfac;
-    k_cell_factors<DIM, NC, T><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, ft, fac); GRMP_LAUNCHED(ctx);
+    const bool lap1 = single_laplace(ft);
+    if (lap1)
+        k_lap_factors<DIM, sizeof(T) == 8, sizeof(T) == 4><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(
+            m->ncells, m->d_coords, m->d_cells, ft.factor[0], ft.coef[0], (double *)fac, (float *)fac);
+    else
+        k_cell_factors<DIM, NC, T><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, ft, fac);
+    GRMP_LAUNCHED(ctx);
     T *vals;
     if (sizeof(T) == 8) {
         if (!A->d_vals64) {
@@ -514,8 +662,7 @@ int run_assembly(grmp_matrix A, const FastTerms &ft, const std::vector<double> &
     }
     // rows per block (autotuned per matrix and precision): their values (the
     // largest block's count) and the reference tensors in shared memory
-    const size_t tens_b = ((tens.size() + 1) & ~(size_t)1) * sizeof(T);
-    const bool lap1 = single_laplace(ft);
+    const size_t tens_b = lap1 ? 0 : ((tens.size() + 1) & ~(size_t)1) * sizeof(T);
     auto go = [&](int tpb, size_t shm) {
         auto launch = [&](auto kern, const auto *slot) {
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
@@ -708,6 +855,7 @@ int grmp_assemble_bilinear_impl(grmp_matrix A, int nterms, const grmp_bilinear_t
         f.op = t.op_kind;
         f.foff = foff;
         f.toff = (int)tens.size();
+        f.exact = t.bonus_quadorder >= 0;
         ft.factor[i] = t.factor;
         ft.mu[i] = t.param[0];
         ft.lambda[i] = t.param[1];

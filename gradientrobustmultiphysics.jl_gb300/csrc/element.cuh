@@ -166,6 +166,7 @@ __device__ __forceinline__ void rhs_eval(const RhsDev &r, int dim, int cell, con
     } else if (r.kind == GRMP_RHS_FOURIER) {
         int stride = 1 + dim, nm = (int)(r.npar / stride);
         double s = 0;
+#pragma unroll 4   // independent sines: one after another they are a chain of latencies
         for (int m = 0; m < nm; m++) {
             double arg = 0;
             for (int j = 0; j < dim; j++) arg += r.par[m * stride + 1 + j] * x[j];
