@@ -590,7 +590,7 @@ int run_assembly_dual(grmp_matrix A, const FastTerms &ft, const std::vector<doub
         int bnz = 0;
         block_nnz_max(A, tpb, &bnz);   // counted by the caller already: no download here
         auto launch = [&](auto kern, const auto *slot) {
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+            grmp_allow_smem(kern);
             kern<<<nblk(A->nrows, tpb), tpb, shm, ctx->stream>>>(A->nrows, s->d_inc_ptr, s->d_inc_cell, s->d_inc_loc,
                                                                 slot, A->d_rowptr, fac64, fac32, dt64, dt32, ft,
                                                                 A->d_vals64, A->d_vals32, bnz);
@@ -665,7 +665,7 @@ int run_assembly(grmp_matrix A, const FastTerms &ft, const std::vector<double> &
     const size_t tens_b = lap1 ? 0 : ((tens.size() + 1) & ~(size_t)1) * sizeof(T);
     auto go = [&](int tpb, size_t shm) {
         auto launch = [&](auto kern, const auto *slot) {
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+            grmp_allow_smem(kern);
             kern<<<nblk(A->nrows, tpb), tpb, shm, ctx->stream>>>(A->nrows, s->d_inc_ptr, s->d_inc_cell, s->d_inc_loc,
                                                                 slot, A->d_rowptr, fac, dtens, ft, vals);
             GRMP_LAUNCHED(ctx);

@@ -1990,7 +1990,7 @@ extern "C" int grmp_stokes_batch_solve(grmp_matrix A, grmp_vector bf, grmp_vecto
         if (!rc && smem > 220 * 1024)
             rc = grmp_fail(ctx, GRMP_ERR_UNSUPPORTED, "batch direct: front of %d DoFs too large", m.max_f);
         if (!rc) {
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            grmp_allow_smem(kern);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 512, smem);
             int grid = std::max(1, std::min(np, std::max(1, per_sm) * ctx->num_sms));
             // one workspace slot per resident block; fewer blocks when memory is short

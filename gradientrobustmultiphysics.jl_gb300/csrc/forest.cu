@@ -888,8 +888,8 @@ void grmp_forest_solve64(grmp_context ctx, MfForest *F, double *w, const int *ac
     double *uv = (double *)F->uv;
     auto smem_f = [](int maxf) { return (size_t)(maxf + 32) * 8; };
     auto smem_b = [](int nt, int maxf) { return ((size_t)nt + maxf) * 8; };
-    cudaFuncSetAttribute(k_fs_fwd<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f(F->max_f));
-    cudaFuncSetAttribute(k_fs_bwd<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b(512, F->max_f));
+    grmp_allow_smem(k_fs_fwd<512>);
+    grmp_allow_smem(k_fs_bwd<512>);
     for (size_t l = 0; l < F->level.size(); l++) {
         const FoItems *c = F->level[l].solve;
         if (c[2].count) k_fs_fwd<512><<<c[2].count, 512, smem_f(c[2].maxf), ctx->stream>>>(F->dev, c[2].d, L, uv, w, active);

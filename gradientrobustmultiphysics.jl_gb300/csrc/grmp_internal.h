@@ -230,6 +230,22 @@ int grmp_upload(grmp_context ctx, T **dst, const T *src, size_t count) {
 
 // ---------------------------------------------------------------- device helpers
 #ifdef __CUDACC__
+// Lets a kernel use all the shared memory that a block can have.  The same
+// value at every call: contexts on other threads launch the same kernels with
+// other sizes, and a smaller limit set between one thread's call and its launch
+// fails that launch.
+template <typename K>
+inline cudaError_t grmp_allow_smem(K kern) {
+    cudaFuncAttributes fa;
+    int dev = 0, most = 0;
+    cudaError_t e = cudaFuncGetAttributes(&fa, (const void *)kern);
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                most - (int)fa.sharedSizeBytes);
+}
+
 // Grid-wide barrier for a cooperative (co-resident) launch.  Every wait is
 // bounded: after `limit` polls (one L2 round trip plus 32 ns each) the
 // waiting block records GRMP_ERR_TIMEOUT in *status and leaves; callers

@@ -652,8 +652,8 @@ int mf_enqueue_inverse(grmp_matrix A) {
     MfCache &C = *A->mf;
     float *uv = (float *)C.F->uv;
     const size_t sf = (size_t)C.S.max_s * 4;
-    cudaFuncSetAttribute(k_fq_fwd<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf);
-    cudaFuncSetAttribute(k_fq_bwd<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((512 + C.S.max_f) * 4));
+    grmp_allow_smem(k_fq_fwd<512>);
+    grmp_allow_smem(k_fq_bwd<512>);
     int k = 0;
     for (const MfCache::Lv &v : C.lv) {
         if (v.nfwdb) {

@@ -1711,13 +1711,12 @@ int launch_pcg_duo_keep(grmp_matrix A, const double *bvec, double *xvec, const g
         const int jt = (int)((n + stride - 1) / stride);
         const size_t sb = (size_t)KW * jt * G * 4;
         if ((long long)sb > dev_max) continue;
-        if (cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb) !=
-            cudaSuccess) {
+        int occ = 0;
+        if (grmp_allow_smem(kern) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, PTPB, sb) != cudaSuccess) {
             cudaGetLastError();
             continue;
         }
-        int occ = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, PTPB, sb);
         if ((long long)occ * ctx->num_sms >= gtry) {
             grid = gtry;
             J = jt;
