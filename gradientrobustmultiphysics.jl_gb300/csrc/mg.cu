@@ -5,12 +5,12 @@
 // and each is bound by the latency of its gathers and grid barriers, so what
 // pays is fewer iterations.  The preconditioner is one multilevel cycle:
 //
-//   z = c D_0 r + P_0 V(P_0^T r)
+//   z = V(r)                        (small and medium systems: fine_mult)
+//   z = c D_0 r + P_0 V(P_0^T r)    (large ones)
 //
-// additive on the fine level (its Jacobi part costs no product with the fine
-// matrix, so an iteration keeps one fine SpMV; multiplicative smoothing there
-// needs two more and saves less than half of the iterations: 47 against 27 on
-// 24^3 P2), and a symmetric V(1,1) cycle below.  P_0 of a P2 space
+// a symmetric V(1,1) cycle, additive on the fine level of large systems (its
+// Jacobi part costs no product with the fine matrix, so an iteration keeps one
+// fine SpMV).  P_0 of a P2 space
 // interpolates from the vertices (P1 is in P2); all other levels are smoothed
 // aggregation, P = (I - w D A) P_agg.  D = 1 / sum_j |a_ij| (l1-Jacobi:
 // convergent for every SPD matrix without an eigenvalue estimate).  With
@@ -57,19 +57,28 @@ constexpr double kMaxReaction = 0.02;
 // gained a digit after kStallBicg, are left to the Jacobi iteration
 constexpr int kMaxBicg = 200, kStallBicg = 40;
 
-// Rows from which the multilevel solver is taken.  An iteration costs three to
-// four Jacobi iterations on small systems (the cycle's phases) and the values
-// about 0.4 ms, so it pays once Jacobi-PCG needs some 150 iterations, about 6
-// per DoF along an axis.  Whole passes, multilevel / Jacobi, lognormal
-// coefficient, ms: 2D 441 rows 0.80 / 0.94, 1,089 rows 0.93 / 1.69; 3D P1
-// mixed 15,625 rows 1.78 / 1.52, FP64 4,913 rows 1.82 / 1.73, 15,625 rows 2.25 /
-// 2.54; 3D P2 mixed 1,331 rows 1.33 / 1.15, 4,913 rows 1.83 / 1.99, FP64 2.64 /
-// 2.54.
+// Rows from which the multilevel solver is taken: where whole passes are no
+// slower than with Jacobi-PCG for constant coefficients (lognormal ones gain
+// more).  Multilevel / Jacobi, constant, ms: 2D mixed 121 rows 0.35 / 0.43; 2D
+// FP64 225 rows 0.73 / 0.70, 441 rows 1.02 / 1.01 (P1), 0.89 / 1.30 (P2); 3D P1
+// mixed 2,197 rows 0.72 / 0.70, 4,913 rows 0.81 / 0.95; 3D P1 FP64 1,000 rows
+// 0.78 / 0.73, 2,197 rows 0.93 / 0.98; 3D P2 mixed 1,331 rows 0.93 / 0.90, 2,197
+// rows 0.94 / 1.02; 3D P2 FP64 729 rows 1.11 / 1.07, 1,331 rows 1.20 / 1.28.
 int min_rows(int dim, int fe, bool mixed) {
-    if (dim == 2) return 600;
-    if (fe == GRMP_FE_H1P2) return mixed ? 4500 : 6000;
-    return mixed ? 30000 : 12000;
+    if (dim == 2) return mixed ? 120 : 440;
+    if (fe == GRMP_FE_H1P2) return mixed ? 2000 : 1300;
+    return mixed ? 2500 : 2000;
 }
+
+// Whether the fine level is smoothed multiplicatively too, which costs a
+// product with the matrix, one with Q_0 and a longer restriction an iteration and saves
+// 30-50 % of the iterations: while an iteration is mostly phases and barriers.
+// Additive / multiplicative, whole passes, ms: 2D P2 1,089 rows 0.76 / 0.72
+// (37 / 21 iterations), 63,001 rows 2.35 / 1.77, FP64 641,601 rows 9.9 / 10.7; 2D
+// P1 491,401 rows mixed 6.3 / 4.7, FP64 10.4 / 7.9; 3D P1 238,328 rows FP64
+// 5.61 / 5.46 (46 / 26), 531,441 rows 10.4 / 10.8; 3D P2 6,859 rows 1.73 / 1.16,
+// 117,649 rows mixed 2.9 / 2.5, FP64 4.2 / 4.4, 804,357 rows mixed 9.4 / 10.5.
+bool fine_mult(int dim, int fe, int n) { return n <= (dim == 3 && fe == GRMP_FE_H1P2 ? 80000 : 400000); }
 
 template <typename T>
 struct alignas(2 * sizeof(T)) Pair {
@@ -99,6 +108,12 @@ struct MgDev {
     const int32_t *rrp, *rci;
     const T *rv;
     const T *D0, *binv;
+    // fine level smoothed multiplicatively: Q_0 (its transpose is in rrp, rci, rv), lanes per row of A
+    // and Q_0, A in the cycle's precision and a vector
+    int mult, flanes, n;
+    const int32_t *frp, *fci, *q0rp, *q0ci;
+    const T *fv, *q0v;
+    T *z0;
     MgLv<T> lv[kMgMaxLevels + 1];
 };
 
@@ -641,6 +656,29 @@ __device__ __forceinline__ T mg_fine(const MgDev<T> &m, int i, T ri) {
     return z;
 }
 
+// z = M^-1 r on the fine level after mg_cycle; epi(i, z_i) by the thread that
+// owns row i.  Multiplicative: z = 2 S r - S A S r + Q e, as on the levels
+// below (no barrier more: S r is formed where it is gathered).
+template <typename T, typename E>
+__device__ __forceinline__ void mg_fine_rows(const MgDev<T> &m, int n, const T *r, E epi) {
+    if (!m.mult) {
+        const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
+#pragma unroll 4
+        for (int i = gtid; i < n; i += gsz) epi(i, mg_fine(m, i, r[i]));
+        return;
+    }
+    const T *D0 = m.D0, *e1 = m.lv[1].e;
+    T *z0 = m.z0;
+    mg_rows(
+        n, m.frp, m.fci, m.fv, m.flanes, [&](int c) { return (T)kSmooth * __ldg(D0 + c) * r[c]; },
+        [&](int i, T s) {
+            const T w = (T)kSmooth * __ldg(D0 + i);
+            z0[i] = T(2) * w * r[i] - w * s;
+        });
+    mg_rows(
+        n, m.q0rp, m.q0ci, m.q0v, m.flanes, [&](int c) { return e1[c]; }, [&](int i, T s) { epi(i, z0[i] + s); });
+}
+
 // ------------------------------------------------------------------ FP64 solver
 template <int TPR, int U, bool PIPE, class SY>
 __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
@@ -674,11 +712,10 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     while (!conv && it < maxit) {
         if (!mg_cycle(m, (const double *)r, eb, sy)) return;
         double w[1] = {0};
-        for (int i = gtid; i < n; i += gsz) {
-            const double ri = r[i], zi = mg_fine(m, i, ri);
+        mg_fine_rows(m, n, (const double *)r, [&](int i, double zi) {
             z[i] = zi;
-            w[0] += ri * zi;
-        }
+            w[0] += r[i] * zi;
+        });
         if (!sy.template sum<1>(w, sh)) return;
         const double beta = it == 0 ? 0.0 : w[0] / rz;
         rz = w[0];
@@ -755,7 +792,7 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     bool conv = sqrt(rr) <= tol, bad = false;
     while (!conv && it < maxit) {
         if (!mg_cycle(m, (const double *)p, eb, sy)) return;
-        for (int i = gtid; i < n; i += gsz) ph[i] = mg_fine(m, i, p[i]);
+        mg_fine_rows(m, n, (const double *)p, [&](int i, double zi) { ph[i] = zi; });
         if (!sy.barrier()) return;
         double d[1];
         d[0] = spmv_grid<TPR, U, PIPE, double, double, double, true, false>(n, rowptr, cols, vals, ph, v, rh, nullptr);
@@ -777,7 +814,7 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
             break;
         }
         if (!mg_cycle(m, (const double *)s, eb, sy)) return;
-        for (int i = gtid; i < n; i += gsz) shv[i] = mg_fine(m, i, s[i]);
+        mg_fine_rows(m, n, (const double *)s, [&](int i, double zi) { shv[i] = zi; });
         if (!sy.barrier()) return;
         double ts[2] = {0, 0};
         spmv_rows<TPR, U, PIPE, double>(
@@ -876,12 +913,10 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     while (!conv && it < maxit && outer < maxouter) {
         if (!mg_cycle(m, (const float *)r, eb, sy)) return;
         float w[1] = {0.f};
-#pragma unroll 4
-        for (int i = gtid; i < n; i += gsz) {
-            const float ri = r[i], zi = mg_fine(m, i, ri);
+        mg_fine_rows(m, n, (const float *)r, [&](int i, float zi) {
             cur[i].x = zi;
-            w[0] += ri * zi;
-        }
+            w[0] += r[i] * zi;
+        });
         if (!sy.template sumf<1>(w, shf)) return;
         const float beta = restart ? 0.f : w[0] / rz;
         rz = w[0];
@@ -984,6 +1019,7 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
 // ---------------------------------------------------------------------- host side
 struct MgCache {
     MgSymbolic S;
+    bool mult = false;   // multiplicative smoothing of the fine level
     std::vector<std::pair<void *, size_t>> bufs;   // patterns
     struct Step {
         int32_t *agg = nullptr, *vrow = nullptr;
@@ -998,7 +1034,7 @@ struct MgCache {
         void *p = nullptr;
         size_t bytes = 0;
         std::vector<char *> pv, av, tv, cv, D, iso, r, y, e;
-        char *rv0 = nullptr, *ellv = nullptr, *binv = nullptr, *part = nullptr, *vec = nullptr;
+        char *rv0 = nullptr, *ellv = nullptr, *binv = nullptr, *part = nullptr, *vec = nullptr, *z0 = nullptr;
         int *bad = nullptr;
     } num[2];
     double react[2] = {0, 0};
@@ -1045,8 +1081,9 @@ int mg_build(grmp_matrix A) {
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multilevel: pattern download");
     MgCache *C = new MgCache;
     A->mg = C;
+    C->mult = fine_mult(s->mesh->dim, s->fe, n);
     if (mg_symbolic_build(n, rp.data(), ci.data(), s->mesh->dim, s->mesh->ncells, s->ldofs, cd.empty() ? nullptr : cd.data(),
-                          coords.data(), cells.data(), &C->S)) {
+                          coords.data(), cells.data(), C->mult, &C->S)) {
         A->mg_state = -1;
         return GRMP_OK;
     }
@@ -1091,7 +1128,7 @@ int mg_build(grmp_matrix A) {
         up(t.AP.ci, &d.aci);
         up(t.Ac.rp, &d.crp);
         up(t.Ac.ci, &d.cci);
-        if (k > 0) {
+        if (k > 0 || C->mult) {
             up(t.QT.rp, &d.trp);
             up(t.QT.ci, &d.tci);
             up(t.QTperm, &d.tperm);
@@ -1150,6 +1187,7 @@ int mg_storage(grmp_matrix A) {
                 N.e[k] = take(n * sizeof(T));
             }
         }
+        N.z0 = take(C.mult ? (size_t)A->nrows * sizeof(T) : 0);
         N.binv = take((size_t)kMgBottom * kMgBottom * sizeof(T));
         N.part = take((size_t)4096 * 16);
         N.bad = (int *)take(4);
@@ -1207,7 +1245,7 @@ constexpr int kShortLevel = 4096, kWideCap = 700;
 template <typename T, bool RAP>
 size_t mg_wide_smem(int longest) {
     const size_t b = (size_t)kWideG * longest * sizeof(T) + (size_t)longest * 4;
-    cudaFuncSetAttribute(k_mg_wide<T, RAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+    grmp_allow_smem(k_mg_wide<T, RAP>);
     return b;
 }
 
@@ -1255,7 +1293,7 @@ void mg_values(grmp_matrix A) {
             k_mg_rap<T><<<std::max(1, std::min(nblk((long long)nc * 16), wide)), kTB, 0, st>>>(
                 nc, d.rrp, d.rci, d.rperm, pv, d.arp, d.aci, av, d.crp, d.cci, cv);
         ctx->launches += 3;
-        if (k > 0) {
+        if (k > 0 || C.mult) {
             k_mg_q<T><<<nblk(n, 128), 128, 0, st>>>(n, d.prp, d.pci, pv, d.arp, d.aci, D, av);
             k_mg_perm<T><<<nblk((long long)d.nt), 256, 0, st>>>((int)d.nt, d.tperm, av, (T *)N.tv[k]);
             ctx->launches += 2;
@@ -1273,7 +1311,7 @@ void mg_values(grmp_matrix A) {
     GRMP_LAUNCHED(ctx);
     if (nb <= kMgBottom) {
         const size_t smem = (size_t)nb * nb * sizeof(T);
-        cudaFuncSetAttribute(k_mg_binv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        grmp_allow_smem(k_mg_binv<T>);
         k_mg_binv<T><<<1, 512, smem, st>>>(nb, rp, ci, v, (T *)N.binv);
         GRMP_LAUNCHED(ctx);
     }
@@ -1302,6 +1340,23 @@ MgDev<T> mg_device(grmp_matrix A) {
         return entries <= (size_t)kShortRow * rows ? 4 : (entries <= (size_t)kLongRow * rows ? 8 : 32);
     };
     m.rlanes = lanes(C.step[0].np, C.S.step[0].nc);
+    m.n = A->nrows;
+    m.mult = C.mult;
+    if (C.mult) {
+        const MgCache::Step &d = C.step[0];
+        m.rrp = d.trp;
+        m.rci = d.tci;
+        m.rv = (const T *)N.tv[0];
+        m.rlanes = lanes(d.nt, C.S.step[0].nc);
+        m.frp = A->d_rowptr;
+        m.fci = A->d_cols;
+        m.fv = fine_values<T>(A);
+        m.q0rp = d.arp;
+        m.q0ci = d.aci;
+        m.q0v = (const T *)N.av[0];
+        m.flanes = lanes(std::max((size_t)A->nnz, d.na), A->nrows);
+        m.z0 = (T *)N.z0;
+    }
     for (int l = 1; l <= ns; l++) {
         MgLv<T> &L = m.lv[l];
         L.n = C.S.step[l - 1].nc;
@@ -1326,13 +1381,13 @@ MgDev<T> mg_device(grmp_matrix A) {
     return m;
 }
 
-// Systems of at most this many rows run in one block (its L1 holds matrix and
-// vectors; on the FP64 pipe of one SM, two FMAs a clock, only smaller ones
-// gain).  2D lognormal, solve in one block / on the grid: mixed 1,089 rows
-// 0.56 / 0.86 ms, 3,249 1.15 / 1.19, 5,041 1.85 / 1.55; FP64 625 0.93 / 1.07,
-// 1,089 1.38 / 1.28.
-constexpr int kOneBlock32 = 3300, kOneBlock64 = 700;
-
+// Systems of at most this many nonzeros run in one block (its L1 holds matrix
+// and vectors; on the FP64 pipe of one SM, two FMAs a clock, only the smallest
+// gain).  One block / the grid, whole passes, lognormal, ms: mixed 2D P2 289
+// rows 0.47 / 0.71, 1,681 rows (19 k nonzeros) 0.88 / 0.88, 2D P1 3,249 rows
+// (22 k) 1.23 / 1.00, 3D P1 1,000 rows (13 k) 0.60 / 0.68; FP64 2D P1 441 rows
+// (3 k) 1.13 / 1.14, 2D P2 441 rows (5 k) 1.06 / 1.05.
+constexpr int kOneBlock32 = 18000, kOneBlock64 = 4000;
 
 // grid: enough blocks for the rows, at most what fits; small systems take
 // one block per SM, which makes the barriers cheaper
@@ -1371,7 +1426,7 @@ int mg_launch(grmp_matrix A, const double *b, double *x, const grmp_solve_params
     cudaMemsetAsync(dst, 0, sizeof(SolveState), ctx->stream);
     cudaError_t e;
     if (!mixed) {
-        const bool one = n <= kOneBlock64 && p->grid_blocks <= 0;
+        const bool one = A->nnz <= kOneBlock64 && p->grid_blocks <= 0;
         auto kern = one ? k_mgcg64<TPR, U, PIPE, BlockSync> : k_mgcg64<TPR, U, PIPE, MgGridSync>;
         MgDev<double> m = mg_device<double>(A);
         double *r = (double *)N.vec, *z = (double *)(N.vec + al(n0 * 8)), *pp = (double *)(N.vec + 2 * al(n0 * 8));
@@ -1379,7 +1434,7 @@ int mg_launch(grmp_matrix A, const double *b, double *x, const grmp_solve_params
         void *args[] = {&n, &rp, &ci, &v64, &b, &x, &r, &z, &pp, &q, &partial, &dst, &at, &rt, &mi, &guess, &spin, &m};
         e = mg_start(ctx, kern, one, n, TPR, p->grid_blocks, args, grid);
     } else {
-        const bool one = n <= kOneBlock32 && p->grid_blocks <= 0;
+        const bool one = A->nnz <= kOneBlock32 && p->grid_blocks <= 0;
         auto kern = one ? k_mgcg_mixed<TPR, U, PIPE, BlockSync> : k_mgcg_mixed<TPR, U, PIPE, MgGridSync>;
         MgDev<float> m = mg_device<float>(A);
         const float *v32 = A->d_vals32;
@@ -1412,7 +1467,7 @@ int mg_launch_bicg(grmp_matrix A, const double *b, double *x, const grmp_solve_p
     const double *v64 = A->d_vals64;
     long long spin = ctx->wait_limit;
     cudaMemsetAsync(dst, 0, sizeof(SolveState), ctx->stream);
-    const bool one = n <= kOneBlock64 && p->grid_blocks <= 0;
+    const bool one = A->nnz <= kOneBlock64 && p->grid_blocks <= 0;
     auto kern = one ? k_mgbicg64<TPR, U, PIPE, BlockSync> : k_mgbicg64<TPR, U, PIPE, MgGridSync>;
     MgDev<double> m = mg_device<double>(A);
     double *w[9];

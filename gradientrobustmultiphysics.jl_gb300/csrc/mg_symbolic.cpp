@@ -195,7 +195,7 @@ void products(MgStep *s, const int32_t *rp, const int32_t *ci) {
 }  // namespace
 
 int mg_symbolic_build(int n, const int32_t *rp, const int32_t *ci, int dim, int ncells, int ld, const int32_t *celldofs,
-                      const double *coords, const int32_t *cells, MgSymbolic *S) {
+                      const double *coords, const int32_t *cells, bool fine_q, MgSymbolic *S) {
     S->step.clear();
     const int32_t *crp = rp, *cci = ci;
     int cn = n;
@@ -245,7 +245,7 @@ int mg_symbolic_build(int n, const int32_t *rp, const int32_t *ci, int dim, int 
         }
         products(&s, crp, cci);
         if (s.geometric) filter_vertex_level(&s, dim, ncells, ld, celldofs, vert, coords, cells);
-        if (!S->step.empty()) transpose(s.n, s.nc, s.AP, &s.QT, &s.QTperm);
+        if (fine_q || !S->step.empty()) transpose(s.n, s.nc, s.AP, &s.QT, &s.QTperm);
         cn = s.nc;
         S->step.push_back(std::move(s));
         crp = S->step.back().Ac.rp.data();   // stays valid: vectors keep their storage when the step is moved
