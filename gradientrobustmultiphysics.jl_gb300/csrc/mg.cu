@@ -41,12 +41,20 @@
 namespace {
 
 constexpr int kTB = 256;
-constexpr int kCl = 8;            // lanes per row of k_mg_rows
 constexpr int kMgT = 384;         // threads per block of the solvers: two blocks fit an SM at 85 registers a thread
-// lanes per row of the coarse operators by mean entries a row: 4 up to
-// kShortRow (vertex level on right angles: 7), 8, and a warp from kLongRow
-// (transposes of wide aggregates: 100-600)
-constexpr int kShortRow = 10, kLongRow = 48;
+// lanes per row of an operator by mean entries a row: 4 up to kShortRow (vertex
+// level on right angles: 7), 8, and a warp from kLongRow (transposes of wide
+// aggregates: 100-600).  FP64 with kManyRows rows and more is bound by the FP64
+// unit (two lanes a clock: a step of the shuffle reduction costs as much as a
+// multiplication of all lanes) and takes fewer: 61^3 P1, phases of an
+// iteration, restriction / up / fine level 27 / 22 / 44 us before, 15 / 19 / 35 us now.
+constexpr int kShortRow = 10, kLongRow = 48, kManyRows = 8192;
+template <typename T>
+int lanes_of(size_t entries, int rows) {
+    if (sizeof(T) == 8 && rows >= kManyRows)
+        return entries <= (size_t)24 * rows ? 2 : (entries <= (size_t)64 * rows ? 4 : (entries <= (size_t)400 * rows ? 8 : 32));
+    return entries <= (size_t)kShortRow * rows ? 4 : (entries <= (size_t)kLongRow * rows ? 8 : 32);
+}
 constexpr double kSmooth = 1.7;   // w of the smoothing steps and c of the fine level (l1-scaled: spectrum in (0, 1])
 constexpr double kProlong = 1.32; // w of the prolongation smoothing
 // reaction-dominated matrices (energy of the constant function against the
@@ -64,7 +72,9 @@ constexpr int kMaxBicg = 200, kStallBicg = 40;
 // mixed 2,197 rows 0.72 / 0.70, 4,913 rows 0.81 / 0.95; 3D P1 FP64 1,000 rows
 // 0.78 / 0.73, 2,197 rows 0.93 / 0.98; 3D P2 mixed 1,331 rows 0.93 / 0.90, 2,197
 // rows 0.94 / 1.02; 3D P2 FP64 729 rows 1.11 / 1.07, 1,331 rows 1.20 / 1.28.
-int min_rows(int dim, int fe, bool mixed) {
+// BiCGStab (a Jacobi iteration there costs 43 us): Newton steps of 441 rows 1.2 / 2.6-2.9.
+int min_rows(int dim, int fe, bool mixed, bool bicg) {
+    if (bicg) return dim == 2 ? 200 : 500;
     if (dim == 2) return mixed ? 120 : 440;
     if (fe == GRMP_FE_H1P2) return mixed ? 2000 : 1300;
     return mixed ? 2500 : 2000;
@@ -120,7 +130,7 @@ struct MgDev {
 // ------------------------------------------------------------------ values of the hierarchy
 // D, the rows without coupling, and (level 0) per-block sums of the positive
 // row sums and diagonals of the rows away from eliminated DoFs, bad diagonals
-template <typename T>
+template <typename T, int kCl>
 __global__ void __launch_bounds__(kTB) k_mg_rows(int n, const int32_t *rp, const int32_t *ci, const T *v, T *D,
                                                  uint8_t *iso, const uint8_t *fixed, double2 *part, int *bad) {
     __shared__ double sh[32 * 2];
@@ -568,7 +578,8 @@ template <typename T, typename G, typename E>
 __device__ __forceinline__ void mg_rows(int n, const int32_t *rp, const int32_t *ci, const T *v, int lanes, G gather,
                                         E epi) {
     const CsrSource<T> src{ci, v};
-    if (lanes == 4) spmv_rows<4, 2, true, T>(n, rp, src, gather, epi);
+    if (sizeof(T) == 8 && lanes == 2) spmv_rows<2, 4, true, T>(n, rp, src, gather, epi);
+    else if (lanes == 4) spmv_rows<4, 2, true, T>(n, rp, src, gather, epi);
     else if (lanes == 8) spmv_rows<8, 2, true, T>(n, rp, src, gather, epi);
     else spmv_rows<32, 4, false, T>(n, rp, src, gather, epi);
 }
@@ -1214,15 +1225,20 @@ const double *fine_values<double>(grmp_matrix A) { return A->d_vals64; }
 template <>
 const float *fine_values<float>(grmp_matrix A) { return A->d_vals32; }
 
+// lanes per row of k_mg_rows (FP64: as in lanes_of)
+template <typename T>
+int rows_lanes(int n) { return sizeof(T) == 8 && n >= kManyRows ? 2 : 8; }
+
 // D of the fine level, the diagonal check and the reaction share
 template <typename T>
 int mg_probe(grmp_matrix A, double *react) {
     grmp_context ctx = A->space->mesh->ctx;
     MgCache &C = *A->mg;
     MgCache::Num &N = C.num[sizeof(T) == 8 ? 0 : 1];
-    const int n = A->nrows, grid = std::max(1, std::min({nblk(n, kTB / kCl), 4 * ctx->num_sms, 2048}));
+    const int n = A->nrows, cl = rows_lanes<T>(n), grid = std::max(1, std::min({nblk(n, kTB / cl), 4 * ctx->num_sms, 2048}));
     cudaMemsetAsync(N.bad, 0, 4, ctx->stream);
-    k_mg_rows<T><<<grid, kTB, 0, ctx->stream>>>(n, A->d_rowptr, A->d_cols, fine_values<T>(A), (T *)N.D[0],
+    auto kern = cl == 2 ? k_mg_rows<T, 2> : k_mg_rows<T, 8>;
+    kern<<<grid, kTB, 0, ctx->stream>>>(n, A->d_rowptr, A->d_cols, fine_values<T>(A), (T *)N.D[0],
                                                 (uint8_t *)N.iso[0], A->eliminated ? A->d_fixed : nullptr,
                                                 (double2 *)N.part, N.bad);
     GRMP_LAUNCHED(ctx);
@@ -1264,7 +1280,9 @@ void mg_values(grmp_matrix A) {
         const int n = C.S.step[k].n, nc = C.S.step[k].nc;
         T *pv = (T *)N.pv[k], *av = (T *)N.av[k], *cv = (T *)N.cv[k], *D = (T *)N.D[k];
         if (k > 0) {
-            k_mg_rows<T><<<std::max(1, std::min(nblk(n, kTB / kCl), wide)), kTB, 0, st>>>(
+            const int cl = rows_lanes<T>(n);
+            auto kern = cl == 2 ? k_mg_rows<T, 2> : k_mg_rows<T, 8>;
+            kern<<<std::max(1, std::min(nblk(n, kTB / cl), wide)), kTB, 0, st>>>(
                 n, rp, ci, v, D, (uint8_t *)N.iso[k], nullptr, nullptr, nullptr);
             GRMP_LAUNCHED(ctx);
         }
@@ -1306,7 +1324,7 @@ void mg_values(grmp_matrix A) {
         v = cv;
     }
     const int nb = C.S.step[ns - 1].nc;
-    k_mg_rows<T><<<std::max(1, std::min(nblk(nb, kTB / kCl), wide)), kTB, 0, st>>>(
+    k_mg_rows<T, 8><<<std::max(1, std::min(nblk(nb, kTB / 8), wide)), kTB, 0, st>>>(
         nb, rp, ci, v, (T *)N.D[ns], (uint8_t *)N.iso[ns], nullptr, nullptr, nullptr);
     GRMP_LAUNCHED(ctx);
     if (nb <= kMgBottom) {
@@ -1336,9 +1354,7 @@ MgDev<T> mg_device(grmp_matrix A) {
     m.D0 = (const T *)N.D[0];
     m.binv = (const T *)N.binv;
     m.dense = C.S.step[ns - 1].nc <= kMgBottom;
-    auto lanes = [](size_t entries, int rows) {
-        return entries <= (size_t)kShortRow * rows ? 4 : (entries <= (size_t)kLongRow * rows ? 8 : 32);
-    };
+    auto lanes = lanes_of<T>;
     m.rlanes = lanes(C.step[0].np, C.S.step[0].nc);
     m.n = A->nrows;
     m.mult = C.mult;
@@ -1491,12 +1507,12 @@ void grmp_mg_free(grmp_matrix A) {
 
 bool grmp_mg_ready(grmp_matrix A, bool mixed) { return A->mg_state > 0 && A->mg && A->mg->num[mixed ? 1 : 0].p; }
 
-int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, int least) {
+int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool bicg) {
     *use = 0;
     grmp_space s = A->space;
     grmp_context ctx = s->mesh->ctx;
     if (A->mg_state < 0 || A->imported || !A->elliptic || s->ncomp != 1 ||
-        (s->fe != GRMP_FE_H1P1 && s->fe != GRMP_FE_H1P2) || A->nrows < std::max(least, min_rows(s->mesh->dim, s->fe, mixed)))
+        (s->fe != GRMP_FE_H1P1 && s->fe != GRMP_FE_H1P2) || A->nrows < min_rows(s->mesh->dim, s->fe, mixed, bicg))
         return GRMP_OK;
     int rc = GRMP_OK;
     if (!A->mg) rc = mg_build(A);

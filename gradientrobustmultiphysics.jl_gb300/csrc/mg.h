@@ -5,14 +5,12 @@
 // spmv_config reported by a solve that the multilevel preconditioner ran
 // (plus the row-loop code of its SpMV, e.g. 90404)
 constexpr int kMgConfig = 90000;
-// rows of a Jacobian from which BiCGStab takes the cycle
-constexpr int kMgBicgRows = 0;
 
 // Whether grmp_solve takes the multilevel solver for this matrix (scalar
 // H1P1 / H1P2 with a diffusion term, not reaction dominated); builds or
 // refreshes what it needs.  *use = 0: the Jacobi solvers.
-// `least`: rows below which it is not taken (besides the rule by element).
-int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, int least = 0);
+// bicg: for grmp_mg_bicgstab, which pays from fewer rows.
+int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool bicg = false);
 // Jacobi-free conjugate gradients with the prepared hierarchy; allocates nothing.
 int grmp_mg_solve(grmp_matrix A, const double *b, double *x, const grmp_solve_params *p, grmp_solve_stats *st);
 // BiCGStab with the prepared FP64 hierarchy for the scalar Jacobian of a Newton

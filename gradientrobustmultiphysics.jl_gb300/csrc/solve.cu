@@ -1968,7 +1968,7 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
     cudaMemsetAsync(dst, 0, sizeof(SolveState), ctx->stream);
     if (bicg) {   // scalar Jacobians: multilevel, else (and where that fails) Jacobi
         int use = 0;
-        int rc = grmp_mg_prepare(A, false, &use, kMgBicgRows);
+        int rc = grmp_mg_prepare(A, false, &use, true);
         if (rc) return rc;
         if (use) {
             double *vv[9];
