@@ -539,11 +539,12 @@ int run_assembly_dual(grmp_matrix A, const FastTerms &ft, const std::vector<doub
     grmp_space s = A->space;
     grmp_mesh m = s->mesh;
     grmp_context ctx = m->ctx;
+    const bool lap1 = single_laplace(ft);   // the closed form needs no tensors
     std::vector<float> tens32(tens64.begin(), tens64.end());
     double *dt64 = nullptr;
     float *dt32 = nullptr;
-    int rc = grmp_upload(ctx, &dt64, tens64.data(), tens64.size());
-    if (!rc) rc = grmp_upload(ctx, &dt32, tens32.data(), tens32.size());
+    int rc = lap1 ? GRMP_OK : grmp_upload(ctx, &dt64, tens64.data(), tens64.size());
+    if (!rc && !lap1) rc = grmp_upload(ctx, &dt32, tens32.data(), tens32.size());
     auto release = [&]() {
         grmp_free(ctx, dt64, tens64.size() * 8);
         grmp_free(ctx, dt32, tens32.size() * 4);
@@ -566,7 +567,6 @@ int run_assembly_dual(grmp_matrix A, const FastTerms &ft, const std::vector<doub
     }
     double *fac64 = (double *)A->d_cellfac;
     float *fac32 = (float *)((char *)A->d_cellfac + ((f64b + 255) & ~(size_t)255));
-    const bool lap1 = single_laplace(ft);
     if (lap1) {
         k_lap_factors<DIM, true, true><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(
             m->ncells, m->d_coords, m->d_cells, ft.factor[0], ft.coef[0], fac64, fac32);
@@ -624,8 +624,9 @@ int run_assembly(grmp_matrix A, const FastTerms &ft, const std::vector<double> &
     grmp_context ctx = m->ctx;
     // reference tensors in precision T
     std::vector<T> tens(tens64.begin(), tens64.end());
+    const bool lap1 = single_laplace(ft);   // the closed form needs no tensors
     T *dtens = nullptr;
-    int rc = grmp_upload(ctx, &dtens, tens.data(), tens.size());
+    int rc = lap1 ? GRMP_OK : grmp_upload(ctx, &dtens, tens.data(), tens.size());
     if (rc) return rc;
     size_t fbytes = (size_t)m->ncells * ft.nf_total * sizeof(T);
     if (A->cellfac_bytes < fbytes) {
@@ -639,7 +640,6 @@ int run_assembly(grmp_matrix A, const FastTerms &ft, const std::vector<double> &
         A->cellfac_bytes = fbytes;
     }
     T *fac = (T *)A->d_cellfac;
-    const bool lap1 = single_laplace(ft);
     if (lap1)
         k_lap_factors<DIM, sizeof(T) == 8, sizeof(T) == 4><<<nblk(m->ncells), TPB, 0, ctx->stream>>>(
             m->ncells, m->d_coords, m->d_cells, ft.factor[0], ft.coef[0], (double *)fac, (float *)fac);
@@ -966,9 +966,12 @@ int grmp_assemble_linear_impl(grmp_space s, const grmp_rhs *rhs, grmp_vector b) 
     if (!rc && !s->d_locbuf) rc = grmp_alloc(ctx, (void **)&s->d_locbuf, ncl * 8);
     if (!rc) {
         RhsDev r{rhs->kind, rhs->ncomponents, dpar, rhs->nparams, rhs->factor, nq, nb, dtab, dtab + nq, dtab + 4 * nq};
-        if (dim == 2) k_linear_cells<2><<<nblk(m->ncells, 128), 128, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells,
+        // FP64 issue is the bound (sines): small meshes spread warp by warp over the SMs
+        // (512 cells of 2D P2, eight sines a point: 30 us in blocks of 128, 19 us now)
+        const int tpb = m->ncells <= 4 * 128 * ctx->num_sms ? 32 : 128;
+        if (dim == 2) k_linear_cells<2><<<nblk(m->ncells, tpb), tpb, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells,
                                                                                     nb, s->ncomp, r, s->d_locbuf);
-        else k_linear_cells<3><<<nblk(m->ncells, 128), 128, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, nb,
+        else k_linear_cells<3><<<nblk(m->ncells, tpb), tpb, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, nb,
                                                                            s->ncomp, r, s->d_locbuf);
         GRMP_LAUNCHED(ctx);
         k_gather_rows<<<nblk(s->ndofs), TPB, 0, ctx->stream>>>(s->ndofs, s->d_inc_ptr, s->d_inc_cell, s->d_inc_loc,

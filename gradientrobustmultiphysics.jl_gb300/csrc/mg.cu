@@ -1046,7 +1046,6 @@ struct MgCache {
         size_t bytes = 0;
         std::vector<char *> pv, av, tv, cv, D, iso, r, y, e;
         char *rv0 = nullptr, *ellv = nullptr, *binv = nullptr, *part = nullptr, *vec = nullptr, *z0 = nullptr;
-        int *bad = nullptr;
     } num[2];
     double react[2] = {0, 0};
     char *state = nullptr;
@@ -1201,7 +1200,6 @@ int mg_storage(grmp_matrix A) {
         N.z0 = take(C.mult ? (size_t)A->nrows * sizeof(T) : 0);
         N.binv = take((size_t)kMgBottom * kMgBottom * sizeof(T));
         N.part = take((size_t)4096 * 16);
-        N.bad = (int *)take(4);
         // FP64: r z p q; mixed: r q xc, two pairs, FP64 residual
         const size_t n0 = A->nrows;
         N.vec = take(sizeof(T) == 8 ? 4 * al(n0 * 8) : 3 * al(n0 * 4) + 2 * al(n0 * 8) + al(n0 * 8));
@@ -1236,16 +1234,17 @@ int mg_probe(grmp_matrix A, double *react) {
     MgCache &C = *A->mg;
     MgCache::Num &N = C.num[sizeof(T) == 8 ? 0 : 1];
     const int n = A->nrows, cl = rows_lanes<T>(n), grid = std::max(1, std::min({nblk(n, kTB / cl), 4 * ctx->num_sms, 2048}));
-    cudaMemsetAsync(N.bad, 0, 4, ctx->stream);
+    cudaMemsetAsync(N.part, 0, 16, ctx->stream);   // the flag of a bad diagonal, then the blocks' sums
     auto kern = cl == 2 ? k_mg_rows<T, 2> : k_mg_rows<T, 8>;
     kern<<<grid, kTB, 0, ctx->stream>>>(n, A->d_rowptr, A->d_cols, fine_values<T>(A), (T *)N.D[0],
                                                 (uint8_t *)N.iso[0], A->eliminated ? A->d_fixed : nullptr,
-                                                (double2 *)N.part, N.bad);
+                                                (double2 *)N.part + 1, (int *)N.part);
     GRMP_LAUNCHED(ctx);
-    double h[2 * 2048];
+    double buf[2 * 2049];
+    cudaError_t e = grmp_readback(ctx, buf, N.part, (size_t)(grid + 1) * 16);
+    const double *h = buf + 2;
     int bad = 0;
-    cudaError_t e = grmp_readback(ctx, h, N.part, (size_t)grid * 16);
-    if (e == cudaSuccess) e = grmp_readback(ctx, &bad, N.bad, 4);
+    std::memcpy(&bad, buf, 4);
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multilevel: diagonal");
     if (bad) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "solve: non-positive or non-finite diagonal entry");
     double s = 0, d = 0;

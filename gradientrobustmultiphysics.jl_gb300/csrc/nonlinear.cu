@@ -90,68 +90,88 @@ __global__ void __launch_bounds__(128) k_nl_cells(int ncells, const double *coor
     double A[3][3], G[3][3], vol;
     simplex_geometry_rn<DIM>(X, A, G, vol);
     double uc[LD];
+#pragma unroll
     for (int b = 0; b < LD; b++) uc[b] = u[celldofs[(size_t)cell * LD + b]];
     const int cj = j / NB, aj = j - cj * NB;
     double lm[LD];
+#pragma unroll
     for (int i = 0; i < LD; i++) lm[i] = 0.0;
     double lb = 0.0;
     for (int q = 0; q < t.tab.nq; q++) {
-        const double *vq = t.tab.vals + (size_t)q * NB;
-        double gr[NB][DIM];
-        for (int a = 0; a < NB; a++)
+        const double *vq = t.tab.vals + (size_t)q * NB, *dq = t.tab.derivs + (size_t)q * NB * DIM;
+        // current iterate's operator evaluations: values, then gradients per component
+        double in[ID];
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            double val = 0.0, rg[DIM];
+#pragma unroll
+            for (int l = 0; l < DIM; l++) rg[l] = 0.0;
+#pragma unroll
+            for (int a = 0; a < NB; a++) {
+                val += uc[c * NB + a] * vq[a];
+#pragma unroll
+                for (int l = 0; l < DIM; l++) rg[l] += uc[c * NB + a] * dq[a * DIM + l];
+            }
+            in[c] = val;
+#pragma unroll
             for (int k = 0; k < DIM; k++) {
                 double s = 0.0;
-                for (int l = 0; l < DIM; l++) s += G[k][l] * t.tab.derivs[((size_t)q * NB + a) * DIM + l];
-                gr[a][k] = s;
-            }
-        // current iterate's operator evaluations (in the DoF order of eval_febe!)
-        double in[ID];
-        for (int m = 0; m < ID; m++) in[m] = 0.0;
-        for (int b = 0; b < LD; b++) {
-            const int c = b / NB, a = b - c * NB;
-            if (NC == 1) {
-                in[0] += uc[b] * vq[a];
-                for (int k = 0; k < DIM; k++) in[1 + k] += uc[b] * gr[a][k];
-            } else {
-                in[c] += uc[b] * vq[a];
-                for (int k = 0; k < DIM; k++) in[DIM + c * DIM + k] += uc[b] * gr[a][k];
+#pragma unroll
+                for (int l = 0; l < DIM; l++) s += G[k][l] * rg[l];
+                in[NC + c * DIM + k] = s;
             }
         }
         double K[DIM], J[DIM][ID];
         nl_kernel<DIM, NC>(t, in, K, J);
-        // test operator of phi_j: gradient (scalar kernels) or identity (convection)
+        // test operator of phi_j: gradient (scalar kernels) or identity (convection), times the weight
         double tv[DIM];
-        for (int k = 0; k < DIM; k++) tv[k] = NC == 1 ? gr[aj][k] : (k == cj ? vq[aj] : 0.0);
-        const double w = t.tab.w[q];
-        for (int i = 0; i < LD; i++) {
-            const int ci = i / NB, ai = i - ci * NB;
-            double in2[ID];
-            for (int m = 0; m < ID; m++) in2[m] = 0.0;
-            if (NC == 1) {
-                in2[0] = vq[ai];
-                for (int k = 0; k < DIM; k++) in2[1 + k] = gr[ai][k];
-            } else {
-                in2[ci] = vq[ai];
-                for (int k = 0; k < DIM; k++) in2[DIM + ci * DIM + k] = gr[ai][k];
-            }
-            double temp = 0.0;
-            for (int k = 0; k < DIM; k++) {
-                double ar = 0.0;
-                for (int m = 0; m < ID; m++) ar += J[k][m] * in2[m];
-                temp += ar * tv[k];
-            }
-            lm[i] += temp * w;
-        }
-        double temp = 0.0;
+#pragma unroll
         for (int k = 0; k < DIM; k++) {
-            double ar = 0.0;
-            for (int m = 0; m < ID; m++) ar += J[k][m] * in[m];
-            temp += (ar - K[k]) * tv[k];
+            double s = 0.0;
+            if (NC == 1) {
+#pragma unroll
+                for (int l = 0; l < DIM; l++) s += G[k][l] * dq[aj * DIM + l];
+            } else {
+                s = k == cj ? vq[aj] : 0.0;
+            }
+            tv[k] = s * t.tab.w[q];
         }
-        lb += temp * w;
+        // w_m = tv . dK / din_m; the contribution of phi_i is sum_m w_m in_m(phi_i).  (With physical
+        // gradients: couplings that vanish by orthogonality are exact zeros, as k_nl_gather expects.)
+        double wm[ID];
+#pragma unroll
+        for (int m = 0; m < ID; m++) {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < DIM; k++) s += tv[k] * J[k][m];
+            wm[m] = s;
+        }
+#pragma unroll
+        for (int m = 0; m < ID; m++) lb += wm[m] * in[m];
+#pragma unroll
+        for (int k = 0; k < DIM; k++) lb -= K[k] * tv[k];
+#pragma unroll
+        for (int a = 0; a < NB; a++) {
+            double gr[DIM];
+#pragma unroll
+            for (int k = 0; k < DIM; k++) {
+                double s = 0.0;
+#pragma unroll
+                for (int l = 0; l < DIM; l++) s += G[k][l] * dq[a * DIM + l];
+                gr[k] = s;
+            }
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+                double s = wm[c] * vq[a];
+#pragma unroll
+                for (int k = 0; k < DIM; k++) s += wm[NC + c * DIM + k] * gr[k];
+                lm[c * NB + a] += s;
+            }
+        }
     }
     const double itemfactor = vol * t.factor;
     double *row = LT + ((size_t)cell * LD + j) * LD;
+#pragma unroll
     for (int i = 0; i < LD; i++) row[i] = lm[i] * itemfactor;
     LB[(size_t)cell * LD + j] = lb * itemfactor;
 }
@@ -196,7 +216,9 @@ template <int DIM, int NB, int NC>
 void launch_nl_cells(grmp_space s, const double *u, const NlDev &t, double *LT, double *LB) {
     grmp_mesh m = s->mesh;
     const long long n = (long long)m->ncells * NB * NC;
-    k_nl_cells<DIM, NB, NC><<<nblk(n, 128), 128, 0, m->ctx->stream>>>(m->ncells, m->d_coords, m->d_cells,
+    // FP64 issue is the bound: small meshes spread warp by warp over the SMs
+    const int tpb = n <= 4LL * 128 * m->ctx->num_sms ? 32 : 128;
+    k_nl_cells<DIM, NB, NC><<<nblk(n, tpb), tpb, 0, m->ctx->stream>>>(m->ncells, m->d_coords, m->d_cells,
                                                                       s->d_celldofs, u, t, LT, LB);
 }
 

@@ -10,6 +10,7 @@
 // the order-4 rule (BDM2) -- integrates f against the Piola-mapped target
 // basis and writes the 14 local values; a row kernel then adds each DoF's
 // cell values in ascending cell order (deterministic, no atomics).
+#include "element.cuh"
 #include "grmp_internal.h"
 
 #include <cstring>
@@ -28,6 +29,7 @@ struct P2bMesh {
 
 struct P2bRhs {
     const double *par;     // [ngroups][nt][5] polynomial terms (component, coef, e1, e2, e3)
+    const PolyTerm *term;  // the same, decoded
     int nt;
     const int32_t *group;  // [ncells] group of each cell (nullptr: one group)
     double factor;
@@ -38,16 +40,6 @@ struct P2bRhs {
     double x4[16][2];
     double w4[16];
 };
-
-__device__ __forceinline__ double p2b_pow(double x, double e) {
-    const int k = (int)e;
-    if ((double)k == e && k >= 0 && k <= 8) {
-        double r = 1.0;
-        for (int i = 0; i < k; i++) r *= x;
-        return r;
-    }
-    return pow(x, e);
-}
 
 // RT1 / BDM2 reference basis (src/fedefs/hdiv_rt1.jl:106-121,
 // src/fedefs/hdiv_bdm2.jl:171-194)
@@ -317,40 +309,36 @@ __global__ void __launch_bounds__(128) k_p2b_rhs_cells(int ncells, P2bMesh m, P2
         }
     }
     // (f, R phi_I) on the rhs rule
-    const double *par = r.par + (size_t)(r.group ? r.group[cell] : 0) * r.nt * 5;
-    double lbv[14];
-    for (int i = 0; i < 14; i++) lbv[i] = 0.0;
+    const size_t g0t = (size_t)(r.group ? r.group[cell] : 0) * r.nt;
+    const double *par = r.par + g0t * 5;
+    const PolyTerm *term = r.term + g0t;
+    // products of f with the target's functions, then with the coefficients: 2 NR
+    // operations a point instead of 28 NR (one of each for every function)
+    double h[NR];
+#pragma unroll
+    for (int j = 0; j < NR; j++) h[j] = 0.0;
     for (int q = 0; q < r.nq; q++) {
         const double xi = r.xref[q][0], eta = r.xref[q][1];
-        double rb[NR][2], te[NR][2];
+        double rb[NR][2];
         recon_basis<NR>(xi, eta, rb);
-        for (int j = 0; j < NR; j++)
-            for (int k = 0; k < 2; k++) {
-                double s = 0;
-                for (int l = 0; l < 2; l++) s += A[k][l] * rb[j][l];
-                s *= coef[j] / det;
-                te[j][k] = s;
-            }
-        double x[2], f[2] = {0, 0};
-        for (int k = 0; k < 2; k++) {
-            x[k] = X[k];
-            for (int j = 0; j < 2; j++) x[k] += A[k][j] * (j == 0 ? xi : eta);
-        }
+        double x[2], f0 = 0.0, f1 = 0.0;
+        for (int k = 0; k < 2; k++) x[k] = X[k] + A[k][0] * xi + A[k][1] * eta;
         for (int t = 0; t < r.nt; t++) {
-            const int c = (int)par[5 * t];
-            double v = par[5 * t + 1];
-            for (int j = 0; j < 2; j++) v *= p2b_pow(x[j], par[5 * t + 2 + j]);
-            f[c] += v;
+            const PolyTerm pt = term[t];
+            double v = poly_factor(pt.coef, x[0], (pt.code >> 4) & 15, par + 5 * t + 2);
+            v = poly_factor(v, x[1], (pt.code >> 8) & 15, par + 5 * t + 3);
+            if ((pt.code & 15) == 0) f0 += v;
+            else f1 += v;
         }
-        for (int i = 0; i < 14; i++) {
-            double cv[2] = {0, 0};
-            for (int j = 0; j < NR; j++)
-                if (R[i][j] != 0)
-                    for (int k = 0; k < 2; k++) cv[k] += R[i][j] * te[j][k];
-            double t = 0;
-            for (int k = 0; k < 2; k++) t += f[k] * cv[k];
-            lbv[i] += t * r.w[q];
-        }
+        const double g0 = r.w[q] * (A[0][0] * f0 + A[1][0] * f1), g1 = r.w[q] * (A[0][1] * f0 + A[1][1] * f1);
+#pragma unroll
+        for (int j = 0; j < NR; j++) h[j] += rb[j][0] * g0 + rb[j][1] * g1;
+    }
+    double lbv[14];
+    for (int i = 0; i < 14; i++) lbv[i] = 0.0;
+    for (int j = 0; j < NR; j++) {
+        const double hj = h[j] * (coef[j] / det);
+        for (int i = 0; i < 14; i++) lbv[i] += R[i][j] * hj;
     }
     const double itemfactor = r.factor * vol;
     for (int i = 0; i < 14; i++) loc[(size_t)cell * 14 + i] = lbv[i] * itemfactor;
@@ -411,10 +399,15 @@ int grmp_p2b_rhs(grmp_space s, const grmp_rhs *rhs, grmp_vector b) {
     double *dpar = nullptr;
     int32_t *dgrp = nullptr;
     int rc = grmp_upload(ctx, &dpar, rhs->params, (size_t)rhs->nparams);
+    std::vector<PolyTerm> term((size_t)(ng * nt));
+    for (size_t t = 0; t < term.size(); t++) term[t] = poly_term(rhs->params + 5 * t);
+    PolyTerm *dterm = nullptr;
+    if (!rc) rc = grmp_upload(ctx, &dterm, term.data(), term.size());
     if (!rc && rhs->cell_group) rc = grmp_upload(ctx, &dgrp, rhs->cell_group, (size_t)m->ncells);
     if (!rc && !s->d_locbuf) rc = grmp_alloc(ctx, (void **)&s->d_locbuf, (size_t)m->ncells * 14 * 8);
     if (!rc) {
         r.par = dpar;
+        r.term = dterm;
         r.group = dgrp;
         const P2bMesh pm{m->d_coords, m->d_cells, m->d_cell_faces, m->d_face_normals, m->d_face_volumes,
                          m->d_cell_face_signs};
@@ -431,6 +424,7 @@ int grmp_p2b_rhs(grmp_space s, const grmp_rhs *rhs, grmp_vector b) {
         if (e != cudaSuccess) rc = grmp_cuda_fail(ctx, e, "H1P2B rhs");
     }
     grmp_free(ctx, dpar, (size_t)rhs->nparams * 8);
+    grmp_free(ctx, dterm, term.size() * sizeof(PolyTerm));
     grmp_free(ctx, dgrp, (size_t)m->ncells * 4);
     return rc;
 }
