@@ -308,6 +308,8 @@ def duo_family(cfg: int) -> bool:
 
 
 def pcg_kernel(cfg: int) -> str:
+    if cfg >= 90000:
+        return "k_mgcg_mixed"
     if 64000 <= cfg < 67000:
         return "k_pcg_mixed_duo_keep"
     if duo_family(cfg):
@@ -323,10 +325,12 @@ def pcg_bytes(stats: dict, n: int, nnz: int, mixed: bool) -> float:
     FP32 iteration the matrix once (4-byte value + 4-byte column per entry)
     and the vector traffic of Jacobi-PCG's update phase (seven 8-byte streams
     per row); per FP64 refinement one FP64 residual.  A format or kernel that
-    moves fewer bytes shows as DRAM traffic below these bytes."""
+    moves fewer bytes shows as DRAM traffic below these bytes.  Multilevel
+    solves (9xxxx) add the first restriction and prolongation, two entries a
+    row each; their coarser levels are not counted."""
     it, outer = stats["iterations"], stats["outer_iterations"]
     if mixed:
-        per_it = 8.0 * nnz + 56.0 * n
+        per_it = 8.0 * nnz + 56.0 * n + (36.0 * n if stats.get("spmv_config", 0) >= 90000 else 0.0)
         per_outer = 12.0 * nnz + 64.0 * n
         return it * per_it + (outer + 1) * per_outer
     return it * (12.0 * nnz + 108.0 * n) + 2 * (12.0 * nnz + 36.0 * n)
