@@ -727,13 +727,17 @@ class GB300PCG:
     """The linear solver handed to solve! as `linsolver` (the LinearSolve
     algorithm slot of default_solver_kwargs, src/solvers.jl:55).
 
-    mode "fp64": Jacobi-PCG in FP64.  mode "mixed": FP32 Jacobi-PCG inside an
-    FP64 refinement loop (FP64 residual b - A x and solution update).
+    mode "fp64": preconditioned CG in FP64.  mode "mixed": FP32 CG inside an
+    FP64 refinement loop (FP64 residual b - A x and solution update).  Scalar
+    H1P1 / H1P2 matrices with a diffusion term are preconditioned by a
+    multilevel cycle (unless spmv_config asks for a Jacobi configuration, the
+    system is small or reaction dominated), all others by Jacobi.
     mode "direct": FP64 multifrontal Cholesky + residual refinement (the
     counterpart of the reference's sparse-direct default).  mode
     "mixed_direct": FP32 multifrontal Cholesky as the preconditioner of FP64
-    conjugate gradients.  mode "bicgstab": FP64 Jacobi-preconditioned
-    BiCGStab for non-symmetric matrices (Newton steps of a NonlinearForm)."""
+    conjugate gradients.  mode "bicgstab": FP64 BiCGStab for
+    non-symmetric matrices (Newton steps of a NonlinearForm), multilevel
+    preconditioned on scalar spaces, else Jacobi."""
     mode: str = "fp64"
     abstol: float = 1e-12
     reltol: float = 1e-12

@@ -1,5 +1,5 @@
 // Batched iterated-penalty Stokes solver: many independent Bernardi-Raugel /
-// P0 problems, one thread block per problem, all in one launch.
+// P0 problems.
 //
 // Reference: solve_fixpoint_subiterations! (src/solvers.jl:1018-1250) with
 // subiterations [[1],[2]] on the operators of
@@ -8,13 +8,16 @@
 //                      = (f, R v) + (p, div v)            [R: BR -> RT0]
 //   pressure update  (p_new, q) = (p, q) - lambda (div u, q)  on P0
 //   FixedIntegralMean(2, 0): the pressure has zero mean (src/globalconstraints.jl:23-44).
-// The velocity system is solved by Jacobi-PCG (FP64, or FP32 inside FP64
-// refinement) warm-started from the previous sweep's velocity.
+// DIRECT factors all problems of a memory-bounded part of the batch together,
+// level by level over the forest of their assembly trees (forest.cu); the
+// sweeps run chunks of 512 rows of all problems a launch, with per-problem
+// sums over the chunks in order and decisions taken on the device (k_sb_*).
 //
-// Scheduling: a persistent grid of blocks pulls problems from a work queue
-// sorted by size (largest first).  A problem never spans blocks, all its
-// reductions are block reductions in a fixed order, so its result does not
-// depend on which block runs it or on the rest of the batch.
+// The iterative modes (Jacobi-PCG, FP64 or FP32 inside FP64 refinement, warm
+// started) and MIXED_DIRECT run a problem per block: a persistent grid pulls
+// problems from a queue sorted by size (largest first), and all reductions
+// are block reductions in a fixed order.  In every mode a problem's result
+// does not depend on the rest of the batch.
 #include <algorithm>
 #include <atomic>
 #include <cmath>

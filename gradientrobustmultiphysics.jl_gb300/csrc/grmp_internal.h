@@ -179,8 +179,8 @@ int grmp_alloc(grmp_context ctx, void **p, size_t bytes);
 void grmp_free(grmp_context ctx, void *p, size_t bytes);
 // Small results to the host and a stream synchronize, through page-locked
 // memory: a copy to pageable memory waits for the stream's kernels inside the
-// driver and keeps other threads' calls out meanwhile, so the solves of four
-// serving slots ran one after another (12 requests 11.5 ms, now 5.9 ms).
+// CUDA library and keeps other threads' calls out meanwhile, so the solves of four
+// serving slots ran one after another (12 requests 11.5 ms, 5.9 ms with it).
 // Called with the context's lock held.
 constexpr size_t kPinBytes = 64 << 10;
 cudaError_t grmp_readback(grmp_context ctx, void *host, const void *dev, size_t bytes);

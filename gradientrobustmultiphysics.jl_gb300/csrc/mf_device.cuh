@@ -1,6 +1,6 @@
-// Dense kernels of the multifrontal Cholesky factorisation, shared by the
-// batched Stokes solver (one problem per block, FP64) and the single-problem
-// direct solvers (FP64, or FP32 as a preconditioner).
+// Dense kernels of the multifrontal Cholesky factorisation of one problem per
+// block: the batched Stokes solver with an FP32 factor (MIXED_DIRECT) and its
+// FP64 fallback.  (The other direct solvers run on forest.cu.)
 #pragma once
 
 constexpr int kPanel = 16;

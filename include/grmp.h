@@ -402,8 +402,8 @@ int grmp_apply_dirichlet(grmp_matrix A, grmp_vector b, int32_t nfixed, const int
 /* ------------------------------------------------------------------ solve */
 
 typedef enum {
-    GRMP_SOLVE_FP64 = 0,   /* plain: FP64 Jacobi-PCG                                                 */
-    GRMP_SOLVE_MIXED = 1,  /* FP32 Jacobi-PCG inside FP64 refinement (outer residual, update in FP64) */
+    GRMP_SOLVE_FP64 = 0,   /* plain: FP64 PCG (multilevel or Jacobi, see grmp_solve)               */
+    GRMP_SOLVE_MIXED = 1,  /* FP32 PCG inside FP64 refinement (outer residual, update in FP64)      */
     GRMP_SOLVE_DIRECT = 2, /* FP64 multifrontal Cholesky (nested-dissection order) + residual
                               refinement against the assembled FP64 matrix; in
                               grmp_stokes_batch_solve one factorisation per problem, reused by
@@ -411,7 +411,7 @@ typedef enum {
     GRMP_SOLVE_MIXED_DIRECT = 3, /* grmp_solve only: FP32 multifrontal Cholesky used as the
                               preconditioner of FP64 conjugate gradients on the FP64 matrix
                               (Dirichlet rows must be eliminated: 1e60 overflows FP32)           */
-    GRMP_SOLVE_BICGSTAB = 4 /* grmp_solve only: FP64 Jacobi-preconditioned BiCGStab in one
+    GRMP_SOLVE_BICGSTAB = 4 /* grmp_solve only: FP64 BiCGStab (multilevel or Jacobi) in one
                               persistent launch, for non-symmetric matrices (the Jacobian of a
                               NonlinearForm's Newton step, where the reference calls a sparse LU) */
 } grmp_solve_mode;
@@ -470,7 +470,13 @@ int grmp_solve_params_default(grmp_solve_params *p);
 /* Solve A x = b.  Stands in for init(LinearProblem(A, b), alg; abstol, reltol)
  * + LinearSolve.solve(cache) (src/solvers.jl:89-101, :658-661).  `x` is
  * overwritten.  Returns GRMP_ERR_NOT_CONVERGED (with x = the last iterate)
- * when the caps are hit; device-side waits are bounded (GRMP_ERR_TIMEOUT). */
+ * when the caps are hit; device-side waits are bounded (GRMP_ERR_TIMEOUT).
+ * FP64, MIXED and BICGSTAB: a matrix of a scalar H1P1 / H1P2 space whose last
+ * assembly had a diffusion term (Laplace, or a diffusion Newton term) is
+ * preconditioned by a multilevel cycle, reported as spmv_config 90000 + ...,
+ * when spmv_config <= 0, the system is large enough and not reaction
+ * dominated, and the hierarchy fits in memory; otherwise by Jacobi.  BICGSTAB
+ * falls back to Jacobi where the cycle does not converge. */
 int grmp_solve(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solve_params *params,
                grmp_solve_stats *stats);
 
@@ -492,7 +498,8 @@ int grmp_spmv(grmp_matrix A, int precision, grmp_vector x, grmp_vector y);
  *     with GRMP_ERR_INVALID_ARG.  params->mode must be GRMP_SOLVE_FP64
  *     (GRMP_ERR_UNSUPPORTED otherwise).  spmv_config 0 uses the matrix's
  *     tuned configuration if grmp_solve has tuned it, else a heuristic; no
- *     tuning runs here.
+ *     tuning runs here.  A matrix whose multilevel hierarchy an FP64
+ *     grmp_solve has built is solved with it, in the hierarchy's storage.
  *   - The first call on a device looks up the scratch address (set-up);
  *     make it before any stream capture on that device begins.
  *   - The grid-barrier counters, the status word and the diagonal check flag
