@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(PTPB, 4) k_bicgstab64(int n, const int32_t *ro
     const double bn = sqrt(w3[2]);
     const double tol = fmax(abstol, reltol * bn);
     double alpha = 1.0, omega = 1.0, beta = 0.0;
-    int it = 0;
+    int it = 0, restarts = 0;
     bool conv = sqrt(rr) <= tol;
     while (!conv && it < maxit) {
         for (int i = gtid; i < n; i += gsz) {
@@ -208,9 +208,17 @@ __global__ void __launch_bounds__(PTPB, 4) k_bicgstab64(int n, const int32_t *ro
         it++;
         rr = w2[1];
         conv = sqrt(rr) <= tol;
-        if (!conv && (!(w2[0] != 0.0) || !(omega != 0.0))) {   // breakdown
-            if (gtid == 0) atomicCAS(&st->status, 0, (int)GRMP_ERR_NAN);
-            break;
+        if (!conv && (!(w2[0] != 0.0) || !(omega != 0.0))) {
+            // breakdown: r has become orthogonal to the shadow vector (rounding, on iterations that
+            // stagnate); go on from r as a new start, a few times
+            if (!isfinite(rr) || !(rr > 0.0) || restarts++ >= 8) {
+                if (gtid == 0) atomicCAS(&st->status, 0, (int)GRMP_ERR_NAN);
+                break;
+            }
+            for (int i = gtid; i < n; i += gsz) rh[i] = r[i];
+            rho = rr;
+            beta = 0.0;
+            continue;
         }
         beta = (w2[0] / rho) * (alpha / omega);
         rho = w2[0];
