@@ -75,6 +75,7 @@ struct grmp_matrix_s {
     int32_t *d_cols = nullptr;      // [nnz]
     void *d_slot = nullptr;         // [ninc][ldofs] uint8 or uint16 (row-relative slot, all-ones = dropped)
     int slot_bytes = 1;
+    bool face_coupled = false;      // the pattern couples face neighbours too (built with face terms)
     double *d_vals64 = nullptr;     // [nnz]
     float *d_vals32 = nullptr;      // [nnz]
     void *d_pack32 = nullptr;       // [nnz] int2 (column, FP32 value bits), built by mixed solves

@@ -515,12 +515,12 @@ int mf_build(grmp_matrix A) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(ci.data(), A->d_cols, (size_t)A->nnz * 4, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multifrontal: pattern download");
-    // separators in the mesh's graph, where the matrix was assembled on one by
-    // cell terms (face terms couple further)
+    // separators in the graph of the mesh's cells, which has to cover the pattern:
+    // face terms couple across its separators, their matrices use the pattern itself
     grmp_space s = A->space;
     NdGraph G;
     bool mesh_graph = false;
-    if (!A->imported && s->d_celldofs && (s->fe == GRMP_FE_H1P1 || s->fe == GRMP_FE_H1P2)) {
+    if (!A->imported && !A->face_coupled && s->d_celldofs && (s->fe == GRMP_FE_H1P1 || s->fe == GRMP_FE_H1P2)) {
         std::vector<int32_t> cd((size_t)s->mesh->ncells * s->ldofs);
         e = cudaMemcpyAsync(cd.data(), s->d_celldofs, cd.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -528,8 +528,7 @@ int mf_build(grmp_matrix A) {
         mesh_graph = nd_cell_graph(n, s->mesh->ncells, s->ldofs, s->ncomp, cd.data(), &G) == 0;
     }
     MfCache *C = new MfCache;
-    int src = nd_symbolic_build(n, rp.data(), ci.data(), &C->S, mesh_graph ? &G : nullptr);
-    if (src == 3 && mesh_graph) src = nd_symbolic_build(n, rp.data(), ci.data(), &C->S);
+    const int src = nd_symbolic_build(n, rp.data(), ci.data(), &C->S, mesh_graph ? &G : nullptr);
     if (src) {
         delete C;
         return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "multifrontal: symbolic analysis failed (%d)", src);

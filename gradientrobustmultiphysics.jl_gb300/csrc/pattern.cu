@@ -539,6 +539,7 @@ int grmp_pattern_build_impl(grmp_space s, int nterms, const grmp_bilinear_term *
     grmp_matrix A = new grmp_matrix_s();
     A->space = s;
     A->nrows = s->ndofs;
+    A->face_coupled = faces;
     int32_t *cnt = nullptr, *dmax = nullptr;
     int *dovf = nullptr;
     rc = grmp_alloc(ctx, (void **)&cnt, ((size_t)A->nrows + 1) * 4);
