@@ -1093,7 +1093,7 @@ int mg_build(grmp_matrix A) {
     A->mg = C;
     C->mult = fine_mult(s->mesh->dim, s->fe, n);
     if (mg_symbolic_build(n, rp.data(), ci.data(), s->mesh->dim, s->mesh->ncells, s->ldofs, cd.empty() ? nullptr : cd.data(),
-                          coords.data(), cells.data(), C->mult, &C->S)) {
+                          coords.data(), cells.data(), !A->face_coupled, C->mult, &C->S)) {
         A->mg_state = -1;
         return GRMP_OK;
     }

@@ -6,7 +6,7 @@
 // its edges.  Every other step aggregates: a row whose neighbours are all
 // free takes them as one aggregate, rows left over join an aggregate next to
 // them (Vanek, Mandel, Brezina 1996).  The vertex level keeps only couplings
-// that P1 stiffness has: on right angles (squares split in triangles, Kuhn
+// that P1 stiffness has on some cell: on right angles (squares split in triangles, Kuhn
 // cubes) half of the neighbours do not couple, and aggregates that take them
 // in span two couplings where the smoothed prolongation reaches one (128 x
 // 128: 56 iterations with them, about half without).  Patterns include the DoFs that a call
@@ -107,9 +107,12 @@ int aggregate(int n, const int32_t *rp, const int32_t *ci, std::vector<int32_t> 
     return na;
 }
 
-// Drops from the vertex level's pattern the pairs without P1 stiffness (unit
-// coefficient): a statement about the mesh, so one hierarchy serves every
-// coefficient.
+// Drops from the vertex level's pattern the pairs that have no P1 stiffness on
+// any of their cells: a statement about the mesh that holds for every
+// coefficient, so one hierarchy serves them all.  (Not the pairs whose cells
+// cancel for the unit coefficient, as the diagonals of isosceles trapezoids:
+// they couple as soon as the coefficient varies, and a coupling that the
+// pattern lacks goes to the diagonal, which then need not stay positive.)
 void filter_vertex_level(MgStep *s, int dim, int ncells, int ld, const int32_t *celldofs, const std::vector<int32_t> &vert,
                          const double *coords, const int32_t *cells) {
     const int nv = dim + 1, nc = s->nc;
@@ -159,7 +162,7 @@ void filter_vertex_level(MgStep *s, int dim, int ncells, int ld, const int32_t *
                 const int J = vert[celldofs[c * ld + b]];
                 const int32_t *r = s->Ac.ci.data() + s->Ac.rp[i], *re = s->Ac.ci.data() + s->Ac.rp[i + 1];
                 const int32_t *f = std::lower_bound(r, re, J);
-                if (f != re && *f == J) K[f - s->Ac.ci.data()] += d / (det != 0 ? std::fabs(det) : 1.0);
+                if (f != re && *f == J) K[f - s->Ac.ci.data()] += std::fabs(d) / (det != 0 ? std::fabs(det) : 1.0);
             }
         }
         for (int k = s->Ac.rp[i]; k < s->Ac.rp[i + 1]; k++)
@@ -169,7 +172,7 @@ void filter_vertex_level(MgStep *s, int dim, int ncells, int ld, const int32_t *
     build_rows(nc, nc, &F, [&](int i, auto add) {
         for (int k = s->Ac.rp[i]; k < s->Ac.rp[i + 1]; k++) {
             const int j = s->Ac.ci[k];
-            if (j == i || std::fabs(K[k]) > 1e-6 * std::sqrt(std::fabs(diag[i] * diag[j]))) add(j);
+            if (j == i || K[k] > 1e-6 * std::sqrt(diag[i] * diag[j])) add(j);
         }
     });
     s->filtered = F.ci.size() < s->Ac.ci.size();
@@ -195,7 +198,7 @@ void products(MgStep *s, const int32_t *rp, const int32_t *ci) {
 }  // namespace
 
 int mg_symbolic_build(int n, const int32_t *rp, const int32_t *ci, int dim, int ncells, int ld, const int32_t *celldofs,
-                      const double *coords, const int32_t *cells, bool fine_q, MgSymbolic *S) {
+                      const double *coords, const int32_t *cells, bool cell_terms, bool fine_q, MgSymbolic *S) {
     S->step.clear();
     const int32_t *crp = rp, *cci = ci;
     int cn = n;
@@ -244,7 +247,7 @@ int mg_symbolic_build(int n, const int32_t *rp, const int32_t *ci, int dim, int 
             });
         }
         products(&s, crp, cci);
-        if (s.geometric) filter_vertex_level(&s, dim, ncells, ld, celldofs, vert, coords, cells);
+        if (s.geometric && cell_terms) filter_vertex_level(&s, dim, ncells, ld, celldofs, vert, coords, cells);
         if (fine_q || !S->step.empty()) transpose(s.n, s.nc, s.AP, &s.QT, &s.QTperm);
         cn = s.nc;
         S->step.push_back(std::move(s));

@@ -31,7 +31,9 @@ constexpr int kMgMaxLevels = 14;
 // Builds the steps of a matrix with pattern (n, rp, ci).  celldofs != nullptr:
 // a P2 space's cell DoFs [ncells][ld] (dim + 1 vertices, then edges) on the
 // mesh (coords, cells); the first step then interpolates from the vertices.
+// cell_terms: the matrix has terms on cells only (face terms couple vertices
+// that have no stiffness in common: nothing is left out then).
 // fine_q: the transpose of Q also for step 0.  Returns 0, or 1 when the matrix
 // does not coarsen.
 int mg_symbolic_build(int n, const int32_t *rp, const int32_t *ci, int dim, int ncells, int ld, const int32_t *celldofs,
-                      const double *coords, const int32_t *cells, bool fine_q, MgSymbolic *S);
+                      const double *coords, const int32_t *cells, bool cell_terms, bool fine_q, MgSymbolic *S);
