@@ -64,6 +64,18 @@ constexpr double kMaxReaction = 0.02;
 // iterates, up to 95 on white noise, where Jacobi takes 200-800), or have not
 // gained a digit after kStallBicg, are left to the Jacobi iteration
 constexpr int kMaxBicg = 200, kStallBicg = 40;
+// Conjugate gradients are given up when, kStall iterations times k = 2, 3, ...
+// on, the residual has not fallen by k digits: mixed solves then go on with the
+// FP64 cycle, FP64 ones with the Jacobi iteration.  Coefficients that jump by
+// 1e5 and more across element sides, and long strips fixed at one end, lose the FP32
+// recurrence its conjugacy (80^2 P1 squares, contrast 1e6, to 1e-8: no convergence in
+// 20,000 FP32 iterations, 274 in FP64; Jacobi 990 / 2,163 in FP64 / mixed).  What converges
+// keeps ahead of that: lognormal coefficients with sigma 3 (435 iterations to 1e-11)
+// have lost five digits at 128; FP64 at contrast 1e6 two at 128, four to six at 256.
+constexpr int kStall32 = 64, kStall64 = 128;
+__device__ __forceinline__ bool mg_stalled(int it, int every, double rn, double rn0) {
+    return it >= 2 * every && it % every == 0 && rn > rn0 * (double)exp10f(-(float)(it / every));
+}
 
 // Rows from which the multilevel solver is taken: where whole passes are no
 // slower than with Jacobi-PCG for constant coefficients (lognormal ones gain
@@ -715,10 +727,10 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
         v[1] += b[i] * b[i];
     }
     if (!sy.template sum<2>(v, sh)) return;
-    const double bn = sqrt(v[1]);
+    const double bn = sqrt(v[1]), rn0 = sqrt(v[0]);
     const double tol = fmax(abstol, reltol * bn);
     int it = 0;
-    bool conv = sqrt(v[0]) <= tol;
+    bool conv = rn0 <= tol;
     double rz = 0.0;
     while (!conv && it < maxit) {
         if (!mg_cycle(m, (const double *)r, eb, sy)) return;
@@ -750,7 +762,9 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
         }
         if (!sy.template sum<1>(rr, sh)) return;
         it++;
-        conv = sqrt(rr[0]) <= tol;
+        const double rn = sqrt(rr[0]);
+        conv = rn <= tol;
+        if (!conv && mg_stalled(it, kStall64, rn, rn0)) break;
     }
     if (!sy.barrier()) return;
     double t[1];
@@ -759,6 +773,7 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     if (gtid == 0) {
         st->iters = it;
         st->outer = 0;
+        st->nearer = sqrt(t[0]) < rn0;
         st->relres = sqrt(t[0]) / (bn > 0 ? bn : 1.0);
         if (st->status == 0 && !(sqrt(t[0]) <= fmax(tol, 0.0) || conv)) st->status = GRMP_ERR_NOT_CONVERGED;
     }
@@ -906,7 +921,8 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     if (!sy.template sum<2>(v, sh)) return;
     const double bn = sqrt(v[1]);
     const double tol = fmax(abstol, reltol * bn);
-    double rn64 = sqrt(v[0]), prev_rn64 = rn64;
+    const double rn0 = sqrt(v[0]);
+    double rn64 = rn0, prev_rn64 = rn64;
     // the FP32 system is solved for the residual scaled to norm 1: the
     // correction and its residual stay in FP32's range at any size of b
     double scale = rn64 > 0 ? rn64 : 1.0;
@@ -984,6 +1000,7 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
         if (!sy.template sumf<1>(u, shf)) return;
         it++;
         const float rn32 = sqrtf(u[0]);
+        if (mg_stalled(it, kStall32, (double)rn32 * scale, rn0)) break;   // x: as of the last refinement
         restart = false;
         if (rn32 <= (float)delta * rmax || (double)rn32 * scale <= tol || it >= maxit) {
             for (int i = gtid; i < n; i += gsz) {
@@ -1020,6 +1037,7 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     if (gtid == 0) {
         st->iters = it;
         st->outer = outer;
+        st->nearer = rn64 < rn0;
         st->relres = rn64 / (bn > 0 ? bn : 1.0);
         if (st->status == 0 && !conv) st->status = GRMP_ERR_NOT_CONVERGED;
     }
@@ -1045,7 +1063,7 @@ struct MgCache {
         void *p = nullptr;
         size_t bytes = 0;
         std::vector<char *> pv, av, tv, cv, D, iso, r, y, e;
-        char *rv0 = nullptr, *ellv = nullptr, *binv = nullptr, *part = nullptr, *vec = nullptr, *z0 = nullptr;
+        char *rv0 = nullptr, *ellv = nullptr, *binv = nullptr, *part = nullptr, *vec = nullptr, *z0 = nullptr, *x0 = nullptr;
     } num[2];
     double react[2] = {0, 0};
     char *state = nullptr;
@@ -1198,6 +1216,7 @@ int mg_storage(grmp_matrix A) {
             }
         }
         N.z0 = take(C.mult ? (size_t)A->nrows * sizeof(T) : 0);
+        N.x0 = take((size_t)A->nrows * 8);   // the caller's start, while it may be needed again
         N.binv = take((size_t)kMgBottom * kMgBottom * sizeof(T));
         N.part = take((size_t)4096 * 16);
         // FP64: r z p q; mixed: r q xc, two pairs, FP64 residual
@@ -1536,15 +1555,18 @@ int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool bicg) {
     return GRMP_OK;
 }
 
-int grmp_mg_solve(grmp_matrix A, const double *b, double *x, const grmp_solve_params *p, grmp_solve_stats *st) {
+int grmp_mg_solve(grmp_matrix A, const double *b, double *x, bool mixed, grmp_solve_params *p, grmp_solve_stats *st,
+                  bool *done) {
     grmp_context ctx = A->space->mesh->ctx;
-    const bool mixed = p->mode == GRMP_SOLVE_MIXED;
     const double avg = (double)A->nnz / std::max(1, A->nrows);
     MgCache::Num &N = A->mg->num[mixed ? 1 : 0];
     const SolveState *dst = (const SolveState *)((char *)N.p + N.bytes - al(sizeof(SolveState)));
+    *done = true;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
+    if (p->use_initial_guess)
+        cudaMemcpyAsync(N.x0, x, (size_t)A->nrows * 8, cudaMemcpyDeviceToDevice, ctx->stream);
     cudaEventRecord(e0, ctx->stream);
     int grid = 0, code, rc;
     if (avg <= 8) {
@@ -1573,11 +1595,26 @@ int grmp_mg_solve(grmp_matrix A, const double *b, double *x, const grmp_solve_pa
     st->spmv_config = kMgConfig + code;
     st->grid_blocks = grid;
     st->solve_ms = ms;
-    if (hs.status == GRMP_ERR_NOT_CONVERGED)
-        return grmp_fail(ctx, GRMP_ERR_NOT_CONVERGED, "PCG: %d iterations, relative residual %.3e", hs.iters, hs.relres);
     if (hs.status == GRMP_ERR_TIMEOUT) return grmp_fail(ctx, GRMP_ERR_TIMEOUT, "PCG: a grid barrier wait timed out");
-    if (hs.status == GRMP_ERR_NAN) return grmp_fail(ctx, GRMP_ERR_NAN, "PCG: breakdown (non-positive or non-finite p.Ap)");
-    return hs.status;
+    if (hs.status != GRMP_ERR_NOT_CONVERGED && hs.status != GRMP_ERR_NAN) return hs.status;
+    // another solver goes on: from x if that is nearer, else from the start
+    *done = false;
+    if (hs.nearer) p->use_initial_guess = 1;
+    else if (p->use_initial_guess)
+        e = cudaMemcpyAsync(x, N.x0, (size_t)A->nrows * 8, cudaMemcpyDeviceToDevice, ctx->stream);
+    return e == cudaSuccess ? GRMP_OK : grmp_cuda_fail(ctx, e, "multilevel solve");
+}
+
+int grmp_mg_cg(grmp_matrix A, const double *b, double *x, grmp_solve_params *p, grmp_solve_stats *st, bool *done) {
+    *done = false;
+    for (int mixed = p->mode == GRMP_SOLVE_MIXED; mixed >= 0; mixed--) {
+        int use = 0;
+        int rc = grmp_mg_prepare(A, mixed, &use);
+        if (rc || !use) return rc;
+        rc = grmp_mg_solve(A, b, x, mixed, p, st, done);
+        if (rc || *done || st->iterations >= p->maxiter) return rc;
+    }
+    return GRMP_OK;
 }
 
 int grmp_mg_bicgstab(grmp_matrix A, const double *b, double *x, const grmp_solve_params *p, double *const vec[9],

@@ -23,7 +23,7 @@ struct SolveState {
     int status;
     int iters;
     int outer;
-    int pad;
+    int nearer;   // multilevel solves: x has a smaller residual than the start
     double relres;
 };
 

@@ -1945,11 +1945,12 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
     if (mixed && !A->has32) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "solve: MIXED needs FP32 values too");
     int n = A->nrows;
     const bool bicg = p->mode == GRMP_SOLVE_BICGSTAB;
+    grmp_solve_params q = *p;
     if (!bicg && p->spmv_config <= 0) {   // no configuration asked for: multilevel where it applies
-        int use = 0;
-        const int rc = grmp_mg_prepare(A, mixed, &use);
-        if (rc) return rc;
-        if (use) return grmp_mg_solve(A, b->d, x->d, p, st);
+        bool done = false;
+        const int rc = grmp_mg_cg(A, b->d, x->d, &q, st, &done);
+        if (rc || done) return rc;
+        std::memset(st, 0, sizeof(*st));
     }
     // workspace, each array 256-byte aligned:
     //   FP64 : dinv r z p q (double)                  | partials | state
@@ -2014,7 +2015,6 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
     A->duo_fresh = false;
     A->duo_sfresh = false;
     int cfg = p->spmv_config;
-    grmp_solve_params q = *p;
     if (cfg == 0) {   // autotuned once per matrix and solver mode (configuration and grid)
         int &slot = mixed ? A->tuned_cfg32 : A->tuned_cfg;
         int &gslot = mixed ? A->tuned_grid32 : A->tuned_grid;
@@ -2197,11 +2197,13 @@ extern "C" int grmp_solve_fp64_noalloc(grmp_matrix A, grmp_vector b, grmp_vector
     std::lock_guard<std::mutex> lk(ctx->mu);
     // the hierarchy that an FP64 grmp_solve of this matrix left: the same solver,
     // in that hierarchy's own storage
+    grmp_solve_params q = *p;
     if (p->spmv_config <= 0 && grmp_mg_ready(A, false)) {
-        int use = 0;
-        const int mrc = grmp_mg_prepare(A, false, &use);
-        if (mrc) return mrc;
-        if (use) return grmp_mg_solve(A, b->d, x->d, p, st);
+        bool done = false;
+        const int mrc = grmp_mg_cg(A, b->d, x->d, &q, st, &done);
+        if (mrc || done) return mrc;
+        std::memset(st, 0, sizeof(*st));
+        p = &q;
     }
     char *work = nullptr;
     int rc = noalloc_scratch(ctx, &work);

@@ -475,8 +475,11 @@ int grmp_solve_params_default(grmp_solve_params *p);
  * assembly had a diffusion term (Laplace, or a diffusion Newton term) is
  * preconditioned by a multilevel cycle, reported as spmv_config 90000 + ...,
  * when spmv_config <= 0, the system is large enough and not reaction
- * dominated, and the hierarchy fits in memory; otherwise by Jacobi.  BICGSTAB
- * falls back to Jacobi where the cycle does not converge. */
+ * dominated, and the hierarchy fits in memory; otherwise by Jacobi.  Where the
+ * cycle does not converge (maxiter, no progress, breakdown) MIXED goes on with
+ * the FP64 cycle and FP64 with Jacobi, each from the nearest x so far and with
+ * maxiter iterations; BICGSTAB goes back to Jacobi from the caller's start.
+ * The stats are those of the solver that ended the call. */
 int grmp_solve(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solve_params *params,
                grmp_solve_stats *stats);
 
