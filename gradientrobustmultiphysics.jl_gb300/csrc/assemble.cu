@@ -794,6 +794,7 @@ int grmp_p2b_rhs(grmp_space s, const grmp_rhs *rhs, grmp_vector b);
 int grmp_assemble_bilinear_impl(grmp_matrix A, int nterms, const grmp_bilinear_term *terms, int precision) {
     grmp_space s = A->space;
     grmp_context ctx = s->mesh->ctx;
+    A->reaction = 0;
     A->elliptic = false;
     for (int i = 0; i < nterms; i++) A->elliptic = A->elliptic || terms[i].op_kind == GRMP_OP_LAPLACE;
     if (s->fe == GRMP_FE_H1BR) {
@@ -992,6 +993,7 @@ int grmp_apply_dirichlet_impl(grmp_matrix A, grmp_vector b, int32_t nfixed, cons
     if (!A->has64 && !A->has32) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "dirichlet: matrix not assembled");
     if (mode == GRMP_DIRICHLET_PENALTY && A->has32)
         return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "dirichlet: the penalty form overflows FP32 values; use ELIMINATE");
+    A->reaction = 0;
     int rc = GRMP_OK;
     if (!A->d_fixed) rc = grmp_alloc(ctx, (void **)&A->d_fixed, (size_t)A->nrows);
     if (rc) return rc;

@@ -145,6 +145,7 @@ struct grmp_matrix_s {
     int mg_state = 0;
     size_t mg_budget = SIZE_MAX;    // device bytes it may take (served requests: what their estimate leaves)
     bool elliptic = false;
+    int reaction = 0;               // the present values are reaction dominated: bit 0 FP64, 1 FP32 (cleared where values are written)
 };
 
 void grmp_duo_free(grmp_matrix A);   // duo copy of mixed solves (solve.cu)

@@ -58,7 +58,9 @@ int lanes_of(size_t entries, int rows) {
 constexpr double kSmooth = 1.7;   // w of the smoothing steps and c of the fine level (l1-scaled: spectrum in (0, 1])
 constexpr double kProlong = 1.32; // w of the prolongation smoothing
 // reaction-dominated matrices (energy of the constant function against the
-// diagonal) converge in a few dozen Jacobi iterations: they keep that solver
+// diagonal) converge in a few dozen Jacobi iterations: they keep that solver.
+// The look costs a pass over the matrix and a stop of the stream (which then
+// serves the Jacobi solver's diagonal check too), once per set of values
 constexpr double kMaxReaction = 0.02;
 // Jacobians that take more BiCGStab iterations than kMaxBicg (15-50 on smooth
 // iterates, up to 95 on white noise, where Jacobi takes 200-800), or have not
@@ -1177,6 +1179,10 @@ size_t mg_bytes(const MgCache &C) {
     return b;
 }
 
+// the probe's flag and per-block sums
+constexpr int kProbeBlocks = 2048;
+constexpr size_t kProbePart = (size_t)(kProbeBlocks + 1) * 16;
+
 // numeric storage of one precision: values of every level, vectors, state
 template <typename T>
 int mg_storage(grmp_matrix A) {
@@ -1218,7 +1224,7 @@ int mg_storage(grmp_matrix A) {
         N.z0 = take(C.mult ? (size_t)A->nrows * sizeof(T) : 0);
         N.x0 = take((size_t)A->nrows * 8);   // the caller's start, while it may be needed again
         N.binv = take((size_t)kMgBottom * kMgBottom * sizeof(T));
-        N.part = take((size_t)4096 * 16);
+        N.part = take(kProbePart);
         // FP64: r z p q; mixed: r q xc, two pairs, FP64 residual
         const size_t n0 = A->nrows;
         N.vec = take(sizeof(T) == 8 ? 4 * al(n0 * 8) : 3 * al(n0 * 4) + 2 * al(n0 * 8) + al(n0 * 8));
@@ -1248,19 +1254,17 @@ int rows_lanes(int n) { return sizeof(T) == 8 && n >= kManyRows ? 2 : 8; }
 
 // D of the fine level, the diagonal check and the reaction share
 template <typename T>
-int mg_probe(grmp_matrix A, double *react) {
+int mg_probe(grmp_matrix A, char *D, char *iso, char *part, double *react) {
     grmp_context ctx = A->space->mesh->ctx;
-    MgCache &C = *A->mg;
-    MgCache::Num &N = C.num[sizeof(T) == 8 ? 0 : 1];
-    const int n = A->nrows, cl = rows_lanes<T>(n), grid = std::max(1, std::min({nblk(n, kTB / cl), 4 * ctx->num_sms, 2048}));
-    cudaMemsetAsync(N.part, 0, 16, ctx->stream);   // the flag of a bad diagonal, then the blocks' sums
+    const int n = A->nrows, cl = rows_lanes<T>(n);
+    const int grid = std::max(1, std::min({nblk(n, kTB / cl), 4 * ctx->num_sms, kProbeBlocks}));
+    cudaMemsetAsync(part, 0, 16, ctx->stream);   // the flag of a bad diagonal, then the blocks' sums
     auto kern = cl == 2 ? k_mg_rows<T, 2> : k_mg_rows<T, 8>;
-    kern<<<grid, kTB, 0, ctx->stream>>>(n, A->d_rowptr, A->d_cols, fine_values<T>(A), (T *)N.D[0],
-                                                (uint8_t *)N.iso[0], A->eliminated ? A->d_fixed : nullptr,
-                                                (double2 *)N.part + 1, (int *)N.part);
+    kern<<<grid, kTB, 0, ctx->stream>>>(n, A->d_rowptr, A->d_cols, fine_values<T>(A), (T *)D, (uint8_t *)iso,
+                                        A->eliminated ? A->d_fixed : nullptr, (double2 *)part + 1, (int *)part);
     GRMP_LAUNCHED(ctx);
-    double buf[2 * 2049];
-    cudaError_t e = grmp_readback(ctx, buf, N.part, (size_t)(grid + 1) * 16);
+    double buf[2 * (kProbeBlocks + 1)];
+    cudaError_t e = grmp_readback(ctx, buf, part, (size_t)(grid + 1) * 16);
     const double *h = buf + 2;
     int bad = 0;
     std::memcpy(&bad, buf, 4);
@@ -1270,6 +1274,19 @@ int mg_probe(grmp_matrix A, double *react) {
     for (int b = 0; b < grid; b++) s += h[2 * b], d += h[2 * b + 1];
     *react = d > 0 ? s / d : 1.0;
     return GRMP_OK;
+}
+
+// the probe before there is a hierarchy, in memory of its own
+template <typename T>
+int mg_probe_first(grmp_matrix A, double *react) {
+    grmp_context ctx = A->space->mesh->ctx;
+    const size_t d = al((size_t)A->nrows * sizeof(T)), i = al((size_t)A->nrows), bytes = d + i + kProbePart;
+    char *w = nullptr;
+    int rc = grmp_alloc(ctx, (void **)&w, bytes);
+    if (rc) return rc;
+    rc = mg_probe<T>(A, w, w + d, w + d + i, react);
+    grmp_free(ctx, w, bytes);
+    return rc;
 }
 
 // levels of at most kShortLevel rows give a row 16 lanes (k_mg_prol_agg) or a
@@ -1525,28 +1542,44 @@ void grmp_mg_free(grmp_matrix A) {
 
 bool grmp_mg_ready(grmp_matrix A, bool mixed) { return A->mg_state > 0 && A->mg && A->mg->num[mixed ? 1 : 0].p; }
 
-int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool bicg) {
+int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool *checked, bool bicg) {
     *use = 0;
+    *checked = false;
     grmp_space s = A->space;
     grmp_context ctx = s->mesh->ctx;
-    if (A->mg_state < 0 || A->imported || !A->elliptic || s->ncomp != 1 ||
+    const int bit = mixed ? 2 : 1;
+    if (A->mg_state < 0 || A->imported || !A->elliptic || (A->reaction & bit) || s->ncomp != 1 ||
         (s->fe != GRMP_FE_H1P1 && s->fe != GRMP_FE_H1P2) || A->nrows < min_rows(s->mesh->dim, s->fe, mixed, bicg))
         return GRMP_OK;
     int rc = GRMP_OK;
-    if (!A->mg) rc = mg_build(A);
-    if (!rc && A->mg_state > 0) rc = mixed ? mg_storage<float>(A) : mg_storage<double>(A);
-    if (rc == GRMP_ERR_BUDGET || rc == GRMP_ERR_OUT_OF_MEMORY) {   // no room for the hierarchy: the Jacobi solvers
-        grmp_mg_free(A);
-        A->mg_state = -1;
-        ctx->last_error.clear();
-        cudaGetLastError();
+    double react = 0.0;
+    if (!grmp_mg_ready(A, mixed)) {
+        // the matrix is looked at first: analysis and storage are for those that the cycle is for
+        rc = mixed ? mg_probe_first<float>(A, &react) : mg_probe_first<double>(A, &react);
+        *checked = !rc;
+        if (!rc && react > kMaxReaction) {
+            A->reaction |= bit;
+            return GRMP_OK;
+        }
+        if (!rc && !A->mg) rc = mg_build(A);
+        if (!rc && A->mg_state > 0) rc = mixed ? mg_storage<float>(A) : mg_storage<double>(A);
+        if (rc == GRMP_ERR_BUDGET || rc == GRMP_ERR_OUT_OF_MEMORY) {   // no room for the hierarchy: the Jacobi solvers
+            grmp_mg_free(A);
+            A->mg_state = -1;
+            ctx->last_error.clear();
+            cudaGetLastError();
+            return GRMP_OK;
+        }
+        if (rc || A->mg_state < 0) return rc;
+    }
+    MgCache::Num &N = A->mg->num[mixed ? 1 : 0];
+    rc = mixed ? mg_probe<float>(A, N.D[0], N.iso[0], N.part, &react) : mg_probe<double>(A, N.D[0], N.iso[0], N.part, &react);
+    if (rc) return rc;
+    *checked = true;
+    if (react > kMaxReaction) {
+        A->reaction |= bit;
         return GRMP_OK;
     }
-    if (rc || A->mg_state < 0) return rc;
-    double react = 0.0;
-    rc = mixed ? mg_probe<float>(A, &react) : mg_probe<double>(A, &react);
-    if (rc) return rc;
-    if (react > kMaxReaction) return GRMP_OK;
     if (mixed) mg_values<float>(A);
     else mg_values<double>(A);
     cudaError_t e = cudaGetLastError();
@@ -1605,11 +1638,14 @@ int grmp_mg_solve(grmp_matrix A, const double *b, double *x, bool mixed, grmp_so
     return e == cudaSuccess ? GRMP_OK : grmp_cuda_fail(ctx, e, "multilevel solve");
 }
 
-int grmp_mg_cg(grmp_matrix A, const double *b, double *x, grmp_solve_params *p, grmp_solve_stats *st, bool *done) {
-    *done = false;
+int grmp_mg_cg(grmp_matrix A, const double *b, double *x, grmp_solve_params *p, grmp_solve_stats *st, bool *done,
+               bool *checked) {
+    *done = *checked = false;
     for (int mixed = p->mode == GRMP_SOLVE_MIXED; mixed >= 0; mixed--) {
         int use = 0;
-        int rc = grmp_mg_prepare(A, mixed, &use);
+        bool ok = false;
+        int rc = grmp_mg_prepare(A, mixed, &use, &ok);
+        *checked = *checked || ok;   // of the caller's precision: the first to be looked at
         if (rc || !use) return rc;
         rc = grmp_mg_solve(A, b, x, mixed, p, st, done);
         if (rc || *done || st->iterations >= p->maxiter) return rc;

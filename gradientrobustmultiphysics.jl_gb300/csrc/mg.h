@@ -8,14 +8,16 @@ constexpr int kMgConfig = 90000;
 
 // Whether grmp_solve takes the multilevel solver for this matrix (scalar
 // H1P1 / H1P2 with a diffusion term, not reaction dominated); builds or
-// refreshes what it needs.  *use = 0: the Jacobi solvers.
+// refreshes what it needs.  *use = 0: the Jacobi solvers.  *checked: the
+// diagonal has been found positive and finite (the Jacobi solvers need not look again).
 // bicg: for grmp_mg_bicgstab, which pays from fewer rows.
-int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool bicg = false);
+int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool *checked, bool bicg = false);
 // Conjugate gradients with the hierarchy where the matrix takes them, mixed
 // ones that fail once more in FP64.  *done = false: not taken or not converged
 // (maxiter, no progress, breakdown); the Jacobi solvers go on with *p, from x
 // if it is nearer than the caller's start, else from that.
-int grmp_mg_cg(grmp_matrix A, const double *b, double *x, grmp_solve_params *p, grmp_solve_stats *st, bool *done);
+int grmp_mg_cg(grmp_matrix A, const double *b, double *x, grmp_solve_params *p, grmp_solve_stats *st, bool *done,
+               bool *checked);
 // BiCGStab with the prepared FP64 hierarchy for the scalar Jacobian of a Newton
 // step; vec: nine vectors of the matrix's rows.  *done = false: it did not
 // converge and x is as it was.

@@ -242,6 +242,7 @@ int grmp_assemble_nonlinear_impl(grmp_matrix A, grmp_vector b, grmp_vector u, co
         return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "convection needs ncomponents == dim");
     if (precision != GRMP_FP64 && precision != GRMP_FP64_FP32)
         return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "nonlinear form: precision FP64 or FP64_FP32");
+    A->reaction = 0;
     A->elliptic = scalar_kind || (add && A->elliptic);
     // quadrature order (src/assemblypatterns.jl:558-565): bonus + sum over the
     // operators of polyorder + shift (Identity 0, Gradient -1)

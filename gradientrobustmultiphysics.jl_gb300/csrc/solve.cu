@@ -1946,9 +1946,10 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
     int n = A->nrows;
     const bool bicg = p->mode == GRMP_SOLVE_BICGSTAB;
     grmp_solve_params q = *p;
+    bool checked = false;   // the diagonal, by the multilevel solver's look at the matrix
     if (!bicg && p->spmv_config <= 0) {   // no configuration asked for: multilevel where it applies
         bool done = false;
-        const int rc = grmp_mg_cg(A, b->d, x->d, &q, st, &done);
+        const int rc = grmp_mg_cg(A, b->d, x->d, &q, st, &done, &checked);
         if (rc || done) return rc;
         std::memset(st, 0, sizeof(*st));
     }
@@ -1977,7 +1978,7 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
     cudaMemsetAsync(dst, 0, sizeof(SolveState), ctx->stream);
     if (bicg) {   // scalar Jacobians: multilevel, else (and where that fails) Jacobi
         int use = 0;
-        int rc = grmp_mg_prepare(A, false, &use, true);
+        int rc = grmp_mg_prepare(A, false, &use, &checked, true);
         if (rc) return rc;
         if (use) {
             double *vv[9];
@@ -2002,7 +2003,7 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
                                                              bad);
         GRMP_LAUNCHED(ctx);
         int hbad = 0;
-        cudaError_t e = grmp_readback(ctx, &hbad, bad, 4);
+        cudaError_t e = checked ? cudaGetLastError() : grmp_readback(ctx, &hbad, bad, 4);
         grmp_free(ctx, bad, 4);
         if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "jacobi diagonal");
         if (hbad) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "solve: non-positive or non-finite diagonal entry");
@@ -2199,8 +2200,8 @@ extern "C" int grmp_solve_fp64_noalloc(grmp_matrix A, grmp_vector b, grmp_vector
     // in that hierarchy's own storage
     grmp_solve_params q = *p;
     if (p->spmv_config <= 0 && grmp_mg_ready(A, false)) {
-        bool done = false;
-        const int mrc = grmp_mg_cg(A, b->d, x->d, &q, st, &done);
+        bool done = false, checked = false;
+        const int mrc = grmp_mg_cg(A, b->d, x->d, &q, st, &done, &checked);
         if (mrc || done) return mrc;
         std::memset(st, 0, sizeof(*st));
         p = &q;
