@@ -56,7 +56,6 @@ int lanes_of(size_t entries, int rows) {
     return entries <= (size_t)kShortRow * rows ? 4 : (entries <= (size_t)kLongRow * rows ? 8 : 32);
 }
 constexpr double kSmooth = 1.7;   // w of the smoothing steps and c of the fine level (l1-scaled: spectrum in (0, 1])
-constexpr double kProlong = 1.32; // w of the prolongation smoothing
 // reaction-dominated matrices (energy of the constant function against the
 // diagonal) converge in a few dozen Jacobi iterations: they keep that solver.
 // The look costs a pass over the matrix and a stop of the stream (which then
@@ -203,6 +202,17 @@ __global__ void k_mg_prol_geo(int n, const int32_t *prp, const int32_t *pci, con
     ellv[i] = Pair<T>{w[0], w[1]};
 }
 
+// position of column c in a row's ascending columns, -1 if it is not there
+__device__ __forceinline__ int mg_find(const int32_t *cols, int n, int c) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (cols[mid] < c) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo < n && cols[lo] == c ? lo : -1;
+}
+
 // P = (I - w D A) P_agg, L lanes a row (1 on long levels; 16 on short ones,
 // whose rows hold hundreds of entries: 3,000 rows 57 us with one lane)
 template <typename T, int L>
@@ -212,7 +222,7 @@ __global__ void k_mg_prol_agg(int n, const int32_t *rp, const int32_t *ci, const
     const bool in = i < n;   // whole warps take part in the shuffles
     const int kb = in ? rp[i] : 0, ke = in ? rp[i + 1] : 0, own = in ? agg[i] : -1;
     const bool lone = in && iso[i];
-    const T w = in ? (T)kProlong * D[i] : T(0);
+    const T w = in ? (T)kMgProlong * D[i] : T(0);
     const int q0 = in ? prp[i] : 0;
     int nq = in ? prp[i + 1] - q0 : 0;
     if (L > 1) nq = __reduce_max_sync(0xffffffffu, nq);
@@ -226,15 +236,21 @@ __global__ void k_mg_prol_agg(int n, const int32_t *rp, const int32_t *ci, const
     }
 }
 
-// position of column c in a row's ascending columns, -1 if it is not there
-__device__ __forceinline__ int mg_find(const int32_t *cols, int n, int c) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (cols[mid] < c) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo < n && cols[lo] == c ? lo : -1;
+// Couplings to aggregates that a row of P lacks (weak ones, on stretched
+// meshes) go to its own aggregate, so that rows without Dirichlet neighbours
+// keep their sum of one; 8 lanes a row
+template <typename T>
+__global__ void k_mg_prol_lump(int n, const int32_t *rp, const int32_t *ci, const T *v, const T *D, const uint8_t *iso,
+                               const int32_t *agg, const int32_t *prp, const int32_t *pci, T *pv) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / 8, lane = threadIdx.x & 7;
+    const bool in = i < n && !iso[i];   // whole warps take part in the shuffles
+    const int q0 = in ? prp[i] : 0, nq = in ? prp[i + 1] - q0 : 0;
+    T s = 0;
+    if (in)
+        for (int k = rp[i] + lane; k < rp[i + 1]; k += 8)
+            if (mg_find(pci + q0, nq, agg[ci[k]]) < 0) s += v[k];
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (in && lane == 0) pv[q0 + mg_find(pci + q0, nq, agg[i])] -= (T)kMgProlong * D[i] * s;
 }
 
 // Sparse products, a group of lanes per row of the result.  The factor rows
@@ -339,6 +355,50 @@ __global__ void __launch_bounds__(kTB) k_mg_ap_geo(int n, const int32_t *__restr
             if (tb < te) av[tb] = acc;
         }
     }
+}
+
+// cells whose longest edge is more than kStretch times their smallest height
+constexpr double kStretch = 4.0;   // 2.0 on squares split in triangles, 2.45 on Kuhn cubes
+template <int DIM>
+__global__ void k_mg_stretched(int ncells, const double *coords, const int32_t *cells, int *count) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    bool s = false;
+    if (c < ncells) {
+        double X[DIM + 1][DIM], longest = 0.0, face = 0.0;
+        for (int v = 0; v <= DIM; v++)
+            for (int k = 0; k < DIM; k++) X[v][k] = coords[(size_t)cells[(size_t)c * (DIM + 1) + v] * DIM + k];
+        for (int a = 0; a < DIM; a++)
+            for (int b = a + 1; b <= DIM; b++) {
+                double l = 0.0;
+                for (int k = 0; k < DIM; k++) l += (X[a][k] - X[b][k]) * (X[a][k] - X[b][k]);
+                longest = fmax(longest, l);
+            }
+        if (DIM == 2) {
+            // longest edge squared against twice the area
+            const double det = (X[1][0] - X[0][0]) * (X[2][1] - X[0][1]) - (X[1][1] - X[0][1]) * (X[2][0] - X[0][0]);
+            s = longest > kStretch * fabs(det);
+        } else {
+            // longest edge times twice the largest face's area against six volumes
+            double det = 0.0;
+            for (int f = 0; f < 4; f++) {
+                const int o = f == 0 ? 1 : 0, a = f <= 1 ? 2 : 1, b = f <= 2 ? 3 : 2;   // the face without vertex f
+                double u[3], w[3], n[3];
+                for (int k = 0; k < 3; k++) {
+                    u[k] = X[a][k % DIM] - X[o][k % DIM];
+                    w[k] = X[b][k % DIM] - X[o][k % DIM];
+                }
+                for (int k = 0; k < 3; k++) n[k] = u[(k + 1) % 3] * w[(k + 2) % 3] - u[(k + 2) % 3] * w[(k + 1) % 3];
+                face = fmax(face, n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+                if (f == 0) {
+                    det = 0.0;
+                    for (int k = 0; k < 3; k++) det += n[k] * (X[0][k % DIM] - X[1][k % DIM]);
+                }
+            }
+            s = sqrt(longest * face) > kStretch * fabs(det);
+        }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, s);
+    if ((threadIdx.x & 31) == 0 && m) atomicAdd(count, __popc(m));
 }
 
 // next level's matrix P^T (A P), 16 lanes a row; a row without values (only
@@ -1088,15 +1148,43 @@ int mg_up_vec(grmp_context ctx, MgCache &C, const std::vector<V> &v, V **out) {
     return e == cudaSuccess ? GRMP_OK : grmp_cuda_fail(ctx, e, "multilevel patterns");
 }
 
+// Whether more than a twentieth of the mesh's cells are stretched: the
+// aggregates then follow strong couplings, for which the host forms the unit
+// stiffness of every level (first solve of a pattern: 160 x 160 P1 9 ms instead of
+// 4, 40^3 P1 32 to 47 instead of 13, 20^3 P2 62 to 77 instead of 15).
+int mg_stretched(grmp_mesh m, bool *out) {
+    grmp_context ctx = m->ctx;
+    int *cnt = nullptr, h = 0;
+    int rc = grmp_alloc(ctx, (void **)&cnt, 4);
+    if (rc) return rc;
+    cudaMemsetAsync(cnt, 0, 4, ctx->stream);
+    if (m->dim == 2) k_mg_stretched<2><<<nblk(m->ncells), 256, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, cnt);
+    else k_mg_stretched<3><<<nblk(m->ncells), 256, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, cnt);
+    GRMP_LAUNCHED(ctx);
+    cudaError_t e = grmp_readback(ctx, &h, cnt, 4);
+    grmp_free(ctx, cnt, 4);
+    if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multilevel: cells");
+    *out = h > m->ncells / 20;
+    return GRMP_OK;
+}
+
 int mg_build(grmp_matrix A) {
     grmp_space s = A->space;
     grmp_context ctx = s->mesh->ctx;
     const int n = A->nrows;
-    std::vector<int32_t> rp((size_t)n + 1), ci((size_t)A->nnz), cd, cells;
+    const bool p2 = s->fe == GRMP_FE_H1P2;
+    bool stretched = false;
+    int rc = mg_stretched(s->mesh, &stretched);
+    if (rc) return rc;
+    MgCsr pattern;
+    std::vector<int32_t> cd, cells;
     std::vector<double> coords;
-    cudaError_t e = cudaMemcpyAsync(rp.data(), A->d_rowptr, rp.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ci.data(), A->d_cols, ci.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (s->fe == GRMP_FE_H1P2) {
+    pattern.rp.resize((size_t)n + 1);
+    pattern.ci.resize((size_t)A->nnz);
+    cudaError_t e = cudaMemcpyAsync(pattern.rp.data(), A->d_rowptr, pattern.rp.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(pattern.ci.data(), A->d_cols, pattern.ci.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
+    if (p2 || stretched) {
         cd.resize((size_t)s->mesh->ncells * s->ldofs);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(cd.data(), s->d_celldofs, cd.size() * 4, cudaMemcpyDeviceToHost, ctx->stream);
@@ -1112,12 +1200,11 @@ int mg_build(grmp_matrix A) {
     MgCache *C = new MgCache;
     A->mg = C;
     C->mult = fine_mult(s->mesh->dim, s->fe, n);
-    if (mg_symbolic_build(n, rp.data(), ci.data(), s->mesh->dim, s->mesh->ncells, s->ldofs, cd.empty() ? nullptr : cd.data(),
-                          coords.data(), cells.data(), !A->face_coupled, C->mult, &C->S)) {
+    const MgCells m{s->mesh->dim, s->mesh->ncells, s->ldofs, cd.data(), cells.data(), coords.data()};
+    if (mg_symbolic_build(n, pattern, m, p2, !A->face_coupled, stretched, C->mult, &C->S)) {
         A->mg_state = -1;
         return GRMP_OK;
     }
-    int rc = GRMP_OK;
     const int ns = (int)C->S.step.size();
     C->step.resize(ns);
     for (int k = 0; k < ns && !rc; k++) {
@@ -1330,6 +1417,11 @@ void mg_values(grmp_matrix A) {
         else
             k_mg_prol_agg<T, 16><<<nblk((long long)n * 16, 128), 128, 0, st>>>(n, rp, ci, v, D, (const uint8_t *)N.iso[k],
                                                                                d.agg, d.prp, d.pci, pv);
+        if (C.S.step[k].lump) {
+            k_mg_prol_lump<T><<<nblk((long long)n * 8, 256), 256, 0, st>>>(n, rp, ci, v, D, (const uint8_t *)N.iso[k], d.agg,
+                                                                          d.prp, d.pci, pv);
+            GRMP_LAUNCHED(ctx);
+        }
         if (d.vrow)
             k_mg_ap_geo<T><<<std::max(1, std::min(nblk((long long)n * 16), wide)), kTB, 0, st>>>(
                 n, rp, ci, v, d.ell, (const Pair<T> *)N.ellv, d.arp, d.aci, av);

@@ -9,7 +9,19 @@
 // that P1 stiffness has on some cell: on right angles (squares split in triangles, Kuhn
 // cubes) half of the neighbours do not couple, and aggregates that take them
 // in span two couplings where the smoothed prolongation reaches one (128 x
-// 128: 56 iterations with them, about half without).  Patterns include the DoFs that a call
+// 128: 56 iterations with them, about half without).
+//
+// On stretched meshes the neighbours are not alike: the error that the
+// smoother leaves is smooth along the short cell sides only, and aggregates
+// that span long sides cannot represent it, nor can the vertices of P2 cells
+// (160 x 160 P1 on strips 1 : 10, 1 : 30 and 1 : 100: 81, 226 and 510 iterations, 19
+// on the square; 80 x 80 P2 98, 272 and 531).  There a row aggregates with strong
+// neighbours only, on every level and P2's first one too: those whose stiffness
+// for the unit coefficient exceeds kStrong of the diagonal (half of that on
+// each coarser level, as in the paper), and the prolongation adds weak
+// couplings to the row's own aggregate: 18 to 27 iterations on the P1 strips and
+// graded meshes, 23 to 25 on the P2 strips; plates and rods of 40^3 P1 cubes 14 to 20
+// (118 at 1 : 20 before), a P2 plate 1 : 20 of 20^3 cubes 51 (157 before).  Patterns include the DoFs that a call
 // fixes later (they are masked by values), so one hierarchy serves every set
 // of boundary DoFs.
 #include <algorithm>
@@ -19,6 +31,10 @@
 #include "mg_symbolic.h"
 
 namespace {
+
+// P1 and coarse levels: 0.05 takes 28 iterations on a strip 1 : 3, 0.08 16; 0.2 leaves nothing strong on Kuhn
+// cubes.  P2: 0.08 takes 38 iterations on a strip 1 : 30 and 105 on a plate 1 : 20, 0.2 24 and 36.
+constexpr double kStrong = 0.08, kStrongP2 = 0.2;
 
 int host_threads(int n) {
     const int hw = std::max(1, (int)std::thread::hardware_concurrency());
@@ -55,6 +71,18 @@ void build_rows(int n, int ncols, MgCsr *out, F fn) {
     out->ci.resize(out->rp[n]);
     for (int t = 0; t < nt; t++)
         std::copy(part[t].begin(), part[t].end(), out->ci.begin() + out->rp[(size_t)((long long)n * t / nt)]);
+}
+
+template <typename F>
+void parallel_rows(int n, F fn) {
+    const int nt = host_threads(n);
+    auto work = [&](int t) {
+        for (int i = (int)((long long)n * t / nt); i < (int)((long long)n * (t + 1) / nt); i++) fn(i);
+    };
+    std::vector<std::thread> pool;
+    for (int t = 1; t < nt; t++) pool.emplace_back(work, t);
+    work(0);
+    for (auto &t : pool) t.join();
 }
 
 void transpose(int n, int nc, const MgCsr &A, MgCsr *T, std::vector<int32_t> *perm) {
@@ -107,41 +135,52 @@ int aggregate(int n, const int32_t *rp, const int32_t *ci, std::vector<int32_t> 
     return na;
 }
 
-// Drops from the vertex level's pattern the pairs that have no P1 stiffness on
-// any of their cells: a statement about the mesh that holds for every
-// coefficient, so one hierarchy serves them all.  (Not the pairs whose cells
-// cancel for the unit coefficient, as the diagonals of isosceles trapezoids:
-// they couple as soon as the coefficient varies, and a coupling that the
-// pattern lacks goes to the diagonal, which then need not stay positive.)
-void filter_vertex_level(MgStep *s, int dim, int ncells, int ld, const int32_t *celldofs, const std::vector<int32_t> &vert,
-                         const double *coords, const int32_t *cells) {
-    const int nv = dim + 1, nc = s->nc;
-    std::vector<int32_t> ptr((size_t)nc + 1, 0);
-    for (long long c = 0; c < ncells; c++)
-        for (int v = 0; v < nv; v++) ptr[vert[celldofs[c * ld + v]] + 1]++;
-    for (int i = 0; i < nc; i++) ptr[i + 1] += ptr[i];
-    std::vector<int32_t> inc(ptr[nc]), at(ptr.begin(), ptr.end() - 1);
-    for (long long c = 0; c < ncells; c++)
-        for (int v = 0; v < nv; v++) inc[at[vert[celldofs[c * ld + v]]]++] = (int32_t)(c * 4 + v);
-    std::vector<double> K(s->Ac.ci.size(), 0.0), diag(nc, 0.0);
-    const int nt = host_threads(nc);
-    auto rows = [&](int t, auto fn) {
-        for (int i = (int)((long long)nc * t / nt); i < (int)((long long)nc * (t + 1) / nt); i++) fn(i);
-    };
-    auto parallel = [&](auto fn) {
-        std::vector<std::thread> pool;
-        for (int t = 1; t < nt; t++) pool.emplace_back([&, t] { rows(t, fn); });
-        rows(0, fn);
-        for (auto &t : pool) t.join();
-    };
-    parallel([&](int i) {
-        for (int q = ptr[i]; q < ptr[i + 1]; q++) {
-            const long long c = inc[q] >> 2;
-            const int a = inc[q] & 3;
-            double E[3][3], G[4][3] = {}, det;
-            const double *x0 = coords + (size_t)cells[c * nv] * dim;
+// vertices of the P2 edge functions
+constexpr int kEdge2[3][2] = {{0, 1}, {1, 2}, {2, 0}};
+constexpr int kEdge3[6][2] = {{0, 1}, {0, 2}, {0, 3}, {1, 2}, {1, 3}, {2, 3}};
+
+// Entry (a, b) of a cell's P1 (p2 = false) or P2 stiffness from h_ij =
+// |T| grad lambda_i . grad lambda_j (assemble.cu derives the P2 form).
+double local_stiffness(int dim, bool p2, const double h[4][4], int a, int b) {
+    const int nv = dim + 1;
+    if (!p2) return h[a][b];
+    const double e = 16.0 / (nv * (nv + 1)), c = 1.0 - 8.0 / nv, g = e - 4.0 / nv;
+    if (a < nv && b < nv) return (a == b ? 2 * e + c : e + c) * h[a][b];
+    if (a < nv) std::swap(a, b);   // a: an edge
+    const int i = dim == 2 ? kEdge2[a - nv][0] : kEdge3[a - nv][0], j = dim == 2 ? kEdge2[a - nv][1] : kEdge3[a - nv][1];
+    if (b < nv) return g * (h[i][b] + h[j][b]) + (b == i || b == j ? e * h[i][j] : 0.0);
+    const int k = dim == 2 ? kEdge2[b - nv][0] : kEdge3[b - nv][0], l = dim == 2 ? kEdge2[b - nv][1] : kEdge3[b - nv][1];
+    double s = h[i][k] + h[j][k] + h[i][l] + h[j][l];
+    if (k == i) s += h[j][l];
+    if (l == i) s += h[j][k];
+    if (k == j) s += h[i][l];
+    if (l == j) s += h[i][k];
+    return e * s;
+}
+
+// Contributions of the cells to the stiffness of the unit coefficient, P2 (all
+// local DoFs) or P1 (the vertex DoFs), in the pattern A of n rows; row[d]: row
+// of the DoF d.  Mode Sum: their sums; Size: the sums of their absolute values.
+enum class Mode { Sum, Size };
+std::vector<double> unit_stiffness(Mode mode, int n, const MgCsr &A, const MgCells &m, bool p2,
+                                   const std::vector<int32_t> &row) {
+    const int dim = m.dim, nv = dim + 1, nb = p2 ? (dim == 2 ? 6 : 10) : nv;
+    std::vector<int64_t> ptr((size_t)n + 1, 0);
+    for (long long c = 0; c < m.ncells; c++)
+        for (int v = 0; v < nb; v++) ptr[row[m.celldofs[c * m.ld + v]] + 1]++;
+    for (int i = 0; i < n; i++) ptr[i + 1] += ptr[i];
+    std::vector<int64_t> inc(ptr[n]), at(ptr.begin(), ptr.end() - 1);
+    for (long long c = 0; c < m.ncells; c++)
+        for (int v = 0; v < nb; v++) inc[at[row[m.celldofs[c * m.ld + v]]]++] = c * 16 + v;
+    std::vector<double> K(A.ci.size(), 0.0);
+    parallel_rows(n, [&](int i) {
+        for (int64_t q = ptr[i]; q < ptr[i + 1]; q++) {
+            const long long c = inc[q] >> 4;
+            const int a = (int)(inc[q] & 15);
+            double E[3][3], G[4][3] = {}, h[4][4], det;
+            const double *x0 = m.coords + (size_t)m.cells[c * nv] * dim;
             for (int j = 0; j < dim; j++)
-                for (int k = 0; k < dim; k++) E[j][k] = coords[(size_t)cells[c * nv + j + 1] * dim + k] - x0[k];
+                for (int k = 0; k < dim; k++) E[j][k] = m.coords[(size_t)m.cells[c * nv + j + 1] * dim + k] - x0[k];
             if (dim == 2) {
                 det = E[0][0] * E[1][1] - E[0][1] * E[1][0];
                 G[1][0] = E[1][1], G[1][1] = -E[1][0];
@@ -156,27 +195,84 @@ void filter_vertex_level(MgStep *s, int dim, int ncells, int ld, const int32_t *
             }
             for (int k = 0; k < dim; k++)
                 for (int j = 1; j <= dim; j++) G[0][k] -= G[j][k];
-            for (int b = 0; b < nv; b++) {
-                double d = 0;
-                for (int k = 0; k < dim; k++) d += G[a][k] * G[b][k];
-                const int J = vert[celldofs[c * ld + b]];
-                const int32_t *r = s->Ac.ci.data() + s->Ac.rp[i], *re = s->Ac.ci.data() + s->Ac.rp[i + 1];
+            for (int j = 0; j < nv; j++)
+                for (int l = 0; l < nv; l++) {
+                    double d = 0;
+                    for (int k = 0; k < dim; k++) d += G[j][k] * G[l][k];
+                    h[j][l] = d / (det != 0 ? std::fabs(det) : 1.0);   // the common factor 1 / dim! does not matter
+                }
+            for (int b = 0; b < nb; b++) {
+                const int J = row[m.celldofs[c * m.ld + b]];
+                const int32_t *r = A.ci.data() + A.rp[i], *re = A.ci.data() + A.rp[i + 1];
                 const int32_t *f = std::lower_bound(r, re, J);
-                if (f != re && *f == J) K[f - s->Ac.ci.data()] += std::fabs(d) / (det != 0 ? std::fabs(det) : 1.0);
+                if (f == re || *f != J) continue;
+                const double v = local_stiffness(dim, p2, h, a, b);
+                K[f - A.ci.data()] += mode == Mode::Size ? std::fabs(v) : v;
             }
         }
-        for (int k = s->Ac.rp[i]; k < s->Ac.rp[i + 1]; k++)
-            if (s->Ac.ci[k] == i) diag[i] = K[k];
+    });
+    return K;
+}
+
+// the pattern's pairs whose entry exceeds theta times the two diagonal entries' mean
+MgCsr strong_pairs(int n, const MgCsr &A, const std::vector<double> &K, double theta) {
+    std::vector<double> d(n, 0.0);
+    parallel_rows(n, [&](int i) {
+        for (int k = A.rp[i]; k < A.rp[i + 1]; k++)
+            if (A.ci[k] == i) d[i] = std::fabs(K[k]);
     });
     MgCsr F;
-    build_rows(nc, nc, &F, [&](int i, auto add) {
-        for (int k = s->Ac.rp[i]; k < s->Ac.rp[i + 1]; k++) {
-            const int j = s->Ac.ci[k];
-            if (j == i || K[k] > 1e-6 * std::sqrt(diag[i] * diag[j])) add(j);
+    build_rows(n, n, &F, [&](int i, auto add) {
+        for (int k = A.rp[i]; k < A.rp[i + 1]; k++) {
+            const int j = A.ci[k];
+            if (j == i || std::fabs(K[k]) > theta * std::sqrt(d[i] * d[j])) add(j);
         }
     });
-    s->filtered = F.ci.size() < s->Ac.ci.size();
-    if (s->filtered) s->Ac = std::move(F);
+    return F;
+}
+
+// Drops from the vertex level's pattern the pairs that have no P1 stiffness on
+// any of their cells: a statement about the mesh that holds for every
+// coefficient, so one hierarchy serves them all.  (Not the pairs whose cells
+// cancel for the unit coefficient, as the diagonals of isosceles trapezoids:
+// they couple as soon as the coefficient varies, and a coupling that the
+// pattern lacks goes to the diagonal, which then need not stay positive.)
+void filter_vertex_level(MgStep *s, const MgCells &m, const std::vector<int32_t> &vert) {
+    const std::vector<double> K = unit_stiffness(Mode::Size, s->nc, s->Ac, m, false, vert);
+    s->Ac = strong_pairs(s->nc, s->Ac, K, 1e-6);
+}
+
+// The next level's unit stiffness, P^T K P with P = (I - w D K) P_agg as on the
+// device: couplings to aggregates that a row of P lacks go to its own.
+std::vector<double> coarse_stiffness(const MgStep &s, const MgCsr &A, const std::vector<double> &K) {
+    const MgCsr &P = s.P, &AP = s.AP;
+    std::vector<double> pv(P.ci.size()), av(AP.ci.size()), cv(s.Ac.ci.size());
+    auto find = [](const MgCsr &M, int i, int c) {
+        const int32_t *b = M.ci.data() + M.rp[i], *e = M.ci.data() + M.rp[i + 1], *f = std::lower_bound(b, e, c);
+        return f != e && *f == c ? (int)(f - M.ci.data()) : -1;
+    };
+    parallel_rows(s.n, [&](int i) {
+        double sum = 0.0;
+        for (int k = A.rp[i]; k < A.rp[i + 1]; k++) sum += std::fabs(K[k]);
+        const double w = sum > 0 ? kMgProlong / sum : 0.0;
+        const int own = find(P, i, s.agg[i]);
+        pv[own] += 1.0;
+        for (int k = A.rp[i]; k < A.rp[i + 1]; k++) {
+            const int q = find(P, i, s.agg[A.ci[k]]);
+            pv[q < 0 ? own : q] -= w * K[k];
+        }
+    });
+    parallel_rows(s.n, [&](int i) {
+        for (int k = A.rp[i]; k < A.rp[i + 1]; k++)
+            for (int q = P.rp[A.ci[k]]; q < P.rp[A.ci[k] + 1]; q++) av[find(AP, i, P.ci[q])] += K[k] * pv[q];
+    });
+    parallel_rows(s.nc, [&](int I) {
+        for (int k = s.R.rp[I]; k < s.R.rp[I + 1]; k++) {
+            const int i = s.R.ci[k];
+            for (int q = AP.rp[i]; q < AP.rp[i + 1]; q++) cv[find(s.Ac, I, AP.ci[q])] += pv[s.Rperm[k]] * av[q];
+        }
+    });
+    return cv;
 }
 
 void products(MgStep *s, const int32_t *rp, const int32_t *ci) {
@@ -197,24 +293,32 @@ void products(MgStep *s, const int32_t *rp, const int32_t *ci) {
 
 }  // namespace
 
-int mg_symbolic_build(int n, const int32_t *rp, const int32_t *ci, int dim, int ncells, int ld, const int32_t *celldofs,
-                      const double *coords, const int32_t *cells, bool cell_terms, bool fine_q, MgSymbolic *S) {
+int mg_symbolic_build(int n, const MgCsr &A, const MgCells &m, bool p2, bool cell_terms, bool stretched, bool fine_q,
+                      MgSymbolic *S) {
     S->step.clear();
-    const int32_t *crp = rp, *cci = ci;
+    S->step.reserve(kMgMaxLevels);   // C points into it
+    const MgCsr *C = &A;
     int cn = n;
+    const int dim = m.dim, ncells = m.ncells, ld = m.ld;
+    const int32_t *celldofs = m.celldofs;
+    std::vector<double> K;   // unit stiffness of the level (stretched meshes)
+    double theta = p2 ? kStrongP2 : kStrong;
+    if (stretched) {
+        std::vector<int32_t> same(n);
+        for (int i = 0; i < n; i++) same[i] = i;
+        K = unit_stiffness(Mode::Sum, n, A, m, p2, same);
+    }
     while ((cn > kMgBottom || S->step.empty()) && (int)S->step.size() + 1 < kMgMaxLevels) {
         MgStep s;
         s.n = cn;
         std::vector<int32_t> vert;
-        if (S->step.empty() && celldofs) {
+        if (S->step.empty() && p2 && !stretched) {
             // coarse number of each vertex DoF, ascending; edge DoFs get their two vertices
             const int nv = dim + 1;
             std::vector<int32_t> e0(n, -1), e1(n, -1);
             vert.assign(n, -1);
             for (long long c = 0; c < ncells; c++)
                 for (int v = 0; v < nv; v++) vert[celldofs[c * ld + v]] = 0;
-            const int ed2[3][2] = {{0, 1}, {1, 2}, {2, 0}};
-            const int ed3[6][2] = {{0, 1}, {0, 2}, {0, 3}, {1, 2}, {1, 3}, {2, 3}};
             const int ne = dim == 2 ? 3 : 6;
             for (int i = 0, k = 0; i < n; i++)
                 if (vert[i] == 0) vert[i] = k++, s.nc = k;
@@ -222,8 +326,8 @@ int mg_symbolic_build(int n, const int32_t *rp, const int32_t *ci, int dim, int 
                 for (int e = 0; e < ne; e++) {
                     const int32_t *d = celldofs + c * ld;
                     const int i = d[nv + e];
-                    e0[i] = vert[d[dim == 2 ? ed2[e][0] : ed3[e][0]]];
-                    e1[i] = vert[d[dim == 2 ? ed2[e][1] : ed3[e][1]]];
+                    e0[i] = vert[d[dim == 2 ? kEdge2[e][0] : kEdge3[e][0]]];
+                    e1[i] = vert[d[dim == 2 ? kEdge2[e][1] : kEdge3[e][1]]];
                 }
             s.geometric = true;
             for (int i = 0; i < n && s.geometric; i++)   // each DoF is a vertex or an edge
@@ -239,20 +343,28 @@ int mg_symbolic_build(int n, const int32_t *rp, const int32_t *ci, int dim, int 
                 });
         }
         if (!s.geometric) {
-            s.nc = aggregate(cn, crp, cci, &s.agg);
+            MgCsr F;
+            if (stretched) F = strong_pairs(cn, *C, K, theta);
+            const MgCsr &N = stretched ? F : *C;
+            s.nc = aggregate(cn, N.rp.data(), N.ci.data(), &s.agg);
             if (s.nc > 0.7 * cn) break;   // does not coarsen further
             build_rows(cn, s.nc, &s.P, [&](int i, auto add) {
                 add(s.agg[i]);
-                for (int k = crp[i]; k < crp[i + 1]; k++) add(s.agg[cci[k]]);
+                for (int k = N.rp[i]; k < N.rp[i + 1]; k++) add(s.agg[N.ci[k]]);
             });
+            s.lump = stretched;
         }
-        products(&s, crp, cci);
-        if (s.geometric && cell_terms) filter_vertex_level(&s, dim, ncells, ld, celldofs, vert, coords, cells);
+        products(&s, C->rp.data(), C->ci.data());
+        if (s.geometric) {
+            if (cell_terms) filter_vertex_level(&s, m, vert);
+        } else if (stretched) {
+            K = coarse_stiffness(s, *C, K);
+            theta = theta > kStrong ? kStrong : 0.5 * theta;
+        }
         if (fine_q || !S->step.empty()) transpose(s.n, s.nc, s.AP, &s.QT, &s.QTperm);
         cn = s.nc;
         S->step.push_back(std::move(s));
-        crp = S->step.back().Ac.rp.data();   // stays valid: vectors keep their storage when the step is moved
-        cci = S->step.back().Ac.ci.data();
+        C = &S->step.back().Ac;
     }
     return S->step.empty() ? 1 : 0;
 }

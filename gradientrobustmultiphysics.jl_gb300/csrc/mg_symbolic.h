@@ -15,7 +15,7 @@ struct MgCsr {
 struct MgStep {
     int n = 0, nc = 0;
     bool geometric = false;              // P2 -> P1 interpolation, else smoothed aggregation
-    bool filtered = false;               // Ac leaves out couplings (their values go to the diagonal)
+    bool lump = false;                   // rows of P lack aggregates that they couple to (their values go to the row's own)
     std::vector<int32_t> agg;            // aggregate of each row (smoothed aggregation)
     MgCsr P, R, AP, QT, Ac;
     std::vector<int32_t> Rperm, QTperm;
@@ -28,12 +28,21 @@ struct MgSymbolic {
 constexpr int kMgBottom = 96;            // rows of a level that is solved densely
 constexpr int kMgMaxLevels = 14;
 
-// Builds the steps of a matrix with pattern (n, rp, ci).  celldofs != nullptr:
-// a P2 space's cell DoFs [ncells][ld] (dim + 1 vertices, then edges) on the
-// mesh (coords, cells); the first step then interpolates from the vertices.
-// cell_terms: the matrix has terms on cells only (face terms couple vertices
-// that have no stiffness in common: nothing is left out then).
-// fine_q: the transpose of Q also for step 0.  Returns 0, or 1 when the matrix
-// does not coarsen.
-int mg_symbolic_build(int n, const int32_t *rp, const int32_t *ci, int dim, int ncells, int ld, const int32_t *celldofs,
-                      const double *coords, const int32_t *cells, bool cell_terms, bool fine_q, MgSymbolic *S);
+constexpr double kMgProlong = 1.32;      // w of the prolongation smoothing, P = (I - w D A) P_agg
+
+// The cells of the matrix's space: cell DoFs [ncells][ld] (dim + 1 vertices,
+// then, P2, edges) and the mesh.
+struct MgCells {
+    int dim = 0, ncells = 0, ld = 0;
+    const int32_t *celldofs = nullptr, *cells = nullptr;
+    const double *coords = nullptr;
+};
+
+// Builds the steps of a matrix with pattern A (n rows).  p2: of a P2 space, the
+// first step then interpolates from the vertices.  cell_terms: the matrix has
+// terms on cells only (face terms couple vertices that have no stiffness in
+// common: nothing is left out then).  stretched: every step aggregates, along
+// strong couplings.  m is read for p2 or stretched only.  fine_q: the
+// transpose of Q also for step 0.  Returns 0, or 1 when the matrix does not coarsen.
+int mg_symbolic_build(int n, const MgCsr &A, const MgCells &m, bool p2, bool cell_terms, bool stretched, bool fine_q,
+                      MgSymbolic *S);
