@@ -1,7 +1,8 @@
 // C-ABI entry points: contexts, meshes, spaces, vectors and the thin
 // wrappers around the pattern / assembly / solve implementations.
-#include <cstring>
+#include <algorithm>
 #include <cstdarg>
+#include <cstring>
 #include <new>
 
 #include "grmp_internal.h"
@@ -46,6 +47,20 @@ void grmp_free(grmp_context ctx, void *p, size_t bytes) {
     if (!p) return;
     cudaFreeAsync(p, ctx->stream);
     ctx->in_use -= bytes;
+}
+
+size_t grmp_room(grmp_context ctx, double share) {
+    size_t room = 0, total = 0;
+    if (cudaMemGetInfo(&room, &total) != cudaSuccess) cudaGetLastError();
+    cudaMemPool_t pool;
+    uint64_t held = 0, used = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+        room += held - used;
+    room = (size_t)(share * (double)room);
+    if (ctx->budget) room = std::min(room, ctx->budget > ctx->in_use ? ctx->budget - ctx->in_use : (size_t)0);
+    return room;
 }
 
 cudaError_t grmp_readback(grmp_context ctx, void *host, const void *dev, size_t bytes) {

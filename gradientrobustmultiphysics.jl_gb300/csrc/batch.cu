@@ -1927,17 +1927,7 @@ extern "C" int grmp_stokes_batch_solve(grmp_matrix A, grmp_vector bf, grmp_vecto
         }
     }
     if (prm->mode == GRMP_SOLVE_DIRECT) {
-        size_t freeb = 0, totalb = 0;
-        cudaMemGetInfo(&freeb, &totalb);
-        // what the pool holds without using it counts as free
-        cudaMemPool_t pool;
-        uint64_t held = 0, used = 0;
-        if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess &&
-            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
-            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
-            freeb += held - used;
-        size_t allow = (size_t)(0.8 * (double)freeb);
-        if (ctx->budget) allow = std::min(allow, ctx->budget > ctx->in_use ? ctx->budget - ctx->in_use : (size_t)0);
+        const size_t allow = grmp_room(ctx, 0.8);
         cudaMemsetAsync(d.u, 0, (size_t)n * 8, ctx->stream);
         cudaMemsetAsync(d.p, 0, (size_t)nc * 8, ctx->stream);
         if (!rc) rc = build_parts(A, order, allow);

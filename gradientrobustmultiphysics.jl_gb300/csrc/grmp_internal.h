@@ -143,6 +143,7 @@ struct grmp_matrix_s {
     // for this matrix; elliptic: the last assembly had a diffusion term
     struct MgCache *mg = nullptr;
     int mg_state = 0;
+    size_t mg_floor[2] = {0, 0};    // FP64, FP32: the room it needs, where it has not been had (not tried with less)
     size_t mg_budget = SIZE_MAX;    // device bytes it may take (served requests: what their estimate leaves)
     bool elliptic = false;
     int reaction = 0;               // the present values are reaction dominated: bit 0 FP64, 1 FP32 (cleared where values are written)
@@ -179,6 +180,9 @@ int grmp_cuda_fail(grmp_context ctx, cudaError_t e, const char *what);
 // device memory accounted against the context budget
 int grmp_alloc(grmp_context ctx, void **p, size_t bytes);
 void grmp_free(grmp_context ctx, void *p, size_t bytes);
+// bytes that can still be had: a share of the device's, with what its pool
+// holds without using it, and no more than the budget's
+size_t grmp_room(grmp_context ctx, double share = 1.0);
 // Small results to the host and a stream synchronize, through page-locked
 // memory: a copy to pageable memory waits for the stream's kernels inside the
 // CUDA library and keeps other threads' calls out meanwhile, so the solves of four

@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "mg.h"
@@ -1127,8 +1128,6 @@ struct MgCache {
         std::vector<char *> pv, av, tv, cv, D, iso, r, y, e;
         char *rv0 = nullptr, *ellv = nullptr, *binv = nullptr, *part = nullptr, *vec = nullptr, *z0 = nullptr, *x0 = nullptr;
     } num[2];
-    double react[2] = {0, 0};
-    char *state = nullptr;
 };
 
 namespace {
@@ -1168,7 +1167,62 @@ int mg_stretched(grmp_mesh m, bool *out) {
     return GRMP_OK;
 }
 
-int mg_build(grmp_matrix A) {
+// the probe's flag and per-block sums
+constexpr int kProbeBlocks = 2048;
+constexpr size_t kProbePart = (size_t)(kProbeBlocks + 1) * 16;
+
+// numeric storage of one precision: values of every level, vectors, state.
+// Its bytes; base: where it lies (nullptr: only the bytes)
+template <typename T>
+size_t mg_layout(grmp_matrix A, MgCache &C, char *base) {
+    MgCache::Num &N = C.num[sizeof(T) == 8 ? 0 : 1];
+    const int ns = (int)C.step.size();
+    size_t at = 0;
+    auto take = [&](size_t bytes) -> char * {
+        const size_t o = at;
+        at += al(bytes);
+        return base ? base + o : nullptr;
+    };
+    N.pv.assign(ns, nullptr);
+    N.av = N.tv = N.cv = N.pv;
+    N.D.assign(ns + 1, nullptr);
+    N.iso = N.r = N.y = N.e = N.D;
+    for (int k = 0; k < ns; k++) {
+        const MgCache::Step &d = C.step[k];
+        N.pv[k] = take(d.np * sizeof(T));
+        N.av[k] = take(d.na * sizeof(T));
+        N.cv[k] = take(d.nc * sizeof(T));
+        N.tv[k] = take(d.nt * sizeof(T));
+    }
+    N.rv0 = take(C.step[0].np * sizeof(T));
+    N.ellv = take(C.S.step[0].geometric ? (size_t)A->nrows * 2 * sizeof(T) : 0);
+    for (int k = 0; k <= ns; k++) {
+        const size_t n = k < ns ? C.S.step[k].n : C.S.step[ns - 1].nc;
+        N.D[k] = take(n * sizeof(T));
+        N.iso[k] = take(n);
+        if (k > 0) {
+            N.r[k] = take(n * sizeof(T));
+            N.y[k] = take(n * sizeof(T));
+            N.e[k] = take(n * sizeof(T));
+        }
+    }
+    N.z0 = take(C.mult ? (size_t)A->nrows * sizeof(T) : 0);
+    N.x0 = take((size_t)A->nrows * 8);   // the caller's start, while it may be needed again
+    N.binv = take((size_t)kMgBottom * kMgBottom * sizeof(T));
+    N.part = take(kProbePart);
+    // FP64: r z p q; mixed: r q xc, two pairs, FP64 residual
+    const size_t n0 = A->nrows;
+    N.vec = take(sizeof(T) == 8 ? 4 * al(n0 * 8) : 3 * al(n0 * 4) + 2 * al(n0 * 8) + al(n0 * 8));
+    return at + al((size_t)2 * kPartStride * 8) + al(sizeof(SolveState));
+}
+
+size_t mg_need(grmp_matrix A, MgCache &C, bool mixed) {
+    return mixed ? mg_layout<float>(A, C, nullptr) : mg_layout<double>(A, C, nullptr);
+}
+
+// The patterns, on the device; A->mg stays nullptr on failure.  GRMP_ERR_BUDGET
+// before anything is taken if they and the storage of this precision do not fit.
+int mg_build(grmp_matrix A, bool mixed) {
     grmp_space s = A->space;
     grmp_context ctx = s->mesh->ctx;
     const int n = A->nrows;
@@ -1197,8 +1251,8 @@ int mg_build(grmp_matrix A) {
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multilevel: pattern download");
-    MgCache *C = new MgCache;
-    A->mg = C;
+    std::unique_ptr<MgCache> own(new MgCache);
+    MgCache *C = own.get();
     C->mult = fine_mult(s->mesh->dim, s->fe, n);
     const MgCells m{s->mesh->dim, s->mesh->ncells, s->ldofs, cd.data(), cells.data(), coords.data()};
     if (mg_symbolic_build(n, pattern, m, p2, !A->face_coupled, stretched, C->mult, &C->S)) {
@@ -1207,8 +1261,9 @@ int mg_build(grmp_matrix A) {
     }
     const int ns = (int)C->S.step.size();
     C->step.resize(ns);
-    for (int k = 0; k < ns && !rc; k++) {
-        MgStep &t = C->S.step[k];
+    size_t need = 0;
+    for (int k = 0; k < ns; k++) {
+        const MgStep &t = C->S.step[k];
         MgCache::Step &d = C->step[k];
         d.np = t.P.ci.size();
         d.na = t.AP.ci.size();
@@ -1221,18 +1276,28 @@ int mg_build(grmp_matrix A) {
         };
         d.longa = longest(t.AP.rp);
         d.longc = longest(t.Ac.rp);
+        for (const MgCsr *x : {&t.P, &t.R, &t.AP, &t.QT, &t.Ac}) need += (x->rp.size() + x->ci.size()) * 4;
+        need += (t.Rperm.size() + t.QTperm.size() + t.agg.size()) * 4 + (t.geometric ? (size_t)t.nc * 4 + (size_t)t.n * 8 : 0);
+    }
+    need += mg_need(A, *C, mixed);
+    A->mg_floor[mixed] = need > A->mg_budget ? SIZE_MAX : need;
+    if (need > A->mg_budget || (ctx->budget && need > ctx->budget - std::min(ctx->budget, ctx->in_use))) return GRMP_ERR_BUDGET;
+    for (int k = 0; k < ns && !rc; k++) {
+        MgStep &t = C->S.step[k];
+        MgCache::Step &d = C->step[k];
         auto up = [&](std::vector<int32_t> &v, int32_t **p) {
             if (!rc) rc = mg_up_vec(ctx, *C, v, p);
         };
+        std::vector<int32_t> vrow;
+        std::vector<int2> ell;
         if (t.geometric) {
-            std::vector<int32_t> vrow(t.nc);
+            vrow.resize(t.nc);
             for (int i = 0; i < t.n; i++)
                 if (t.P.rp[i + 1] - t.P.rp[i] == 1) vrow[t.P.ci[t.P.rp[i]]] = i;
             up(vrow, &d.vrow);
-            std::vector<int2> ell(t.n);
+            ell.resize(t.n);
             for (int i = 0; i < t.n; i++) ell[i] = make_int2(t.P.ci[t.P.rp[i]], t.P.ci[t.P.rp[i + 1] - 1]);
             if (!rc) rc = mg_up_vec(ctx, *C, ell, &d.ell);
-            if (!rc && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = GRMP_ERR_DEVICE;
         } else {
             up(t.agg, &d.agg);
         }
@@ -1250,11 +1315,15 @@ int mg_build(grmp_matrix A) {
             up(t.QT.ci, &d.tci);
             up(t.QTperm, &d.tperm);
         }
-        if (!rc && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = GRMP_ERR_DEVICE;
+        if (cudaStreamSynchronize(ctx->stream) != cudaSuccess && !rc) rc = GRMP_ERR_DEVICE;
         t.P = t.R = t.AP = t.QT = t.Ac = MgCsr();   // the sizes stay
         t.Rperm = t.QTperm = t.agg = std::vector<int32_t>();
     }
-    if (rc) return rc;
+    if (rc) {
+        for (auto &b : C->bufs) grmp_free(ctx, b.first, b.second);
+        return rc;
+    }
+    A->mg = own.release();
     A->mg_state = 1;
     return GRMP_OK;
 }
@@ -1262,69 +1331,58 @@ int mg_build(grmp_matrix A) {
 size_t mg_bytes(const MgCache &C) {
     size_t b = 0;
     for (auto &x : C.bufs) b += x.second;
-    for (auto &N : C.num) b += N.bytes;
     return b;
 }
 
-// the probe's flag and per-block sums
-constexpr int kProbeBlocks = 2048;
-constexpr size_t kProbePart = (size_t)(kProbeBlocks + 1) * 16;
-
-// numeric storage of one precision: values of every level, vectors, state
-template <typename T>
-int mg_storage(grmp_matrix A) {
+// whether there is still less room than this precision needs (the other one's storage counts as room)
+bool mg_no_room(grmp_matrix A, bool mixed) {
     grmp_context ctx = A->space->mesh->ctx;
-    MgCache &C = *A->mg;
-    MgCache::Num &N = C.num[sizeof(T) == 8 ? 0 : 1];
-    if (N.p) return GRMP_OK;
-    const int ns = (int)C.step.size();
-    for (int pass = 0; pass < 2; pass++) {
-        size_t at = 0;
-        auto take = [&](size_t bytes) -> char * {
-            const size_t o = at;
-            at += al(bytes);
-            return pass ? (char *)N.p + o : nullptr;
-        };
-        N.pv.assign(ns, nullptr);
-        N.av = N.tv = N.cv = N.pv;
-        N.D.assign(ns + 1, nullptr);
-        N.iso = N.r = N.y = N.e = N.D;
-        for (int k = 0; k < ns; k++) {
-            const MgCache::Step &d = C.step[k];
-            N.pv[k] = take(d.np * sizeof(T));
-            N.av[k] = take(d.na * sizeof(T));
-            N.cv[k] = take(d.nc * sizeof(T));
-            N.tv[k] = take(d.nt * sizeof(T));
+    const size_t floor = A->mg_floor[mixed], other = A->mg ? A->mg->num[!mixed].bytes : 0;
+    if (floor == 0 || floor == SIZE_MAX) return floor > 0;
+    if (ctx->budget && ctx->in_use - other + floor > ctx->budget) return true;
+    return grmp_room(ctx) + other < floor;
+}
+
+// The hierarchy with storage of this precision.  *fits = false: there is no
+// room for it now; the patterns and the other precision's storage then stay if
+// that is in use.  Of two precisions that do not fit together the one asked for
+// has the room, whatever was solved before.
+int mg_make(grmp_matrix A, bool mixed, bool *fits) {
+    grmp_context ctx = A->space->mesh->ctx;
+    *fits = false;
+    int rc = A->mg ? GRMP_OK : mg_build(A, mixed);
+    if (!rc && A->mg_state < 0) return GRMP_OK;
+    if (!rc) {
+        MgCache &C = *A->mg;
+        MgCache::Num &N = C.num[mixed], &O = C.num[!mixed];
+        const size_t need = mg_need(A, C, mixed), pat = mg_bytes(C);
+        A->mg_floor[mixed] = pat + need > A->mg_budget ? SIZE_MAX : need;
+        rc = GRMP_ERR_BUDGET;
+        if (pat + need + O.bytes <= A->mg_budget) rc = grmp_alloc(ctx, &N.p, need);
+        if ((rc == GRMP_ERR_BUDGET || rc == GRMP_ERR_OUT_OF_MEMORY) && O.p && pat + need <= A->mg_budget &&
+            (!ctx->budget || ctx->in_use - O.bytes + need <= ctx->budget)) {
+            cudaGetLastError();
+            grmp_free(ctx, O.p, O.bytes);
+            O.p = nullptr;
+            O.bytes = 0;
+            rc = grmp_alloc(ctx, &N.p, need);
         }
-        N.rv0 = take(C.step[0].np * sizeof(T));
-        N.ellv = take(C.step[0].ell ? (size_t)A->nrows * 2 * sizeof(T) : 0);
-        for (int k = 0; k <= ns; k++) {
-            const size_t n = k < ns ? C.S.step[k].n : C.S.step[ns - 1].nc;
-            N.D[k] = take(n * sizeof(T));
-            N.iso[k] = take(n);
-            if (k > 0) {
-                N.r[k] = take(n * sizeof(T));
-                N.y[k] = take(n * sizeof(T));
-                N.e[k] = take(n * sizeof(T));
-            }
-        }
-        N.z0 = take(C.mult ? (size_t)A->nrows * sizeof(T) : 0);
-        N.x0 = take((size_t)A->nrows * 8);   // the caller's start, while it may be needed again
-        N.binv = take((size_t)kMgBottom * kMgBottom * sizeof(T));
-        N.part = take(kProbePart);
-        // FP64: r z p q; mixed: r q xc, two pairs, FP64 residual
-        const size_t n0 = A->nrows;
-        N.vec = take(sizeof(T) == 8 ? 4 * al(n0 * 8) : 3 * al(n0 * 4) + 2 * al(n0 * 8) + al(n0 * 8));
-        if (pass == 0) {
-            N.bytes = at + al((size_t)2 * kPartStride * 8) + al(sizeof(SolveState));
-            int rc = mg_bytes(C) > A->mg_budget ? (int)GRMP_ERR_BUDGET : grmp_alloc(ctx, &N.p, N.bytes);
-            if (rc) {
-                N.p = nullptr;
-                N.bytes = 0;
-                return rc;
-            }
+        if (!rc) {
+            N.bytes = need;
+            mixed ? mg_layout<float>(A, C, (char *)N.p) : mg_layout<double>(A, C, (char *)N.p);
+        } else if (!O.p) {   // patterns alone are of no use
+            if (A->mg_floor[mixed] != SIZE_MAX) A->mg_floor[mixed] += pat;
+            grmp_mg_free(A);
         }
     }
+    if (rc == GRMP_ERR_BUDGET || rc == GRMP_ERR_OUT_OF_MEMORY) {
+        ctx->last_error.clear();
+        cudaGetLastError();
+        return GRMP_OK;
+    }
+    if (rc) return rc;
+    A->mg_floor[mixed] = 0;
+    *fits = true;
     return GRMP_OK;
 }
 
@@ -1646,6 +1704,7 @@ int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool *checked, bool bic
     int rc = GRMP_OK;
     double react = 0.0;
     if (!grmp_mg_ready(A, mixed)) {
+        if (mg_no_room(A, mixed)) return GRMP_OK;
         // the matrix is looked at first: analysis and storage are for those that the cycle is for
         rc = mixed ? mg_probe_first<float>(A, &react) : mg_probe_first<double>(A, &react);
         *checked = !rc;
@@ -1653,16 +1712,14 @@ int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool *checked, bool bic
             A->reaction |= bit;
             return GRMP_OK;
         }
-        if (!rc && !A->mg) rc = mg_build(A);
-        if (!rc && A->mg_state > 0) rc = mixed ? mg_storage<float>(A) : mg_storage<double>(A);
-        if (rc == GRMP_ERR_BUDGET || rc == GRMP_ERR_OUT_OF_MEMORY) {   // no room for the hierarchy: the Jacobi solvers
-            grmp_mg_free(A);
-            A->mg_state = -1;
+        bool fits = false;
+        if (!rc) rc = mg_make(A, mixed, &fits);
+        if (rc == GRMP_ERR_BUDGET || rc == GRMP_ERR_OUT_OF_MEMORY) {   // not even room to look
             ctx->last_error.clear();
             cudaGetLastError();
             return GRMP_OK;
         }
-        if (rc || A->mg_state < 0) return rc;
+        if (rc || !fits) return rc;
     }
     MgCache::Num &N = A->mg->num[mixed ? 1 : 0];
     rc = mixed ? mg_probe<float>(A, N.D[0], N.iso[0], N.part, &react) : mg_probe<double>(A, N.D[0], N.iso[0], N.part, &react);

@@ -1969,6 +1969,11 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
         grmp_free(ctx, A->d_work, A->work_bytes);
         A->work_bytes = 0;
         int rc = grmp_alloc(ctx, &A->d_work, need);
+        if (rc && A->mg) {   // the hierarchy's memory first goes to what solves without it
+            cudaGetLastError();
+            grmp_mg_free(A);
+            rc = grmp_alloc(ctx, &A->d_work, need);
+        }
         if (rc) return rc;
         A->work_bytes = need;
     }
