@@ -6,6 +6,7 @@
 #include <new>
 
 #include "grmp_internal.h"
+#include "mg.h"
 
 namespace {
 bool valid_ctx(grmp_context c) { return c != nullptr && c->stream != nullptr; }
@@ -28,7 +29,7 @@ int grmp_cuda_fail(grmp_context ctx, cudaError_t e, const char *what) {
     return grmp_fail(ctx, code, "%s: %s", what, cudaGetErrorString(e));
 }
 
-int grmp_alloc(grmp_context ctx, void **p, size_t bytes) {
+int grmp_alloc_spare(grmp_context ctx, void **p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) return GRMP_OK;
     if (ctx->budget && ctx->in_use + bytes > ctx->budget)
@@ -41,6 +42,16 @@ int grmp_alloc(grmp_context ctx, void **p, size_t bytes) {
     }
     ctx->in_use += bytes;
     return GRMP_OK;
+}
+
+int grmp_alloc(grmp_context ctx, void **p, size_t bytes) {
+    int rc = grmp_alloc_spare(ctx, p, bytes);
+    if (rc != GRMP_ERR_BUDGET && rc != GRMP_ERR_OUT_OF_MEMORY) return rc;
+    cudaGetLastError();
+    if (!grmp_mg_reclaim(ctx, bytes)) return rc;
+    rc = grmp_alloc_spare(ctx, p, bytes);
+    if (!rc) ctx->last_error.clear();
+    return rc;
 }
 
 void grmp_free(grmp_context ctx, void *p, size_t bytes) {

@@ -32,6 +32,7 @@ struct grmp_context_s {
     std::string last_error;
     void *pin = nullptr;     // kPinBytes of page-locked host memory for grmp_readback
     std::mutex mu;
+    std::vector<grmp_matrix> hier;   // matrices with a multilevel hierarchy
 };
 
 struct grmp_mesh_s {
@@ -144,6 +145,7 @@ struct grmp_matrix_s {
     struct MgCache *mg = nullptr;
     int mg_state = 0;
     size_t mg_floor[2] = {0, 0};    // FP64, FP32: the room it needs, where it has not been had (not tried with less)
+    int mg_reclaimed = 0;           // how often other allocations have taken its memory
     size_t mg_budget = SIZE_MAX;    // device bytes it may take (served requests: what their estimate leaves)
     bool elliptic = false;
     int reaction = 0;               // the present values are reaction dominated: bit 0 FP64, 1 FP32 (cleared where values are written)
@@ -177,8 +179,11 @@ int grmp_cuda_fail(grmp_context ctx, cudaError_t e, const char *what);
 // count one kernel launch of a context
 #define GRMP_LAUNCHED(ctx) ((ctx)->launches.fetch_add(1, std::memory_order_relaxed))
 
-// device memory accounted against the context budget
+// device memory accounted against the context budget; multilevel hierarchies
+// give theirs up where there is not enough
 int grmp_alloc(grmp_context ctx, void **p, size_t bytes);
+// the same for what can be done without: takes nothing from a hierarchy
+int grmp_alloc_spare(grmp_context ctx, void **p, size_t bytes);
 void grmp_free(grmp_context ctx, void *p, size_t bytes);
 // bytes that can still be had: a share of the device's, with what its pool
 // holds without using it, and no more than the budget's

@@ -1138,7 +1138,7 @@ template <typename V>
 int mg_up_vec(grmp_context ctx, MgCache &C, const std::vector<V> &v, V **out) {
     const size_t bytes = std::max<size_t>(1, v.size()) * sizeof(V);
     void *p = nullptr;
-    int rc = grmp_alloc(ctx, &p, bytes);
+    int rc = grmp_alloc_spare(ctx, &p, bytes);
     if (rc) return rc;
     C.bufs.push_back({p, bytes});
     *out = (V *)p;
@@ -1154,7 +1154,7 @@ int mg_up_vec(grmp_context ctx, MgCache &C, const std::vector<V> &v, V **out) {
 int mg_stretched(grmp_mesh m, bool *out) {
     grmp_context ctx = m->ctx;
     int *cnt = nullptr, h = 0;
-    int rc = grmp_alloc(ctx, (void **)&cnt, 4);
+    int rc = grmp_alloc_spare(ctx, (void **)&cnt, 4);
     if (rc) return rc;
     cudaMemsetAsync(cnt, 0, 4, ctx->stream);
     if (m->dim == 2) k_mg_stretched<2><<<nblk(m->ncells), 256, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, cnt);
@@ -1324,6 +1324,7 @@ int mg_build(grmp_matrix A, bool mixed) {
         return rc;
     }
     A->mg = own.release();
+    ctx->hier.push_back(A);
     A->mg_state = 1;
     return GRMP_OK;
 }
@@ -1358,14 +1359,14 @@ int mg_make(grmp_matrix A, bool mixed, bool *fits) {
         const size_t need = mg_need(A, C, mixed), pat = mg_bytes(C);
         A->mg_floor[mixed] = pat + need > A->mg_budget ? SIZE_MAX : need;
         rc = GRMP_ERR_BUDGET;
-        if (pat + need + O.bytes <= A->mg_budget) rc = grmp_alloc(ctx, &N.p, need);
+        if (pat + need + O.bytes <= A->mg_budget) rc = grmp_alloc_spare(ctx, &N.p, need);
         if ((rc == GRMP_ERR_BUDGET || rc == GRMP_ERR_OUT_OF_MEMORY) && O.p && pat + need <= A->mg_budget &&
             (!ctx->budget || ctx->in_use - O.bytes + need <= ctx->budget)) {
             cudaGetLastError();
             grmp_free(ctx, O.p, O.bytes);
             O.p = nullptr;
             O.bytes = 0;
-            rc = grmp_alloc(ctx, &N.p, need);
+            rc = grmp_alloc_spare(ctx, &N.p, need);
         }
         if (!rc) {
             N.bytes = need;
@@ -1427,7 +1428,7 @@ int mg_probe_first(grmp_matrix A, double *react) {
     grmp_context ctx = A->space->mesh->ctx;
     const size_t d = al((size_t)A->nrows * sizeof(T)), i = al((size_t)A->nrows), bytes = d + i + kProbePart;
     char *w = nullptr;
-    int rc = grmp_alloc(ctx, (void **)&w, bytes);
+    int rc = grmp_alloc_spare(ctx, (void **)&w, bytes);
     if (rc) return rc;
     rc = mg_probe<T>(A, w, w + d, w + d + i, react);
     grmp_free(ctx, w, bytes);
@@ -1688,11 +1689,32 @@ void grmp_mg_free(grmp_matrix A) {
     for (auto &N : A->mg->num) grmp_free(ctx, N.p, N.bytes);
     delete A->mg;
     A->mg = nullptr;
+    ctx->hier.erase(std::find(ctx->hier.begin(), ctx->hier.end(), A));
 }
 
-bool grmp_mg_ready(grmp_matrix A, bool mixed) { return A->mg_state > 0 && A->mg && A->mg->num[mixed ? 1 : 0].p; }
+bool grmp_mg_reclaim(grmp_context ctx, size_t bytes) {
+    bool any = false;
+    while (!ctx->hier.empty() && !(any && ctx->budget && ctx->in_use + bytes <= ctx->budget)) {
+        grmp_matrix A = ctx->hier.back();
+        const size_t pat = mg_bytes(*A->mg), both = ++A->mg_reclaimed > 2 ? bytes : 0;
+        for (int k = 0; k < 2; k++)
+            if (A->mg_floor[k] != SIZE_MAX)
+                A->mg_floor[k] = pat + both + (A->mg->num[k].p ? A->mg->num[k].bytes : mg_need(A, *A->mg, k));
+        grmp_mg_free(A);
+        any = true;
+    }
+    return any;
+}
 
-int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool *checked, bool bicg) {
+namespace {
+
+// whether a hierarchy with numeric storage of this precision exists
+bool mg_ready(grmp_matrix A, bool mixed) { return A->mg_state > 0 && A->mg && A->mg->num[mixed ? 1 : 0].p; }
+
+// Whether the multilevel solver is for this matrix (scalar H1P1 / H1P2 with a
+// diffusion term, not reaction dominated); builds or refreshes what it needs.
+// *use = 0: the Jacobi solvers.  bicg: for BiCGStab, which pays from fewer rows.
+int mg_prepare(grmp_matrix A, bool mixed, int *use, bool *checked, bool bicg = false) {
     *use = 0;
     *checked = false;
     grmp_space s = A->space;
@@ -1703,7 +1725,7 @@ int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool *checked, bool bic
         return GRMP_OK;
     int rc = GRMP_OK;
     double react = 0.0;
-    if (!grmp_mg_ready(A, mixed)) {
+    if (!mg_ready(A, mixed)) {
         if (mg_no_room(A, mixed)) return GRMP_OK;
         // the matrix is looked at first: analysis and storage are for those that the cycle is for
         rc = mixed ? mg_probe_first<float>(A, &react) : mg_probe_first<double>(A, &react);
@@ -1737,7 +1759,7 @@ int grmp_mg_prepare(grmp_matrix A, bool mixed, int *use, bool *checked, bool bic
     return GRMP_OK;
 }
 
-int grmp_mg_solve(grmp_matrix A, const double *b, double *x, bool mixed, grmp_solve_params *p, grmp_solve_stats *st,
+int mg_solve(grmp_matrix A, const double *b, double *x, bool mixed, grmp_solve_params *p, grmp_solve_stats *st,
                   bool *done) {
     grmp_context ctx = A->space->mesh->ctx;
     const double avg = (double)A->nnz / std::max(1, A->nrows);
@@ -1787,27 +1809,33 @@ int grmp_mg_solve(grmp_matrix A, const double *b, double *x, bool mixed, grmp_so
     return e == cudaSuccess ? GRMP_OK : grmp_cuda_fail(ctx, e, "multilevel solve");
 }
 
+}  // namespace
+
 int grmp_mg_cg(grmp_matrix A, const double *b, double *x, grmp_solve_params *p, grmp_solve_stats *st, bool *done,
-               bool *checked) {
+               bool *checked, bool present) {
     *done = *checked = false;
     for (int mixed = p->mode == GRMP_SOLVE_MIXED; mixed >= 0; mixed--) {
+        if (present && !mg_ready(A, mixed)) return GRMP_OK;
         int use = 0;
         bool ok = false;
-        int rc = grmp_mg_prepare(A, mixed, &use, &ok);
+        int rc = mg_prepare(A, mixed, &use, &ok);
         *checked = *checked || ok;   // of the caller's precision: the first to be looked at
         if (rc || !use) return rc;
-        rc = grmp_mg_solve(A, b, x, mixed, p, st, done);
+        rc = mg_solve(A, b, x, mixed, p, st, done);
         if (rc || *done || st->iterations >= p->maxiter) return rc;
     }
     return GRMP_OK;
 }
 
 int grmp_mg_bicgstab(grmp_matrix A, const double *b, double *x, const grmp_solve_params *p, double *const vec[9],
-                     double *partial, void *state, grmp_solve_stats *st, bool *done) {
+                     double *partial, void *state, grmp_solve_stats *st, bool *done, bool *checked) {
     grmp_context ctx = A->space->mesh->ctx;
     const double avg = (double)A->nnz / std::max(1, A->nrows);
     SolveState *dst = (SolveState *)state;
     *done = false;
+    int use = 0;
+    const int prc = mg_prepare(A, false, &use, checked, true);
+    if (prc || !use) return prc;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);

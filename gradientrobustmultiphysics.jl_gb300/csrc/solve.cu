@@ -1969,11 +1969,6 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
         grmp_free(ctx, A->d_work, A->work_bytes);
         A->work_bytes = 0;
         int rc = grmp_alloc(ctx, &A->d_work, need);
-        if (rc && A->mg) {   // the hierarchy's memory first goes to what solves without it
-            cudaGetLastError();
-            grmp_mg_free(A);
-            rc = grmp_alloc(ctx, &A->d_work, need);
-        }
         if (rc) return rc;
         A->work_bytes = need;
     }
@@ -1982,16 +1977,11 @@ int grmp_solve_impl(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solv
     WorkLayout lay{vec, off_r64, off_part};
     cudaMemsetAsync(dst, 0, sizeof(SolveState), ctx->stream);
     if (bicg) {   // scalar Jacobians: multilevel, else (and where that fails) Jacobi
-        int use = 0;
-        int rc = grmp_mg_prepare(A, false, &use, &checked, true);
-        if (rc) return rc;
-        if (use) {
-            double *vv[9];
-            for (int k = 0; k < 9; k++) vv[k] = (double *)(work + (size_t)k * vec);
-            bool done = false;
-            rc = grmp_mg_bicgstab(A, b->d, x->d, p, vv, (double *)(work + off_part), dst, st, &done);
-            if (rc || done) return rc;
-        }
+        double *vv[9];
+        for (int k = 0; k < 9; k++) vv[k] = (double *)(work + (size_t)k * vec);
+        bool done = false;
+        const int rc = grmp_mg_bicgstab(A, b->d, x->d, p, vv, (double *)(work + off_part), dst, st, &done, &checked);
+        if (rc || done) return rc;
     }
     // Jacobi preconditioner (not for the Jacobi-scaled configurations, which
     // form and check their own row scales)
@@ -2204,9 +2194,9 @@ extern "C" int grmp_solve_fp64_noalloc(grmp_matrix A, grmp_vector b, grmp_vector
     // the hierarchy that an FP64 grmp_solve of this matrix left: the same solver,
     // in that hierarchy's own storage
     grmp_solve_params q = *p;
-    if (p->spmv_config <= 0 && grmp_mg_ready(A, false)) {
+    if (p->spmv_config <= 0) {
         bool done = false, checked = false;
-        const int mrc = grmp_mg_cg(A, b->d, x->d, &q, st, &done, &checked);
+        const int mrc = grmp_mg_cg(A, b->d, x->d, &q, st, &done, &checked, true);
         if (mrc || done) return mrc;
         std::memset(st, 0, sizeof(*st));
         p = &q;

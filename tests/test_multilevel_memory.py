@@ -101,3 +101,32 @@ def test_the_jacobi_workspace_comes_first(G):
     assert p.solve("mixed")[0]
     assert not p.solve("fp64")[0]
     p.solve("mixed")
+
+
+def test_memory_goes_to_what_is_allocated_later(G):
+    """A vector and a second matrix that fit beside the first matrix, not beside
+    its hierarchy too: they are had, and the hierarchy is made again when they are gone."""
+    base, one, both, x64, x32 = _sizes(G)
+    budget = one + (1 << 20)
+    c = G.GB300Context(0, hbm_budget_bytes=budget)
+    p = _Problem(G, c)
+    assert p.solve("fp64")[0]
+    big = _vector(G, c, budget - base - (1 << 20))
+    big.fill(2.0)
+    took, x = p.solve("fp64")   # the Jacobi workspace fits beside the vector
+    assert not took and np.linalg.norm(x - x64) <= 1e-8 * np.linalg.norm(x64)
+    assert np.array_equal(big.entries, np.full(big.n, 2.0))
+    del big
+    took, x = p.solve("fp64")
+    assert took and np.array_equal(x, x64)
+    for _ in range(3):   # again and again: then the analysis is no longer made for one solve each
+        big = _vector(G, c, budget - base - (1 << 20))
+        del big
+        took, x = p.solve("fp64")
+    assert not took and np.linalg.norm(x - x64) <= 1e-8 * np.linalg.norm(x64)
+    A2 = G.FEMatrix(c, p.S, p.ops)
+    G.assemble(A2, p.ops, G.FP64)
+    y = G.FEVector(c, p.S)
+    G.spmv(A2, p.x, y, G.FP64)
+    assert np.all(np.isfinite(y.entries))
+
