@@ -106,12 +106,12 @@ __device__ __forceinline__ void basis_grad(int a, const double lam[DIM + 1], con
     if (a <= DIM) {
         const double c = NB == DIM + 1 ? 1.0 : 4.0 * lam[a] - 1.0;
 #pragma unroll
-        for (int k = 0; k < DIM; k++) g[k] = c * gl[a][k];
+        for (int k = 0; k < DIM; k++) g[k] = __dmul_rn(c, gl[a][k]);
     } else {
         const int i = edge_vertex<DIM>(a - DIM - 1, 0), j = edge_vertex<DIM>(a - DIM - 1, 1);
         const double ci = 4.0 * lam[i], cj = 4.0 * lam[j];
 #pragma unroll
-        for (int k = 0; k < DIM; k++) g[k] = ci * gl[j][k] + cj * gl[i][k];
+        for (int k = 0; k < DIM; k++) g[k] = fma(ci, gl[j][k], __dmul_rn(cj, gl[i][k]));
     }
 }
 
@@ -203,6 +203,38 @@ struct FaceTermDev {
 };
 
 // ------------------------------------------------------------------ face bilinear terms
+// one point's contribution to an entry of a face's matrix from the jumps of two
+// functions (explicit fma: both kernels that form entries round alike)
+template <int DIM>
+__device__ __forceinline__ double face_point_entry(const double a[DIM], const double b[DIM], double w, double s) {
+    double d = 0.0;
+#pragma unroll
+    for (int k = 0; k < DIM; k++) d = fma(a[k], b[k], d);
+    return fma(w, d, s);
+}
+
+// adds v to the entry of column col in the row [r0, r1)
+__device__ __forceinline__ void add_entry(int r0, int r1, const int32_t *cols, int32_t col, double v, double *v64,
+                                          float *v32, int *missing) {
+    int lo = r0, hi = r1;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (cols[mid] < col) lo = mid + 1;
+        else hi = mid;
+    }
+    if (lo >= r1 || cols[lo] != col) {
+        atomicExch(missing, 1);
+        return;
+    }
+    v64[lo] += v;
+    if (v32) v32[lo] += (float)v;
+}
+
+struct FaceGeom {
+    const int32_t *cell_faces, *cells, *celldofs;
+    const double *coords, *gl, *fvol;
+};
+
 // Face matrices, then rows.  k_face_mats: a block takes fb faces; a thread per
 // (face, point) puts the jump of every function of the two cells into shared
 // memory, then a thread per entry i <= j of a face's matrix sums over the
@@ -211,8 +243,9 @@ struct FaceTermDev {
 // fn: their number).  k_face_add: LPR lanes per row, a lane per column, walk
 // the row's cells in ascending order and their interior faces (a face that two
 // cells of the row share comes from the lower one) and add the row of the
-// face's matrix: the same order of additions as adding face by face in one
-// thread, no atomics.
+// face's matrix: within a chunk of faces (kFaceBytes) the same order of
+// additions as adding face by face in one thread, no atomics.  The chunks depend
+// on the mesh alone, so the bits do too.
 //
 // Bound by FP64 issue in k_face_mats (45 entries x 2 points x 3 operations a
 // face for P2 triangles) and by the face matrices' write and read (63 MB for
@@ -300,10 +333,10 @@ __global__ void __launch_bounds__(128) k_face_mats(int F0, int nf, int fb, const
         const double *Ja = J + (size_t)i * r.nq * NC * DIM + a * DIM, *Jb = Ja + (b - a) * DIM;
         double s = 0.0;
         for (int q = 0; q < r.nq; q++, Ja += NC * DIM, Jb += NC * DIM) {
-            double d = 0.0;
+            double a_[DIM], b_[DIM];
 #pragma unroll
-            for (int k = 0; k < DIM; k++) d += Ja[k] * Jb[k];
-            s += r.w[q] * d;
+            for (int k = 0; k < DIM; k++) a_[k] = Ja[k], b_[k] = Jb[k];
+            s = face_point_entry<DIM>(a_, b_, r.w[q], s);
         }
         s *= sc[i];
         double *M = mats + (size_t)(base + i) * NC * NC;
@@ -337,22 +370,77 @@ __global__ void __launch_bounds__(128) k_face_add(int32_t nrows, int F0, int nf,
             const unsigned own = __ballot_sync(mask, col == row);
             const int a = __ffs(own >> first) - 1;
             if (c2 < c && a < NB) continue;   // taken from the lower of the row's two cells
-            if (col >= 0) {
-                int lo = r0, hi = r1;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (cols[mid] < col) lo = mid + 1;
-                    else hi = mid;
-                }
-                if (lo >= r1 || cols[lo] != col) {
-                    atomicExch(missing, 1);
-                } else {
-                    const double v = mats[(size_t)i * NC * NC + a * n + sub];
-                    v64[lo] += v;
-                    if (v32) v32[lo] += (float)v;
-                }
-            }
+            if (col >= 0) add_entry(r0, r1, cols, col, mats[(size_t)i * NC * NC + a * n + sub], v64, v32, missing);
             __syncwarp(mask);   // the next face may meet the same entries from other lanes
+        }
+    }
+}
+
+// The same without face matrices, where there is no memory for them: a thread
+// per row takes the row's faces in the same order and forms every entry as
+// k_face_mats does, bit for bit.  129,600 P2 rows: assembly 1.4 ms (0.32 with matrices).
+template <int DIM, int NB>
+__global__ void __launch_bounds__(128) k_face_rows(int32_t nrows, int F0, int nf, const int32_t *inc_ptr,
+                                                   const int32_t *inc_cell, const int32_t *nbr, const int32_t *rowptr,
+                                                   const int32_t *cols, double *v64, float *v32, int *missing, FaceGeom m,
+                                                   FaceTermDev t, FaceRule r) {
+    constexpr int NF = DIM + 1, NC = 2 * NB;
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= nrows) return;
+    const int r0 = rowptr[row], r1 = rowptr[row + 1];
+    for (int p = inc_ptr[row]; p < inc_ptr[row + 1]; p++) {
+        const int c = inc_cell[p];
+        for (int f = 0; f < NF; f++) {
+            const int o = nbr[(size_t)c * NF + f];
+            if (o < 0) continue;
+            const int F = m.cell_faces[(size_t)c * NF + f];
+            if (F < F0 || F >= F0 + nf) continue;
+            const int c1 = min(c, o), c2 = max(c, o);
+            // the functions as k_face_mats numbers them, and the row's own
+            int32_t col[NC];
+            int map[NB], n = NB, a = -1;
+            for (int b = 0; b < NB; b++) {
+                col[b] = m.celldofs[(size_t)c1 * NB + b];
+                if (col[b] == row) a = b;
+            }
+            if (o < c && a >= 0) continue;   // taken from the lower of the row's two cells
+            for (int b = 0; b < NB; b++) {
+                const int32_t d = m.celldofs[(size_t)c2 * NB + b];
+                int k = -1;
+                for (int e = 0; e < NB; e++)
+                    if (col[e] == d) k = e;
+                if (k < 0) {
+                    k = n++;
+                    col[k] = d;
+                    if (d == row) a = k;
+                }
+                map[b] = k;
+            }
+            if (a < 0) continue;   // (the row is a function of its own cell)
+            double s[NC];
+            for (int e = 0; e < n; e++) s[e] = 0.0;
+            for (int q = 0; q < r.nq; q++) {
+                double J[NC][DIM];
+                for (int side = 0; side < 2; side++) {
+                    const int cc = side ? c2 : c1;
+                    int loc[DIM];
+                    double lam[DIM + 1], g[DIM + 1][DIM];
+                    face_canon<DIM>(m.cells, cc, face_in_cell<DIM>(m.cell_faces, cc, F), loc);
+                    face_point<DIM>(r.lam[q], loc, lam);
+                    load_grads<DIM>(m.gl, m.coords, m.cells, cc, g);
+#pragma unroll
+                    for (int b = 0; b < NB; b++) {
+                        double d[DIM];
+                        basis_grad<DIM, NB>(b, lam, g, d);
+                        const int e = side ? map[b] : b;
+#pragma unroll
+                        for (int k = 0; k < DIM; k++) J[e][k] = !side ? d[k] : (e < NB ? J[e][k] - d[k] : -d[k]);
+                    }
+                }
+                for (int e = 0; e < n; e++) s[e] = face_point_entry<DIM>(J[a], J[e], r.w[q], s[e]);
+            }
+            const double fv = m.fvol[F], sc = t.factor * fv * power_of(fv, t.power);
+            for (int e = 0; e < n; e++) add_entry(r0, r1, cols, col[e], __dmul_rn(s[e], sc), v64, v32, missing);
         }
     }
 }
@@ -439,8 +527,9 @@ __global__ void __launch_bounds__(128) k_face_jumps(int32_t nfaces, const int32_
 double *cell_grads(grmp_mesh m) {
     grmp_context ctx = m->ctx;
     double *gl = nullptr;
-    if (grmp_alloc(ctx, (void **)&gl, (size_t)m->ncells * (m->dim + 1) * m->dim * 8)) {
+    if (grmp_alloc_spare(ctx, (void **)&gl, (size_t)m->ncells * (m->dim + 1) * m->dim * 8)) {
         cudaGetLastError();
+        ctx->last_error.clear();
         return nullptr;
     }
     if (m->dim == 2) k_cell_grads<2><<<nblk(m->ncells, 128), 128, 0, ctx->stream>>>(m->ncells, m->d_coords, m->d_cells, gl);
@@ -533,19 +622,19 @@ int grmp_face_assemble(grmp_matrix A, int nterms, const grmp_bilinear_term *term
     rc = grmp_alloc(ctx, (void **)&dmiss, 4);
     if (rc) return rc;
     cudaMemsetAsync(dmiss, 0, 4, ctx->stream);
-    // scratch: gradients of the cells, matrices and columns of a chunk of faces (halved until it fits)
+    // scratch: gradients of the cells, matrices and columns of a chunk of faces; without room for them
+    // the rows form their entries themselves
     double *gl = nullptr, *mats = nullptr;
     int32_t *fcol = nullptr, *fn = nullptr;
     const int nc = 2 * s->nb;
     const size_t per = (size_t)nc * nc * 8;
-    int chunk = (int)std::min<size_t>((size_t)m->nfaces, kFaceBytes / per);
+    const int chunk = (int)std::min<size_t>((size_t)m->nfaces, kFaceBytes / per);
     gl = cell_grads(m);
     // matrices, columns and numbers of a chunk in one piece
-    while ((rc = grmp_alloc(ctx, (void **)&mats, (size_t)chunk * (per + nc * 4 + 4))) && chunk > 32) {
+    if (grmp_alloc_spare(ctx, (void **)&mats, (size_t)chunk * (per + nc * 4 + 4))) {
         cudaGetLastError();
-        chunk = (chunk + 1) / 2;
-    }
-    if (!rc) {
+        ctx->last_error.clear();
+    } else {
         fcol = reinterpret_cast<int32_t *>(mats + (size_t)chunk * nc * nc);
         fn = fcol + (size_t)chunk * nc;
     }
@@ -554,10 +643,7 @@ int grmp_face_assemble(grmp_matrix A, int nterms, const grmp_bilinear_term *term
         grmp_free(ctx, gl, (size_t)m->ncells * (dim + 1) * dim * 8);
         grmp_free(ctx, mats, (size_t)chunk * (per + nc * 4 + 4));
     };
-    if (rc) {
-        release();
-        return rc;
-    }
+    const FaceGeom geo{m->d_cell_faces, m->d_cells, s->d_celldofs, m->d_coords, gl, m->d_face_volumes};
     double *v64 = precision != GRMP_FP32 ? A->d_vals64 : nullptr;
     float *v32 = precision != GRMP_FP64 ? A->d_vals32 : nullptr;
     const int p = grmp_fe_polyorder(s->fe, dim);
@@ -577,12 +663,19 @@ int grmp_face_assemble(grmp_matrix A, int nterms, const grmp_bilinear_term *term
             rc = grmp_fail(ctx, GRMP_ERR_UNSUPPORTED, "face terms: FP64 values are required (use FP64 or FP64_FP32)");
             break;
         }
-        auto go = [&](auto mat, auto add, int nb, int lpr) {
+        auto go = [&](auto mat, auto add, auto rows, int nb, int lpr) {
             const int nc = 2 * nb;
             const size_t fsm = ((size_t)r.nq * nc * dim + 1) * 8 + (1 + nb) * 4;
             const int fb = (int)std::max<size_t>(1, std::min<size_t>(32, (size_t)46 * 1024 / fsm));
             for (int F0 = 0; F0 < m->nfaces; F0 += chunk) {
                 const int nf = std::min(chunk, m->nfaces - F0);
+                if (!mats) {
+                    rows<<<nblk(A->nrows, 128), 128, 0, ctx->stream>>>(
+                        A->nrows, F0, nf, s->d_inc_ptr, s->d_inc_cell, m->d_cell_nbr, A->d_rowptr, A->d_cols, w64, w32,
+                        dmiss, geo, t, r);
+                    GRMP_LAUNCHED(ctx);
+                    continue;
+                }
                 mat<<<nblk(nf, fb), 128, fb * fsm + 8, ctx->stream>>>(F0, nf, fb, m->d_face_cells, m->d_cell_faces,
                                                                       m->d_cells, m->d_coords, s->d_celldofs, gl, m->d_face_volumes,
                                                                       t, r, mats, fcol, fn);
@@ -593,10 +686,10 @@ int grmp_face_assemble(grmp_matrix A, int nterms, const grmp_bilinear_term *term
                 GRMP_LAUNCHED(ctx);
             }
         };
-        if (dim == 2 && s->nb == 3) go(k_face_mats<2, 3>, k_face_add<2, 3, 8>, 3, 8);
-        else if (dim == 2 && s->nb == 6) go(k_face_mats<2, 6>, k_face_add<2, 6, 16>, 6, 16);
-        else if (dim == 3 && s->nb == 4) go(k_face_mats<3, 4>, k_face_add<3, 4, 8>, 4, 8);
-        else go(k_face_mats<3, 10>, k_face_add<3, 10, 32>, 10, 32);
+        if (dim == 2 && s->nb == 3) go(k_face_mats<2, 3>, k_face_add<2, 3, 8>, k_face_rows<2, 3>, 3, 8);
+        else if (dim == 2 && s->nb == 6) go(k_face_mats<2, 6>, k_face_add<2, 6, 16>, k_face_rows<2, 6>, 6, 16);
+        else if (dim == 3 && s->nb == 4) go(k_face_mats<3, 4>, k_face_add<3, 4, 8>, k_face_rows<3, 4>, 4, 8);
+        else go(k_face_mats<3, 10>, k_face_add<3, 10, 32>, k_face_rows<3, 10>, 10, 32);
     }
     int hmiss = 0;
     cudaError_t e = cudaGetLastError();
