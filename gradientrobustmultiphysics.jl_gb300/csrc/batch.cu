@@ -1195,7 +1195,7 @@ struct SweepDev {
     const int *pid;         // problem in the batch
     const int *err;         // factorisation failures
     double *part;           // [chunk][3]
-    double *anorm, *bn, *prev, *rel, *worst;
+    double *anorm, *bn, *prev, *worst;
     int *act, *fin, *ok, *nsolve, *sweeps, *count;
     int max_solves;
 };
@@ -1650,23 +1650,21 @@ int build_parts(grmp_matrix A, const std::vector<int32_t> &order, size_t allow) 
     if (!C.parts.empty() && C.parts_allow <= allow) return GRMP_OK;
     free_parts(ctx, C);
     size_t need = 0;
+    const FoNeed none(groups, 8);
+    allow -= std::min(allow, none.trees());
     for (size_t at = 0; at < order.size();) {
         std::vector<FoProblem> probs;
         std::vector<int> pid;
-        size_t bytes = 0;
+        FoNeed part = none;
         while (at < order.size()) {
-            const int k = order[at];
-            probs.push_back(FoProblem{C.group_of[k], C.row_offsets[k], C.nnz0[k]});
-            const size_t b = grmp_forest_bytes(groups, probs, 8);
-            if (probs.size() > 1 && b > allow) {
-                probs.pop_back();
-                break;
-            }
-            bytes = b;
+            const int k = order[at], g = C.group_of[k];
+            if (!pid.empty() && part.with(g) > allow) break;
+            part.add(g);
+            probs.push_back(FoProblem{g, C.row_offsets[k], C.nnz0[k]});
             pid.push_back(k);
             at++;
         }
-        need = std::max(need, bytes);
+        need = std::max(need, part.bytes());
         std::vector<int4> chunk;
         std::vector<int2> pchunk;
         for (size_t q = 0; q < pid.size(); q++) {
@@ -1688,7 +1686,7 @@ int build_parts(grmp_matrix A, const std::vector<int32_t> &order, size_t allow) 
             return rc;
         }
     }
-    C.parts_allow = need;
+    C.parts_allow = need;   // (the trees are there by then)
     return GRMP_OK;
 }
 
@@ -1696,7 +1694,7 @@ int build_parts(grmp_matrix A, const std::vector<int32_t> &order, size_t allow) 
 int run_part(grmp_context ctx, DirectCache::Part &P, const BatchDev &d) {
     const int np = P.np;
     char *w = nullptr;
-    const size_t dbl = (size_t)P.nchunk * 3 + 5 * (size_t)np, bytes = dbl * 8 + ((size_t)np * 6 + 2) * 4;
+    const size_t dbl = (size_t)P.nchunk * 3 + 4 * (size_t)np, bytes = dbl * 8 + ((size_t)np * 6 + 2) * 4;
     int rc = grmp_alloc(ctx, (void **)&w, bytes);
     if (rc) return rc;
     SweepDev s;
@@ -1707,8 +1705,7 @@ int run_part(grmp_context ctx, DirectCache::Part &P, const BatchDev &d) {
     s.anorm = s.part + (size_t)P.nchunk * 3;
     s.bn = s.anorm + np;
     s.prev = s.bn + np;
-    s.rel = s.prev + np;
-    s.worst = s.rel + np;
+    s.worst = s.prev + np;
     int *iw = (int *)(w + dbl * 8);
     s.act = iw;
     s.fin = iw + np;

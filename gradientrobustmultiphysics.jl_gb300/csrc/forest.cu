@@ -636,21 +636,23 @@ int fo_storage(grmp_context ctx, MfForest *F, int esize) {
     int rc = grmp_alloc(ctx, &F->L, F->Lb);
     if (!rc) rc = grmp_alloc(ctx, &F->U, F->Ub);
     if (!rc) rc = grmp_alloc(ctx, &F->uv, F->uvb);
+    if (!rc) rc = grmp_alloc(ctx, &F->cs, kMaxGroups * sizeof(CoopState));
     // short of memory or budget: fewer groups of blocks, down to one front's
     size_t one = 256;
     for (const FoLevel &l : F->level)
         if (l.big.count) one = std::max<size_t>(one, (size_t)slot_elems(l.big.maxf) * esize);
     if (!rc) {
-        while ((rc = grmp_alloc(ctx, &F->pool, F->poolb)) && F->poolb > one) F->poolb = std::max(one, F->poolb / 2);
+        while ((rc = F->poolb > one ? grmp_alloc_spare(ctx, &F->pool, F->poolb) : grmp_alloc(ctx, &F->pool, F->poolb)) &&
+               F->poolb > one)
+            F->poolb = std::max(one, F->poolb / 2);
         if (!rc) ctx->last_error.clear();
         cudaGetLastError();
     }
-    if (!rc) rc = grmp_alloc(ctx, &F->cs, kMaxGroups * sizeof(CoopState));
     if (rc) {
         grmp_free(ctx, F->L, F->Lb);
         grmp_free(ctx, F->U, F->Ub);
         grmp_free(ctx, F->uv, F->uvb);
-        grmp_free(ctx, F->pool, F->poolb);
+        grmp_free(ctx, F->cs, kMaxGroups * sizeof(CoopState));
         F->L = F->U = F->uv = F->pool = F->cs = nullptr;
         return rc;
     }
@@ -713,11 +715,33 @@ int fo_factor(grmp_context ctx, MfForest *F, const double *vals, int *err) {
 
 }  // namespace
 
-size_t grmp_forest_bytes(const std::vector<const NdSymbolic *> &groups, const std::vector<FoProblem> &probs, int esize) {
-    size_t b = kPoolBound / 4;
-    for (const FoProblem &p : probs) b += (size_t)(groups[p.group]->L_size + groups[p.group]->U_size + groups[p.group]->uv_size) * esize;
-    return b;
+FoNeed::FoNeed(const std::vector<const NdSymbolic *> &groups, int esize) {
+    const int large = class_limit(esize, 3);
+    for (const NdSymbolic *S : groups) {
+        Group g{(size_t)(S->L_size + S->U_size + S->uv_size) * esize, 0, 0};
+        for (size_t l = 0; l + 1 < S->level_ptr.size(); l++) {
+            size_t level = 0;
+            for (int q = S->level_ptr[l]; q < S->level_ptr[l + 1]; q++) {
+                const int f = S->node[S->level_nodes[q]].f;
+                if (f <= large) continue;
+                level += (size_t)slot_elems(f) * esize;
+                g.slot = std::max(g.slot, (size_t)slot_elems(f) * esize);
+            }
+            g.pool = std::max(g.pool, level);
+        }
+        of.push_back(g);
+        tree += S->node.size() * sizeof(FoNode) + S->front.size() * 12 + (S->child.size() + S->ext.size()) * 4 + S->ent_rel.size() * 8;
+    }
 }
+void FoNeed::add(int group) {
+    fac += of[group].fac;
+    pool += of[group].pool;
+    slot = std::max(slot, of[group].slot);
+}
+size_t FoNeed::with(int group) const {
+    return total(fac + of[group].fac, pool + of[group].pool, std::max(slot, of[group].slot));
+}
+size_t FoNeed::total(size_t fac, size_t pool, size_t slot) { return fac + std::max(slot, std::min(pool, kPoolBound / 4)); }
 
 int grmp_forest_create(grmp_context ctx, const std::vector<const NdSymbolic *> &groups, const std::vector<FoProblem> &probs,
                        int esize, MfForest **out) {
@@ -729,8 +753,11 @@ int grmp_forest_create(grmp_context ctx, const std::vector<const NdSymbolic *> &
     std::vector<int32_t> front, child, ent_rel, ent_pos, ext;
     std::vector<int2> src;
     std::vector<int> node0(ng);
+    std::vector<char> used(ng, 0);   // a part of a batch holds the trees of its own problems only
+    for (const FoProblem &p : probs) used[p.group] = 1;
     size_t nlev = 0;
     for (int g = 0; g < ng; g++) {
+        if (!used[g]) continue;
         const NdSymbolic &S = *groups[g];
         const int nb = (int)node.size(), fb = (int)front.size(), cb = (int)child.size(), eb = (int)ent_rel.size(),
                   xb = (int)ext.size();

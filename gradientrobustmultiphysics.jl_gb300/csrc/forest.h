@@ -61,8 +61,25 @@ struct FoProblem {
     long long nnz0;
 };
 
-// device bytes of the numeric storage
-size_t grmp_forest_bytes(const std::vector<const NdSymbolic *> &groups, const std::vector<FoProblem> &probs, int esize);
+// device bytes of the numeric storage of a growing set of problems: factors and
+// updates, and the buffers of the fronts that groups of blocks work on (as many
+// as a level of theirs needs, within a quarter of the pool's bound, one at the least)
+class FoNeed {
+  public:
+    FoNeed(const std::vector<const NdSymbolic *> &groups, int esize);
+    void add(int group);
+    size_t with(int group) const;    // bytes with one more problem of this group
+    size_t bytes() const { return total(fac, pool, slot); }
+    size_t trees() const { return tree; }   // of all groups' trees, which every part keeps for its problems
+
+  private:
+    struct Group {
+        size_t fac, pool, slot;
+    };
+    std::vector<Group> of;
+    size_t fac = 0, pool = 0, slot = 0, tree = 0;
+    static size_t total(size_t fac, size_t pool, size_t slot);
+};
 // esize: precision the size classes are made for
 int grmp_forest_create(grmp_context ctx, const std::vector<const NdSymbolic *> &groups, const std::vector<FoProblem> &probs,
                        int esize, MfForest **out);
