@@ -632,32 +632,37 @@ int fo_storage(grmp_context ctx, MfForest *F, int esize) {
     F->Lb = std::max<size_t>(1, F->L_size) * esize;
     F->Ub = std::max<size_t>(1, F->U_size) * esize;
     F->uvb = std::max<size_t>(1, F->uv_size) * esize;
-    F->poolb = std::max<size_t>(256, pool_bytes(*F, ctx->num_sms, esize));
     int rc = grmp_alloc(ctx, &F->L, F->Lb);
     if (!rc) rc = grmp_alloc(ctx, &F->U, F->Ub);
     if (!rc) rc = grmp_alloc(ctx, &F->uv, F->uvb);
     if (!rc) rc = grmp_alloc(ctx, &F->cs, kMaxGroups * sizeof(CoopState));
-    // short of memory or budget: fewer groups of blocks, down to one front's
-    size_t one = 256;
-    for (const FoLevel &l : F->level)
-        if (l.big.count) one = std::max<size_t>(one, (size_t)slot_elems(l.big.maxf) * esize);
-    if (!rc) {
-        while ((rc = F->poolb > one ? grmp_alloc_spare(ctx, &F->pool, F->poolb) : grmp_alloc(ctx, &F->pool, F->poolb)) &&
-               F->poolb > one)
-            F->poolb = std::max(one, F->poolb / 2);
-        if (!rc) ctx->last_error.clear();
-        cudaGetLastError();
-    }
     if (rc) {
         grmp_free(ctx, F->L, F->Lb);
         grmp_free(ctx, F->U, F->Ub);
         grmp_free(ctx, F->uv, F->uvb);
-        grmp_free(ctx, F->cs, kMaxGroups * sizeof(CoopState));
-        F->L = F->U = F->uv = F->pool = F->cs = nullptr;
+        F->L = F->U = F->uv = F->cs = nullptr;
         return rc;
     }
     F->esize = esize;
     return GRMP_OK;
+}
+
+// Buffers of the large fronts, for one factorisation (nothing else needs them,
+// and they can be larger than the factor).  Short of memory or budget: fewer
+// groups of blocks, down to one front's.
+int fo_pool(grmp_context ctx, MfForest *F, int esize) {
+    size_t one = 256;
+    for (const FoLevel &l : F->level)
+        if (l.big.count) one = std::max<size_t>(one, (size_t)slot_elems(l.big.maxf) * esize);
+    F->poolb = std::max<size_t>(one, pool_bytes(*F, ctx->num_sms, esize));
+    int rc;
+    while ((rc = F->poolb > one ? grmp_alloc_spare(ctx, &F->pool, F->poolb) : grmp_alloc(ctx, &F->pool, F->poolb)) &&
+           F->poolb > one) {
+        cudaGetLastError();
+        F->poolb = std::max(one, F->poolb / 2);
+    }
+    if (!rc) ctx->last_error.clear();
+    return rc;
 }
 
 template <typename T, int NT, bool WB>
@@ -670,9 +675,7 @@ void launch_small(grmp_context ctx, MfForest *F, const FoItems &it, const double
 }
 
 template <typename T, bool WB>
-int fo_factor(grmp_context ctx, MfForest *F, const double *vals, int *err) {
-    int rc = fo_storage(ctx, F, sizeof(T));
-    if (rc) return rc;
+int fo_factor_levels(grmp_context ctx, MfForest *F, const double *vals, int *err) {
     cudaMemsetAsync(err, 0, (size_t)F->nprob * 4, ctx->stream);
     const size_t bsmem = ((size_t)2 * kWide * kWs + 32 * kWs + 16 * 17 + kWide) * sizeof(T);
     int coop = 0;
@@ -711,6 +714,17 @@ int fo_factor(grmp_context ctx, MfForest *F, const double *vals, int *err) {
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     return e == cudaSuccess ? GRMP_OK : grmp_cuda_fail(ctx, e, "multifrontal factorisation");
+}
+
+template <typename T, bool WB>
+int fo_factor(grmp_context ctx, MfForest *F, const double *vals, int *err) {
+    int rc = fo_storage(ctx, F, sizeof(T));
+    if (!rc) rc = fo_pool(ctx, F, sizeof(T));
+    if (rc) return rc;
+    rc = fo_factor_levels<T, WB>(ctx, F, vals, err);
+    grmp_free(ctx, F->pool, F->poolb);
+    F->pool = nullptr;
+    return rc;
 }
 
 }  // namespace
@@ -890,9 +904,8 @@ void grmp_forest_release(grmp_context ctx, MfForest *F) {
     grmp_free(ctx, F->L, F->Lb);
     grmp_free(ctx, F->U, F->Ub);
     grmp_free(ctx, F->uv, F->uvb);
-    grmp_free(ctx, F->pool, F->poolb);
     grmp_free(ctx, F->cs, kMaxGroups * sizeof(CoopState));
-    F->L = F->U = F->uv = F->pool = F->cs = nullptr;
+    F->L = F->U = F->uv = F->cs = nullptr;
     F->esize = 0;
 }
 
