@@ -1220,9 +1220,10 @@ size_t mg_need(grmp_matrix A, MgCache &C, bool mixed) {
     return mixed ? mg_layout<float>(A, C, nullptr) : mg_layout<double>(A, C, nullptr);
 }
 
-// The patterns, on the device; A->mg stays nullptr on failure.  GRMP_ERR_BUDGET
-// before anything is taken if they and the storage of this precision do not fit.
-int mg_build(grmp_matrix A, bool mixed) {
+// The patterns, on the device.  GRMP_ERR_BUDGET before anything is taken if they
+// and the storage of this precision do not fit; A->mg_state = -1 if the matrix
+// does not coarsen.
+int mg_build(grmp_matrix A, bool mixed, MgCache *C) {
     grmp_space s = A->space;
     grmp_context ctx = s->mesh->ctx;
     const int n = A->nrows;
@@ -1251,8 +1252,6 @@ int mg_build(grmp_matrix A, bool mixed) {
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "multilevel: pattern download");
-    std::unique_ptr<MgCache> own(new MgCache);
-    MgCache *C = own.get();
     C->mult = fine_mult(s->mesh->dim, s->fe, n);
     const MgCells m{s->mesh->dim, s->mesh->ncells, s->ldofs, cd.data(), cells.data(), coords.data()};
     if (mg_symbolic_build(n, pattern, m, p2, !A->face_coupled, stretched, C->mult, &C->S)) {
@@ -1319,14 +1318,8 @@ int mg_build(grmp_matrix A, bool mixed) {
         t.P = t.R = t.AP = t.QT = t.Ac = MgCsr();   // the sizes stay
         t.Rperm = t.QTperm = t.agg = std::vector<int32_t>();
     }
-    if (rc) {
-        for (auto &b : C->bufs) grmp_free(ctx, b.first, b.second);
-        return rc;
-    }
-    A->mg = own.release();
-    ctx->hier.push_back(A);
-    A->mg_state = 1;
-    return GRMP_OK;
+    if (!rc) A->mg_state = 1;
+    return rc;
 }
 
 size_t mg_bytes(const MgCache &C) {
@@ -1351,7 +1344,23 @@ bool mg_no_room(grmp_matrix A, bool mixed) {
 int mg_make(grmp_matrix A, bool mixed, bool *fits) {
     grmp_context ctx = A->space->mesh->ctx;
     *fits = false;
-    int rc = A->mg ? GRMP_OK : mg_build(A, mixed);
+    int rc = GRMP_OK;
+    if (!A->mg) {
+        std::unique_ptr<MgCache> C;
+        try {
+            C.reset(new MgCache);
+            rc = mg_build(A, mixed, C.get());
+        } catch (const std::exception &) {   // host memory: solved without the hierarchy, as when the device's is short
+            cudaStreamSynchronize(ctx->stream);
+            rc = GRMP_ERR_OUT_OF_MEMORY;
+        }
+        if (!rc && A->mg_state > 0) {
+            A->mg = C.release();
+            ctx->hier.push_back(A);
+        } else if (C) {
+            for (auto &b : C->bufs) grmp_free(ctx, b.first, b.second);
+        }
+    }
     if (!rc && A->mg_state < 0) return GRMP_OK;
     if (!rc) {
         MgCache &C = *A->mg;

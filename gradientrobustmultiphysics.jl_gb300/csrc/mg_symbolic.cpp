@@ -26,6 +26,8 @@
 // of boundary DoFs.
 #include <algorithm>
 #include <cmath>
+#include <exception>
+#include <mutex>
 #include <thread>
 
 #include "mg_symbolic.h"
@@ -39,6 +41,33 @@ constexpr double kStrong = 0.08, kStrongP2 = 0.2;
 int host_threads(int n) {
     const int hw = std::max(1, (int)std::thread::hardware_concurrency());
     return std::max(1, std::min({hw, 16, n / 4096}));
+}
+
+// work(0), ..., work(nt - 1), a thread each; what one throws is thrown here
+// after all have ended.  Where threads cannot be had this one does their work.
+template <typename F>
+void run_threads(int nt, F work) {
+    std::exception_ptr thrown;
+    std::mutex mu;
+    auto guarded = [&](int t) {
+        try {
+            work(t);
+        } catch (...) {
+            std::lock_guard<std::mutex> lk(mu);
+            if (!thrown) thrown = std::current_exception();
+        }
+    };
+    std::vector<std::thread> pool;
+    pool.reserve(nt);
+    int t = 1;
+    try {
+        for (; t < nt; t++) pool.emplace_back(guarded, t);
+    } catch (const std::exception &) {
+    }
+    guarded(0);
+    for (; t < nt; t++) guarded(t);
+    for (auto &p : pool) p.join();
+    if (thrown) std::rethrow_exception(thrown);
 }
 
 // out row i = sorted distinct columns that fn(i, add) names; rows in parallel
@@ -63,10 +92,7 @@ void build_rows(int n, int ncols, MgCsr *out, F fn) {
             out->rp[(size_t)i + 1] = (int32_t)(c.size() - b);
         }
     };
-    std::vector<std::thread> pool;
-    for (int t = 1; t < nt; t++) pool.emplace_back(work, t);
-    work(0);
-    for (auto &t : pool) t.join();
+    run_threads(nt, work);
     for (int i = 0; i < n; i++) out->rp[i + 1] += out->rp[i];
     out->ci.resize(out->rp[n]);
     for (int t = 0; t < nt; t++)
@@ -76,13 +102,9 @@ void build_rows(int n, int ncols, MgCsr *out, F fn) {
 template <typename F>
 void parallel_rows(int n, F fn) {
     const int nt = host_threads(n);
-    auto work = [&](int t) {
+    run_threads(nt, [&](int t) {
         for (int i = (int)((long long)n * t / nt); i < (int)((long long)n * (t + 1) / nt); i++) fn(i);
-    };
-    std::vector<std::thread> pool;
-    for (int t = 1; t < nt; t++) pool.emplace_back(work, t);
-    work(0);
-    for (auto &t : pool) t.join();
+    });
 }
 
 void transpose(int n, int nc, const MgCsr &A, MgCsr *T, std::vector<int32_t> *perm) {
