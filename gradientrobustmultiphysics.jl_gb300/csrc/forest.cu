@@ -479,7 +479,8 @@ __device__ __forceinline__ double rows8(const double *Lt, int s, int i, bool in,
     for (int j = 0; j < 8; j++) l[j] = in && c0 + j < nb ? r[j] : 0.0;
     double a = 0.0;
 #pragma unroll
-    for (int j = 0; j < 8; j++) a += l[j] * v[kb + c0 + j];
+    for (int j = 0; j < 8; j++)
+        if (c0 + j < nb) a += l[j] * v[kb + c0 + j];   // beyond nb: structure rows, which other warps write meanwhile
     a += __shfl_xor_sync(0xffffffffu, a, 1);
     a += __shfl_xor_sync(0xffffffffu, a, 2);
     return a;
@@ -494,7 +495,7 @@ template <int NT>
 __global__ void __launch_bounds__(NT) k_fs_fwd(FoDev m, const int2 *items, const double *L, double *uv, double *w,
                                                const int *active) {
     extern __shared__ __align__(16) unsigned char fo_ssmem[];
-    double *v = reinterpret_cast<double *>(fo_ssmem);   // f + 32 (the last columns' reads run past s)
+    double *v = reinterpret_cast<double *>(fo_ssmem);   // f
     const int2 it = items[blockIdx.x];
     if (active && !active[it.x]) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -506,14 +507,10 @@ __global__ void __launch_bounds__(NT) k_fs_fwd(FoDev m, const int2 *items, const
     const int2 *src = m.src + nd.front_off;
     const double *Lt = L + pr.Lb + nd.L_off;
     double *u = uv + pr.uvb;
-    for (int k = tid; k < f + 32; k += NT) {
-        double x = 0.0;
-        if (k < f) {
-            const int2 q = src[k];
-            const double c = (q.x >= 0 ? u[q.x] : 0.0) + (q.y >= 0 ? u[q.y] : 0.0);
-            x = k < s ? w[pr.row0 + fr[k]] - c : c;
-        }
-        v[k] = x;
+    for (int k = tid; k < f; k += NT) {
+        const int2 q = src[k];
+        const double c = (q.x >= 0 ? u[q.x] : 0.0) + (q.y >= 0 ? u[q.y] : 0.0);
+        v[k] = k < s ? w[pr.row0 + fr[k]] - c : c;
     }
     __syncthreads();
     for (int kb = 0; kb < s; kb += 32) {
@@ -926,7 +923,7 @@ int grmp_forest_factor32(grmp_context ctx, MfForest *F, const double *vals, int 
 void grmp_forest_solve64(grmp_context ctx, MfForest *F, double *w, const int *active) {
     const double *L = (const double *)F->L;
     double *uv = (double *)F->uv;
-    auto smem_f = [](int maxf) { return (size_t)(maxf + 32) * 8; };
+    auto smem_f = [](int maxf) { return (size_t)maxf * 8; };
     auto smem_b = [](int nt, int maxf) { return ((size_t)nt + maxf) * 8; };
     grmp_allow_smem(k_fs_fwd<512>);
     grmp_allow_smem(k_fs_bwd<512>);
