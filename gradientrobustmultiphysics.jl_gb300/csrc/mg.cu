@@ -75,8 +75,12 @@ constexpr int kMaxBicg = 200, kStallBicg = 40;
 // keeps ahead of that: lognormal coefficients with sigma 3 (435 iterations to 1e-11)
 // have lost five digits at 128; FP64 at contrast 1e6 two at 128, four to six at 256.
 constexpr int kStall32 = 64, kStall64 = 128;
-__device__ __forceinline__ bool mg_stalled(int it, int every, double rn, double rn0) {
-    return it >= 2 * every && it % every == 0 && rn > rn0 * (double)exp10f(-(float)(it / every));
+// (rn0, the start's residual, waits in shared memory: it is needed once in kStall
+// iterations, and registers are what the iterations are short of)
+__device__ __forceinline__ bool mg_behind(int it, int every, double rn, const double *rn0) {
+    double lim = *rn0;
+    for (int k = it / every; k > 0; k--) lim *= 0.1;
+    return rn > lim;
 }
 
 // Rows from which the multilevel solver is taken: where whole passes are no
@@ -772,7 +776,7 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
              double *z, double *p, double *q, double *partial, SolveState *st, double abstol, double reltol, int maxit,
              int guess, long long spin, const __grid_constant__ MgDev<double> m) {
     __shared__ double sh[32 * 4];
-    __shared__ double eb[2 * kMgBottom];
+    __shared__ double eb[2 * kMgBottom], rn0;
     SY sy(st, partial, spin);
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gsz = gridDim.x * blockDim.x;
@@ -790,10 +794,11 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
         v[1] += b[i] * b[i];
     }
     if (!sy.template sum<2>(v, sh)) return;
-    const double bn = sqrt(v[1]), rn0 = sqrt(v[0]);
+    const double bn = sqrt(v[1]);
     const double tol = fmax(abstol, reltol * bn);
+    if (threadIdx.x == 0) rn0 = sqrt(v[0]);
     int it = 0;
-    bool conv = rn0 <= tol;
+    bool conv = sqrt(v[0]) <= tol;
     double rz = 0.0;
     while (!conv && it < maxit) {
         if (!mg_cycle(m, (const double *)r, eb, sy)) return;
@@ -825,9 +830,8 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
         }
         if (!sy.template sum<1>(rr, sh)) return;
         it++;
-        const double rn = sqrt(rr[0]);
-        conv = rn <= tol;
-        if (!conv && mg_stalled(it, kStall64, rn, rn0)) break;
+        conv = sqrt(rr[0]) <= tol;
+        if (it % kStall64 == 0 && it > kStall64 && !conv && mg_behind(it, kStall64, sqrt(rr[0]), &rn0)) break;
     }
     if (!sy.barrier()) return;
     double t[1];
@@ -967,6 +971,7 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     __shared__ double sh[32 * 4];
     __shared__ float shf[32 * 4];
     __shared__ float eb[2 * kMgBottom];
+    __shared__ double rn0;
     SY sy(st, partial, spin);
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gsz = gridDim.x * blockDim.x;
@@ -984,8 +989,8 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     if (!sy.template sum<2>(v, sh)) return;
     const double bn = sqrt(v[1]);
     const double tol = fmax(abstol, reltol * bn);
-    const double rn0 = sqrt(v[0]);
-    double rn64 = rn0, prev_rn64 = rn64;
+    double rn64 = sqrt(v[0]), prev_rn64 = rn64;
+    if (threadIdx.x == 0) rn0 = rn64;
     // the FP32 system is solved for the residual scaled to norm 1: the
     // correction and its residual stay in FP32's range at any size of b
     double scale = rn64 > 0 ? rn64 : 1.0;
@@ -1063,7 +1068,8 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
         if (!sy.template sumf<1>(u, shf)) return;
         it++;
         const float rn32 = sqrtf(u[0]);
-        if (mg_stalled(it, kStall32, (double)rn32 * scale, rn0)) break;   // x: as of the last refinement
+        if (it % kStall32 == 0 && it > kStall32 && mg_behind(it, kStall32, (double)rn32 * scale, &rn0))
+            break;   // x: as of the last refinement
         restart = false;
         if (rn32 <= (float)delta * rmax || (double)rn32 * scale <= tol || it >= maxit) {
             for (int i = gtid; i < n; i += gsz) {
