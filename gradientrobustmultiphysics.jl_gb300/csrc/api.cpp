@@ -34,7 +34,7 @@ int grmp_alloc_spare(grmp_context ctx, void **p, size_t bytes) {
     if (bytes == 0) return GRMP_OK;
     if (ctx->budget && ctx->in_use + bytes > ctx->budget)
         return grmp_fail(ctx, GRMP_ERR_BUDGET, "allocation of %zu bytes exceeds the HBM budget (%zu of %zu in use)",
-                         bytes, ctx->in_use, ctx->budget);
+                         bytes, ctx->in_use.load(), ctx->budget);
     cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
     if (e != cudaSuccess) {
         *p = nullptr;
@@ -159,7 +159,7 @@ int grmp_context_launches(grmp_context ctx, uint64_t *launches) {
 
 int grmp_context_set_wait_limit(grmp_context ctx, int64_t polls) {
     if (!valid_ctx(ctx) || polls < 0) return GRMP_ERR_INVALID_ARG;
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     ctx->wait_limit = polls > 0 ? (long long)polls : GRMP_SPIN_LIMIT;
     return GRMP_OK;
 }
@@ -355,7 +355,7 @@ int grmp_vector_download(grmp_vector v, double *host) {
 int grmp_pattern_build(grmp_space space, int nterms, const grmp_bilinear_term *terms, grmp_matrix *out) {
     if (!space || !out || nterms <= 0 || nterms > GRMP_MAX_TERMS || !terms) return GRMP_ERR_INVALID_ARG;
     cudaSetDevice(space->mesh->ctx->device);
-    std::lock_guard<std::mutex> lk(space->mesh->ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(space->mesh->ctx->mu);
     return grmp_pattern_build_impl(space, nterms, terms, out);
 }
 
@@ -366,7 +366,7 @@ int grmp_assemble_bilinear(grmp_matrix A, int nterms, const grmp_bilinear_term *
                          "assemble: the matrix was imported from a CSC (no assembly space); use grmp_matrix_update_values");
     if (precision != GRMP_FP64 && precision != GRMP_FP32 && precision != GRMP_FP64_FP32) return GRMP_ERR_INVALID_ARG;
     cudaSetDevice(A->space->mesh->ctx->device);
-    std::lock_guard<std::mutex> lk(A->space->mesh->ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(A->space->mesh->ctx->mu);
     return grmp_assemble_bilinear_impl(A, nterms, terms, precision);
 }
 
@@ -377,7 +377,7 @@ int grmp_assemble_nonlinear(grmp_matrix A, grmp_vector b, grmp_vector u, const g
     if (b->n != A->nrows || u->n != A->nrows || b->ctx != ctx || u->ctx != ctx)
         return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "nonlinear form: vector length or context mismatch");
     cudaSetDevice(ctx->device);
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     return grmp_assemble_nonlinear_impl(A, b, u, term, precision, add);
 }
 
@@ -387,7 +387,7 @@ int grmp_assemble_linear(grmp_space space, const grmp_rhs *rhs, grmp_vector b) {
         return grmp_fail(space->mesh->ctx, GRMP_ERR_INVALID_ARG, "linear form: vector length %d != ndofs %d", b->n,
                          space->ndofs);
     cudaSetDevice(space->mesh->ctx->device);
-    std::lock_guard<std::mutex> lk(space->mesh->ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(space->mesh->ctx->mu);
     return grmp_assemble_linear_impl(space, rhs, b);
 }
 
@@ -396,7 +396,7 @@ int grmp_item_l2error(grmp_space space, grmp_vector u, grmp_vector v, int op, co
     if (!space || !u) return GRMP_ERR_INVALID_ARG;
     if (u->ctx != space->mesh->ctx || (v && v->ctx != space->mesh->ctx)) return GRMP_ERR_INVALID_ARG;
     cudaSetDevice(space->mesh->ctx->device);
-    std::lock_guard<std::mutex> lk(space->mesh->ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(space->mesh->ctx->mu);
     return grmp_item_l2error_impl(space, u, v, op, data, factor, quadorder, cell_values, total);
 }
 
@@ -410,7 +410,7 @@ int grmp_apply_dirichlet(grmp_matrix A, grmp_vector b, int32_t nfixed, const int
         if (fixed[i] < 0 || fixed[i] >= A->nrows)
             return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "dirichlet: fixed dof %d out of range", fixed[i]);
     cudaSetDevice(ctx->device);
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     return grmp_apply_dirichlet_impl(A, b, nfixed, fixed, values, mode, penalty);
 }
 
@@ -433,7 +433,7 @@ int grmp_solve(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solve_par
     if (p->mode < GRMP_SOLVE_FP64 || p->mode > GRMP_SOLVE_BICGSTAB) return GRMP_ERR_INVALID_ARG;
     if (!(p->reltol >= 0) || !(p->abstol >= 0) || p->maxiter <= 0) return GRMP_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     grmp_solve_stats local;
     if (!st) st = &local;
     std::memset(st, 0, sizeof(*st));
@@ -449,7 +449,7 @@ int grmp_solve(grmp_matrix A, grmp_vector b, grmp_vector x, const grmp_solve_par
 int grmp_spmv(grmp_matrix A, int precision, grmp_vector x, grmp_vector y) {
     if (!A || !x || !y || x->n != A->nrows || y->n != A->nrows) return GRMP_ERR_INVALID_ARG;
     cudaSetDevice(A->space->mesh->ctx->device);
-    std::lock_guard<std::mutex> lk(A->space->mesh->ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(A->space->mesh->ctx->mu);
     return grmp_spmv_impl(A, precision, x, y);
 }
 

@@ -1778,7 +1778,7 @@ extern "C" int grmp_stokes_batch_solve(grmp_matrix A, grmp_vector bf, grmp_vecto
     grmp_context ctx = m->ctx;
     std::memset(stats, 0, sizeof(*stats));
     cudaSetDevice(ctx->device);
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     const int np = prm->nproblems;
     if (s->fe != GRMP_FE_H1BR) return grmp_fail(ctx, GRMP_ERR_UNSUPPORTED, "batched Stokes needs an H1BR space");
     if (np <= 0 || !prm->row_offsets || !prm->cell_offsets) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "batch: offsets");

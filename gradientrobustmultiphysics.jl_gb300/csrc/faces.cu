@@ -709,7 +709,7 @@ extern "C" int grmp_item_face_jumps(grmp_space s, grmp_vector u, int kind, doubl
     grmp_context ctx = m->ctx;
     if (u->ctx != ctx || u->n != s->ndofs) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "face jumps: vector mismatch");
     cudaSetDevice(ctx->device);
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     if (s->ncomp != 1 || (s->fe != GRMP_FE_H1P1 && s->fe != GRMP_FE_H1P2))
         return grmp_fail(ctx, GRMP_ERR_UNSUPPORTED, "face jumps: scalar H1P1 / H1P2 spaces");
     int rc = grmp_mesh_neighbors(m);

@@ -25,14 +25,15 @@ struct grmp_context_s {
     int device = 0;
     cudaStream_t stream = nullptr;
     size_t budget = 0;       // 0 = unlimited
-    size_t in_use = 0;
+    std::atomic<size_t> in_use{0};
     int num_sms = 0;
     long long wait_limit = GRMP_SPIN_LIMIT;   // polls of a bounded device wait in this context's solves
     std::atomic<unsigned long long> launches{0};
     std::string last_error;
     void *pin = nullptr;     // kPinBytes of page-locked host memory for grmp_readback
-    std::mutex mu;
-    std::vector<grmp_matrix> hier;   // matrices with a multilevel hierarchy
+    // re-entrant: what gives memory up or destroys a matrix takes it too, inside entry points that hold it
+    std::recursive_mutex mu;
+    std::vector<grmp_matrix> hier;   // matrices with a multilevel hierarchy (under mu)
 };
 
 struct grmp_mesh_s {

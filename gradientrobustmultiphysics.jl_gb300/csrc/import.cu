@@ -208,7 +208,7 @@ extern "C" int grmp_matrix_from_csc(grmp_context ctx, int32_t n, const int64_t *
     }
     cudaError_t se = cudaSetDevice(ctx->device);
     if (se != cudaSuccess) return grmp_cuda_fail(ctx, se, "CSC import: cudaSetDevice");
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     // a matrix without an assembly space: a placeholder mesh / space carry the context
     grmp_mesh m = new (std::nothrow) grmp_mesh_s();
     grmp_space s = new (std::nothrow) grmp_space_s();
@@ -256,7 +256,7 @@ extern "C" int grmp_matrix_update_values(grmp_matrix A, const double *nzval) {
     if (!A->imported) return grmp_fail(ctx, GRMP_ERR_INVALID_ARG, "update values: the matrix was not imported from a CSC");
     cudaError_t se = cudaSetDevice(ctx->device);
     if (se != cudaSuccess) return grmp_cuda_fail(ctx, se, "update values: cudaSetDevice");
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     int rc = load_values(A, nzval);
     if (!rc) rc = refresh_values(A);
     return rc;

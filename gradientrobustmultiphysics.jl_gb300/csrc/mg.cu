@@ -1286,7 +1286,7 @@ int mg_build(grmp_matrix A, bool mixed, MgCache *C) {
     }
     need += mg_need(A, *C, mixed);
     A->mg_floor[mixed] = need > A->mg_budget ? SIZE_MAX : need;
-    if (need > A->mg_budget || (ctx->budget && need > ctx->budget - std::min(ctx->budget, ctx->in_use))) return GRMP_ERR_BUDGET;
+    if (need > A->mg_budget || (ctx->budget && need > ctx->budget - std::min(ctx->budget, ctx->in_use.load()))) return GRMP_ERR_BUDGET;
     for (int k = 0; k < ns && !rc; k++) {
         MgStep &t = C->S.step[k];
         MgCache::Step &d = C->step[k];
@@ -1698,8 +1698,11 @@ int mg_launch_bicg(grmp_matrix A, const double *b, double *x, const grmp_solve_p
 }  // namespace
 
 void grmp_mg_free(grmp_matrix A) {
-    if (!A || !A->mg) return;
+    if (!A) return;
     grmp_context ctx = A->space->mesh->ctx;
+    // a garbage collector may destroy matrices on another thread than the one that allocates or solves
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+    if (!A->mg) return;
     for (auto &b : A->mg->bufs) grmp_free(ctx, b.first, b.second);
     for (auto &N : A->mg->num) grmp_free(ctx, N.p, N.bytes);
     delete A->mg;
@@ -1708,6 +1711,7 @@ void grmp_mg_free(grmp_matrix A) {
 }
 
 bool grmp_mg_reclaim(grmp_context ctx, size_t bytes) {
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     bool any = false;
     while (!ctx->hier.empty() && !(any && ctx->budget && ctx->in_use + bytes <= ctx->budget)) {
         grmp_matrix A = ctx->hier.back();

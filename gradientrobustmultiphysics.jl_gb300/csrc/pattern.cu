@@ -643,7 +643,7 @@ extern "C" int grmp_matrix_download(grmp_matrix A, int precision, int64_t *rowpt
     if (!A) return GRMP_ERR_INVALID_ARG;
     grmp_context ctx = A->space->mesh->ctx;
     cudaSetDevice(ctx->device);
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     if (rowptr) {
         int64_t *d = nullptr;
         int rc = grmp_alloc(ctx, (void **)&d, ((size_t)A->nrows + 1) * 8);

@@ -2079,7 +2079,7 @@ extern "C" int grmp_selftest_wait_timeout(grmp_context ctx, int64_t polls, int32
     if (!ctx || !ctx->stream || polls < 0 || !grid_status || !mbar_status) return GRMP_ERR_INVALID_ARG;
     cudaError_t se = cudaSetDevice(ctx->device);
     if (se != cudaSuccess) return grmp_cuda_fail(ctx, se, "wait self-test: cudaSetDevice");
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     struct Words {
         GridBarrier bar;
         int grid_status, mbar_status;
@@ -2190,7 +2190,7 @@ extern "C" int grmp_solve_fp64_noalloc(grmp_matrix A, grmp_vector b, grmp_vector
     const auto t0 = std::chrono::steady_clock::now();
     cudaError_t se = cudaSetDevice(ctx->device);
     if (se != cudaSuccess) return grmp_cuda_fail(ctx, se, "noalloc solve: cudaSetDevice");
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    std::lock_guard<std::recursive_mutex> lk(ctx->mu);
     // the hierarchy that an FP64 grmp_solve of this matrix left: the same solver,
     // in that hierarchy's own storage
     grmp_solve_params q = *p;
