@@ -138,7 +138,7 @@ struct MgDev {
     const T *D0, *binv;
     // fine level smoothed multiplicatively: Q_0 (its transpose is in rrp, rci, rv), lanes per row of A
     // and Q_0, A in the cycle's precision and a vector
-    int mult, flanes, n;
+    int mult, flanes;
     const int32_t *frp, *fci, *q0rp, *q0ci;
     const T *fv, *q0v;
     T *z0;
@@ -1557,7 +1557,6 @@ MgDev<T> mg_device(grmp_matrix A) {
     m.dense = C.S.step[ns - 1].nc <= kMgBottom;
     auto lanes = lanes_of<T>;
     m.rlanes = lanes(C.step[0].np, C.S.step[0].nc);
-    m.n = A->nrows;
     m.mult = C.mult;
     if (C.mult) {
         const MgCache::Step &d = C.step[0];

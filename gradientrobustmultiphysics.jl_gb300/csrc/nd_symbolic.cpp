@@ -44,7 +44,7 @@ struct Builder {
     const int32_t *mptr = nullptr, *mem = nullptr;   // DoFs of each node (nullptr: node = DoF)
     std::vector<int> stamp;      // membership stamps
     int cur = 0;
-    std::vector<int> level, queue;
+    std::vector<int> level;
     std::vector<std::vector<int>> own;   // own DoFs per node (creation = post-order)
     std::vector<std::vector<int>> kids;
 
