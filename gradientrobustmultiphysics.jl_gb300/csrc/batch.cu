@@ -1420,7 +1420,8 @@ struct DirectCache {
         const int *pid = nullptr;
     };
     std::vector<Part> parts;
-    size_t parts_allow = 0;
+    size_t parts_allow = 0;               // of the largest part that could be split
+    std::vector<std::pair<void *, size_t>> part_bufs;
     bool tables = false;                  // MIXED_DIRECT's arrays are uploaded
     std::vector<std::pair<void *, size_t>> bufs;
     const DNode *node = nullptr;
@@ -1434,12 +1435,12 @@ struct DirectCache {
 namespace {
 
 template <typename T>
-int upload_vec(grmp_context ctx, DirectCache &C, const std::vector<T> &v, const T **out) {
+int upload_vec(grmp_context ctx, std::vector<std::pair<void *, size_t>> &bufs, const std::vector<T> &v, const T **out) {
     T *p = nullptr;
     const size_t bytes = std::max<size_t>(1, v.size()) * sizeof(T);
     int rc = grmp_alloc(ctx, (void **)&p, bytes);
     if (rc) return rc;
-    C.bufs.push_back({p, bytes});
+    bufs.push_back({p, bytes});
     if (!v.empty()) {
         cudaError_t e = cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, ctx->stream);
         if (e != cudaSuccess) return grmp_cuda_fail(ctx, e, "direct cache upload");
@@ -1614,18 +1615,18 @@ int build_direct_tables(grmp_matrix A, int np) {
         pl0[k] = glvl0[group_of[k]];
         pnl[k] = gnlev[group_of[k]];
     }
-    rc = upload_vec(ctx, *C, node, &C->node);
-    if (!rc) rc = upload_vec(ctx, *C, front, &C->front);
-    if (!rc) rc = upload_vec(ctx, *C, child, &C->child);
-    if (!rc) rc = upload_vec(ctx, *C, ent_rel, &C->ent_rel);
-    if (!rc) rc = upload_vec(ctx, *C, ent_pos, &C->ent_pos);
-    if (!rc) rc = upload_vec(ctx, *C, ext, &C->ext);
-    if (!rc) rc = upload_vec(ctx, *C, pn0, &C->prob_node0);
-    if (!rc) rc = upload_vec(ctx, *C, pnn, &C->prob_nnodes);
-    if (!rc) rc = upload_vec(ctx, *C, lvl_ptr, &C->lvl_ptr);
-    if (!rc) rc = upload_vec(ctx, *C, lvl_nodes, &C->lvl_nodes);
-    if (!rc) rc = upload_vec(ctx, *C, pl0, &C->prob_lvl0);
-    if (!rc) rc = upload_vec(ctx, *C, pnl, &C->prob_nlev);
+    rc = upload_vec(ctx, C->bufs, node, &C->node);
+    if (!rc) rc = upload_vec(ctx, C->bufs, front, &C->front);
+    if (!rc) rc = upload_vec(ctx, C->bufs, child, &C->child);
+    if (!rc) rc = upload_vec(ctx, C->bufs, ent_rel, &C->ent_rel);
+    if (!rc) rc = upload_vec(ctx, C->bufs, ent_pos, &C->ent_pos);
+    if (!rc) rc = upload_vec(ctx, C->bufs, ext, &C->ext);
+    if (!rc) rc = upload_vec(ctx, C->bufs, pn0, &C->prob_node0);
+    if (!rc) rc = upload_vec(ctx, C->bufs, pnn, &C->prob_nnodes);
+    if (!rc) rc = upload_vec(ctx, C->bufs, lvl_ptr, &C->lvl_ptr);
+    if (!rc) rc = upload_vec(ctx, C->bufs, lvl_nodes, &C->lvl_nodes);
+    if (!rc) rc = upload_vec(ctx, C->bufs, pl0, &C->prob_lvl0);
+    if (!rc) rc = upload_vec(ctx, C->bufs, pnl, &C->prob_nlev);
     if (!rc) {
         cudaError_t e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) rc = grmp_cuda_fail(ctx, e, "direct cache upload");
@@ -1636,7 +1637,9 @@ int build_direct_tables(grmp_matrix A, int np) {
 
 void free_parts(grmp_context ctx, DirectCache &C) {
     for (auto &p : C.parts) grmp_forest_free(ctx, p.F);
+    for (auto &b : C.part_bufs) grmp_free(ctx, b.first, b.second);
     C.parts.clear();
+    C.part_bufs.clear();
     C.parts_allow = 0;
 }
 
@@ -1664,7 +1667,7 @@ int build_parts(grmp_matrix A, const std::vector<int32_t> &order, size_t allow) 
             pid.push_back(k);
             at++;
         }
-        need = std::max(need, part.bytes());
+        if (pid.size() > 1) need = std::max(need, part.bytes());   // (a part of one stays as it is)
         std::vector<int4> chunk;
         std::vector<int2> pchunk;
         for (size_t q = 0; q < pid.size(); q++) {
@@ -1677,9 +1680,9 @@ int build_parts(grmp_matrix A, const std::vector<int32_t> &order, size_t allow) 
         p.np = (int)pid.size();
         p.nchunk = (int)chunk.size();
         int rc = grmp_forest_create(ctx, groups, probs, 8, &p.F);
-        if (!rc) rc = upload_vec(ctx, C, chunk, &p.chunk);
-        if (!rc) rc = upload_vec(ctx, C, pchunk, &p.pchunk);
-        if (!rc) rc = upload_vec(ctx, C, pid, &p.pid);
+        if (!rc) rc = upload_vec(ctx, C.part_bufs, chunk, &p.chunk);
+        if (!rc) rc = upload_vec(ctx, C.part_bufs, pchunk, &p.pchunk);
+        if (!rc) rc = upload_vec(ctx, C.part_bufs, pid, &p.pid);
         if (!rc && cudaStreamSynchronize(ctx->stream) != cudaSuccess) rc = GRMP_ERR_DEVICE;
         if (rc) {
             free_parts(ctx, C);
