@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
 // caller falls back to the Jacobi iteration from the same start otherwise.
 // Bound like the other solvers by the latency of the cycle's phases, two
 // cycles an iteration.  41^2 P2 Jacobian (6,889 rows, relres 1e-11): Jacobi
-// 278-308 iterations, 11.9 ms; here 16 iterations, 1.4 ms.
+// 278-308 iterations, 11.9 ms; here 9 to 13 iterations, 0.87 to 1.10 ms.
 template <int TPR, int U, bool PIPE, class SY>
 __global__ void __launch_bounds__(SY::kThreads, SY::kBlocks)
     k_mgbicg64(int n, const int32_t *rowptr, const int32_t *cols, const double *vals, const double *b, double *x,
@@ -1662,7 +1662,7 @@ int mg_launch(grmp_matrix A, const double *b, double *x, const grmp_solve_params
         // an iteration of this solver gains about as much as ten of the Jacobi one and
         // a refinement costs the same, so it waits for twice as many digits; not for
         // three times as many: FP32 directions of 128^2 P2 (condition 1e5) are noise by
-        // then (33 iterations at 1e-2, 33 to 142 at 1e-3, depending on the right-hand side)
+        // then (22 to 23 iterations at 1e-2, 23 to 43 at 1e-3, depending on the right-hand side)
         const double d1 = p->inner_reltol > 0 && p->inner_reltol < 1 ? p->inner_reltol : 0.1;
         double delta = std::max(1e-3, d1 * d1);
         if (one) delta = std::max(1e-4, delta * delta);   // small systems: FP32 directions stay good
