@@ -191,14 +191,17 @@ std::vector<double> unit_stiffness(Mode mode, int n, const MgCsr &A, const MgCel
     for (long long c = 0; c < m.ncells; c++)
         for (int v = 0; v < nb; v++) ptr[row[m.celldofs[c * m.ld + v]] + 1]++;
     for (int i = 0; i < n; i++) ptr[i + 1] += ptr[i];
-    std::vector<int64_t> inc(ptr[n]), at(ptr.begin(), ptr.end() - 1);
+    std::vector<int32_t> inc(ptr[n]);   // cells of each row, ascending
+    std::vector<int64_t> at(ptr.begin(), ptr.end() - 1);
     for (long long c = 0; c < m.ncells; c++)
-        for (int v = 0; v < nb; v++) inc[at[row[m.celldofs[c * m.ld + v]]]++] = c * 16 + v;
+        for (int v = 0; v < nb; v++) inc[at[row[m.celldofs[c * m.ld + v]]]++] = (int32_t)c;
     std::vector<double> K(A.ci.size(), 0.0);
     parallel_rows(n, [&](int i) {
+        int a = 0;
         for (int64_t q = ptr[i]; q < ptr[i + 1]; q++) {
-            const long long c = inc[q] >> 4;
-            const int a = (int)(inc[q] & 15);
+            const long long c = inc[q];
+            a = q > ptr[i] && inc[q - 1] == c ? a + 1 : 0;   // the row's function in the cell (the next one if it has two)
+            while (row[m.celldofs[c * m.ld + a]] != i) a++;
             double E[3][3], G[4][3] = {}, h[4][4], det;
             const double *x0 = m.coords + (size_t)m.cells[c * nv] * dim;
             for (int j = 0; j < dim; j++)
@@ -217,7 +220,7 @@ std::vector<double> unit_stiffness(Mode mode, int n, const MgCsr &A, const MgCel
             }
             for (int k = 0; k < dim; k++)
                 for (int j = 1; j <= dim; j++) G[0][k] -= G[j][k];
-            for (int j = 0; j < nv; j++)
+            for (int j = p2 ? 0 : a; j < (p2 ? nv : a + 1); j++)   // (P1: the row's own)
                 for (int l = 0; l < nv; l++) {
                     double d = 0;
                     for (int k = 0; k < dim; k++) d += G[j][k] * G[l][k];
